@@ -309,6 +309,26 @@ def run(state):
                                                                                      _run_codec)(state)
 
 
+# ------------------------------------------------------------------------------------------- exact
+def exact(case, seed):
+    """The three PowerSGD stages in 64 bits.  The codecs' results are defined bit for bit and need none; a training
+    step's are a whole model's."""
+    if case["kind"] != "powersgd":
+        return None
+    s = _prepare_powersgd(case, seed)
+    n, m, r = case["rows"], case["cols"], case["rank"]
+    grad = s["grad"].double().view(n, m)
+    mat = grad + s["residual"].double().view(n, m)
+    P = mat @ s["Q"].double()
+    for j in range(r):      # modified Gram-Schmidt, left to right
+        P[:, j] /= P[:, j].norm() + 1e-8
+        for c in range(j + 1, r):
+            P[:, c] -= (P[:, j] @ P[:, c]) * P[:, j]
+    Q = mat.t() @ P
+    approx = P @ Q.t()
+    return {"P": P, "Q": Q, "M": approx, "residual": (grad - approx).view(-1), "grad": approx.reshape(-1)}
+
+
 # ------------------------------------------------------------------------------------------- work, tolerance
 # parameters, forward multiply-adds per image or per token
 MODEL_SIZE = {"resnet50": (25.6e6, 4.1e9), "vgg19": (143.7e6, 19.6e9), "bert_large": (335e6, 303e6)}
