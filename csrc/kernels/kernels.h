@@ -164,10 +164,14 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
 // candidates dropped so far for lack of pool space} of the last call on `scratch`; asynchronous
 // copies to host4 on `stream`.
 cudaError_t sparse_read_stats(const void* scratch, unsigned int* host4, cudaStream_t stream);
-// add == 0 zero-fills out first.  Payloads are applied one after another in
+// add == 0 writes every element of out.  Payloads are applied one after another in
 // rank order so that the fp32 sum is reproducible on every replica.
+// redo: two zeroed words of scratch that belong to the stream (left zeroed); with them, and with
+// add == 0, out is written in one pass over tiles (see sparse.cu).  Null: memset, then one scatter
+// per payload.
 cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
-                                float post_scale, int* status, cudaStream_t stream);
+                                float post_scale, int* status, cudaStream_t stream,
+                                unsigned int* redo = nullptr);
 
 // out[idx] = 0 for every index of every payload (one launch): after the optimizer has consumed a
 // dense gradient that only held scattered payload entries, this leaves it all zero again

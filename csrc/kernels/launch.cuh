@@ -1,0 +1,43 @@
+// Launches whose start overlaps the end of the kernel before them in the stream (programmatic
+// dependent launch).  A chain of short kernels otherwise pays, between any two of them, the drain
+// of one and the ramp-up of the next.
+//
+// Rules the kernels here follow.  A kernel launched by launch_after() calls wait_for_previous()
+// before it touches memory; the wait covers the whole kernel before it, so a chain is ordered
+// exactly as plain launches are.  Pointers that are read through the read-only path afterwards are
+// passed through after_wait(), so that no such load can be moved above the wait.  The kernel before
+// it calls let_next_start() (its result is only about when the next one is brought in, never about
+// what it may read).  The first kernel of a chain is launched plainly: its inputs come from kernels
+// of the caller, which know nothing of this.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace hipress {
+namespace cuda {
+
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                         Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+}  // namespace cuda
+}  // namespace hipress

@@ -77,6 +77,10 @@ void cpu_accumulate(size_t world, int64_t n, float* out, bool add, double post_s
     for (int64_t i = 0; i < n; ++i) out[i] = hp_mul(out[i], float(post_scale));
 }
 
+// Places in a stream's scratch (see scratch_for): the min/max state of the quantisers at 0, the
+// sum of squares of DGC's clipping, the words of the sparse decode, and from 16,384 the sparse state.
+constexpr size_t kSumsqOffset = 12288, kRedoOffset = 12352, kSparseOffset = 16384;
+
 struct DeviceState {
   std::map<std::pair<int, cudaStream_t>, torch::Tensor> scratch;
   std::map<int, torch::Tensor> status;
@@ -267,7 +271,7 @@ void sparse_compress(const c10::optional<torch::Tensor>& grad, torch::Tensor R, 
   if (R.is_cuda()) {
     c10::cuda::CUDAGuard guard(R.device());
     // the sparse state lives behind the min/max state other codecs keep in the same scratch
-    void* scratch = static_cast<uint8_t*>(scratch_for(R, 16384 + cuda::sparse_scratch_bytes(n))) + 16384;
+    void* scratch = static_cast<uint8_t*>(scratch_for(R, kSparseOffset + cuda::sparse_scratch_bytes(n))) + kSparseOffset;
     HP_CHECK_CUDA(cuda::sparse_compress(g, R.data_ptr<float>(), n, sample_rate, keep_fraction,
                                         uint64_t(seed), accumulate ? 1 : 0, local_target(out),
                                         scratch, at::cuda::getCurrentCUDAStream()));
@@ -296,17 +300,17 @@ void dgc_momentum_compress(torch::Tensor grad, torch::Tensor u, torch::Tensor v,
   TORCH_CHECK(out.numel() >= sparse_payload_bytes(n, keep_fraction), "out needs ",
               sparse_payload_bytes(n, keep_fraction), " bytes");
   c10::cuda::CUDAGuard guard(v.device());
-  uint8_t* base = static_cast<uint8_t*>(scratch_for(v, 16384 + cuda::sparse_scratch_bytes(n)));
+  uint8_t* base = static_cast<uint8_t*>(scratch_for(v, kSparseOffset + cuda::sparse_scratch_bytes(n)));
   cuda::SparseFuse fuse;
   fuse.mode = 2;
   fuse.grad = grad.data_ptr<float>();
   fuse.u = u.data_ptr<float>();
   fuse.momentum = float(momentum);
   fuse.clip = float(clip);
-  fuse.sumsq = reinterpret_cast<float*>(base + 12288);
+  fuse.sumsq = reinterpret_cast<float*>(base + kSumsqOffset);
   fuse.zero_grad = zero_grad ? 1 : 0;
   HP_CHECK_CUDA(cuda::sparse_compress_fused(fuse, v.data_ptr<float>(), n, sample_rate, keep_fraction, uint64_t(seed),
-                                            local_target(out), base + 16384, at::cuda::getCurrentCUDAStream()));
+                                            local_target(out), base + kSparseOffset, at::cuda::getCurrentCUDAStream()));
 }
 
 void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,
@@ -316,9 +320,16 @@ void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor
   TORCH_CHECK(n > 0, "empty tensor");
   if (out.is_cuda()) {
     c10::cuda::CUDAGuard guard(out.device());
+    auto stream = at::cuda::getCurrentCUDAStream();
+    // The one-pass decode needs two words of the stream's scratch.  A captured graph may outlive
+    // that scratch, or run beside later calls on the stream, and takes the form without them.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    HP_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
+    unsigned int* redo = nullptr;
+    if (!add && capture == cudaStreamCaptureStatusNone)
+      redo = reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(scratch_for(out, kSparseOffset)) + kRedoOffset);
     HP_CHECK_CUDA(cuda::sparse_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
-                                            add ? 1 : 0, float(post_scale), status_word_for(out),
-                                            at::cuda::getCurrentCUDAStream()));
+                                            add ? 1 : 0, float(post_scale), status_word_for(out), stream, redo));
   } else {
     TORCH_CHECK(!payloads.empty(), "at least one payload expected");
     if (!add) out.zero_();

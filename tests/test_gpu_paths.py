@@ -1,0 +1,80 @@
+"""Edges of the size- and alignment-dependent paths of the kernels, against the CPU codecs or 64-bit restatements."""
+import pytest
+import torch
+
+from hipress_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def gauss(n, std=0.01, seed=0):
+    return torch.randn(n, generator=torch.Generator().manual_seed(seed)) * std
+
+
+def sparse_payload(idx, val):
+    k = idx.numel()
+    head = torch.tensor([4 + 8 * k], dtype=torch.int32)
+    return torch.cat([head.view(torch.uint8), idx.to(torch.int32).view(torch.uint8), val.view(torch.uint8)])
+
+
+def random_payload(n, k, seed, order="ascending"):
+    g = torch.Generator().manual_seed(seed)
+    idx = torch.randperm(n, generator=g)[:k]
+    if order == "ascending":
+        idx = idx.sort().values
+    return sparse_payload(idx, torch.randn(k, generator=g))
+
+
+# ----------------------------------------------------------------------------- sparse decode in tiles
+@pytest.mark.parametrize("n,k", [(1, 1), (5, 0), (1023, 7), (1024, 1024), (1025, 33), (8192 * 3, 1), (700001, 32),
+                                 (700001, 1025), (5000000, 1300000)])
+@pytest.mark.parametrize("world", [1, 2, 3, 8])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sparse_decode_tiles(n, k, world, offset):
+    payloads = [random_payload(n, min(n, k + 3 * s), s) for s in range(world)]
+    ref = torch.empty(n)
+    ops.sparse_decompress(payloads, ref, post_scale=1.0 / world)
+    out = torch.full((n + offset,), 7.0, device="cuda")[offset:]
+    ops.sparse_decompress([p.cuda() for p in payloads], out, post_scale=1.0 / world)
+    assert torch.equal(out.cpu(), ref)
+    assert ops.read_status(out) == 0
+
+
+@pytest.mark.parametrize("world", [1, 3])
+def test_sparse_decode_of_unordered_payloads(world):
+    """Order is a property of this library's compressor, not of the format: any order decodes, and the calls after
+    it are not affected."""
+    n, k = 300000, 9000
+    for order in ("random", "ascending", "random", "random", "ascending"):
+        payloads = [random_payload(n, k, 5 + s, order if s == world - 1 else "ascending") for s in range(world)]
+        ref = torch.empty(n)
+        ops.sparse_decompress(payloads, ref, post_scale=0.5)
+        out = torch.full((n,), 7.0, device="cuda")
+        ops.sparse_decompress([p.cuda() for p in payloads], out, post_scale=0.5)
+        assert torch.equal(out.cpu(), ref), order
+
+
+def test_sparse_decode_reports_indices_past_the_end():
+    n = 50000
+    idx = torch.arange(0, 60000, 100)           # the last hundred lie past the tensor
+    val = torch.ones(idx.numel())
+    out = torch.empty(n, device="cuda")
+    ops.sparse_decompress(sparse_payload(idx, val).cuda(), out)
+    assert ops.read_status(out) == 2
+    ref = torch.zeros(n)
+    ref[idx[idx < n]] = 1.0
+    assert torch.equal(out.cpu(), ref)
+
+
+def test_sparse_decode_under_capture():
+    n = 100000
+    p = [random_payload(n, 500, s).cuda() for s in range(2)]
+    out = torch.empty(n, device="cuda")
+    ops.sparse_decompress(p, out)
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.sparse_decompress(p, out)
+    out.fill_(3.0)
+    graph.replay()
+    assert torch.equal(out, want)
