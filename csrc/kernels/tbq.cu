@@ -146,37 +146,51 @@ tbq_compress_kernel(const float* __restrict__ grad, float* __restrict__ residual
   publish_when_grid_done(dst);
 }
 
-// Table-driven unpack (see unpack_lut.cuh): one table shared by all ranks.  MODE is chosen by the
-// launcher so that each form is its own kernel with its own register budget: kPair = pair table
-// (aligned dense arrays), kConcat = concatenated shards, kGeneric = nibble table.
-enum UnpackMode : int { kGeneric = 0, kPair = 1, kConcat = 2 };
+// Aligned dense arrays: one index table shared by all groups of four ranks (see unpack_lut.cuh).
+template <bool APPLY, int WORLD>
+__global__ void __launch_bounds__(kIndexThreads, WORLD > 4 ? 2 : 3)
+tbq_unpack_index_kernel(UnpackSources src, float thr, float* __restrict__ out, int64_t n, int add, float post_scale,
+                        SgdApply apply, int align) {
+  if (unpack_guarded(src)) return;
+  resolve_epoch(src);
+  extern __shared__ __align__(16) float smem[];
+  PayloadWords<WORLD> w;
+  index_prefetch<2, WORLD>(src, 0, n, align, w);
+  build_index_tables<2, WORLD, true, false>(smem, [&](int, uint32_t q) { return tbq_dequant(q, thr); });
+  __syncthreads();
+  // a rank that is not there counts as "zero" fields, which decode to +0.0
+  unpack_index_body<2, APPLY, WORLD, true, false>(smem, w, 0x55555555u, src, src.parity_off, align, out, n, add, post_scale,
+                                                  apply);
+}
 
-template <bool APPLY, int MODE, int WORLD>
-__global__ void __launch_bounds__(kUnpackThreads, MODE == kGeneric ? 1 : 4)
+// Everything else: the plain nibble table [16][2], for concatenated shards (aligned dense arrays) or any
+// alignment.
+template <bool APPLY, bool CONCAT>
+__global__ void __launch_bounds__(kUnpackThreads, CONCAT ? 4 : 1)
 tbq_unpack_lut_kernel(UnpackSources src, float thr, float* __restrict__ out, int64_t n, int add,
                       float post_scale, SgdApply apply) {
   if (unpack_guarded(src)) return;
   resolve_epoch(src);
-  // pair table [256][2] (2 KB): row (b << 4) | a = decode(a) + decode(b); otherwise the plain
-  // nibble table [16][2]
-  __shared__ __align__(128) float tab[MODE == kPair ? kPairRows * 2 : 32];
+  __shared__ __align__(128) float tab[32];
   uint32_t first[kMaxWorld];
-  if constexpr (MODE != kConcat) unpack_nibble_prefetch<2>(src, 0, src.parity_off, n, first);
-  if constexpr (MODE == kPair) {
-    build_pair_tables<true>(tab, src.world, [&](int, int nibble, int which) {
-      return tbq_dequant((uint32_t(nibble) >> (2 * which)) & 3u, thr);
-    });
-    __syncthreads();
-    // a rank without a partner pairs with four "zero" fields, which decode to +0.0
-    unpack_pair_body<APPLY, true, (WORLD > 0 ? WORLD : 1)>(tab, 0x55555555u, first, src, src.parity_off, out, n, add, post_scale, apply);
-  } else {
-    if (threadIdx.x < 32) tab[threadIdx.x] = tbq_dequant((uint32_t(threadIdx.x) >> 1 >> (2 * (threadIdx.x & 1))) & 3u, thr);
-    __syncthreads();
-    if constexpr (MODE == kConcat)
-      unpack_concat_body<APPLY, true>(tab, src, src.parity_off, out, n, add, post_scale, apply);
-    else
-      unpack_nibble_body<2, APPLY, true>(tab, first, src, src.parity_off, out, n, add, post_scale, apply);
-  }
+  if constexpr (!CONCAT) unpack_nibble_prefetch<2>(src, 0, src.parity_off, n, first);
+  if (threadIdx.x < 32) tab[threadIdx.x] = tbq_dequant((uint32_t(threadIdx.x) >> 1 >> (2 * (threadIdx.x & 1))) & 3u, thr);
+  __syncthreads();
+  if constexpr (CONCAT)
+    unpack_concat_body<APPLY, true>(tab, src, src.parity_off, out, n, add, post_scale, apply);
+  else
+    unpack_nibble_body<2, APPLY, true>(tab, first, src, src.parity_off, out, n, add, post_scale, apply);
+}
+
+template <bool APPLY, int WORLD>
+cudaError_t launch_tbq_index(const UnpackSources& src, float thr, float* out, int64_t n, int add, float post_scale,
+                             const SgdApply& apply, cudaStream_t stream) {
+  using L = IndexLayout<2, WORLD, true, false>;
+  static_assert(L::kBytes <= 48 * 1024, "fits the default shared-memory limit");
+  const int grid = index_grid(n, IndexForm<2>::kChunk, L::kBytes);
+  tbq_unpack_index_kernel<APPLY, WORLD><<<grid, kIndexThreads, L::kBytes, stream>>>(
+      src, thr, out, n, add, post_scale, apply, payload_alignment(src, 0));
+  return cudaGetLastError();
 }
 
 inline int grid_for(int64_t items, int threads, int max_blocks) {
@@ -224,30 +238,30 @@ cudaError_t tbq_unpack_accum(const UnpackSources& src, float threshold, float* o
     if (apply.param != nullptr) ok = ok && aligned16(apply.param) && aligned16(apply.momentum);
     if (!ok) return cudaErrorInvalidValue;
   }
-  // one thread decodes 16 elements per iteration
-  const int grid = grid_for((n + 15) >> 4, kUnpackThreads, 148 * 4);
   bool aligned = aligned16(out);
   if (apply.param != nullptr) aligned = aligned && aligned16(apply.param) && aligned16(apply.momentum);
-  const int mode = src.shard_elems > 0 ? kConcat : (aligned ? kPair : kGeneric);
-#define HP_LAUNCH(AP, MODE, W) \
-  tbq_unpack_lut_kernel<AP, MODE, W><<<grid, kUnpackThreads, 0, stream>>>(src, threshold, out, n, add, post_scale, apply)
-#define HP_PAIR(AP)                                                                                     \
-  switch (src.world) {                                                                                  \
-    case 1: HP_LAUNCH(AP, kPair, 1); break;  case 2: HP_LAUNCH(AP, kPair, 2); break;                    \
-    case 3: HP_LAUNCH(AP, kPair, 3); break;  case 4: HP_LAUNCH(AP, kPair, 4); break;                    \
-    case 5: HP_LAUNCH(AP, kPair, 5); break;  case 6: HP_LAUNCH(AP, kPair, 6); break;                    \
-    case 7: HP_LAUNCH(AP, kPair, 7); break;  default: HP_LAUNCH(AP, kPair, 8); break;                   \
+  if (src.shard_elems == 0 && aligned) {
+#define HP_INDEX(W)                                                                                               \
+  case W:                                                                                                         \
+    return apply.param != nullptr                                                                                 \
+               ? launch_tbq_index<true, W>(src, threshold, out, n, add, post_scale, apply, stream)                \
+               : launch_tbq_index<false, W>(src, threshold, out, n, add, post_scale, apply, stream)
+    switch (src.world) {
+      HP_INDEX(1); HP_INDEX(2); HP_INDEX(3); HP_INDEX(4); HP_INDEX(5); HP_INDEX(6); HP_INDEX(7); HP_INDEX(8);
+    }
+#undef HP_INDEX
   }
+  // one thread decodes 16 elements per iteration
+  const int grid = grid_for((n + 15) >> 4, kUnpackThreads, 148 * 4);
+#define HP_LAUNCH(AP, CONCAT) \
+  tbq_unpack_lut_kernel<AP, CONCAT><<<grid, kUnpackThreads, 0, stream>>>(src, threshold, out, n, add, post_scale, apply)
   if (apply.param != nullptr) {
-    if (mode == kConcat) HP_LAUNCH(true, kConcat, 0);
-    else if (mode == kPair) { HP_PAIR(true) }
-    else HP_LAUNCH(true, kGeneric, 0);
+    if (src.shard_elems > 0) HP_LAUNCH(true, true);
+    else HP_LAUNCH(true, false);
   } else {
-    if (mode == kConcat) HP_LAUNCH(false, kConcat, 0);
-    else if (mode == kPair) { HP_PAIR(false) }
-    else HP_LAUNCH(false, kGeneric, 0);
+    if (src.shard_elems > 0) HP_LAUNCH(false, true);
+    else HP_LAUNCH(false, false);
   }
-#undef HP_PAIR
 #undef HP_LAUNCH
   return cudaGetLastError();
 }

@@ -342,39 +342,18 @@ __device__ __forceinline__ TernHeader read_header(const uint8_t* p, int64_t cap,
   return h;
 }
 
-// Table-driven unpack (see unpack_lut.cuh).  All payloads of one call must
-// carry the same bitwidth; it is read from the headers, so the host never has
-// to look at a payload.  BW > 0 compiles the decode loop for that bitwidth only
-// (fewer registers, more resident CTAs); BW == 0 dispatches on the header at
-// run time for callers that do not know the bitwidth.
-// MODE (chosen by the launcher, so that each form is its own kernel with its own register
-// budget): kPair = pair tables (2 bits, aligned), kConcat = concatenated shards (2 bits,
-// aligned), kGeneric = nibble or byte tables.
-enum UnpackMode : int { kGeneric = 0, kPair = 1, kConcat = 2 };
-
-template <int BW, bool APPLY, int MODE, int WORLD>
-__global__ void __launch_bounds__(kUnpackThreads, MODE == kGeneric ? 1 : 4)
-tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add,
-                       float post_scale, SgdApply apply, int* status) {
-  if (unpack_guarded(src)) return;
-  resolve_epoch(src);
-  extern __shared__ __align__(16) float lut[];  // [world][256][dpb], byte-table path only
-  // BW == 2: pair tables [slots][256][2] (8 KB), whose first 1 KB doubles as the per-rank nibble
-  // tables of the unaligned and concatenated forms; BW == 1, 4: nibble tables only
-  __shared__ __align__(128) float tab[MODE == kPair ? (kMaxWorld / 2) * kPairRows * 2
-                                                   : ((BW == 1 || BW == 2 || BW == 4) ? kMaxWorld * 16 * (4 / (BW ? BW : 1)) : 1)];
-  __shared__ TernHeader hdr[kMaxWorld];
+// Headers of all payloads -> hdr (shared memory), their common bitwidth -> bw; false, with the status
+// word set, when one of them does not fit.  BW > 0: the bitwidth they must have.  concat: payload r holds
+// shard r only, possibly nothing.  Whole CTA.
+template <int BW>
+__device__ __forceinline__ bool read_headers(const UnpackSources& src, int64_t n, bool concat, TernHeader* hdr, int* status,
+                                             int& bw) {
   __shared__ int all_ok;
-  constexpr bool concat = MODE == kConcat;
-  uint32_t first[kMaxWorld];
-  if constexpr ((BW == 1 || BW == 2 || BW == 4) && !concat)
-    unpack_nibble_prefetch<BW>(src, kTernHeaderBytes, src.parity_off, n, first);
   if (threadIdx.x == 0) all_ok = 1;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kMaxWorld; ++r) {   // thread r reads header r; compile-time index into src
     if (int(threadIdx.x) == r && r < src.world) {
-      // concatenated shards: payload r holds shard r only (possibly nothing)
       const int64_t count = concat ? shard_count(n, src.shard_elems, r) : n;
       if (count > 0) {
         hdr[r] = read_header(src.payload[r] + src.parity_off, src.payload_bytes[r], count);
@@ -385,7 +364,7 @@ tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, in
     }
   }
   __syncthreads();
-  int bw = BW;
+  bw = BW;
   if (all_ok) {
     for (int r = 0; r < src.world; ++r) {  // every thread computes the same verdict
       if (hdr[r].bw == 0) continue;        // empty shard
@@ -394,19 +373,64 @@ tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, in
     }
   }
   __syncthreads();
-  if (!all_ok || bw == 0) {
-    if (!all_ok && blockIdx.x == 0 && threadIdx.x == 0 && status) atomicExch(status, int(kBadHeader));
-    return;
-  }
+  if (all_ok && bw != 0) return true;
+  if (!all_ok && blockIdx.x == 0 && threadIdx.x == 0 && status) atomicExch(status, int(kBadHeader));
+  return false;
+}
+
+// Known bitwidth and 16-byte aligned dense arrays: index tables, or arithmetic at 8 bits.
+template <int BW, bool APPLY, int WORLD>
+__global__ void __launch_bounds__(kIndexThreads, WORLD > 4 ? 2 : 3)
+tern_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add, float post_scale, SgdApply apply,
+                         int* status, int align) {
+  if (unpack_guarded(src)) return;
+  resolve_epoch(src);
+  extern __shared__ __align__(16) float smem[];
+  __shared__ TernHeader hdr[kMaxWorld];
   const int64_t data_offset = kTernHeaderBytes + src.parity_off;
-  if constexpr (MODE == kPair) {
-    build_pair_tables<false>(tab, src.world, [&](int r, int nibble, int which) {
-      return tern_dequant((uint32_t(nibble) >> (2 * which)) & 3u, hdr[r].gap, hdr[r].mn);
-    });
+  int bw;
+  if constexpr (BW == 8) {
+    if (!read_headers<8>(src, n, false, hdr, status, bw)) return;
+    float mn[WORLD], gap[WORLD];
+#pragma unroll
+    for (int r = 0; r < WORLD; ++r) {
+      mn[r] = hdr[r].mn;
+      gap[r] = hdr[r].gap;
+    }
+    unpack_bytes_body<APPLY, WORLD, false>(src, data_offset, align, out, n, add, post_scale, apply,
+                                           [&](int r, uint32_t q) { return tern_dequant(q, gap[r], mn[r]); });
+  } else {
+    PayloadWords<WORLD> w;
+    index_prefetch<BW, WORLD>(src, kTernHeaderBytes, n, align, w);
+    if (!read_headers<BW>(src, n, false, hdr, status, bw)) return;
+    build_index_tables<BW, WORLD, false, false>(
+        smem, [&](int r, uint32_t q) { return tern_dequant(q, hdr[r].gap, hdr[r].mn); });
     __syncthreads();
-    unpack_pair_body<APPLY, false, (WORLD > 0 ? WORLD : 1)>(tab, 0u, first, src, data_offset, out, n, add, post_scale, apply);
-    return;
-  } else if constexpr (BW == 1 || BW == 2 || BW == 4) {
+    unpack_index_body<BW, APPLY, WORLD, false, false>(smem, w, 0u, src, data_offset, align, out, n, add, post_scale, apply);
+  }
+}
+
+// Table-driven unpack of everything else (see unpack_lut.cuh).  All payloads of one call must carry the
+// same bitwidth; it is read from the headers, so the host never has to look at a payload.  BW > 0
+// compiles the decode loop for that bitwidth only (fewer registers, more resident CTAs); BW == 0
+// dispatches on the header at run time for callers that do not know the bitwidth.
+// CONCAT: concatenated shards (2 bits, aligned dense arrays); otherwise nibble or byte tables.
+template <int BW, bool APPLY, bool CONCAT>
+__global__ void __launch_bounds__(kUnpackThreads, CONCAT ? 4 : 1)
+tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add,
+                       float post_scale, SgdApply apply, int* status) {
+  if (unpack_guarded(src)) return;
+  resolve_epoch(src);
+  extern __shared__ __align__(16) float lut[];  // [world][256][dpb], byte-table path only
+  constexpr bool nibbles = BW == 1 || BW == 2 || BW == 4;
+  __shared__ __align__(128) float tab[nibbles ? kMaxWorld * 16 * (4 / (BW ? BW : 1)) : 1];
+  __shared__ TernHeader hdr[kMaxWorld];
+  uint32_t first[kMaxWorld];
+  if constexpr (nibbles && !CONCAT) unpack_nibble_prefetch<BW>(src, kTernHeaderBytes, src.parity_off, n, first);
+  int bw;
+  if (!read_headers<BW>(src, n, CONCAT, hdr, status, bw)) return;
+  const int64_t data_offset = kTernHeaderBytes + src.parity_off;
+  if constexpr (nibbles) {
     // nibble tables (see unpack_lut.cuh): entry (rank, nibble, slot)
     constexpr int DPN = 4 / BW;
     for (int i = threadIdx.x; i < src.world * 16 * DPN; i += blockDim.x) {
@@ -414,7 +438,7 @@ tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, in
       tab[i] = tern_dequant((uint32_t(v) >> (BW * j)) & ((1u << BW) - 1u), hdr[r].gap, hdr[r].mn);
     }
     __syncthreads();
-    if constexpr (concat)
+    if constexpr (CONCAT)
       unpack_concat_body<APPLY, false>(tab, src, data_offset, out, n, add, post_scale, apply);
     else
       unpack_nibble_body<BW, APPLY, false>(tab, first, src, data_offset, out, n, add, post_scale, apply);
@@ -442,41 +466,62 @@ tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, in
   }
 }
 
+template <int BW, bool APPLY, int WORLD>
+cudaError_t launch_tern_index(const UnpackSources& src, float* out, int64_t n, int add, float post_scale,
+                              const SgdApply& apply, int* status, cudaStream_t stream) {
+  const int align = payload_alignment(src, kTernHeaderBytes);
+  int grid = grid_for((n + 3) >> 2, kIndexThreads, 148 * 8);
+  size_t smem = 0;
+  if constexpr (BW != 8) {
+    using L = IndexLayout<BW, WORLD, false, false>;
+    smem = L::kBytes;
+    grid = index_grid(n, IndexForm<BW>::kChunk, smem);
+    if (smem > 40 * 1024) {   // with the static part, past the default limit; per device, and cheap: set on every launch rather than remembered per process
+      const cudaError_t e = cudaFuncSetAttribute(tern_unpack_index_kernel<BW, APPLY, WORLD>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+      if (e != cudaSuccess) return e;
+    }
+  }
+  tern_unpack_index_kernel<BW, APPLY, WORLD><<<grid, kIndexThreads, smem, stream>>>(src, out, n, add, post_scale, apply,
+                                                                                  status, align);
+  return cudaGetLastError();
+}
+
 template <int BW, bool APPLY>
 cudaError_t launch_tern_unpack(const UnpackSources& src, float* out, int64_t n, int add, float post_scale,
                                const SgdApply& apply, int* status, cudaStream_t stream) {
+  bool aligned = aligned16(out);
+  if (APPLY) aligned = aligned && aligned16(apply.param) && aligned16(apply.momentum);
+  if constexpr (BW == 2) {
+    if (src.shard_elems > 0) {
+      const int grid = grid_for((n + 15) >> 4, kUnpackThreads, 148 * 4);
+      tern_unpack_lut_kernel<2, APPLY, true><<<grid, kUnpackThreads, 0, stream>>>(src, out, n, add, post_scale, apply, status);
+      return cudaGetLastError();
+    }
+  }
+  if constexpr (BW > 0) {
+    if (aligned) {
+#define HP_INDEX(W) case W: return launch_tern_index<BW, APPLY, W>(src, out, n, add, post_scale, apply, status, stream)
+      switch (src.world) {
+        HP_INDEX(1); HP_INDEX(2); HP_INDEX(3); HP_INDEX(4); HP_INDEX(5); HP_INDEX(6); HP_INDEX(7); HP_INDEX(8);
+        default: return cudaErrorInvalidValue;
+      }
+#undef HP_INDEX
+    }
+  }
   // table size: world x 256 x dpb floats; without a known bitwidth, room for 1-bit payloads (dpb = 8)
   const int dpb = BW > 0 ? 8 / BW : 8;
   const bool nibble = BW == 1 || BW == 2 || BW == 4;
   const size_t smem = nibble ? 0 : size_t(src.world) * 256 * dpb * sizeof(float);
   if (!nibble) {
-    // per device, and cheap: set on every launch rather than remembered per process
-    cudaError_t e = cudaFuncSetAttribute(tern_unpack_lut_kernel<BW, APPLY, kGeneric, 0>,
+    cudaError_t e = cudaFuncSetAttribute(tern_unpack_lut_kernel<BW, APPLY, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 256 * 8 * 4);
     if (e != cudaSuccess) return e;
   }
   // a CTA decodes many groups so that building its tables stays small against the decode work
   const int64_t groups = (n + 4 * dpb - 1) / (4 * dpb);
   const int grid = grid_for(groups, kUnpackThreads, nibble ? 148 * 4 : 148 * 8);
-  bool aligned = aligned16(out);
-  if (APPLY) aligned = aligned && aligned16(apply.param) && aligned16(apply.momentum);
-  if constexpr (BW == 2) {
-    if (src.shard_elems > 0) {
-      tern_unpack_lut_kernel<2, APPLY, kConcat, 0><<<grid, kUnpackThreads, 0, stream>>>(src, out, n, add, post_scale, apply, status);
-      return cudaGetLastError();
-    }
-    if (aligned) {
-#define HP_PAIR(W) \
-  case W: tern_unpack_lut_kernel<2, APPLY, kPair, W><<<grid, kUnpackThreads, 0, stream>>>(src, out, n, add, post_scale, apply, status); break
-      switch (src.world) {
-        HP_PAIR(1); HP_PAIR(2); HP_PAIR(3); HP_PAIR(4); HP_PAIR(5); HP_PAIR(6); HP_PAIR(7); HP_PAIR(8);
-        default: return cudaErrorInvalidValue;
-      }
-#undef HP_PAIR
-      return cudaGetLastError();
-    }
-  }
-  tern_unpack_lut_kernel<BW, APPLY, kGeneric, 0><<<grid, kUnpackThreads, smem, stream>>>(src, out, n, add, post_scale, apply, status);
+  tern_unpack_lut_kernel<BW, APPLY, false><<<grid, kUnpackThreads, smem, stream>>>(src, out, n, add, post_scale, apply, status);
   return cudaGetLastError();
 }
 

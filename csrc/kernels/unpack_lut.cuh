@@ -9,12 +9,11 @@
 // The decoded values of the ranks are summed in the canonical pairwise order (tree_sum in
 // codec_math.h), so the result is bit-identical to the CPU codec on every replica.  Three table
 // forms, fastest first:
-//   pair tables     2-bit payloads, 16-byte aligned dense arrays: ranks (2s, 2s+1) share a table
-//                   indexed by one nibble of each, whose entry already holds the pair's sum
-//                   (the first level of the canonical order), so eight ranks cost four
-//                   shared-memory reads and three adds per two elements
+//   index tables    bitwidths 1, 2, 4 and 16-byte aligned dense arrays: the fields of 8, 4 or 2 ranks
+//                   make up one index, whose entry already holds those ranks' sum
 //   nibble tables   bitwidths 1, 2, 4 at any alignment
-//   byte tables     bitwidth 8 or unknown
+//   byte tables     bitwidth 8 at any alignment, or unknown
+// At 8 bits and with aligned dense arrays the levels are decoded arithmetically.
 #pragma once
 #include "../common/codec_math.h"
 #include "kernels.h"
@@ -26,7 +25,10 @@ namespace cuda {
 constexpr int kUnpackThreads = 256;
 
 __device__ __forceinline__ uint32_t load_u32_any(const uint8_t* p) {
-  if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) return *reinterpret_cast<const uint32_t*>(p);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if ((a & 3) == 0) return *reinterpret_cast<const uint32_t*>(p);
+  if ((a & 1) == 0)
+    return uint32_t(reinterpret_cast<const uint16_t*>(p)[0]) | (uint32_t(reinterpret_cast<const uint16_t*>(p)[1]) << 16);
   return uint32_t(p[0]) | (uint32_t(p[1]) << 8) | (uint32_t(p[2]) << 16) | (uint32_t(p[3]) << 24);
 }
 
@@ -289,125 +291,328 @@ __device__ __forceinline__ void unpack_nibble_body(const float* lut, uint32_t (&
   }
 }
 
-// ---------------------------------------------------------------- pair tables, 2 bits
-// Slot s covers ranks (2s, 2s+1).  Its table has 256 rows of two floats: row (b << 4) | a holds
-// decode_{2s}(a) + decode_{2s+1}(b) for the two elements of nibbles a and b, i.e. the first
-// level of the canonical sum is read, not computed.  A last rank without a partner uses rows
-// 0..15 of its slot (b = 0), which hold its decoded values alone.
+// ---------------------------------------------------------------- index tables: 1, 2 and 4 bits
+// What bounds a decode of several payloads is not the dense store but the work per element and rank.
+// Here one table read covers 8 / BW ranks of an element: the BW-bit fields of those ranks side by side
+// are a byte, and row `byte` of the group's table holds their sum in the canonical order (the order
+// adds neighbours first, so a group of 2, 4 or 8 ranks is a subtree of it).  Eight ranks at 2 bits are
+// two reads and one add per element.  Every row is stored 32 times, once per bank: lane L reads its own
+// column, so no read conflicts whatever the data is; the price is 32 KB per group, built once by each
+// of the few resident CTAs.
 //
-// Index words: for payload words wa, wb of the two ranks, lo = (wa & 0x0f0f0f0f) | ((wb << 4) &
-// 0xf0f0f0f0) packs the four row numbers of the even nibbles into the bytes of one register and
-// hi = ((wa >> 4) & 0x0f0f0f0f) | (wb & 0xf0f0f0f0) those of the odd nibbles: eight look-ups
-// cost four logic instructions to prepare.  Rows are stored swizzled, row ^ ((row >> 4) & 5):
-// gradient nibbles are mostly 5, 6, 9 or 10 (both fields on a middle level), and without the
-// swizzle two lanes that agree in a and differ in b hit the same bank on different rows.
-//
-// Mapping: lane L of a warp handles payload byte j*32 + L (j = 0..3) of the warp's 128-byte
-// chunk, i.e. elements (j*32 + L)*4 .. +3 of the chunk's 512: every dense access is a 512-byte
-// contiguous run across the warp.  Payloads are loaded one 32-bit word per lane and rank; index
-// words reach their lanes by shuffle.
-constexpr int kPairRows = 256;
-__device__ __forceinline__ uint32_t pair_swizzle(uint32_t packed_rows) {
-  return packed_rows ^ ((packed_rows >> 4) & 0x05050505u);
-}
+// A lane loads 32 payload bits of each rank, turns the words of a group into one index byte per element
+// (a shift and a bit select per field, then a byte transposition), and writes those bytes to a buffer of
+// its warp; the lanes read them back so that every dense access is a 512-byte run across the warp.
+// The form before this one read a table entry per pair of ranks and two elements, with bank conflicts,
+// and moved every index word by shuffle:
+// 4 bits, one payload, 2.4 M elements (ncu, cold): 15.8 us before, 6.9 now; 2 bits, eight payloads, 25 MB,
+// compress and decode together: 62.7 us before, 58 now.
+constexpr int kIndexThreads = 256;
 
-// value(r, nibble, which): decoded value of element `which` (0/1) of a nibble of rank r.
-// tables: [slots][256][2] floats; slots = (world + 1) / 2, or one table when SHARED (all ranks
-// decode alike, and the lone rank of an odd world reads the pair rows of a partner that decodes
-// to zero: lone_nibble is that partner's nibble).
-template <bool SHARED, typename Value>
-__device__ __forceinline__ void build_pair_tables(float* tables, int world, Value value) {
-  const int slots = SHARED ? 1 : (world + 1) / 2;
-  for (int i = threadIdx.x; i < slots * kPairRows; i += blockDim.x) {
-    const int s = i >> 8, row = i & 255, a = row & 15, b = row >> 4;
-    const int ra = 2 * s, rb = 2 * s + 1;
-    const bool lone = !SHARED && rb >= world;
-    if (lone && b != 0) continue;
-    float x = value(ra, a, 0), y = value(ra, a, 1);
-    if (!lone) {
-      x = hp_add(x, value(rb, b, 0));
-      y = hp_add(y, value(rb, b, 1));
+template <int BW>
+struct IndexForm {
+  static constexpr int kRanks = 8 / BW;        // ranks per group
+  static constexpr int kElems = 32 / BW;       // elements per payload word = index bytes per lane and group
+  static constexpr int kChunk = 32 * kElems;   // elements a warp decodes per iteration
+  static constexpr int kDpb = 8 / BW;
+};
+// Sequential sums (the order of the ECQ codec: ascending ranks, one by one) read the first group's sum
+// from its table and every later rank from a table of its own.
+template <int BW, int WORLD, bool SHARED, bool SEQ>
+struct IndexLayout {
+  using F = IndexForm<BW>;
+  static constexpr int kGroups = (WORLD + F::kRanks - 1) / F::kRanks;
+  static constexpr int kFirst = WORLD < F::kRanks ? WORLD : F::kRanks;      // ranks of the first group
+  static constexpr int kLast = WORLD - (kGroups - 1) * F::kRanks;            // ranks of the last one
+  static constexpr int rows(int g) { return 1 << (BW * (g + 1 < kGroups || SHARED ? kFirst : kLast)); }
+  static constexpr int kFull = 1 << (BW * kFirst);                           // rows before group 1
+  static constexpr int kRows = SEQ ? kFull + (WORLD - kFirst) * (1 << BW)
+                                   : (SHARED ? kFull : kFull * (kGroups - 1) + rows(kGroups - 1));
+  static constexpr int kStage = 32 * F::kElems * kGroups;                    // bytes per warp
+  static constexpr size_t kBytes = size_t(kRows) * 128 + size_t(kIndexThreads / 32) * kStage;
+};
+
+// value(r, q): decoded value of level q of rank r.
+template <int BW, int WORLD, bool SHARED, bool SEQ, typename Value>
+__device__ __forceinline__ void build_index_tables(float* tables, Value value) {
+  using L = IndexLayout<BW, WORLD, SHARED, SEQ>;
+  constexpr int R = IndexForm<BW>::kRanks;
+  constexpr uint32_t mask = (1u << BW) - 1u;
+  for (int i = threadIdx.x; i < L::kRows; i += blockDim.x) {
+    float x;
+    if (SEQ && i >= L::kFull) {
+      const int at = i - L::kFull;
+      x = value(L::kFirst + (at >> BW), uint32_t(at) & mask);
+    } else {
+      const int g = SHARED || SEQ ? 0 : i / L::kFull;
+      const uint32_t byte = uint32_t(i - g * L::kFull);
+      float v[R];
+#pragma unroll
+      for (int p = 0; p < R; ++p) v[p] = g * R + p < WORLD ? value(g * R + p, (byte >> (BW * p)) & mask) : 0.0f;
+      const int ranks = WORLD - g * R < R ? WORLD - g * R : R;
+      if (SEQ) {
+        x = v[0];
+#pragma unroll
+        for (int p = 1; p < R; ++p)
+          if (p < ranks) x = hp_add(x, v[p]);
+      } else {
+        x = tree_sum(v, ranks);
+      }
     }
-    const int at = row ^ ((row >> 4) & 5);
-    reinterpret_cast<float2*>(tables)[s * kPairRows + at] = make_float2(x, y);
+    // 32 copies; the lanes start at different columns, so that the stores spread over the banks
+    float4* row = reinterpret_cast<float4*>(tables + i * 32);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) row[(c + threadIdx.x) & 7] = make_float4(x, x, x, x);
   }
 }
 
-// WORLD is a template parameter: with the rank count known at compile time the loops below are
-// straight-line code (a first version that tested `r < src.world` everywhere spent 60 % of its
-// instructions on those tests and their branches).
-template <bool APPLY, bool SHARED, int WORLD>
-__device__ __forceinline__ void unpack_pair_body(const float* tables, uint32_t lone_word, uint32_t (&w)[kMaxWorld],
-                                                 const UnpackSources& src, int64_t data_offset,
-                                                 float* __restrict__ out, int64_t n, int add,
-                                                 float post_scale, const SgdApply& apply) {
-  constexpr int kSlots = (WORLD + 1) / 2;
-  const int64_t full_chunks = n / 512;  // complete 128-byte warp chunks
-  const int lane = threadIdx.x & 31;
-  const uint32_t sel = 0x4440u | uint32_t(lane & 3);  // byte (lane & 3) of a register, zero-extended
-  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-  int64_t chunk = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  for (; chunk < full_chunks; chunk += warps) {
-    const int64_t nxt = (chunk + warps) * 32 + lane;
-    const bool more = chunk + warps < full_chunks;
-    uint32_t wn[WORLD];
+// Index bytes of one group: u[] holds them in element order.  w: the payload words of the group's ranks.
+template <int BW, int N>
+__device__ __forceinline__ void index_bytes(const uint32_t (&w)[N], uint32_t (&u)[IndexForm<BW>::kElems / 4]) {
+  constexpr int D = IndexForm<BW>::kDpb;
+  constexpr uint32_t field = BW == 4 ? 0x0f0f0f0fu : (BW == 2 ? 0x03030303u : 0x01010101u);
+  uint32_t t[D];   // t[j], byte b: index of element b * D + j
 #pragma unroll
-    for (int r = 0; r < WORLD; ++r)
-      wn[r] = more ? load_u32_any(src.payload[r] + data_offset + nxt * 4) : 0u;
-    uint32_t lo[kSlots], hi[kSlots];
+  for (int j = 0; j < D; ++j) {
+    t[j] = 0;
 #pragma unroll
-    for (int s = 0; s < kSlots; ++s) {
-      const uint32_t wa = w[2 * s];
-      const uint32_t wb = (2 * s + 1 < WORLD) ? w[2 * s + 1] : lone_word;
-      lo[s] = pair_swizzle((wa & 0x0f0f0f0fu) | ((wb << 4) & 0xf0f0f0f0u));
-      hi[s] = pair_swizzle(((wa >> 4) & 0x0f0f0f0fu) | (wb & 0xf0f0f0f0u));
+    for (int p = 0; p < N; ++p) {
+      const uint32_t moved = j >= p ? w[p] >> (BW * (j - p)) : w[p] << (BW * (p - j));
+      t[j] |= moved & (field << (BW * p));
     }
-    float* const o = out + chunk * 512 + lane * 4;
+  }
+  if constexpr (D == 2) {
+    u[0] = __byte_perm(t[0], t[1], 0x5140);
+    u[1] = __byte_perm(t[0], t[1], 0x7362);
+  } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int from = j * 8 + (lane >> 2);
-      float v[4][kSlots];
+    for (int q = 0; q < D / 4; ++q) {
+      const uint32_t a = __byte_perm(t[4 * q], t[4 * q + 1], 0x5140), b = __byte_perm(t[4 * q + 2], t[4 * q + 3], 0x5140);
+      const uint32_t c = __byte_perm(t[4 * q], t[4 * q + 1], 0x7362), d = __byte_perm(t[4 * q + 2], t[4 * q + 3], 0x7362);
+      u[0 * (D / 4) + q] = __byte_perm(a, b, 0x5410);
+      u[1 * (D / 4) + q] = __byte_perm(a, b, 0x7632);
+      u[2 * (D / 4) + q] = __byte_perm(c, d, 0x5410);
+      u[3 * (D / 4) + q] = __byte_perm(c, d, 0x7632);
+    }
+  }
+}
+
+// Payload words in flight.  `align` says how every payload's packed data lies (payload_alignment): on
+// 4-byte boundaries (the receive slots of the exchange), on 2-byte ones (behind a 10-byte header at the
+// start of a tensor), or anyhow.  It is the same for the whole call, and the halves of a 2-byte aligned word
+// are only put together where the word is used: a load that decides by its own address, and combines what
+// it loaded, waits for memory once per rank instead of once for all.
+template <int WORLD>
+struct PayloadWords {
+  uint32_t lo[WORLD], hi[WORLD];
+  __device__ __forceinline__ void clear() {
 #pragma unroll
-      for (int s = 0; s < kSlots; ++s) {
-        const uint32_t l = __shfl_sync(0xffffffffu, lo[s], from);
-        const uint32_t h = __shfl_sync(0xffffffffu, hi[s], from);
-        const char* table = reinterpret_cast<const char*>(tables) + (SHARED ? 0 : s * kPairRows * 8);
-        const float2 a = *reinterpret_cast<const float2*>(table + (__byte_perm(l, 0u, sel) << 3));
-        const float2 b = *reinterpret_cast<const float2*>(table + (__byte_perm(h, 0u, sel) << 3));
-        v[0][s] = a.x; v[1][s] = a.y; v[2][s] = b.x; v[3][s] = b.y;
+    for (int r = 0; r < WORLD; ++r) lo[r] = hi[r] = 0;
+  }
+  __device__ __forceinline__ void load(const UnpackSources& src, int64_t at, int align) {
+    if (align == 4) {
+#pragma unroll
+      for (int r = 0; r < WORLD; ++r) {
+        lo[r] = __ldg(reinterpret_cast<const uint32_t*>(src.payload[r] + at));
+        hi[r] = 0;
       }
+    } else if (align == 2) {
+#pragma unroll
+      for (int r = 0; r < WORLD; ++r) {
+        const uint16_t* p = reinterpret_cast<const uint16_t*>(src.payload[r] + at);
+        lo[r] = __ldg(p);
+        hi[r] = __ldg(p + 1);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < WORLD; ++r) {
+        lo[r] = load_u32_any(src.payload[r] + at);
+        hi[r] = 0;
+      }
+    }
+  }
+  __device__ __forceinline__ uint32_t word(int r) const { return lo[r] | (hi[r] << 16); }
+};
+
+// The first words of a thread, requested before the kernel reads headers and builds its tables.  A word
+// is only requested when it lies inside the slot, whatever the header will turn out to say.
+template <int BW, int WORLD>
+__device__ __forceinline__ void index_prefetch(const UnpackSources& src, int header_bytes, int64_t n, int align,
+                                               PayloadWords<WORLD>& w) {
+  const int64_t warp = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t word = warp * 32 + (threadIdx.x & 31);
+  bool ok = warp < n / IndexForm<BW>::kChunk;
+#pragma unroll
+  for (int r = 0; r < WORLD; ++r) ok = ok && header_bytes + (word + 1) * 4 <= src.payload_bytes[r];
+  w.clear();
+  if (ok) w.load(src, src.parity_off + header_bytes + word * 4, align);
+}
+
+// smem: tables, then the warps' index buffers.  pad: payload word of a rank that is not there in a
+// SHARED table's last group (fields that decode to +0).
+template <int BW, bool APPLY, int WORLD, bool SHARED, bool SEQ>
+__device__ __forceinline__ void unpack_index_body(float* smem, PayloadWords<WORLD>& w, uint32_t pad, const UnpackSources& src,
+                                                  int64_t data_offset, int align, float* __restrict__ out, int64_t n,
+                                                  int add, float post_scale, const SgdApply& apply) {
+  using F = IndexForm<BW>;
+  using L = IndexLayout<BW, WORLD, SHARED, SEQ>;
+  constexpr int R = F::kRanks, G = L::kGroups, V = F::kElems / 4;
+  constexpr uint32_t mask = (1u << BW) - 1u;
+  const int lane = threadIdx.x & 31;
+  uint32_t* stage = reinterpret_cast<uint32_t*>(smem + L::kRows * 32) + (threadIdx.x >> 5) * (L::kStage / 4);
+  const float* table = smem + lane;
+  auto sum_of = [&](const uint32_t (&byte)[G]) -> float {
+    if constexpr (SEQ) {
+      float x = table[byte[0] * 32];
+#pragma unroll
+      for (int r = L::kFirst; r < WORLD; ++r)
+        x = hp_add(x, table[(L::kFull + ((r - L::kFirst) << BW) + ((byte[r / R] >> (BW * (r % R))) & mask)) * 32]);
+      return x;
+    } else {
+      float v[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) v[g] = table[((SHARED ? 0 : g * L::kFull) + byte[g]) * 32];
+      return tree_sum(v, G);
+    }
+  };
+  const int64_t chunks = n / F::kChunk;
+  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t c = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); c < chunks; c += warps) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      uint32_t u[V];
+      if (SHARED || g + 1 < G) {
+        constexpr int N = SHARED && G > 1 ? R : L::kFirst;
+        uint32_t x[N];
+#pragma unroll
+        for (int p = 0; p < N; ++p) x[p] = g * R + p < WORLD ? w.word((g * R + p) % WORLD) : pad;
+        index_bytes<BW>(x, u);
+      } else {
+        uint32_t x[L::kLast];
+#pragma unroll
+        for (int p = 0; p < L::kLast; ++p) x[p] = w.word((g * R + p) % WORLD);
+        index_bytes<BW>(x, u);
+      }
+      uint32_t* mine = stage + g * (8 * F::kElems) + lane * V;
+      if constexpr (V == 2) {
+        *reinterpret_cast<uint2*>(mine) = make_uint2(u[0], u[1]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < V / 4; ++q)
+          reinterpret_cast<uint4*>(mine)[q] = make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+      }
+    }
+    if (c + warps < chunks) w.load(src, data_offset + ((c + warps) * 32 + lane) * 4, align);
+    __syncwarp();
+    float* const o = out + c * F::kChunk + lane * 4;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      uint32_t four[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) four[g] = stage[g * (8 * F::kElems) + j * 32 + lane];
       float acc[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = tree_sum(v[k], kSlots);
-      unpack_finish4<APPLY>(acc, o, j * 128, add, post_scale, apply, chunk * 512 + lane * 4 + j * 128);
-    }
+      for (int k = 0; k < 4; ++k) {
+        uint32_t byte[G];
 #pragma unroll
-    for (int r = 0; r < WORLD; ++r) w[r] = wn[r];
-  }
-  // elements past the last complete chunk (fewer than 512): block 0, element by element,
-  // through the same tables (rank pairs, then the canonical order over the slots)
-  if (blockIdx.x == 0) {
-    const uint32_t lone_nib = lone_word & 15u;
-    for (int64_t e = full_chunks * 512 + threadIdx.x; e < n; e += blockDim.x) {
-      float v[kSlots];
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s) {
-        const int sh = 4 * int((e & 3) >> 1);
-        const uint32_t a = (uint32_t(src.payload[2 * s][data_offset + (e >> 2)]) >> sh) & 15u;
-        uint32_t b = lone_nib;
-        if (2 * s + 1 < WORLD) b = (uint32_t(src.payload[(2 * s + 1) % kMaxWorld][data_offset + (e >> 2)]) >> sh) & 15u;
-        const uint32_t row = (b << 4) | a;
-        v[s] = tables[((SHARED ? 0 : s) * kPairRows + (row ^ ((row >> 4) & 5u))) * 2 + (e & 1)];
+        for (int g = 0; g < G; ++g) byte[g] = (four[g] >> (8 * k)) & 255u;
+        acc[k] = sum_of(byte);
       }
-      unpack_finish1<APPLY>(tree_sum(v, kSlots), out, e, add, post_scale, apply);
+      unpack_finish4<APPLY>(acc, o, j * 128, add, post_scale, apply, c * F::kChunk + lane * 4 + j * 128);
+    }
+    __syncwarp();
+  }
+  // elements past the last complete chunk: block 0, element by element, through the same tables
+  if (blockIdx.x == 0) {
+    for (int64_t e = chunks * F::kChunk + threadIdx.x; e < n; e += blockDim.x) {
+      const int sh = BW * int(e % F::kDpb);
+      uint32_t byte[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        byte[g] = 0;
+#pragma unroll
+        for (int p = 0; p < R; ++p) {
+          const int r = g * R + p;
+          uint32_t q = 0;
+          if (r < WORLD) q = (uint32_t(src.payload[r % kMaxWorld][data_offset + e / F::kDpb]) >> sh) & mask;
+          else if (SHARED && G > 1) q = pad & mask;
+          byte[g] |= q << (BW * p);
+        }
+      }
+      unpack_finish1<APPLY>(sum_of(byte), out, e, add, post_scale, apply);
     }
   }
+}
+
+// ---------------------------------------------------------------- 8 bits
+// A payload word is four elements: the lane that loads it stores them, and a level is decoded by its own
+// two rounded operations (a table per rank would fill shared memory for no fewer instructions).
+template <bool APPLY, int WORLD, bool SEQ, typename Value>
+__device__ __forceinline__ void unpack_bytes_body(const UnpackSources& src, int64_t data_offset, int align,
+                                                  float* __restrict__ out, int64_t n, int add, float post_scale,
+                                                  const SgdApply& apply, Value value) {
+  auto sum_of = [&](const uint32_t (&q)[WORLD]) -> float {
+    float v[WORLD];
+#pragma unroll
+    for (int r = 0; r < WORLD; ++r) v[r] = value(r, q[r]);
+    if constexpr (SEQ) {
+#pragma unroll
+      for (int r = 1; r < WORLD; ++r) v[0] = hp_add(v[0], v[r]);
+      return v[0];
+    } else {
+      return tree_sum(v, WORLD);
+    }
+  };
+  const int64_t words = n >> 2;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  PayloadWords<WORLD> w;
+  if (i < words) w.load(src, data_offset + i * 4, align);
+  for (; i < words; i += stride) {
+    uint32_t now[WORLD];
+#pragma unroll
+    for (int r = 0; r < WORLD; ++r) now[r] = w.word(r);
+    if (i + stride < words) w.load(src, data_offset + (i + stride) * 4, align);
+    float acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint32_t q[WORLD];
+#pragma unroll
+      for (int r = 0; r < WORLD; ++r) q[r] = (now[r] >> (8 * k)) & 255u;
+      acc[k] = sum_of(q);
+    }
+    unpack_finish4<APPLY>(acc, out, i * 4, add, post_scale, apply);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < (n & 3)) {
+    const int64_t e = (words << 2) + threadIdx.x;
+    uint32_t q[WORLD];
+#pragma unroll
+    for (int r = 0; r < WORLD; ++r) q[r] = src.payload[r][data_offset + e];
+    unpack_finish1<APPLY>(sum_of(q), out, e, add, post_scale, apply);
+  }
+}
+
+// 4, 2 or 1: the alignment of every payload's packed data (and, with slots double-buffered by parity, of the
+// other slot's).
+inline int payload_alignment(const UnpackSources& src, int header_bytes) {
+  uintptr_t bits = uintptr_t(src.parity_stride);
+  for (int r = 0; r < src.world; ++r) bits |= reinterpret_cast<uintptr_t>(src.payload[r] + header_bytes);
+  return (bits & 3) == 0 ? 4 : ((bits & 1) == 0 ? 2 : 1);
+}
+// Resident CTAs of an index-table kernel: by shared memory, and no more than three per SM by registers.
+inline int index_grid(int64_t n, int chunk, size_t smem_bytes) {
+  const int warps = kIndexThreads / 32;
+  int64_t blocks = (n / chunk + warps - 1) / warps;
+  int per_sm = int((size_t(227) * 1024) / (smem_bytes + 1024));
+  per_sm = per_sm < 1 ? 1 : (per_sm > 3 ? 3 : per_sm);
+  if (blocks > 148 * per_sm) blocks = 148 * per_sm;
+  return blocks < 1 ? 1 : int(blocks);
 }
 
 // ---------------------------------------------------------------- concatenated shards, 2 bits
 // Sharded exchange, last phase: payload[j] encodes shard j alone.  nib: [world or 1][16][2]
-// nibble tables (rank j's at nib + j*32 floats; one table when SHARED).  Same lane mapping as
-// the pair body; a 512-element chunk never straddles two shards (shard_elems % 2048 == 0).
+// nibble tables (rank j's at nib + j*32 floats; one table when SHARED).  Lane L
+// decodes payload byte j*32 + L (j = 0..3) of the warp's 128-byte chunk; a 512-element chunk never straddles two shards (shard_elems % 2048 == 0).
 // header_bytes + slot_shift: where the packed data starts inside payload[j].
 template <bool APPLY, bool SHARED>
 __device__ __forceinline__ void unpack_concat_body(const float* nib, const UnpackSources& src, int64_t data_offset,
@@ -443,13 +648,6 @@ __device__ __forceinline__ void unpack_concat_body(const float* nib, const Unpac
       unpack_finish1<APPLY>(nib[((SHARED ? 0 : j) * 16 + nb) * 2 + (le & 1)], out, e, add, post_scale, apply);
     }
   }
-}
-
-// True when the dense arrays allow the 16-byte accesses of the pair and concat bodies.
-__device__ __forceinline__ bool unpack_coalesced_ok(const float* out, bool apply_on, const SgdApply& apply) {
-  uintptr_t bits = reinterpret_cast<uintptr_t>(out);
-  if (apply_on) bits |= reinterpret_cast<uintptr_t>(apply.param) | reinterpret_cast<uintptr_t>(apply.momentum);
-  return (bits & 15) == 0;
 }
 
 }  // namespace cuda

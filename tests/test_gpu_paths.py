@@ -78,3 +78,59 @@ def test_sparse_decode_under_capture():
     out.fill_(3.0)
     graph.replay()
     assert torch.equal(out, want)
+
+
+# ----------------------------------------------------------------------------- quantisers: decode
+def at_offset(payload, offset):
+    """The payload `offset` bytes past an allocation's start (16-byte aligned): 6 puts data behind a 10-byte header on
+    a 16-byte boundary, as in the exchange's receive slots."""
+    buf = torch.zeros(payload.numel() + offset, dtype=torch.uint8, device="cuda")
+    buf[offset:] = payload.cuda()
+    return buf[offset:]
+
+
+@pytest.mark.parametrize("bw", [1, 2, 4, 8])
+@pytest.mark.parametrize("world", range(1, 9))
+@pytest.mark.parametrize("offset", [0, 1, 6])
+def test_terngrad_decode_tables(bw, world, offset):
+    chunk = 1024 // bw
+    for n in (1, chunk - 1, chunk, 9 * chunk + 5):
+        payloads = [ops.terngrad_compress(gauss(n, seed=s), bw, True, seed=s) for s in range(world)]
+        for add in (False, True):
+            ref = gauss(n, 1.0, seed=99)
+            out = ref.cuda()
+            ops.terngrad_decompress(payloads, ref, add=add, post_scale=1.0 / world, bitwidth=bw)
+            ops.terngrad_decompress([at_offset(p, offset) for p in payloads], out, add=add, post_scale=1.0 / world,
+                                    bitwidth=bw)
+            assert torch.equal(out.cpu(), ref), (n, add)
+    assert ops.read_status(out) == 0
+
+
+@pytest.mark.parametrize("world", range(1, 9))
+@pytest.mark.parametrize("offset", [0, 2, 3])
+def test_tbq_decode_tables(world, offset):
+    for n in (1, 511, 512, 4613):
+        payloads = [ops.tbq_compress(gauss(n, 0.03, seed=s), torch.zeros(n), 0.02) for s in range(world)]
+        for add in (False, True):
+            ref = gauss(n, 1.0, seed=99)
+            out = ref.cuda()
+            ops.tbq_decompress(payloads, ref, 0.02, add=add, post_scale=1.0 / world)
+            ops.tbq_decompress([at_offset(p, offset) for p in payloads], out, 0.02, add=add, post_scale=1.0 / world)
+            assert torch.equal(out.cpu(), ref), (n, add)
+
+
+@pytest.mark.parametrize("bw", [2, 4, 8])
+@pytest.mark.parametrize("world", range(1, 9))
+def test_ecq_decode_tables(bw, world):
+    chunk = 1024 // bw
+    for n in (1, chunk, 9 * chunk + 5):
+        payloads = [ops.ecq_compress(gauss(n, seed=s), torch.zeros(n), 1.0, 0.9, bw, seed=s) for s in range(world)]
+        for add in (False, True):
+            ref = gauss(n, 1.0, seed=99)
+            ops_ref = ref.clone()
+            ops.ecq_decompress(payloads, ops_ref, add=add, post_scale=0.5)
+            for offset, shift in ((0, 0), (6, 0), (0, 1)):
+                out = torch.empty(n + shift, device="cuda")[shift:]
+                out.copy_(ref)
+                ops.ecq_decompress([at_offset(p, offset) for p in payloads], out, add=add, post_scale=0.5)
+                assert torch.equal(out.cpu(), ops_ref), (n, add, offset, shift)
