@@ -14,6 +14,7 @@
 // kernel of the step recorded a failure.
 #include "../common/codec_math.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "p2p.cuh"
 #include "reduce.cuh"
 #include "unpack_lut.cuh"
@@ -44,14 +45,26 @@ ecq_absmax_header_kernel(const float* __restrict__ grad, const float* __restrict
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t nv = VEC ? (n >> 2) : 0;  // 16-byte loads when both arrays are aligned
-  for (int64_t i = tid; i < nv; i += stride) {
-    const float4 g = __ldg(reinterpret_cast<const float4*>(grad) + i);
-    const float4 h = __ldg(reinterpret_cast<const float4*>(hist) + i);
+  auto fold = [&](float4 g, float4 h) {
     mx = fmaxf(mx, fmaxf(fmaxf(fabsf(ecq_compensated(g.x, h.x, alpha)), fabsf(ecq_compensated(g.y, h.y, alpha))),
                          fmaxf(fabsf(ecq_compensated(g.z, h.z, alpha)), fabsf(ecq_compensated(g.w, h.w, alpha)))));
+  };
+  int64_t q = tid;
+  for (; q + 3 * stride < nv; q += 4 * stride) {   // four loads of each array in flight
+    float4 g[4], h[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      g[u] = __ldg(reinterpret_cast<const float4*>(grad) + q + u * stride);
+      h[u] = __ldg(reinterpret_cast<const float4*>(hist) + q + u * stride);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) fold(g[u], h[u]);
   }
+  for (; q < nv; q += stride)
+    fold(__ldg(reinterpret_cast<const float4*>(grad) + q), __ldg(reinterpret_cast<const float4*>(hist) + q));
   for (int64_t i = (nv << 2) + tid; i < n; i += stride)
     mx = fmaxf(mx, fabsf(ecq_compensated(grad[i], hist[i], alpha)));
+  let_next_start();
   float gmn, gmx;
   if (!grid_minmax_last_block<kThreads>(scratch, unused, mx, gmn, gmx)) return;
   if (threadIdx.x == 0) {
@@ -78,14 +91,19 @@ ecq_absmax_header_kernel(const float* __restrict__ grad, const float* __restrict
   }
 }
 
+constexpr int kStageBytes = 512;  // payload bytes a warp gathers before it stores them
+
 // One thread quantises four consecutive elements (one 16-byte load of the gradient and of the
 // history, one 16-byte store of the history) into BW/2 payload bytes; lanes then combine their
 // bytes into 32-bit words, so that every destination gets word stores.  The random generator is
-// seeded per payload byte, as in the CPU codec.
+// seeded per payload byte, as in the CPU codec.  shift >= 0: large tensors whose destinations start
+// equally far past a 16-byte boundary; a warp then gathers 512 payload bytes in shared memory, with the
+// loads of four sub-steps in flight, and stores them 16 bytes per lane (put_chunk512).
 template <int BW, bool VEC>
 __global__ void __launch_bounds__(kThreads)
 ecq_quant_kernel(const float* __restrict__ grad, float* __restrict__ hist, int64_t n, float alpha,
-                 float beta, uint64_t seed, PushTargets dst, const MinMaxScratch* scratch) {
+                 float beta, uint64_t seed, PushTargets dst, const MinMaxScratch* scratch, int shift) {
+  wait_for_previous();
   if (push_guarded(dst)) return;
   resolve_epoch(dst);
   if (dst.epoch_dev != nullptr) seed += uint64_t(dst.epoch) * kEpochSeedStride;
@@ -109,10 +127,58 @@ ecq_quant_kernel(const float* __restrict__ grad, float* __restrict__ hist, int64
     }
     return q;
   };
+  int64_t unit0 = 0;   // first unit of the rest
+  if (VEC && shift >= 0) {
+    constexpr int64_t CU = int64_t(kStageBytes) / BPT;   // units per chunk
+    __shared__ __align__(16) uint8_t stages[kThreads / 32][kStageBytes + 16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint8_t* const stage = stages[warp] + shift;
+    const PushCursor all{nullptr};
+    const int64_t chunks = (n >> 2) / CU;
+    const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t c = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp; c < chunks; c += warps) {
+#pragma unroll 1
+      for (int j = 0; j < int(CU) / 32; j += 4) {
+        float4 gv[4], hv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int64_t u = c * CU + (j + k) * 32 + lane;
+          gv[k] = __ldg(reinterpret_cast<const float4*>(grad) + u);
+          hv[k] = reinterpret_cast<const float4*>(hist)[u];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int at = (j + k) * 32 + lane;
+          const int64_t u = c * CU + at;
+          const float g[4] = {gv[k].x, gv[k].y, gv[k].z, gv[k].w};
+          float h[4] = {hv[k].x, hv[k].y, hv[k].z, hv[k].w};
+          uint32_t bytes = 0;
+#pragma unroll
+          for (int b = 0; b < BPT; ++b)
+            bytes |= quant_byte(g + b * DPB, h + b * DPB, DPB, u * BPT + b) << (8 * b);
+          reinterpret_cast<float4*>(hist)[u] = make_float4(h[0], h[1], h[2], h[3]);
+          if (BPT == 1) {
+            stage[at] = uint8_t(bytes);
+          } else if (BPT == 2) {
+            reinterpret_cast<uint16_t*>(stage)[at] = uint16_t(bytes);
+          } else if ((shift & 3) == 0) {
+            reinterpret_cast<uint32_t*>(stage)[at] = bytes;
+          } else {
+            reinterpret_cast<uint16_t*>(stage)[2 * at] = uint16_t(bytes);
+            reinterpret_cast<uint16_t*>(stage)[2 * at + 1] = uint16_t(bytes >> 16);
+          }
+        }
+      }
+      __syncwarp();
+      put_chunk512(dst, all, kEcqHeaderBytes + c * kStageBytes, stages[warp], shift, lane);
+      __syncwarp();
+    }
+    unit0 = chunks * CU;
+  }
   const int64_t units = n >> 2;
-  const int64_t units_padded = (units + 31) & ~int64_t(31);
+  const int64_t units_padded = (units + 31) & ~int64_t(31);   // unit0 is a multiple of 32
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t u = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; u < units_padded; u += stride) {
+  for (int64_t u = unit0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; u < units_padded; u += stride) {
     uint32_t bytes = 0;
     if (u < units) {
       float g[4], h[4];
@@ -318,19 +384,23 @@ cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alp
   const int hgrid = grid_for((n + 3) >> 2, kThreads, 148 * 4);
   if (vec) ecq_absmax_header_kernel<true><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
   else ecq_absmax_header_kernel<false><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
-  const int grid = grid_for((n + 3) >> 2, kThreads, 148 * 8);
-#define HP_ECQ(BW)                                                                                               \
-  do {                                                                                                           \
-    if (vec) ecq_quant_kernel<BW, true><<<grid, kThreads, 0, stream>>>(grad, history, n, alpha, beta, seed, dst, s);  \
-    else ecq_quant_kernel<BW, false><<<grid, kThreads, 0, stream>>>(grad, history, n, alpha, beta, seed, dst, s);     \
-  } while (0)
+  // chunked path once there is a chunk per warp of a half-filled GPU
+  const int shift = chunk_shift(dst, kEcqHeaderBytes);
+  const int64_t chunks = n / (int64_t(kStageBytes) * (8 / bitwidth));
+  const bool wide = vec && shift >= 0 && chunks >= 148 * 2;
+  const int threads = wide ? 128 : kThreads;
+  const int grid = wide ? grid_for(chunks * 32, threads, 148 * 16) : grid_for((n + 3) >> 2, kThreads, 148 * 8);
+#define HP_ECQ(BW)                                                                                                   \
+  return vec ? launch_after(ecq_quant_kernel<BW, true>, dim3(grid), dim3(threads), 0, stream, grad, history, n,      \
+                            alpha, beta, seed, dst, s, wide ? shift : -1)                                            \
+             : launch_after(ecq_quant_kernel<BW, false>, dim3(grid), dim3(threads), 0, stream, grad, history, n,     \
+                            alpha, beta, seed, dst, s, -1)
   switch (bitwidth) {
-    case 2: HP_ECQ(2); break;
-    case 4: HP_ECQ(4); break;
-    default: HP_ECQ(8); break;
+    case 2: HP_ECQ(2);
+    case 4: HP_ECQ(4);
+    default: HP_ECQ(8);
   }
 #undef HP_ECQ
-  return cudaGetLastError();
 }
 
 cudaError_t ecq_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,

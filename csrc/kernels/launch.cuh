@@ -7,7 +7,8 @@
 // exactly as plain launches are.  Pointers that are read through the read-only path afterwards are
 // passed through after_wait(), so that no such load can be moved above the wait.  The kernel before
 // it calls let_next_start() (its result is only about when the next one is brought in, never about
-// what it may read).  The first kernel of a chain is launched plainly: its inputs come from kernels
+// what it may read), and a long one only when its work is nearly done: CTAs that wait hold registers and
+// shared memory which kernels of other streams, the backward pass above all, could use.  The first kernel of a chain is launched plainly: its inputs come from kernels
 // of the caller, which know nothing of this.
 #pragma once
 #include <cuda_runtime.h>

@@ -98,6 +98,11 @@ __device__ __forceinline__ bool push_aligned16(const PushTargets& t, int64_t dat
     if (p < t.world) bits |= reinterpret_cast<uintptr_t>(t.payload[p] + t.parity_off + data_off);
   return (bits & 15) == 0;
 }
+__device__ __forceinline__ void push_u16(const PushTargets& t, int64_t byte_off, uint16_t v) {
+#pragma unroll
+  for (int p = 0; p < kMaxWorld; ++p)
+    if (p < t.world) *reinterpret_cast<uint16_t*>(t.payload[p] + t.parity_off + byte_off) = v;
+}
 // payload[j] (+ parity offset) for a run-time j: selects over compile-time indices, so that the
 // kernel argument stays in parameter space (see resolve_epoch).
 __device__ __forceinline__ uint8_t* select_dest(const PushTargets& t, int j) {
@@ -153,6 +158,37 @@ __device__ __forceinline__ void put_bytes(const PushTargets& t, const PushCursor
   } else {
     push_bytes(t, off, src, count);
   }
+}
+
+// 512 payload bytes of a warp, gathered in shared memory, to every destination.  `shift` (0 to 14, even)
+// is how far the bytes start past a 16-byte boundary in every destination; they lie at stage + shift, so
+// that 16-byte words of the buffer are 16-byte words of the destination.  Lane L stores word L; with a
+// shift, the bytes of the first and the last, partial word go out as eight 2-byte stores.  stage: 16-byte
+// aligned, 528 bytes.
+__device__ __forceinline__ void put_chunk512(const PushTargets& t, const PushCursor& c, int64_t off, const uint8_t* stage,
+                                             int shift, int lane) {
+  const uint4 v = reinterpret_cast<const uint4*>(stage)[lane];
+  if (shift == 0) {
+    put_u128(t, c, off + lane * 16, v);
+    return;
+  }
+  if (lane > 0) put_u128(t, c, off - shift + lane * 16, v);
+  if (lane < 8) {
+    const int at = 2 * lane >= shift ? 2 * lane : 512 + 2 * lane;   // in the buffer
+    const uint16_t h = *reinterpret_cast<const uint16_t*>(stage + at);
+    if (c.one) *reinterpret_cast<uint16_t*>(c.one + off - shift + at) = h;
+    else push_u16(t, off - shift + at, h);
+  }
+}
+// That shift for packed data behind `data_off` bytes of payload, or -1 when the destinations differ in it
+// or it is odd.
+inline int chunk_shift(const PushTargets& t, int data_off) {
+  const int shift = int(reinterpret_cast<uintptr_t>(t.payload[0] + data_off) & 15);
+  if ((shift & 1) != 0 || (t.parity_stride & 15) != 0) return -1;
+  for (int p = 1; p < t.world; ++p)
+    if (int(reinterpret_cast<uintptr_t>(t.payload[p] + data_off) & 15) != shift) return -1;
+  if (t.mc != nullptr && int(reinterpret_cast<uintptr_t>(t.mc + data_off) & 15) != shift) return -1;
+  return shift;
 }
 
 // Called by every thread at the end of a compressing kernel.  Elects the last

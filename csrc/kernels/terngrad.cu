@@ -16,16 +16,21 @@
 // its own header, in ascending rank order.
 #include "../common/codec_math.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "p2p.cuh"
 #include "reduce.cuh"
 #include "unpack_lut.cuh"
 
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 namespace hipress {
 namespace cuda {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kThreads = 256;
 
@@ -35,6 +40,20 @@ inline int grid_for(int64_t items, int threads, int max_blocks) {
   if (blocks < 1) blocks = 1;
   if (blocks > max_blocks) blocks = max_blocks;
   return int(blocks);
+}
+
+__device__ __forceinline__ void put_header(const PushTargets& dst, const PushCursor& cur, int64_t n, int bw, float mn,
+                                           float mx) {
+  uint8_t header[kTernHeaderBytes];
+  header[0] = uint8_t(bw);
+  header[1] = uint8_t(tern_tail(n, bw));
+  const uint32_t a = __float_as_uint(mn), b = __float_as_uint(mx);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    header[2 + k] = uint8_t(a >> (8 * k));
+    header[6 + k] = uint8_t(b >> (8 * k));
+  }
+  put_bytes(dst, cur, 0, header, kTernHeaderBytes);
 }
 
 template <bool VEC, bool EF>
@@ -60,16 +79,28 @@ minmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ r
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (VEC) {
     const int64_t nv = n >> 2;
-    for (int64_t i = tid; i < nv; i += stride) {
-      float4 g = __ldg(reinterpret_cast<const float4*>(grad) + i);
+    auto fold = [&](float4 g, float4 r) {
       if (EF) {
-        const float4 r = __ldg(reinterpret_cast<const float4*>(residual) + i);
         g.x = hp_add(g.x, r.x); g.y = hp_add(g.y, r.y);
         g.z = hp_add(g.z, r.z); g.w = hp_add(g.w, r.w);
       }
       mn = fminf(mn, fminf(fminf(g.x, g.y), fminf(g.z, g.w)));
       mx = fmaxf(mx, fmaxf(fmaxf(g.x, g.y), fmaxf(g.z, g.w)));
+    };
+    int64_t i = tid;
+    for (; i + 3 * stride < nv; i += 4 * stride) {   // four loads of each array in flight
+      float4 g[4], r[4] = {};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        g[u] = __ldg(reinterpret_cast<const float4*>(grad) + i + u * stride);
+        if (EF) r[u] = __ldg(reinterpret_cast<const float4*>(residual) + i + u * stride);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) fold(g[u], r[u]);
     }
+    for (; i < nv; i += stride)
+      fold(__ldg(reinterpret_cast<const float4*>(grad) + i),
+           EF ? __ldg(reinterpret_cast<const float4*>(residual) + i) : make_float4(0.f, 0.f, 0.f, 0.f));
     for (int64_t i = (nv << 2) + tid; i < n; i += stride) {
       const float v = EF ? hp_add(grad[i], residual[i]) : grad[i];
       mn = fminf(mn, v);
@@ -82,6 +113,7 @@ minmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ r
       mx = fmaxf(mx, v);
     }
   }
+  let_next_start();
   float gmn, gmx;
   if (!grid_minmax_last_block<kThreads>(scratch, mn, mx, gmn, gmx)) return;
   if (threadIdx.x == 0) {
@@ -90,16 +122,7 @@ minmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ r
     scratch->mx = gmx;
     scratch->gap = gap;
     scratch->inv = tern_gap_inverse(gap);
-    uint8_t header[kTernHeaderBytes];
-    header[0] = uint8_t(bw);
-    header[1] = uint8_t(tern_tail(n, bw));
-    const uint32_t a = __float_as_uint(gmn), b = __float_as_uint(gmx);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      header[2 + k] = uint8_t(a >> (8 * k));
-      header[6 + k] = uint8_t(b >> (8 * k));
-    }
-    put_bytes(dst, cur, 0, header, kTernHeaderBytes);
+    put_header(dst, cur, n, bw, gmn, gmx);
   }
 }
 
@@ -129,16 +152,72 @@ __device__ __forceinline__ uint32_t tern_quant_unit(float (&x)[Unit<BW>::EPT], i
   return bytes;
 }
 
-// wide: large tensors with 16-byte aligned destinations.  A warp then works on chunks of
-// 512 payload bytes: in each of J = 16/BPT sub-steps lane L quantises unit j*32+L of the chunk
-// (coalesced 16-byte loads), the bytes are gathered in shared memory, and every lane stores
-// 16 of them to each destination -- 512 contiguous bytes per warp and destination, against the
-// 32 bytes per warp of the word path, which is what NVLink peer stores need to run near link
-// speed.  The rest of the tensor (less than one chunk) takes the word path.
+// The payload bytes of unit u, one unit per lane: the lanes combine theirs into 32-bit words.  Whole
+// warp; u < units tells the lanes that hold one.
+template <int BPT>
+__device__ __forceinline__ void put_unit_bytes(const PushTargets& dst, const PushCursor& cur, int64_t u, int64_t units,
+                                               uint32_t bytes) {
+  if (BPT == 1) {
+    const uint32_t word = gather4_bytes(bytes);
+    if ((threadIdx.x & 3) == 0 && u < units) {
+      if (u + 3 < units) {
+        put_u32(dst, cur, kTernHeaderBytes + u, word);
+      } else {
+        for (int64_t b = u; b < units; ++b)
+          put_u8(dst, cur, kTernHeaderBytes + b, uint8_t(word >> (8 * (b - u))));
+      }
+    }
+  } else if (BPT == 2) {
+    const uint32_t word = gather2_halves(bytes);
+    if ((threadIdx.x & 1) == 0 && u < units) {
+      if (u + 1 < units) {
+        put_u32(dst, cur, kTernHeaderBytes + 2 * u, word);
+      } else {
+        put_u8(dst, cur, kTernHeaderBytes + 2 * u, uint8_t(word));
+        put_u8(dst, cur, kTernHeaderBytes + 2 * u + 1, uint8_t(word >> 8));
+      }
+    }
+  } else {
+    if (u < units) put_u32(dst, cur, kTernHeaderBytes + 4 * u, bytes);
+  }
+}
+
+// Elements from `done` to the end of a tensor (or shard), fewer than a unit: whole bytes keep the
+// requested rounding mode, the partial last byte is always deterministic.  One thread.
+template <int BW, bool EF>
+__device__ __forceinline__ void tern_leftover(const float* grad, float* residual, int64_t done, int64_t n, float mn,
+                                              float inv, float gap, int random, uint64_t seed, const PushTargets& dst,
+                                              const PushCursor& cur) {
+  constexpr int DPB = 8 / BW;
+  int64_t byte_index = done / DPB;
+  for (int64_t e = done; e < n; e += DPB, ++byte_index) {
+    const int count = (n - e) >= DPB ? DPB : int(n - e);
+    float x[DPB], ef[DPB];
+    for (int j = 0; j < count; ++j) x[j] = EF ? hp_add(grad[e + j], residual[e + j]) : grad[e + j];
+    const bool rnd = random != 0 && count == DPB;
+    const uint8_t q = tern_pack_byte<BW>(x, count, mn, inv, rnd, tern_byte_seed(seed, byte_index), gap,
+                                         EF ? ef : nullptr);
+    put_u8(dst, cur, kTernHeaderBytes + byte_index, q);
+    if (EF)
+      for (int j = 0; j < count; ++j) residual[e + j] = ef[j];
+  }
+}
+
+// shift >= 0: large tensors whose destinations start equally far past a 16-byte boundary.  A warp
+// then works on chunks of 512 payload bytes: in each of J = 16/BPT sub-steps lane L quantises unit
+// j*32+L of the chunk (coalesced 16-byte loads), the bytes are gathered in shared memory, and every
+// lane stores 16 of them to each destination (put_chunk512) -- 512 contiguous bytes per warp and
+// destination, against the 32 bytes per warp of the word path, which is what NVLink peer stores need
+// to run near link speed, and half the instructions.  The rest of the tensor (less than one chunk)
+// takes the word path.  A payload at the start of a tensor has its packed data 10 bytes past a
+// boundary:
+// compress and decode of 9.4 MB at 4 bits 20.5 us with 2-byte stores, 18.4 now; of 25 MB
+// with ECQ 56.8 and 52.6 us (both with the cheaper draws of Lcg32::unit_from_raw).
 template <int BW, bool VEC, bool EF>
 __global__ void __launch_bounds__(kThreads)
 tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n,
-                  int random, uint64_t seed, PushTargets dst, const MinMaxScratch* scratch, int wide) {
+                  int random, uint64_t seed, PushTargets dst, const MinMaxScratch* scratch, int shift) {
+  wait_for_previous();
   if (push_guarded(dst)) return;
   resolve_epoch(dst);
   if (dst.epoch_dev != nullptr) seed += uint64_t(dst.epoch) * kEpochSeedStride;
@@ -164,12 +243,13 @@ tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
   // ---- chunks of 512 payload bytes
   constexpr int64_t CH = int64_t(kStageBytes) * DPB;
   int64_t chunks = 0;
-  if (VEC && wide) {
-    __shared__ __align__(16) uint8_t stage[kThreads / 32][kStageBytes];
+  if (VEC && shift >= 0) {
+    __shared__ __align__(16) uint8_t stages[kThreads / 32][kStageBytes + 16];
     constexpr int J = 16 / BPT;           // sub-steps per chunk
     constexpr int U = EPT == 8 ? 2 : 4;   // sub-steps whose loads are issued together
     chunks = n / CH;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint8_t* const stage = stages[warp] + shift;
     const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
     for (int64_t c = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp; c < chunks; c += warps) {
       int64_t ebase = c * CH;        // first element of the chunk in the tensor
@@ -209,14 +289,20 @@ tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
               reinterpret_cast<float4*>(residual + e0)[v] =
                   make_float4(ef[u][4 * v], ef[u][4 * v + 1], ef[u][4 * v + 2], ef[u][4 * v + 3]);
           }
-          if (BPT == 1) stage[warp][unit] = uint8_t(bytes);
-          else if (BPT == 2) reinterpret_cast<uint16_t*>(stage[warp])[unit] = uint16_t(bytes);
-          else reinterpret_cast<uint32_t*>(stage[warp])[unit] = bytes;
+          if (BPT == 1) {
+            stage[unit] = uint8_t(bytes);
+          } else if (BPT == 2) {
+            reinterpret_cast<uint16_t*>(stage)[unit] = uint16_t(bytes);
+          } else if ((shift & 3) == 0) {
+            reinterpret_cast<uint32_t*>(stage)[unit] = bytes;
+          } else {
+            reinterpret_cast<uint16_t*>(stage)[2 * unit] = uint16_t(bytes);
+            reinterpret_cast<uint16_t*>(stage)[2 * unit + 1] = uint16_t(bytes >> 16);
+          }
         }
       }
       __syncwarp();
-      const uint4 v = reinterpret_cast<const uint4*>(stage[warp])[lane];
-      put_u128(dst, cur, kTernHeaderBytes + bbase + lane * 16, v);
+      put_chunk512(dst, cur, kTernHeaderBytes + bbase, stages[warp], shift, lane);
       __syncwarp();
     }
   }
@@ -273,51 +359,129 @@ tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
         }
       }
     }
-    // combine lanes into 32-bit words and store them (k and u differ by a multiple of 32 units
-    // only when unit0 is one; the lane pattern below depends on the lane, not on u)
-    if (BPT == 1) {
-      const uint32_t word = gather4_bytes(bytes);
-      if ((threadIdx.x & 3) == 0 && u < units) {
-        if (u + 3 < units) {
-          put_u32(dst, cur, kTernHeaderBytes + u, word);
-        } else {
-          for (int64_t b = u; b < units; ++b)
-            put_u8(dst, cur, kTernHeaderBytes + b, uint8_t(word >> (8 * (b - u))));
+    // (k and u differ by a multiple of 32 units only when unit0 is one; the lane pattern of
+    // put_unit_bytes depends on the lane, not on u)
+    put_unit_bytes<BPT>(dst, cur, u, units, bytes);
+  }
+  if (units * EPT < rest_n && blockIdx.x == 0 && threadIdx.x == 0)
+    tern_leftover<BW, EF>(g_rest, r_rest, units * EPT, rest_n, mn, inv, gap, random, cur_seed, dst, cur);
+  publish_when_grid_done(dst);
+}
+
+// Small tensors: both passes in one launch.  A cluster of eight CTAs holds the tensor in registers (16
+// elements per thread), the CTAs exchange their extremes through distributed shared memory, and the
+// quantising pass starts from the registers.  At these sizes a launch costs more than the work: eight
+// SMs take the tensor in and quantise it in less time than the second launch and its ramp-up need.
+// 256 KB, compress and decode of two payloads: 16.4 us in three launches, 14.3 in two.
+constexpr int kSmallCtas = 8, kSmallThreads = 1024, kSmallPerThread = 16;
+constexpr int64_t kSmallElems = int64_t(kSmallCtas) * kSmallThreads * kSmallPerThread;
+template <int BW, bool VEC, bool EF>
+__global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
+tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int random, uint64_t seed,
+                  PushTargets dst) {
+  // The CTAs may read the guard at different times and must not part before they have met: each tells
+  // the others what it saw.
+  const bool skip = push_guarded(dst);
+  resolve_epoch(dst);
+  if (dst.epoch_dev != nullptr) seed += uint64_t(dst.epoch) * kEpochSeedStride;
+  constexpr int EPT = Unit<BW>::EPT, BPT = Unit<BW>::BPT, UPT = kSmallPerThread / EPT;
+  __shared__ float ext_mn[kSmallCtas], ext_mx[kSmallCtas], scale[4];
+  __shared__ int ext_skip[kSmallCtas];
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int64_t units = n / EPT;
+  const int64_t tid = int64_t(blockIdx.x) * kSmallThreads + threadIdx.x;
+  constexpr int64_t kStride = int64_t(kSmallCtas) * kSmallThreads;
+  float x[UPT][EPT];
+  float mn = INFINITY, mx = -INFINITY;
+#pragma unroll
+  for (int q = 0; q < UPT; ++q) {
+    const int64_t u = tid + q * kStride;
+    if (u < units) {
+      if (VEC) {
+#pragma unroll
+        for (int v = 0; v < EPT / 4; ++v) {
+          float4 g = __ldg(reinterpret_cast<const float4*>(grad + u * EPT) + v);
+          if (EF) {
+            const float4 r = reinterpret_cast<const float4*>(residual + u * EPT)[v];
+            g.x = hp_add(g.x, r.x); g.y = hp_add(g.y, r.y);
+            g.z = hp_add(g.z, r.z); g.w = hp_add(g.w, r.w);
+          }
+          x[q][4 * v] = g.x; x[q][4 * v + 1] = g.y; x[q][4 * v + 2] = g.z; x[q][4 * v + 3] = g.w;
         }
+      } else {
+#pragma unroll
+        for (int i = 0; i < EPT; ++i)
+          x[q][i] = EF ? hp_add(grad[u * EPT + i], residual[u * EPT + i]) : grad[u * EPT + i];
       }
-    } else if (BPT == 2) {
-      const uint32_t word = gather2_halves(bytes);
-      if ((threadIdx.x & 1) == 0 && u < units) {
-        if (u + 1 < units) {
-          put_u32(dst, cur, kTernHeaderBytes + 2 * u, word);
-        } else {
-          put_u8(dst, cur, kTernHeaderBytes + 2 * u, uint8_t(word));
-          put_u8(dst, cur, kTernHeaderBytes + 2 * u + 1, uint8_t(word >> 8));
-        }
+#pragma unroll
+      for (int i = 0; i < EPT; ++i) {
+        mn = fminf(mn, x[q][i]);
+        mx = fmaxf(mx, x[q][i]);
       }
-    } else {
-      if (u < units) put_u32(dst, cur, kTernHeaderBytes + 4 * u, bytes);
     }
   }
-  // leftover elements (fewer than EPT): whole bytes keep the requested rounding
-  // mode, the partial last byte is always deterministic
-  const int64_t done_elems = units * EPT;
-  if (done_elems < rest_n && blockIdx.x == 0 && threadIdx.x == 0) {
-    int64_t byte_index = done_elems / DPB;
-    for (int64_t e = done_elems; e < rest_n; e += DPB, ++byte_index) {
-      const int count = (rest_n - e) >= DPB ? DPB : int(rest_n - e);
-      float x[DPB], ef[DPB];
-      for (int j = 0; j < count; ++j)
-        x[j] = EF ? hp_add(g_rest[e + j], r_rest[e + j]) : g_rest[e + j];
-      const bool rnd = random != 0 && count == DPB;
-      const uint8_t q = tern_pack_byte<BW>(x, count, mn, inv, rnd,
-                                           tern_byte_seed(cur_seed, byte_index), gap,
-                                           EF ? ef : nullptr);
-      put_u8(dst, cur, kTernHeaderBytes + byte_index, q);
-      if (EF)
-        for (int j = 0; j < count; ++j) r_rest[e + j] = ef[j];
+  if (tid == 0) {
+    for (int64_t e = units * EPT; e < n; ++e) {
+      const float v = EF ? hp_add(grad[e], residual[e]) : grad[e];
+      mn = fminf(mn, v);
+      mx = fmaxf(mx, v);
     }
   }
+  block_minmax<kSmallThreads>(mn, mx);
+  cluster.sync();   // the other CTAs' shared memory exists from here on
+  if (threadIdx.x == 0) {
+    for (int c = 0; c < kSmallCtas; ++c) {
+      cluster.map_shared_rank(ext_mn, c)[blockIdx.x] = mn;
+      cluster.map_shared_rank(ext_mx, c)[blockIdx.x] = mx;
+      cluster.map_shared_rank(ext_skip, c)[blockIdx.x] = skip ? 1 : 0;
+    }
+  }
+  cluster.sync();
+  int any_skip = 0;
+#pragma unroll
+  for (int c = 0; c < kSmallCtas; ++c) any_skip |= ext_skip[c];
+  if (any_skip) return;   // the whole cluster
+  PushCursor cur{nullptr};
+  if (threadIdx.x == 0) {
+    mn = ext_mn[0];
+    mx = ext_mx[0];
+    for (int c = 1; c < kSmallCtas; ++c) {
+      mn = fminf(mn, ext_mn[c]);
+      mx = fmaxf(mx, ext_mx[c]);
+    }
+    const float gap = tern_gap(mn, mx, BW);
+    scale[0] = mn;
+    scale[1] = gap;
+    scale[2] = tern_gap_inverse(gap);
+    if (blockIdx.x == 0) put_header(dst, cur, n, BW, mn, mx);
+  }
+  __syncthreads();
+  mn = scale[0];
+  const float gap = scale[1], inv = scale[2];
+#pragma unroll
+  for (int q = 0; q < UPT; ++q) {
+    const int64_t u = tid + q * kStride;
+    if (q * kStride + (tid & ~int64_t(31)) >= units) break;   // whole warps leave together
+    uint32_t bytes = 0;
+    if (u < units) {
+      float ef[EPT];
+      bytes = tern_quant_unit<BW, EF>(x[q], u * BPT, mn, inv, gap, random, seed, ef);
+      if (EF) {
+        if (VEC) {
+#pragma unroll
+          for (int v = 0; v < EPT / 4; ++v)
+            reinterpret_cast<float4*>(residual + u * EPT)[v] =
+                make_float4(ef[4 * v], ef[4 * v + 1], ef[4 * v + 2], ef[4 * v + 3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < EPT; ++i) residual[u * EPT + i] = ef[i];
+        }
+      }
+    }
+    put_unit_bytes<BPT>(dst, cur, u, units, bytes);
+  }
+  if (tid == 0 && units * EPT < n)
+    tern_leftover<BW, EF>(grad, residual, units * EPT, n, mn, inv, gap, random, seed, dst, cur);
   publish_when_grid_done(dst);
 }
 
@@ -537,11 +701,30 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
   const bool ef = residual != nullptr;
   const bool vec = aligned16(grad) && (!ef || aligned16(residual));
   const int64_t S = dst.shard_elems;
-  bool dst16 = (dst.parity_stride & 15) == 0;
-  for (int p = 0; p < dst.world; ++p) dst16 = dst16 && aligned16(dst.payload[p] + kTernHeaderBytes);
-  if (dst.mc != nullptr) dst16 = dst16 && aligned16(dst.mc + kTernHeaderBytes);
+  const int shift = chunk_shift(dst, kTernHeaderBytes);
   // scatter mode runs on the chunked path only (see tern_quant_kernel)
-  if (S > 0 && (!vec || !dst16 || S % 4096 != 0 || (n + S - 1) / S > dst.world)) return cudaErrorInvalidValue;
+  if (S > 0 && (!vec || shift != 0 || S % 4096 != 0 || (n + S - 1) / S > dst.world)) return cudaErrorInvalidValue;
+#define LAUNCH_FORMS(LAUNCH, BW)              \
+  do {                                        \
+    if (vec && ef) LAUNCH(BW, true, true);    \
+    else if (vec) LAUNCH(BW, true, false);    \
+    else if (ef) LAUNCH(BW, false, true);     \
+    else LAUNCH(BW, false, false);            \
+  } while (0)
+#define LAUNCH_BITS(LAUNCH)                   \
+  switch (bitwidth) {                         \
+    case 1: LAUNCH_FORMS(LAUNCH, 1); break;   \
+    case 2: LAUNCH_FORMS(LAUNCH, 2); break;   \
+    case 4: LAUNCH_FORMS(LAUNCH, 4); break;   \
+    default: LAUNCH_FORMS(LAUNCH, 8); break;  \
+  }
+  if (S == 0 && n <= kSmallElems) {
+#define LAUNCH_SMALL(BW, V, E) \
+  tern_small_kernel<BW, V, E><<<kSmallCtas, kSmallThreads, 0, stream>>>(grad, residual, n, enable_random, seed, dst)
+    LAUNCH_BITS(LAUNCH_SMALL);
+#undef LAUNCH_SMALL
+    return cudaGetLastError();
+  }
   const int shards = S > 0 ? int((n + S - 1) / S) : 1;
   PushTargets hdr_dst = dst;
   hdr_dst.done = nullptr;  // only the quantising kernel publishes
@@ -562,28 +745,20 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
     // chunked path with 16-byte stores once there is a chunk per warp of a half-filled GPU
     const int dpb = 8 / bitwidth;
     const int64_t chunks = n / (int64_t(kStageBytes) * dpb);
-    const int wide = (vec && dst16 && (S > 0 || chunks >= 148 * 2)) ? 1 : 0;
+    const bool wide = vec && shift >= 0 && (S > 0 || chunks >= 148 * 2);
     const int threads = wide ? 128 : kThreads;
     const int grid = wide ? grid_for(chunks * 32, threads, 148 * 16)
                           : grid_for(n / (dpb > 4 ? dpb : 4), kThreads, 148 * 8);
-#define LAUNCH2(BW, V, E) \
-  tern_quant_kernel<BW, V, E><<<grid, threads, 0, stream>>>(grad, residual, n, enable_random, seed, dst, s, wide)
-#define LAUNCH_BW(BW)                         \
-  do {                                        \
-    if (vec && ef) LAUNCH2(BW, true, true);   \
-    else if (vec) LAUNCH2(BW, true, false);   \
-    else if (ef) LAUNCH2(BW, false, true);    \
-    else LAUNCH2(BW, false, false);           \
-  } while (0)
-    switch (bitwidth) {
-      case 1: LAUNCH_BW(1); break;
-      case 2: LAUNCH_BW(2); break;
-      case 4: LAUNCH_BW(4); break;
-      default: LAUNCH_BW(8); break;
-    }
-#undef LAUNCH_BW
-#undef LAUNCH2
+    cudaError_t e = cudaSuccess;
+#define LAUNCH_QUANT(BW, V, E)                                                                                   \
+  e = launch_after(tern_quant_kernel<BW, V, E>, dim3(grid), dim3(threads), 0, stream, grad, residual, n,         \
+                   enable_random, seed, dst, s, wide ? shift : -1)
+    LAUNCH_BITS(LAUNCH_QUANT);
+#undef LAUNCH_QUANT
+    if (e != cudaSuccess) return e;
   }
+#undef LAUNCH_BITS
+#undef LAUNCH_FORMS
   return cudaGetLastError();
 }
 

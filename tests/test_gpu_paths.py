@@ -134,3 +134,46 @@ def test_ecq_decode_tables(bw, world):
                 out.copy_(ref)
                 ops.ecq_decompress([at_offset(p, offset) for p in payloads], out, add=add, post_scale=0.5)
                 assert torch.equal(out.cpu(), ops_ref), (n, add, offset, shift)
+
+
+# ----------------------------------------------------------------------------- quantisers: compress
+@pytest.mark.parametrize("bw", [1, 2, 4, 8])
+@pytest.mark.parametrize("feedback", [False, True])
+@pytest.mark.parametrize("offset", [0, 1, 2, 6])
+def test_terngrad_compress_paths(bw, feedback, offset):
+    """Both sides of the one-launch limit (131,072 elements) and of the chunked path (296 chunks of 512 bytes)."""
+    chunked = 296 * 512 * 8 // bw
+    for n in (131072, 131073, chunked - 1, chunked + 777):
+        g, r = gauss(n, seed=n), gauss(n, 0.004, seed=n + 1)
+        rc = r.clone() if feedback else None
+        rg = r.cuda() if feedback else None
+        ref = ops.terngrad_compress(g, bw, True, seed=7, residual=rc)
+        out = torch.zeros(ref.numel() + offset + 64, dtype=torch.uint8, device="cuda")
+        ops.terngrad_compress(g.cuda(), bw, True, seed=7, residual=rg, out=out[offset:offset + ref.numel()])
+        assert torch.equal(out[offset:offset + ref.numel()].cpu(), ref), n
+        assert int(out[:offset].sum()) == 0 and int(out[offset + ref.numel():].sum()) == 0, n
+        if feedback:
+            assert torch.equal(rg.cpu(), rc), n
+
+
+@pytest.mark.parametrize("n", [1, 3, 33, 4096 * 3 + 1])
+def test_terngrad_small_unaligned(n):
+    g, r = gauss(n + 1, seed=1), gauss(n + 1, 0.004, seed=2)
+    rc, rg = r[1:].clone(), r.cuda()
+    ref = ops.terngrad_compress(g[1:].clone(), 2, True, seed=3, residual=rc)
+    out = ops.terngrad_compress(g.cuda()[1:], 2, True, seed=3, residual=rg[1:])
+    assert torch.equal(out.cpu(), ref) and torch.equal(rg[1:].cpu(), rc)
+
+
+@pytest.mark.parametrize("bw", [2, 4, 8])
+@pytest.mark.parametrize("offset", [0, 1, 6])
+def test_ecq_compress_paths(bw, offset):
+    chunked = 296 * 512 * 8 // bw
+    for n in (chunked - 1, chunked + 777):
+        g, h = gauss(n, seed=n), gauss(n, 0.002, seed=n + 1)
+        hc, hg = h.clone(), h.cuda()
+        ref = ops.ecq_compress(g, hc, 1.0, 0.9, bw, seed=4)
+        out = torch.zeros(ref.numel() + offset + 64, dtype=torch.uint8, device="cuda")
+        ops.ecq_compress(g.cuda(), hg, 1.0, 0.9, bw, seed=4, out=out[offset:offset + ref.numel()])
+        assert torch.equal(out[offset:offset + ref.numel()].cpu(), ref), n
+        assert torch.equal(hg.cpu(), hc), n
