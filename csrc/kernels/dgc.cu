@@ -8,6 +8,7 @@
 //     before it enters u (clip already divided by sqrt(world) by the caller)
 // The selector itself is sparse_compress (sparse.cu) run on v.
 #include "kernels.h"
+#include "launch.cuh"
 #include "p2p.cuh"
 
 namespace hipress {
@@ -31,11 +32,20 @@ sumsq_kernel(const float* __restrict__ g, int64_t n, float* __restrict__ out) {
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t nv = (reinterpret_cast<uintptr_t>(g) & 15) == 0 ? (n >> 2) : 0;  // 16-byte loads when aligned
-  for (int64_t i = tid; i < nv; i += stride) {
-    const float4 a = reinterpret_cast<const float4*>(g)[i];
+  int64_t q = tid;
+  for (; q + 3 * stride < nv; q += 4 * stride) {   // four loads in flight
+    float4 a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = __ldg(reinterpret_cast<const float4*>(g) + q + u * stride);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc += a[u].x * a[u].x + a[u].y * a[u].y + a[u].z * a[u].z + a[u].w * a[u].w;
+  }
+  for (; q < nv; q += stride) {
+    const float4 a = reinterpret_cast<const float4*>(g)[q];
     acc += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
   }
   for (int64_t i = (nv << 2) + tid; i < n; i += stride) acc += g[i] * g[i];
+  let_next_start();
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
@@ -149,7 +159,7 @@ adamw_kernel(float* __restrict__ grad, float scale, AdamWApply a, int64_t n) {
 
 cudaError_t dgc_sumsq(const float* g, int64_t n, float* out, cudaStream_t stream) {
   if (n <= 0 || g == nullptr || out == nullptr) return cudaErrorInvalidValue;
-  sumsq_kernel<<<grid_for(n, 148 * 4), kThreads, 0, stream>>>(g, n, out);
+  sumsq_kernel<<<grid_for((n + 3) >> 2, 148 * 4), kThreads, 0, stream>>>(g, n, out);
   return cudaGetLastError();
 }
 

@@ -24,20 +24,35 @@ __device__ __forceinline__ T* after_wait(T* p) {
   return p;
 }
 
+// overlap: start while the kernel before is still running.  cluster: CTAs per cluster (1: none).
 template <typename... Params, typename... Args>
-cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                         Args... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+cudaError_t launch_with(bool overlap, int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                        cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr[2]{};
+  unsigned count = 0;
+  if (overlap) {
+    attr[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[count++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[count].id = cudaLaunchAttributeClusterDimension;
+    attr[count].val.clusterDim.x = unsigned(cluster);
+    attr[count].val.clusterDim.y = attr[count].val.clusterDim.z = 1;
+    ++count;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = count;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                         Args... args) {
+  return launch_with(true, 1, kernel, grid, block, smem, stream, args...);
 }
 
 }  // namespace cuda

@@ -5,28 +5,24 @@
 // -> copy_if (implicit sync) -> sort + truncate -> H2D+sync -> for_each(gather)
 // (gd_body.h:121-229): four host synchronisations and two sorts.  Here:
 //
-//   sample x3   The k-th largest |value| of the random sample is found by a
-//               3-digit radix select (11+11+10 bits of the order-preserving key).
-//               Samples are *recomputed* from the LCG in every round instead of
-//               being stored and sorted, so no sample buffer exists.
-//   count       One pass: R += G (GradDrop), per-CTA count of |R| > threshold and
-//               first-digit histogram of those candidates.
-//   trim x2     Only when more than ceil(N*keep) candidates qualified (decided on
-//               the device; otherwise the kernels return at once): radix select of
-//               the exact cut among the candidates.
-//   recount     Per-CTA counts against the cut (only when trimming).
-//   scan        One CTA: exclusive offsets per CTA, k, the 4-byte header to every
-//               destination, and clearing of the histograms for the next call.
-//   write       Ordered compaction: indices ascending, values, residual zeroing,
-//               stored into every destination (local and NVLink peers), then the
-//               completion flag.
+//   sample      Draws the sample, stores every key (the order-preserving bits of |value|) and counts
+//               the first of three digits (11 + 11 + 10 bits).
+//   select      The k-th largest key of the sample: the CTAs pick the first digit's bin and collect the
+//               few keys in it; the last CTA finds the threshold among those.
+//   count       One pass: the codec's state update, the number of |R| > threshold, and a histogram of
+//               those candidates above the threshold.
+//   trim x2     Only when more than ceil(N*keep) candidates qualified (decided on the device; otherwise
+//               the kernels return at once): the exact cut.  One pass over R; the second kernel only
+//               has work when the cut lies more than a factor of two above the threshold.
+//   write       Ordered compaction: indices ascending, values, residual zeroing, stored into every
+//               destination (local and NVLink peers), then the completion flag.
 //
 // Content rule (identical to the CPU codec): keep |R[i]| > threshold in
 // ascending index order; when over-selected keep the largest magnitudes, ties
 // toward the lower index.
 //
 // Two forms of everything after the sampling.  The passes above ("scan form") read the whole
-// tensor up to five times.  For keep fractions up to 1 % the "list form" reads it ONCE:
+// tensor three or four times.  For keep fractions up to 1 % the "list form" reads it ONCE:
 //
 //   count+collect  the one pass over the tensor.  It applies the codec's state update (R += G
 //               for GradDrop; u = m*u + s*g, v += u and g = 0 for DGC with momentum correction;
@@ -34,17 +30,20 @@
 //               (index, value), to a per-warp list in index order.  A warp owns a contiguous
 //               part of its CTA's chunk, so the lists, taken in order, are sorted by index.
 //               Lists grow in blocks of 16 entries taken from a pool with one atomic.
-//   cut         One CTA, only when more than ceil(N*keep) candidates qualified: their keys
-//               (35 K for a 128 MB bucket at 0.1 %) are gathered into shared memory with batched
-//               loads and the exact cut is found by a radix select there.
-//   count+scan  One warp per list counts what it keeps against the cut; the last CTA to finish
-//               turns the per-CTA totals into exclusive offsets, k and the header.
+//   cut         One CTA (eight for large selections): when more than ceil(N*keep) candidates qualified,
+//               their keys (35 K for a 128 MB bucket at 0.1 %) are gathered into shared memory with
+//               batched loads and the exact cut is found by a radix select there.  It then counts what
+//               each CTA's lists keep and turns the counts into offsets, k and the header.
 //   emit        One warp per list: indices and values to every destination, residual (and
 //               DGC's momentum u) cleared at the emitted positions, then the completion flag.
 //
-// The sample keys are stored by the first sampling round and re-read by the other two (the
-// scan form recomputes them, three random gathers per sample and round with momentum
-// correction).  The pool is sized for many times the expected number of candidates (see
+// The kernels of a call overlap at their ends (launch.cuh): at 25 MB none but the pass over the tensor
+// takes longer than the gap between two plain launches.
+// 64 MB, GradDrop at 0.1 %, compress and decode: 129 us with eight plain launches, 112 now;
+// 25 MB, DGC: 102 and 81 us.
+//
+// A sample of more than a hundredth of the elements does not fit the key array; its keys are then drawn
+// again in each of three rounds, one per digit.  The pool is sized for many times the expected number of candidates (see
 // list_plan); should it still run out, the candidates that did not fit stay in the residual
 // and are sent in a later step (counted in SparseScratch::dropped).
 #include "../common/codec_math.h"
@@ -55,10 +54,14 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 namespace hipress {
 namespace cuda {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kThreads = 256;
 constexpr int kBins = 2048;
@@ -69,30 +72,44 @@ constexpr int kBlockEntries = 16;
 constexpr unsigned int kNoBlock = 0xffffffffu;
 constexpr double kListMaxKeep = 0.01;   // the list form serves keep fractions up to this
 
+constexpr int kFineBins = 512, kFineShift = 14;       // histogram above the threshold: one octave
+constexpr int kExactBins = 1 << kFineShift;           // the keys of one of its bins
+constexpr int kMaxSampleBlocks = kMaxBlocks;
+
 struct SparseScratch {
-  unsigned int shist[3][kBins];  // sample radix-select rounds
-  unsigned int thist[3][kBins];  // trim radix-select rounds
-  unsigned int cnt_gt[kMaxBlocks], cnt_eq[kMaxBlocks];
-  unsigned int off_gt[kMaxBlocks], off_eq[kMaxBlocks];
-  // state words
-  // Radix-select progress, one slot per round: a kernel reads the slot of the
-  // previous round and writes its own, so no word is read and written by
-  // different CTAs of the same launch.
-  unsigned int s_prefix[3], s_rank[3];  // sample select
-  unsigned int t_prefix[3], t_rank[3];  // trim select
-  unsigned int thr_key;                 // threshold (key of a positive float)
-  unsigned int cand;                    // candidates over the threshold
-  unsigned int cut_key, ties_kept;      // final rule
+  // Cleared by the first kernel of a call (clear_call_state).
+  struct Call {
+    unsigned int fine[kFineBins];      // candidates by (key - threshold) >> kFineShift; the last bin: all above
+    unsigned int thist[3][kBins];      // digits of the candidates in that last bin
+    unsigned int exact[kExactBins];    // keys inside the bin that holds the cut
+    unsigned long long agg[kMaxBlocks];  // write kernel: what each chunk keeps, once known
+    unsigned int ticket;               // write kernel: chunks handed out
+    unsigned int trim_done[2];         // CTA arrivals of the trim kernels
+    unsigned int t_prefix, t_rank;     // progress of the trim digits
+    unsigned int clipped;              // the cut lies in the last fine bin
+    unsigned int thr_key;              // threshold (key of a positive float)
+    unsigned int cand;                 // candidates over the threshold
+    unsigned int cut_key, ties_kept;   // final rule
+    unsigned int pool_used;            // list form: blocks handed out
+  } call;
+  // Sampling: zero between calls.
+  unsigned int shist[3][kBins];
+  unsigned int s_prefix[3], s_rank[3];  // written by a round for the next
+  unsigned int s_kept, s_done;
   unsigned int k;                       // elements emitted
-  // list form
-  unsigned int pool_used;               // blocks handed out (reset by select)
   unsigned int dropped;                 // candidates that found no block (cumulative)
   unsigned int last_cand;               // candidates seen by the last call (metrics)
-  unsigned int lists_done;              // CTA arrival counter of the count+scan kernel (left at zero)
+  unsigned int gave_up;                 // waits of the write kernel that ran out (never, see there)
+  unsigned int off_gt[kMaxBlocks], off_eq[kMaxBlocks];
   unsigned int list_head[kMaxLists];    // first block of each warp's list, kNoBlock when empty
-  unsigned int list_gt[kMaxLists], list_eq[kMaxLists];   // kept counts per list (above / at the cut)
 };
 
+__device__ __forceinline__ void clear_call_state(SparseScratch* s) {
+  static_assert(sizeof(SparseScratch::Call) % 4 == 0, "cleared word by word");
+  unsigned int* w = reinterpret_cast<unsigned int*>(&s->call);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < int(sizeof(SparseScratch::Call) / 4); i += gridDim.x * blockDim.x)
+    w[i] = 0u;
+}
 
 __device__ __forceinline__ int digit_of(uint32_t key, int round) {
   return round == 0 ? int(key >> 21) : round == 1 ? int((key >> 10) & 0x7ffu) : int(key & 0x3ffu);
@@ -104,53 +121,74 @@ __device__ __forceinline__ uint32_t extend_prefix(uint32_t prefix, int round, ui
   return round == 0 ? digit : round == 1 ? (prefix << 11) | digit : (prefix << 10) | digit;
 }
 
-// Block-wide: find the bin holding the element of 0-indexed `rank` counted from
-// the top bin down.  Every thread returns the same (bin, rank inside bin).
-__device__ void pick_from_top(const unsigned int* hist, unsigned int rank, unsigned int& bin,
-                              unsigned int& rank_in_bin) {
-  __shared__ unsigned int part[kThreads];
+// Block-wide over kThreads threads: the bin holding the element of 0-indexed `rank` counted from the top
+// bin down, and the rank inside that bin.  Every thread returns the same pair.  hist: BINS counters,
+// 16-byte aligned, in shared or global memory.
+template <int BINS>
+__device__ __forceinline__ void pick_from_top(const unsigned int* hist, unsigned int rank, unsigned int& bin,
+                                              unsigned int& rank_in_bin) {
+  __shared__ unsigned int warp_sum[kThreads / 32];
   __shared__ unsigned int res[2];
-  constexpr int PER = kBins / kThreads;  // 8 bins per thread
-  const int t = threadIdx.x;
-  unsigned int local[PER];
+  constexpr int PER = BINS / kThreads;
+  static_assert(PER >= 4 ? PER % 4 == 0 : PER == 2, "a thread's bins are read in whole vectors");
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int base = BINS - (t + 1) * PER;   // this thread's bins, the highest last
   unsigned int sum = 0;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    local[j] = hist[kBins - 1 - (t * PER + j)];
-    sum += local[j];
-  }
-  part[t] = sum;
-  if (t == 0) {
-    res[0] = 0;
-    res[1] = 0;
-  }
-  __syncthreads();
-  // serial prefix by warp 0 is enough for 256 entries
-  if (t == 0) {
-    unsigned int run = 0;
-    for (int i = 0; i < kThreads; ++i) {
-      const unsigned int v = part[i];
-      part[i] = run;
-      run += v;
+  if (PER >= 4) {
+#pragma unroll 4
+    for (int j = 0; j < PER / 4; ++j) {
+      const uint4 v = *reinterpret_cast<const uint4*>(hist + base + 4 * j);
+      sum += v.x + v.y + v.z + v.w;
     }
+  } else {
+    for (int j = 0; j < PER; ++j) sum += hist[base + j];
   }
-  __syncthreads();
-  const unsigned int before = part[t];
-  if (rank >= before && rank < before + sum) {
-    unsigned int run = before;
+  unsigned int inc = sum;
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      if (rank >= run && rank < run + local[j]) {
-        res[0] = kBins - 1 - (t * PER + j);
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned int a = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += a;
+  }
+  if (lane == 31) warp_sum[warp] = inc;
+  if (t == 0) res[0] = res[1] = 0;
+  __syncthreads();
+  unsigned int before = inc - sum;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w)
+    if (w < warp) before += warp_sum[w];
+  if (rank >= before && rank - before < sum) {
+    unsigned int run = before;
+    for (int j = PER - 1; j >= 0; --j) {
+      const unsigned int c = hist[base + j];
+      if (rank - run < c) {
+        res[0] = base + j;
         res[1] = rank - run;
+        break;
       }
-      run += local[j];
+      run += c;
     }
   }
   __syncthreads();
   bin = res[0];
   rank_in_bin = res[1];
   __syncthreads();
+}
+
+// True in every thread of exactly one CTA: the last of the grid to get here; it sees what all others
+// wrote before.  The counter is left at zero.
+__device__ __forceinline__ bool last_cta(unsigned int* counter) {
+  __shared__ bool is_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    if (is_last) {
+      *counter = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return is_last;
 }
 
 __device__ __forceinline__ void hist_flush(unsigned int* sh, unsigned int* gh) {
@@ -212,22 +250,34 @@ __device__ __forceinline__ float fused_value(const SparseFuseDev& f, const float
   return __fadd_rn(R[i], dgc_new_u(f.u[i], f.grad[i], f.momentum, scale));
 }
 
-// ---- sample rounds
-// keys: when non-null, round 0 stores every sample's key there and rounds 1 and 2 read them
-// back instead of drawing and gathering again.
+// ---- sampling
+// Counts the digits of sampled keys: sampled magnitudes share their leading bits, so the lanes that hit
+// the same bin are counted by one of them (one shared-memory atomic per bin and warp).  Whole warp;
+// bin < 0: nothing to count.
+__device__ __forceinline__ void count_digit(unsigned int* sh, int bin) {
+  const unsigned int same = __match_any_sync(0xffffffffu, bin);
+  if (bin >= 0 && int(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&sh[bin], unsigned(__popc(same)));
+}
+
+// Round 0 stores every sample's key in `keys` when that is non-null (select_kernel goes on from there).
+// Without the array each round draws the sample again and counts its own digit; the last CTA of round 2
+// has the threshold.
 template <int ROUND>
 __global__ void __launch_bounds__(kThreads)
-sample_round_kernel(SparseFuseDev fuse, const float* __restrict__ R, int64_t n,
+sample_round_kernel(SparseFuseDev fuse, const float* R, int64_t n,
                     int64_t sample_cnt, unsigned int rank0, uint64_t seed,
-                    SparseScratch* s, uint32_t* __restrict__ keys, const uint32_t* epoch_dev) {
+                    SparseScratch* s, uint32_t* keys, const uint32_t* epoch_dev) {
+  wait_for_previous();
+  let_next_start();
+  if (ROUND == 0) clear_call_state(s);
   if (epoch_dev != nullptr) seed += uint64_t(*epoch_dev) * kEpochSeedStride;  // see PushTargets
-  __shared__ unsigned int sh[kBins];
+  __shared__ __align__(16) unsigned int sh[kBins];
   for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
   uint32_t prefix = 0;
   if (ROUND > 0) {
     const unsigned int rank = ROUND == 1 ? rank0 : s->s_rank[ROUND - 1];
     unsigned int bin, rin;
-    pick_from_top(s->shist[ROUND - 1], rank, bin, rin);
+    pick_from_top<kBins>(s->shist[ROUND - 1], rank, bin, rin);
     prefix = extend_prefix(ROUND == 1 ? 0u : s->s_prefix[ROUND - 1], ROUND - 1, bin);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       // consumed by the next kernel in the stream
@@ -238,234 +288,293 @@ sample_round_kernel(SparseFuseDev fuse, const float* __restrict__ R, int64_t n,
   __syncthreads();
   const float scale = dgc_clip_scale(fuse);
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  // whole warps iterate together; sampled magnitudes share their leading bits, so the lanes that
-  // hit the same bin are counted by one of them (one shared-memory atomic per bin and warp)
-  const int64_t padded = (sample_cnt + 31) & ~int64_t(31);
+  const int64_t padded = (sample_cnt + 31) & ~int64_t(31);   // whole warps iterate together
   for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < padded; x += stride) {
-    uint32_t key = 0;
-    bool live = x < sample_cnt;
-    if (live) {
-      if (ROUND > 0 && keys != nullptr) {
-        key = keys[x];
-      } else {
-        const uint32_t idx = sparse_sample_index(seed, x, uint32_t(n));
-        key = abs_key(fused_value(fuse, R, idx, scale));
-        if (keys != nullptr) keys[x] = key;
-      }
-      live = prefix_matches(key, ROUND, prefix);
+    int bin = -1;
+    if (x < sample_cnt) {
+      const uint32_t idx = sparse_sample_index(seed, x, uint32_t(n));
+      const uint32_t key = abs_key(fused_value(fuse, R, idx, scale));
+      if (ROUND == 0 && keys != nullptr) keys[x] = key;
+      if (prefix_matches(key, ROUND, prefix)) bin = digit_of(key, ROUND);
     }
-    const int bin = live ? digit_of(key, ROUND) : -1;
-    const unsigned int same = __match_any_sync(0xffffffffu, bin);
-    if (live && int(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&sh[bin], unsigned(__popc(same)));
+    count_digit(sh, bin);
   }
   hist_flush(sh, s->shist[ROUND]);
+  if (ROUND == 2) {
+    if (!last_cta(&s->s_done)) return;
+    unsigned int bin, rin;
+    pick_from_top<kBins>(s->shist[2], s->s_rank[2], bin, rin);
+    if (threadIdx.x == 0) s->call.thr_key = extend_prefix(s->s_prefix[2], 2, bin);
+    for (int i = threadIdx.x; i < 3 * kBins; i += kThreads) (&s->shist[0][0])[i] = 0u;
+  }
 }
 
-// ---- count pass (also performs R += G)
+// The rest of the selection when the keys are stored: the keys in the first digit's bin (around the
+// threshold of a 0.1 % selection, an eighth of an octave: hundreds of a 65,536-element sample) are
+// collected in `kept`, and the last CTA finds the remaining digits among them.
 __global__ void __launch_bounds__(kThreads)
-count_kernel(const float* __restrict__ grad, float* __restrict__ R, int64_t n, int64_t chunk,
-             int64_t sample_cnt, unsigned int rank0, int accumulate, int zero_grad, SparseScratch* s) {
-  __shared__ unsigned int sh[kBins];
-  __shared__ unsigned int blk_cnt;
-  for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
-  if (threadIdx.x == 0) blk_cnt = 0;
-  uint32_t thr_key = 0;
-  if (sample_cnt > 0) {
-    unsigned int bin, rin;
-    pick_from_top(s->shist[2], s->s_rank[2], bin, rin);
-    thr_key = extend_prefix(s->s_prefix[2], 2, bin);
+select_kernel(int64_t sample_cnt, unsigned int rank0, SparseScratch* s, const uint32_t* keys, uint32_t* kept) {
+  wait_for_previous();
+  let_next_start();
+  __shared__ __align__(16) unsigned int sh[kBins];
+  unsigned int bin, rank;
+  pick_from_top<kBins>(s->shist[0], rank0, bin, rank);
+  uint32_t prefix = bin;
+  __shared__ unsigned int mine[kThreads], held, place;
+  const int64_t stride = int64_t(gridDim.x) * kThreads;
+  for (int64_t x0 = int64_t(blockIdx.x) * kThreads; x0 < sample_cnt; x0 += stride) {
+    const int64_t x = x0 + threadIdx.x;
+    if (threadIdx.x == 0) held = 0;
+    __syncthreads();
+    const uint32_t key = x < sample_cnt ? keys[x] : 0u;
+    if (x < sample_cnt && prefix_matches(key, 1, prefix)) mine[atomicAdd(&held, 1u)] = key;
+    __syncthreads();
+    if (threadIdx.x == 0 && held != 0) place = atomicAdd(&s->s_kept, held);   // one per CTA, not one per warp
+    __syncthreads();
+    if (threadIdx.x < held) kept[place + threadIdx.x] = mine[threadIdx.x];
   }
+  if (!last_cta(&s->s_done)) return;
+  const unsigned int count = *reinterpret_cast<volatile unsigned int*>(&s->s_kept);
+#pragma unroll
+  for (int round = 1; round < 3; ++round) {   // inside one bin of the first digit the rest spreads evenly
+    for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
+    __syncthreads();
+    for (unsigned int i = threadIdx.x; i < count; i += kThreads) {
+      const uint32_t key = __ldcg(kept + i);
+      if (prefix_matches(key, round, prefix)) atomicAdd(&sh[digit_of(key, round)], 1u);
+    }
+    __syncthreads();
+    unsigned int rin;
+    pick_from_top<kBins>(sh, rank, bin, rin);
+    prefix = extend_prefix(prefix, round, bin);
+    rank = rin;
+  }
+  if (threadIdx.x == 0) {
+    s->call.thr_key = prefix;
+    s->s_kept = 0u;
+  }
+  for (int i = threadIdx.x; i < kBins; i += kThreads) s->shist[0][i] = 0u;
+}
+
+// ---- scan form: the pass that updates the state, counts the candidates and files them by magnitude
+// MODE = fuse.mode as a template parameter.  Candidates are filed by their distance from the threshold:
+// the cut, when one is needed, lies a few per cent above the threshold, and its bin of this histogram
+// holds few enough keys for the next kernel to count every key by itself.  What lies more than an octave
+// above is filed by its first digit as well.
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 4)
+count_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s) {
+  wait_for_previous();
+  constexpr int U = MODE == 2 ? 2 : 4;   // 16-byte loads of each array in flight per thread
+  __shared__ unsigned int fine[kFineBins], coarse[kBins];
+  __shared__ unsigned int blk_cnt;
+  for (int i = threadIdx.x; i < kFineBins; i += kThreads) fine[i] = 0;
+  for (int i = threadIdx.x; i < kBins; i += kThreads) coarse[i] = 0;
+  if (threadIdx.x == 0) blk_cnt = 0;
+  const uint32_t thr_key = s->call.thr_key;
+  const float scale = MODE == 2 ? dgc_clip_scale(fuse) : 1.0f;
   __syncthreads();
-  if (blockIdx.x == 0 && threadIdx.x == 0) s->thr_key = thr_key;
   const int64_t begin = int64_t(blockIdx.x) * chunk;
   const int64_t end = begin + chunk < n ? begin + chunk : n;
+  const float* grad = fuse.grad;
+  float* gw = const_cast<float*>(fuse.grad);
   unsigned int mine = 0;
-  if (!accumulate) {
-    // read-only pass (DGC: the velocity was accumulated by its own kernel): 16-byte loads
-    for_each_value(R, begin, end, [&](float r) {
-      const uint32_t key = abs_key(r);
-      if (key > thr_key) {
-        ++mine;
-        atomicAdd(&sh[digit_of(key, 0)], 1u);
-      }
-    });
-  } else {
-    for (int64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-      const float r = hp_add(grad[i], R[i]);
-      R[i] = r;
-      if (zero_grad) const_cast<float*>(grad)[i] = 0.f;
-      const uint32_t key = abs_key(r);
-      if (key > thr_key) {
-        ++mine;
-        atomicAdd(&sh[digit_of(key, 0)], 1u);
+  auto file = [&](float r) {
+    const uint32_t key = abs_key(r);
+    if (key > thr_key) {
+      ++mine;
+      const uint32_t d = (key - thr_key) >> kFineShift;
+      if (d < kFineBins - 1) {
+        atomicAdd(&fine[d], 1u);
+      } else {
+        atomicAdd(&fine[kFineBins - 1], 1u);
+        atomicAdd(&coarse[digit_of(key, 0)], 1u);
       }
     }
+  };
+  auto update = [&](float r, float g, float& u) -> float {
+    if (MODE == 1) return hp_add(g, r);
+    if (MODE == 2) {
+      u = dgc_new_u(u, g, fuse.momentum, scale);
+      return __fadd_rn(r, u);
+    }
+    return r;
+  };
+  uintptr_t bits = reinterpret_cast<uintptr_t>(R);
+  if (MODE >= 1) bits |= reinterpret_cast<uintptr_t>(grad);
+  if (MODE == 2) bits |= reinterpret_cast<uintptr_t>(fuse.u);
+  int64_t rest = begin;
+  if ((bits & 15) == 0 && (begin & 3) == 0) {
+    const int64_t nv = (end - begin) >> 2;
+    auto step = [&](int64_t e, float4 r4, float4 g4, float4 u4) {
+      float r[4] = {r4.x, r4.y, r4.z, r4.w};
+      const float g[4] = {g4.x, g4.y, g4.z, g4.w};
+      float u[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = update(r[j], g[j], u[j]);
+      if (MODE >= 1) {
+        *reinterpret_cast<float4*>(R + e) = make_float4(r[0], r[1], r[2], r[3]);
+        if (MODE == 2) *reinterpret_cast<float4*>(fuse.u + e) = make_float4(u[0], u[1], u[2], u[3]);
+        if (fuse.zero_grad) *reinterpret_cast<float4*>(gw + e) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) file(r[j]);
+    };
+    int64_t i = threadIdx.x;
+    for (; i + (U - 1) * kThreads < nv; i += U * kThreads) {
+      float4 r4[U], g4[U] = {}, u4[U] = {};
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int64_t e = begin + 4 * (i + q * kThreads);
+        r4[q] = *reinterpret_cast<const float4*>(R + e);
+        if (MODE >= 1) g4[q] = *reinterpret_cast<const float4*>(grad + e);
+        if (MODE == 2) u4[q] = *reinterpret_cast<const float4*>(fuse.u + e);
+      }
+#pragma unroll
+      for (int q = 0; q < U; ++q) step(begin + 4 * (i + q * kThreads), r4[q], g4[q], u4[q]);
+    }
+    for (; i < nv; i += kThreads) {
+      const int64_t e = begin + 4 * i;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      step(e, *reinterpret_cast<const float4*>(R + e), MODE >= 1 ? *reinterpret_cast<const float4*>(grad + e) : zero,
+           MODE == 2 ? *reinterpret_cast<const float4*>(fuse.u + e) : zero);
+    }
+    rest = begin + 4 * nv;
   }
-  atomicAdd(&blk_cnt, mine);
-  hist_flush(sh, s->thist[0]);
+  for (int64_t e = rest + threadIdx.x; e < end; e += kThreads) {
+    float u = MODE == 2 ? fuse.u[e] : 0.f;
+    const float r = update(R[e], MODE >= 1 ? grad[e] : 0.f, u);
+    if (MODE >= 1) {
+      R[e] = r;
+      if (MODE == 2) fuse.u[e] = u;
+      if (fuse.zero_grad) gw[e] = 0.f;
+    }
+    file(r);
+  }
+  let_next_start();
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if ((threadIdx.x & 31) == 0 && mine != 0) atomicAdd(&blk_cnt, mine);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    s->cnt_gt[blockIdx.x] = blk_cnt;
-    s->cnt_eq[blockIdx.x] = 0;
-    atomicAdd(&s->cand, blk_cnt);
-  }
+  for (int i = threadIdx.x; i < kFineBins; i += kThreads)
+    if (fine[i]) atomicAdd(&s->call.fine[i], fine[i]);
+  if (fine[kFineBins - 1]) hist_flush(coarse, s->call.thist[0]);
+  if (threadIdx.x == 0) atomicAdd(&s->call.cand, blk_cnt);
 }
 
-// ---- trim rounds 1 and 2 (return at once when not over-selected)
+// ---- the exact cut (returns at once when not over-selected)
+// ROUND 0: the keys in the cut's bin of the fine histogram, counted one by one; the last CTA has the cut.
+// Should the cut lie in the histogram's last bin, this round counts the second digit of the keys there,
+// and ROUND 1, which otherwise has nothing to do, the third.
 template <int ROUND>
 __global__ void __launch_bounds__(kThreads)
-trim_round_kernel(const float* __restrict__ R, int64_t n, int64_t chunk, unsigned int expected,
-                  SparseScratch* s) {
-  if (s->cand <= expected) return;
-  __shared__ unsigned int sh[kBins];
-  for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
-  const unsigned int rank = ROUND == 1 ? expected - 1 : s->t_rank[ROUND - 1];
-  unsigned int bin, rin;
-  pick_from_top(s->thist[ROUND - 1], rank, bin, rin);
-  const uint32_t prefix = extend_prefix(ROUND == 1 ? 0u : s->t_prefix[ROUND - 1], ROUND - 1, bin);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    s->t_prefix[ROUND] = prefix;
-    s->t_rank[ROUND] = rin;
+trim_kernel(const float* R, int64_t n, int64_t chunk, unsigned int expected, SparseScratch* s) {
+  wait_for_previous();
+  let_next_start();
+  SparseScratch::Call& c = s->call;
+  const uint32_t thr_key = c.thr_key;
+  if (c.cand <= expected) {
+    if (ROUND == 0 && blockIdx.x == 0 && threadIdx.x == 0) c.cut_key = thr_key;   // ties_kept stays 0
+    return;
   }
-  const uint32_t thr_key = s->thr_key;
-  __syncthreads();
+  __shared__ __align__(16) unsigned int sh[kBins];
   const int64_t begin = int64_t(blockIdx.x) * chunk;
   const int64_t end = begin + chunk < n ? begin + chunk : n;
-  for_each_value(R, begin, end, [&](float x) {
-    const uint32_t key = abs_key(x);
-    if (key > thr_key && prefix_matches(key, ROUND, prefix))
-      atomicAdd(&sh[digit_of(key, ROUND)], 1u);
-  });
-  hist_flush(sh, s->thist[ROUND]);
-}
-
-// ---- final rule + per-CTA counts against the cut
-__global__ void __launch_bounds__(kThreads)
-recount_kernel(const float* __restrict__ R, int64_t n, int64_t chunk, unsigned int expected,
-               SparseScratch* s) {
-  if (s->cand <= expected) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      s->cut_key = s->thr_key;
-      s->ties_kept = 0;
-    }
-    return;  // counts of the count pass stand
-  }
   unsigned int bin, rin;
-  pick_from_top(s->thist[2], s->t_rank[2], bin, rin);
-  const uint32_t cut = extend_prefix(s->t_prefix[2], 2, bin);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    s->cut_key = cut;
-    s->ties_kept = rin + 1;
-  }
-  __shared__ unsigned int c_gt, c_eq;
-  if (threadIdx.x == 0) {
-    c_gt = 0;
-    c_eq = 0;
-  }
-  __syncthreads();
-  const int64_t begin = int64_t(blockIdx.x) * chunk;
-  const int64_t end = begin + chunk < n ? begin + chunk : n;
-  unsigned int g = 0, e = 0;
-  for_each_value(R, begin, end, [&](float x) {
-    const uint32_t key = abs_key(x);
-    g += key > cut;
-    e += key == cut;
-  });
-  atomicAdd(&c_gt, g);
-  atomicAdd(&c_eq, e);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s->cnt_gt[blockIdx.x] = c_gt;
-    s->cnt_eq[blockIdx.x] = c_eq;
-  }
-}
-
-// ---- one CTA: offsets, k, header, housekeeping
-// thread t scans the totals of CTA t: the count / write kernels may not have more CTAs than this
-// kernel has threads
-static_assert(kMaxBlocks <= 1024, "scan_kernel scans one per-CTA total per thread");
-__global__ void __launch_bounds__(1024)
-scan_kernel(int blocks, PushTargets dst, SparseScratch* s) {
-  resolve_epoch(dst);
-  __shared__ unsigned int wa[32], wb[32], tot[2];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const unsigned int va = t < blocks ? s->cnt_gt[t] : 0u;
-  const unsigned int vb = t < blocks ? s->cnt_eq[t] : 0u;
-  unsigned int ia = va, ib = vb;  // inclusive scans inside the warp
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned int x = __shfl_up_sync(0xffffffffu, ia, o);
-    const unsigned int y = __shfl_up_sync(0xffffffffu, ib, o);
-    if (lane >= o) {
-      ia += x;
-      ib += y;
-    }
-  }
-  if (lane == 31) {
-    wa[warp] = ia;
-    wb[warp] = ib;
-  }
-  __syncthreads();
-  if (warp == 0) {  // exclusive scan of the 32 warp totals
-    const unsigned int xa = wa[lane], xb = wb[lane];
-    unsigned int sa = xa, sb = xb;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int x = __shfl_up_sync(0xffffffffu, sa, o);
-      const unsigned int y = __shfl_up_sync(0xffffffffu, sb, o);
-      if (lane >= o) {
-        sa += x;
-        sb += y;
+  if (ROUND == 0) {
+    pick_from_top<kFineBins>(c.fine, expected - 1, bin, rin);
+    if (bin < kFineBins - 1) {
+      const uint32_t base = thr_key + (bin << kFineShift);   // keys of the bin: base .. base + 2^14 - 1
+      for_each_value(R, begin, end, [&](float x) {
+        const uint32_t key = abs_key(x);
+        if (key > thr_key && key - base < kExactBins) {
+          // equal keys of a warp are counted by one lane: a tensor may hold one magnitude many times
+          const unsigned int active = __activemask();
+          const unsigned int same = __match_any_sync(active, key);
+          if (int(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&c.exact[key - base], unsigned(__popc(same)));
+        }
+      });
+      if (!last_cta(&c.trim_done[0])) return;
+      pick_from_top<kExactBins>(c.exact, rin, bin, rin);
+      if (threadIdx.x == 0) {
+        c.cut_key = base + bin;
+        c.ties_kept = rin + 1;
       }
+      return;
     }
-    wa[lane] = sa - xa;
-    wb[lane] = sb - xb;
-    if (lane == 31) {
-      tot[0] = sa;
-      tot[1] = sb;
-    }
+  } else if (c.clipped == 0) {
+    return;
   }
+  const unsigned int rank = ROUND == 0 ? expected - 1 : c.t_rank;
+  pick_from_top<kBins>(c.thist[ROUND], rank, bin, rin);
+  const uint32_t prefix = extend_prefix(ROUND == 0 ? 0u : c.t_prefix, ROUND, bin);
+  for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
   __syncthreads();
-  if (t < blocks) {
-    s->off_gt[t] = wa[warp] + ia - va;
-    s->off_eq[t] = wb[warp] + ib - vb;
+  for_each_value(R, begin, end, [&](float x) {
+    const uint32_t key = abs_key(x);
+    if (key > thr_key && ((key - thr_key) >> kFineShift) >= kFineBins - 1 && prefix_matches(key, ROUND + 1, prefix))
+      atomicAdd(&sh[digit_of(key, ROUND + 1)], 1u);
+  });
+  hist_flush(sh, c.thist[ROUND + 1]);
+  if (!last_cta(&c.trim_done[ROUND])) return;
+  if (ROUND == 0) {
+    if (threadIdx.x == 0) {
+      c.clipped = 1u;
+      c.t_prefix = prefix;
+      c.t_rank = rin;
+    }
+  } else {
+    unsigned int low, in_low;
+    pick_from_top<kBins>(c.thist[2], rin, low, in_low);
+    if (threadIdx.x == 0) {
+      c.cut_key = extend_prefix(prefix, 2, low);
+      c.ties_kept = in_low + 1;
+    }
   }
-  if (t == 0) {
-    const unsigned int ties = s->ties_kept;
-    const unsigned int k = tot[0] + (tot[1] < ties ? tot[1] : ties);
-    s->k = k;
-    const uint32_t total = 4u + 8u * k;
-    uint8_t header[4];
-    for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
-    push_bytes(dst, 0, header, 4);
-    s->last_cand = s->cand;
-    s->cand = 0;
-  }
-  unsigned int* h = &s->shist[0][0];
-  for (int i = t; i < 6 * kBins; i += 1024) h[i] = 0;
 }
 
 // ---- ordered compaction and delivery
 // Output order is index order; position of an element = (elements above the cut before it) +
-// min(ties kept, elements equal to the cut before it).  The CTA's starting counts come from the
-// scan; inside the CTA each warp owns a contiguous part of the chunk: a first walk counts what
-// the warp will emit, one barrier turns the counts into per-warp offsets, and a second walk
-// (its data now in L1 / L2) emits with warp-level scans only.  99.9 % of the data is below the
-// cut, so most 128-element steps are a ballot and nothing else.  (A first version scanned
-// across the whole CTA per 1,024-element tile -- five barriers per tile that held a hit -- and
-// took 64 us for 64 MB where the reads cost 12.)
+// min(ties kept, elements equal to the cut before it).  A chunk's starting counts are what the chunks
+// before it keep: every CTA publishes its own counts as soon as it has them and adds up those of its
+// predecessors.  Chunks are handed out by a ticket, so the ones waited for belong to CTAs that already
+// run, and each publishes before it waits: the wait ends.  (It is bounded all the same.)
+// Inside the CTA each warp owns a contiguous part of the chunk: a first walk counts what the warp will
+// emit, one barrier turns the counts into per-warp offsets, and a second walk (its data now in L1 / L2)
+// emits with warp-level ballots only.
+// 25 MB, 6.25 % kept (ncu, cold): 50 us when every lane stored its own entries, 28 now.
+constexpr unsigned long long kAggReady = 1ull << 62;
+constexpr uint64_t kAggWaitNs = 2000000000ull;
 __global__ void __launch_bounds__(kThreads)
-write_kernel(float* __restrict__ R, float* __restrict__ u_mask, float* sumsq_to_clear, int64_t n,
-             int64_t chunk, PushTargets dst, const SparseScratch* s) {
+write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t chunk, unsigned int expected,
+             PushTargets dst, SparseScratch* s) {
+  wait_for_previous();
   resolve_epoch(dst);
   constexpr int kWarps = kThreads / 32;
-  __shared__ unsigned int warp_gt[kWarps], warp_eq[kWarps];
-  const uint32_t cut = s->cut_key;
-  const unsigned int ties = s->ties_kept;
-  const unsigned int k_total = s->k;
+  __shared__ unsigned int warp_gt[kWarps], warp_eq[kWarps], before_gt, before_eq;
+  __shared__ uint2 packs[kWarps][512];
+  __shared__ int ticket;
+  if (threadIdx.x == 0) {
+    ticket = int(atomicAdd(&s->call.ticket, 1u));
+    before_gt = before_eq = 0;
+  }
+  const uint32_t cut = s->call.cut_key;
+  const unsigned int ties = s->call.ties_kept;
+  const unsigned int cand = s->call.cand;
+  const unsigned int k_total = cand < expected ? cand : expected;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t begin = int64_t(blockIdx.x) * chunk;
+  __syncthreads();
+  const int block = ticket;
+  const int64_t begin = int64_t(block) * chunk;
   const int64_t end = begin + chunk < n ? begin + chunk : n;
+  if (block == 0 && threadIdx.x == 0) {
+    s->k = k_total;
+    s->last_cand = cand;
+    const uint32_t total = 4u + 8u * k_total;
+    uint8_t header[4];
+    for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
+    push_bytes(dst, 0, header, 4);
+    if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
+  }
   // warp ranges: multiples of 128 elements so that every step is 32 lanes x 4 elements
   int64_t wlen = (end - begin + kWarps - 1) / kWarps;
   wlen = (wlen + 127) / 128 * 128;
@@ -527,60 +636,115 @@ write_kernel(float* __restrict__ R, float* __restrict__ u_mask, float* sumsq_to_
     warp_eq[warp] = my_eq;
   }
   __syncthreads();
-  unsigned int run_gt = s->off_gt[blockIdx.x], run_eq = s->off_eq[blockIdx.x];
+  if (threadIdx.x == 0) {
+    unsigned long long g = 0, q = 0;
+    for (int w = 0; w < kWarps; ++w) {
+      g += warp_gt[w];
+      q += warp_eq[w];
+    }
+    atomicExch(&s->call.agg[block], kAggReady | (g << 31) | q);   // the one word is the whole message
+  }
+  unsigned int add_gt = 0, add_eq = 0;
+  const uint64_t t0 = globaltimer_ns();
+  for (int b = threadIdx.x; b < block; b += kThreads) {
+    unsigned long long v;
+    while (((v = *reinterpret_cast<volatile unsigned long long*>(&s->call.agg[b])) & kAggReady) == 0) {
+      if (globaltimer_ns() - t0 > kAggWaitNs) {
+        s->gave_up = 1u;
+        break;
+      }
+    }
+    add_gt += unsigned((v & ~kAggReady) >> 31);
+    add_eq += unsigned(v & 0x7fffffffull);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    add_gt += __shfl_xor_sync(0xffffffffu, add_gt, o);
+    add_eq += __shfl_xor_sync(0xffffffffu, add_eq, o);
+  }
+  if (lane == 0 && (add_gt | add_eq) != 0) {
+    atomicAdd(&before_gt, add_gt);
+    atomicAdd(&before_eq, add_eq);
+  }
+  __syncthreads();
+  unsigned int run_gt = before_gt, run_eq = before_eq;
   for (int w = 0; w < warp; ++w) {
     run_gt += warp_gt[w];
     run_eq += warp_eq[w];
   }
 
   // ---- second walk: emit
+  // 512 elements at a time: what is kept is packed in shared memory first, so that the stores to the
+  // payload (which loop over the destinations) are made by full warps of neighbouring entries.
   if (my_gt != 0 || (ties > 0 && my_eq != 0)) {
-    for (int64_t step = wbegin; step < wend; step += 128) {
-      const int64_t e0 = step + lane * 4;
-      float v[4];
-      uint32_t key[4];
-      load4(e0, v, key);
-      unsigned int n_gt = 0, n_eq = 0;
+    uint2* const packed = packs[warp];
+    unsigned int run_kept = run_gt + (run_eq < ties ? run_eq : ties);
+    const unsigned int lt = (1u << lane) - 1u;
+    for (int64_t base2 = wbegin; base2 < wend; base2 += 512) {
+      float v[4][4];
+      uint32_t key[4][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool in = e0 + j < wend;
-        n_gt += in && key[j] > cut;
-        n_eq += in && key[j] == cut;
-      }
-      if (__ballot_sync(0xffffffffu, (n_gt | n_eq) != 0) == 0) continue;
-      unsigned int inc_gt = n_gt, inc_eq = n_eq;   // inclusive scans over the lanes
+      for (int u = 0; u < 4; ++u) load4(base2 + u * 128 + lane * 4, v[u], key[u]);
+      unsigned int held = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int a = __shfl_up_sync(0xffffffffu, inc_gt, o);
-        const unsigned int b = __shfl_up_sync(0xffffffffu, inc_eq, o);
-        if (lane >= o) {
-          inc_gt += a;
-          inc_eq += b;
+      for (int u = 0; u < 4; ++u) {
+        const int64_t e0 = base2 + u * 128 + lane * 4;
+        bool keep[4], at_cut = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          keep[j] = e0 + j < wend && key[u][j] > cut;
+          at_cut = at_cut || (e0 + j < wend && key[u][j] == cut);
         }
-      }
-      unsigned int gt_before = run_gt + inc_gt - n_gt, eq_before = run_eq + inc_eq - n_eq;
+        if (ties > 0 && __any_sync(0xffffffffu, at_cut)) {
+          // ties are kept from the lower index on: element order is lane by lane
+          unsigned int before = run_eq, total = 0;
+          unsigned int at[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (e0 + j >= wend) break;
-        const bool above = key[j] > cut, at = key[j] == cut;
-        const bool keep = above || (at && eq_before < ties);
-        if (keep) {
-          const unsigned int pos = gt_before + (eq_before < ties ? eq_before : ties);
-          if (pos < k_total) {
-            push_u32(dst, 4 + 4 * int64_t(pos), uint32_t(e0 + j));
-            push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), __float_as_uint(v[j]));
-            R[e0 + j] = 0.0f;
-            if (u_mask != nullptr) u_mask[e0 + j] = 0.0f;   // DGC's momentum factor masking
+          for (int j = 0; j < 4; ++j) {
+            at[j] = __ballot_sync(0xffffffffu, e0 + j < wend && key[u][j] == cut);
+            before += __popc(at[j] & lt);
+            total += __popc(at[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if ((at[j] >> lane) & 1u) {
+              keep[j] = before < ties;
+              ++before;
+            }
+          }
+          run_eq += total;
+        }
+        unsigned int at_pos = held;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const unsigned int m = __ballot_sync(0xffffffffu, keep[j]);
+          at_pos += __popc(m & lt);
+          held += __popc(m);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (keep[j]) {
+            packed[at_pos] = make_uint2(uint32_t(e0 + j), __float_as_uint(v[u][j]));
+            if (run_kept + at_pos < k_total) {
+              R[e0 + j] = 0.0f;
+              if (u_mask != nullptr) u_mask[e0 + j] = 0.0f;   // DGC's momentum factor masking
+            }
+            ++at_pos;
           }
         }
-        gt_before += above;
-        eq_before += at;
       }
-      run_gt += __shfl_sync(0xffffffffu, inc_gt, 31);
-      run_eq += __shfl_sync(0xffffffffu, inc_eq, 31);
+      __syncwarp();
+      for (unsigned int i = lane; i < held; i += 32) {
+        const unsigned int pos = run_kept + i;
+        if (pos < k_total) {
+          push_u32(dst, 4 + 4 * int64_t(pos), packed[i].x);
+          push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), packed[i].y);
+        }
+      }
+      __syncwarp();
+      run_kept += held;
     }
   }
-  if (sumsq_to_clear != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *sumsq_to_clear = 0.f;
   publish_when_grid_done(dst);
 }
 
@@ -613,30 +777,15 @@ scatter_kernel(const uint8_t* __restrict__ payload, int64_t cap, float* __restri
   }
 }
 
-// Scan form, DGC with momentum correction: the state update as a pass of its own
-// (u = m*u + s*g, v += u, g = 0), with the same rounding as the list form's collect pass.
-__global__ void __launch_bounds__(kThreads)
-dgc_update_kernel(SparseFuseDev fuse, float* __restrict__ R, int64_t n) {
-  const float scale = dgc_clip_scale(fuse);
-  float* gw = const_cast<float*>(fuse.grad);
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const float u = dgc_new_u(fuse.u[i], fuse.grad[i], fuse.momentum, scale);
-    fuse.u[i] = u;
-    R[i] = __fadd_rn(R[i], u);
-    if (fuse.zero_grad) gw[i] = 0.f;
-  }
-}
-
 // ================================================================ list form
 // Pool of list blocks, behind the sample keys in the scratch: block b holds count[b] (index,
-// value bits) pairs in entry[b * 16 ..] and continues in block next[b].  Three flat arrays, so
-// that the cut kernel can sweep all entries with coalesced, independent loads.
+// value bits) pairs in entry[b * 16 ..] and continues in block next[b].  
 struct ListPool {
   unsigned int* count;
   unsigned int* next;
   uint2* entry;
-  uint32_t* dense;        // the candidates' keys once more, densely packed in no particular order
+  uint32_t* dense;        // the candidates' keys once more, densely packed in no particular order,
+  uint16_t* dense_cta;    // and the CTA that found each
   unsigned int capacity;  // blocks
 };
 
@@ -669,7 +818,7 @@ __device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& po
         continue;
       }
       if (cur.block == kNoBlock || cur.fill == kBlockEntries) {
-        const unsigned int id = atomicAdd(&s->pool_used, 1u);
+        const unsigned int id = atomicAdd(&s->call.pool_used, 1u);
         if (id >= pool.capacity) {
           cur.exhausted = true;
           ++cur.lost;
@@ -694,19 +843,12 @@ __device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& po
 // CTAs per SM, so that the whole grid of 4 x 148 CTAs is resident at once.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 4)
-collect_kernel(SparseFuseDev fuse, float* __restrict__ R, int64_t n, int64_t chunk, int64_t sample_cnt,
-               SparseScratch* s, ListPool pool) {
+collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s, ListPool pool) {
+  wait_for_previous();
   fuse.mode = MODE;
   constexpr int kWarps = kThreads / 32;
   constexpr int U = MODE == 2 ? 2 : 4;   // steps whose loads are issued together
-  uint32_t thr_key = 0;
-  if (sample_cnt > 0) {
-    unsigned int bin, rin;
-    pick_from_top(s->shist[2], s->s_rank[2], bin, rin);
-    thr_key = extend_prefix(s->s_prefix[2], 2, bin);
-  }
-  __syncthreads();
-  if (blockIdx.x == 0 && threadIdx.x == 0) s->thr_key = thr_key;
+  const uint32_t thr_key = s->call.thr_key;
   const float scale = dgc_clip_scale(fuse);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int list = blockIdx.x * kWarps + warp;
@@ -773,7 +915,7 @@ collect_kernel(SparseFuseDev fuse, float* __restrict__ R, int64_t n, int64_t chu
       for (int q = 0; q < U; ++q) {
         const int64_t e0 = base + q * 128 + lane * 4;
         r4[q] = *reinterpret_cast<const float4*>(R + e0);
-        if (MODE >= 1) g4[MODE >= 1 ? q : 0] = __ldg(reinterpret_cast<const float4*>(fuse.grad + e0));
+        if (MODE >= 1) g4[MODE >= 1 ? q : 0] = *reinterpret_cast<const float4*>(fuse.grad + e0);
         if (MODE == 2) u4[MODE == 2 ? q : 0] = *reinterpret_cast<const float4*>(fuse.u + e0);
       }
 #pragma unroll
@@ -820,274 +962,284 @@ collect_kernel(SparseFuseDev fuse, float* __restrict__ R, int64_t n, int64_t chu
     }
     if (__ballot_sync(0xffffffffu, count != 0) != 0) list_append(s, pool, list, lane, count, idx, val, cur);
   }
-  // The cut kernel wants all candidate keys in one flat array (it is a single CTA: a sweep over
-  // the half-empty list blocks cost it 70 us).  Each warp copies the keys of its own list, which
+  let_next_start();
+  // The cut kernel wants all candidate keys in one flat array (it is one CTA, or eight: a sweep over
+  // the half-empty list blocks cost a single one 70 us).  Each warp copies the keys of its own list, which
   // it has just written, to a range it reserves with one atomic.
   if (lane == 0 && cur.lost != 0) atomicAdd(&s->dropped, cur.lost);
   const unsigned int total = __shfl_sync(0xffffffffu, cur.total, 0);
   if (total != 0) {
     unsigned int base = 0;
-    if (lane == 0) base = atomicAdd(&s->cand, total);
+    if (lane == 0) base = atomicAdd(&s->call.cand, total);
     base = __shfl_sync(0xffffffffu, base, 0);
     __syncwarp();   // lane 0's list writes are visible to the other lanes
     unsigned int done = 0;
     for (unsigned int b = s->list_head[list]; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
       const unsigned int c = pool.count[b];
-      if (lane < int(c)) pool.dense[base + done + lane] = pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu;
+      if (lane < int(c)) {
+        pool.dense[base + done + lane] = pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu;
+        pool.dense_cta[base + done + lane] = uint16_t(blockIdx.x);
+      }
       done += c;
     }
   }
 }
 
-// ---- one CTA: the exact cut among the candidates, when there are more than wanted
+// ---- the exact cut among the candidates, and where every CTA's lists go in the payload
+// CTAS = 1, or a cluster of eight that share the candidates: each counts its share of a digit, the
+// counts are added through distributed shared memory, and every CTA picks the same bin.
+// Two digits of the distance from the threshold (2,048 bins of 4,096 keys: one octave above it, then the
+// keys of one bin) find the cut of ordinary data, and they spread: the leading bits of the keys themselves
+// are nearly all the same, which costs either colliding atomics or a match instruction per warp (38 us for
+// the 17,000 candidates of a 64 MB tensor, 21 us now).  Only when the cut lies in the last bin are the
+// three digits of the keys counted.
 constexpr int kCutThreads = 1024;
-constexpr int kCutSmemKeys = 48 * 1024;   // keys held in shared memory (192 KB)
+constexpr int kCutCluster = 8;
+template <int CTAS> struct CutForm {
+  static constexpr int kKeys = CTAS == 1 ? 48 * 1024 : 24 * 1024;   // keys a CTA holds in shared memory
+};
+constexpr int64_t kCutOneCta = 40 * 1024;   // selections up to this leave a single CTA's array room for the surplus
+static_assert(kMaxBlocks <= kCutThreads, "one thread scans one CTA's total");
 
-// Block-wide over kCutThreads threads: the bin holding the element of 0-indexed `rank` counted
-// from the top bin down, and the rank inside that bin.  Every thread returns the same pair.
-__device__ void pick_from_top_1024(const unsigned int* hist, unsigned int rank, unsigned int& bin,
-                                   unsigned int& rank_in_bin, unsigned int* part /* [kCutThreads] */,
-                                   unsigned int* res /* [2] */) {
-  constexpr int PER = kBins / kCutThreads;  // 2 bins per thread
-  const int t = threadIdx.x;
-  unsigned int local[PER];
-  unsigned int sum = 0;
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    local[j] = hist[kBins - 1 - (t * PER + j)];
-    sum += local[j];
-  }
-  // inclusive scan of the per-thread sums: warp scans, then a scan of the 32 warp totals
-  const int lane = t & 31, warp = t >> 5;
-  unsigned int inc = sum;
+// Exclusive scan over kCutThreads values, one per thread; total: their sum.  ws: 33 words of shared memory.
+__device__ __forceinline__ unsigned int exclusive_scan_1024(unsigned int v, unsigned int* ws, unsigned int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned int inc = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned int a = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += a;
   }
-  if (lane == 31) part[warp] = inc;
+  __syncthreads();
+  if (lane == 31) ws[warp] = inc;
   __syncthreads();
   if (warp == 0) {
-    const unsigned int x = part[lane];
+    const unsigned int x = ws[lane];
     unsigned int sx = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned int a = __shfl_up_sync(0xffffffffu, sx, o);
       if (lane >= o) sx += a;
     }
-    part[lane] = sx - x;   // exclusive
+    ws[lane] = sx - x;
+    if (lane == 31) ws[32] = sx;
   }
   __syncthreads();
-  const unsigned int before = part[warp] + inc - sum;
-  if (rank >= before && rank < before + sum) {
-    unsigned int run = before;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      if (rank >= run && rank < run + local[j]) {
-        res[0] = kBins - 1 - (t * PER + j);
-        res[1] = rank - run;
-      }
-      run += local[j];
-    }
-  }
-  __syncthreads();
-  bin = res[0];
-  rank_in_bin = res[1];
-  __syncthreads();
+  total = ws[32];
+  return ws[warp] + inc - v;
 }
 
+template <int CTAS>
 __global__ void __launch_bounds__(kCutThreads)
-cut_kernel(unsigned int expected, SparseScratch* s, ListPool pool) {
-  extern __shared__ uint32_t keys[];   // kCutSmemKeys
-  __shared__ unsigned int sh[kBins];
-  __shared__ unsigned int part[kCutThreads];
-  __shared__ unsigned int res[2];
-  const unsigned int cand = s->cand;
-  if (cand <= expected) {
-    if (threadIdx.x == 0) {
-      s->cut_key = s->thr_key;
-      s->ties_kept = 0;
-    }
-    return;
-  }
-  const bool in_smem = cand <= unsigned(kCutSmemKeys);
+cut_kernel(unsigned int expected, int blocks, PushTargets dst, SparseScratch* s, ListPool pool, float* sumsq_to_clear) {
+  wait_for_previous();
+  resolve_epoch(dst);
+  extern __shared__ uint32_t keys[];   // CutForm<CTAS>::kKeys
+  __shared__ unsigned int sh[kBins];   // this CTA's counts
+  __shared__ unsigned int all[CTAS > 1 ? kBins : 1];   // the cluster's
+  __shared__ unsigned int kept_gt[kMaxBlocks], kept_eq[kMaxBlocks];
+  __shared__ unsigned int ws[33], res[2];
+  const int t = threadIdx.x, lane = t & 31;
+  const int part = CTAS > 1 ? int(blockIdx.x) : 0;
+  const unsigned int cand = s->call.cand;
+  const unsigned int share = (cand + CTAS - 1) / CTAS;
+  const unsigned int first = share * part < cand ? share * part : cand;
+  const unsigned int count = first + share < cand ? share : cand - first;
+  for (int i = t; i < kMaxBlocks; i += kCutThreads) kept_gt[i] = kept_eq[i] = 0;
+  const bool in_smem = count <= unsigned(CutForm<CTAS>::kKeys);
   if (in_smem) {
     // eight independent loads per thread and iteration
-    for (unsigned int base = 0; base < cand; base += kCutThreads * 8) {
+    for (unsigned int base = 0; base < count; base += kCutThreads * 8) {
       uint32_t k[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const unsigned int i = base + u * kCutThreads + threadIdx.x;
-        k[u] = i < cand ? pool.dense[i] : 0u;
+        const unsigned int i = base + u * kCutThreads + t;
+        k[u] = i < count ? pool.dense[first + i] : 0u;
       }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const unsigned int i = base + u * kCutThreads + threadIdx.x;
-        if (i < cand) keys[i] = k[u];
+        const unsigned int i = base + u * kCutThreads + t;
+        if (i < count) keys[i] = k[u];
       }
     }
-    __syncthreads();
   }
-  const unsigned int count = cand;
-  uint32_t prefix = 0;
-  unsigned int rank = expected - 1;   // 0-based from the top
-  for (int round = 0; round < 3; ++round) {
-    for (int i = threadIdx.x; i < kBins; i += kCutThreads) sh[i] = 0;
-    __syncthreads();
-    // whole warps iterate together: candidate keys share their leading bits (same exponent), so
-    // the lanes that hit the same bin are counted by one of them (one atomic per bin and warp)
-    const unsigned int count_padded = (count + 31u) & ~31u;
-    for (unsigned int i = threadIdx.x; i < count_padded; i += kCutThreads) {
-      uint32_t key = 0;
-      bool live = i < count;
-      if (live) {
-        key = in_smem ? keys[i] : pool.dense[i];   // more candidates than shared memory holds: from L2
+  auto key_at = [&](unsigned int i) { return in_smem ? keys[i] : pool.dense[first + i]; };   // else from L2
+  uint32_t cut = s->call.thr_key;
+  unsigned int ties = 0;
+  if (cand > expected) {   // the same in every CTA
+    const uint32_t thr = cut;
+    unsigned int rank = expected - 1;   // 0-based from the top
+    // one digit: bin(key) below kBins, or negative for a key that does not count
+    auto find = [&](bool collide, auto bin_of) -> uint32_t {
+      for (int i = t; i < kBins; i += kCutThreads) sh[i] = 0;
+      if (t == 0) res[0] = res[1] = 0;
+      __syncthreads();
+      if (collide) {
+        const unsigned int count_padded = (count + 31u) & ~31u;   // whole warps iterate together
+        for (unsigned int i = t; i < count_padded; i += kCutThreads) count_digit(sh, i < count ? bin_of(key_at(i)) : -1);
+      } else {
+        for (unsigned int i = t; i < count; i += kCutThreads) {
+          const int bin = bin_of(key_at(i));
+          if (bin >= 0) atomicAdd(&sh[bin], 1u);
+        }
       }
-      live = live && prefix_matches(key, round, prefix);
-      const int bin = live ? digit_of(key, round) : -1;
-      const unsigned int same = __match_any_sync(0xffffffffu, bin);
-      if (live && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&sh[bin], unsigned(__popc(same)));
+      const unsigned int* hist = sh;
+      if constexpr (CTAS > 1) {
+        const cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        constexpr int kMine = kBins / CTAS;   // bins that this CTA adds up for all
+        if (t < kMine) {
+          const int bin = part * kMine + t;
+          unsigned int sum = 0;
+#pragma unroll
+          for (int c = 0; c < CTAS; ++c) sum += cluster.map_shared_rank(sh, c)[bin];
+#pragma unroll
+          for (int c = 0; c < CTAS; ++c) cluster.map_shared_rank(all, c)[bin] = sum;
+        }
+        cluster.sync();   // also: nobody clears sh while another CTA still reads it
+        hist = all;
+      } else {
+        __syncthreads();
+      }
+      // bin holding the element of that rank, from the top: two bins per thread
+      const int hi = kBins - 1 - 2 * t;
+      const unsigned int a = hist[hi], b = hist[hi - 1];
+      unsigned int unused;
+      const unsigned int before = exclusive_scan_1024(a + b, ws, unused);
+      if (rank >= before && rank - before < a + b) {
+        const bool upper = rank - before < a;
+        res[0] = upper ? hi : hi - 1;
+        res[1] = upper ? rank - before : rank - before - a;
+      }
+      __syncthreads();
+      const uint32_t bin = res[0];
+      rank = res[1];
+      __syncthreads();
+      return bin;
+    };
+    constexpr int kFar = 12;   // log2 of the keys per bin of the first digit
+    const uint32_t far = find(false, [&](uint32_t key) {
+      const uint32_t d = (key - thr) >> kFar;
+      return int(d < kBins - 1 ? d : kBins - 1);
+    });
+    if (far < kBins - 1) {
+      // the bin's 4,096 keys in two steps of the same kind: pairs of keys, then the one of the pair
+      const uint32_t base = thr + (far << kFar);
+      const uint32_t pair = find(false, [&](uint32_t key) { return key - base < (1u << kFar) ? int((key - base) >> 1) : -1; });
+      const uint32_t last = find(false, [&](uint32_t key) { return (key - base) >> 1 == pair ? int((key - base) & 1u) : -1; });
+      cut = base + 2 * pair + last;
+    } else {
+      rank = expected - 1;
+      uint32_t prefix = 0;
+      for (int round = 0; round < 3; ++round) {
+        const uint32_t bin = find(true, [&](uint32_t key) { return prefix_matches(key, round, prefix) ? digit_of(key, round) : -1; });
+        prefix = extend_prefix(prefix, round, bin);
+      }
+      cut = prefix;
     }
+    ties = rank + 1;
+  } else {
     __syncthreads();
-    unsigned int bin, rin;
-    pick_from_top_1024(sh, rank, bin, rin, part, res);
-    prefix = extend_prefix(prefix, round, bin);
-    rank = rin;
   }
-  if (threadIdx.x == 0) {
-    s->cut_key = prefix;
-    s->ties_kept = rank + 1;
+  for (unsigned int i = t; i < count; i += kCutThreads) {
+    const uint32_t key = key_at(i);
+    if (key >= cut) {
+      const int cta = pool.dense_cta[first + i];
+      if (key > cut) atomicAdd(&kept_gt[cta], 1u);
+      else if (ties != 0) atomicAdd(&kept_eq[cta], 1u);
+    }
   }
+  __syncthreads();
+  if constexpr (CTAS > 1) cg::this_cluster().sync();
+  if (part == 0) {
+    unsigned int gt = 0, eq = 0;
+    if (t < blocks) {
+      if constexpr (CTAS > 1) {
+        const cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+        for (int c = 0; c < CTAS; ++c) {
+          gt += cluster.map_shared_rank(kept_gt, c)[t];
+          eq += cluster.map_shared_rank(kept_eq, c)[t];
+        }
+      } else {
+        gt = kept_gt[t];
+        eq = kept_eq[t];
+      }
+    }
+    unsigned int total_gt, total_eq;
+    const unsigned int before_gt = exclusive_scan_1024(gt, ws, total_gt);
+    const unsigned int before_eq = exclusive_scan_1024(eq, ws, total_eq);
+    if (t < blocks) {
+      s->off_gt[t] = before_gt;
+      s->off_eq[t] = before_eq;
+    }
+    if (t == 0) {
+      const unsigned int k = total_gt + (total_eq < ties ? total_eq : ties);
+      s->call.cut_key = cut;
+      s->call.ties_kept = ties;
+      s->k = k;
+      s->last_cand = cand;
+      const uint32_t total = 4u + 8u * k;
+      uint8_t header[4];
+      for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
+      push_bytes(dst, 0, header, 4);
+      if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
+    }
+  }
+  if constexpr (CTAS > 1) cg::this_cluster().sync();   // the counts were read from every CTA
 }
 
-// ---- one warp per list: kept counts against the cut; the last CTA: offsets, k, header, housekeeping
+// ---- one warp per list: deliver, clear the emitted positions, publish
 __global__ void __launch_bounds__(kThreads)
-count_scan_kernel(int lists, PushTargets dst, SparseScratch* s, ListPool pool, float* sumsq_to_clear) {
+emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScratch* s, ListPool pool) {
+  wait_for_previous();
   resolve_epoch(dst);
   constexpr int kWarps = kThreads / 32;
   __shared__ unsigned int w_gt[kWarps], w_eq[kWarps];
-  __shared__ bool is_last;
-  __shared__ unsigned int part_gt[kThreads], part_eq[kThreads];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int list = blockIdx.x * kWarps + warp;
-  const uint32_t cut = s->cut_key;
+  const uint32_t cut = s->call.cut_key;
+  const unsigned int ties = s->call.ties_kept, k_total = s->k;
+  const unsigned int head = list < lists ? s->list_head[list] : kNoBlock;
+  // first walk: what this list keeps
   unsigned int gt = 0, eq = 0;
-  if (list < lists) {
-    for (unsigned int b = s->list_head[list]; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
-      const unsigned int c = pool.count[b];
-      const uint32_t key = lane < int(c) ? (pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu) : 0u;
-      gt += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key > cut));
-      eq += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key == cut));
-    }
-    if (lane == 0) {
-      s->list_gt[list] = gt;
-      s->list_eq[list] = eq;
-    }
+  for (unsigned int b = head; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
+    const unsigned int c = pool.count[b];
+    const uint32_t key = lane < int(c) ? (pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu) : 0u;
+    gt += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key > cut));
+    eq += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key == cut));
   }
   if (lane == 0) {
     w_gt[warp] = gt;
     w_eq[warp] = eq;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int a = 0, b = 0;
-    for (int w = 0; w < kWarps; ++w) {
-      a += w_gt[w];
-      b += w_eq[w];
-    }
-    s->cnt_gt[blockIdx.x] = a;
-    s->cnt_eq[blockIdx.x] = b;
-    __threadfence();
-    is_last = atomicAdd(&s->lists_done, 1u) == gridDim.x - 1;
+  // what the lists before this one keep: the CTA's offset plus the earlier warps of the CTA
+  unsigned int run_gt = s->off_gt[blockIdx.x], run_eq = s->off_eq[blockIdx.x];
+  for (int w = 0; w < warp; ++w) {
+    run_gt += w_gt[w];
+    run_eq += w_eq[w];
   }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  // exclusive scan of the per-CTA totals (at most kMaxBlocks of them)
-  const int ctas = gridDim.x;
-  const int per = (ctas + kThreads - 1) / kThreads;
-  const int c0 = threadIdx.x * per, c1 = (c0 + per < ctas) ? c0 + per : ctas;
-  unsigned int a = 0, b = 0;
-  for (int c = c0; c < c1; ++c) {
-    const unsigned int x = reinterpret_cast<volatile unsigned int*>(s->cnt_gt)[c];
-    const unsigned int y = reinterpret_cast<volatile unsigned int*>(s->cnt_eq)[c];
-    s->off_gt[c] = a;   // exclusive within this thread's run; the run's base is added below
-    s->off_eq[c] = b;
-    a += x;
-    b += y;
-  }
-  part_gt[threadIdx.x] = a;
-  part_eq[threadIdx.x] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int rg = 0, re = 0;
-    for (int i = 0; i < kThreads; ++i) {
-      const unsigned int x = part_gt[i], y = part_eq[i];
-      part_gt[i] = rg;
-      part_eq[i] = re;
-      rg += x;
-      re += y;
-    }
-    const unsigned int ties = s->ties_kept;
-    const unsigned int k = rg + (re < ties ? re : ties);
-    s->k = k;
-    s->last_cand = s->cand;
-    const uint32_t total = 4u + 8u * k;
-    uint8_t header[4];
-    for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
-    push_bytes(dst, 0, header, 4);
-    s->pool_used = 0;
-    s->cand = 0;
-    s->lists_done = 0;
-    if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
-  }
-  __syncthreads();
-  for (int c = c0; c < c1; ++c) {
-    s->off_gt[c] += part_gt[threadIdx.x];
-    s->off_eq[c] += part_eq[threadIdx.x];
-  }
-  unsigned int* h = &s->shist[0][0];
-  for (int i = threadIdx.x; i < 3 * kBins; i += kThreads) h[i] = 0;
-}
-
-// ---- one warp per list: deliver, clear the emitted positions, publish
-__global__ void __launch_bounds__(kThreads)
-emit_kernel(float* __restrict__ R, float* __restrict__ u_mask, int lists, PushTargets dst,
-            const SparseScratch* s, ListPool pool) {
-  resolve_epoch(dst);
-  constexpr int kWarps = kThreads / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int list = blockIdx.x * kWarps + warp;
-  const uint32_t cut = s->cut_key;
-  const unsigned int ties = s->ties_kept, k_total = s->k;
-  if (list < lists) {
-    // what the lists before this one keep: the CTA's offset plus the earlier warps of the CTA
-    unsigned int run_gt = s->off_gt[blockIdx.x], run_eq = s->off_eq[blockIdx.x];
-    for (int w = 0; w < warp; ++w) {
-      run_gt += s->list_gt[blockIdx.x * kWarps + w];
-      run_eq += s->list_eq[blockIdx.x * kWarps + w];
-    }
-    for (unsigned int b = s->list_head[list]; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
-      const unsigned int c = pool.count[b];
-      uint2 en = make_uint2(0u, 0u);
-      if (lane < int(c)) en = pool.entry[size_t(b) * kBlockEntries + lane];
-      const uint32_t key = en.y & 0x7fffffffu;
-      const bool above = lane < int(c) && key > cut, at = lane < int(c) && key == cut;
-      const unsigned int ma = __ballot_sync(0xffffffffu, above), me = __ballot_sync(0xffffffffu, at);
-      const unsigned int lt = (1u << lane) - 1u;
-      const unsigned int gt_before = run_gt + __popc(ma & lt), eq_before = run_eq + __popc(me & lt);
-      if (above || (at && eq_before < ties)) {
-        const unsigned int pos = gt_before + (eq_before < ties ? eq_before : ties);
-        if (pos < k_total) {
-          push_u32(dst, 4 + 4 * int64_t(pos), en.x);
-          push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), en.y);
-          R[en.x] = 0.0f;
-          if (u_mask != nullptr) u_mask[en.x] = 0.0f;
-        }
+  for (unsigned int b = head; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
+    const unsigned int c = pool.count[b];
+    uint2 en = make_uint2(0u, 0u);
+    if (lane < int(c)) en = pool.entry[size_t(b) * kBlockEntries + lane];
+    const uint32_t key = en.y & 0x7fffffffu;
+    const bool above = lane < int(c) && key > cut, at = lane < int(c) && key == cut;
+    const unsigned int ma = __ballot_sync(0xffffffffu, above), me = __ballot_sync(0xffffffffu, at);
+    const unsigned int lt = (1u << lane) - 1u;
+    const unsigned int gt_before = run_gt + __popc(ma & lt), eq_before = run_eq + __popc(me & lt);
+    if (above || (at && eq_before < ties)) {
+      const unsigned int pos = gt_before + (eq_before < ties ? eq_before : ties);
+      if (pos < k_total) {
+        push_u32(dst, 4 + 4 * int64_t(pos), en.x);
+        push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), en.y);
+        R[en.x] = 0.0f;
+        if (u_mask != nullptr) u_mask[en.x] = 0.0f;
       }
-      run_gt += __popc(ma);
-      run_eq += __popc(me);
     }
+    run_gt += __popc(ma);
+    run_eq += __popc(me);
   }
   publish_when_grid_done(dst);
 }
@@ -1370,7 +1522,7 @@ namespace {
 // caller may pick later; a call whose sample or expected candidate count does not fit takes the
 // scan form, which needs neither.
 struct ListPlan {
-  int64_t key_capacity;    // sample keys
+  int64_t key_capacity;    // sample keys, and as many places for the ones select_kernel keeps
   int64_t pool_blocks;
   size_t keys_offset, pool_offset, total_bytes;
 };
@@ -1382,9 +1534,9 @@ inline ListPlan list_plan(int64_t n) {
   const int64_t entries = n / 100 * 6 + 65536;
   p.pool_blocks = entries / kBlockEntries + kMaxLists;
   p.keys_offset = (sizeof(SparseScratch) + 255) / 256 * 256;
-  p.pool_offset = (p.keys_offset + size_t(p.key_capacity) * 4 + 255) / 256 * 256;
-  // count[blocks], next[blocks], entry[blocks][16], dense[blocks * 16]
-  p.total_bytes = p.pool_offset + size_t(p.pool_blocks) * (8 + kBlockEntries * (sizeof(uint2) + 4)) + 512;
+  p.pool_offset = (p.keys_offset + size_t(p.key_capacity) * 8 + 255) / 256 * 256;
+  // count[blocks], next[blocks], entry[blocks][16], dense[blocks * 16], dense_cta[blocks * 16]
+  p.total_bytes = p.pool_offset + size_t(p.pool_blocks) * (8 + kBlockEntries * (sizeof(uint2) + 6)) + 512;
   return p;
 }
 
@@ -1422,19 +1574,39 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
   }
   if (fuse.mode == 2 && fuse.clip > 0.f) {
     if (fuse.sumsq == nullptr) return cudaErrorInvalidValue;
-    cudaError_t e = dgc_sumsq(fuse.grad, n, const_cast<float*>(fuse.sumsq), stream);
-    if (e != cudaSuccess) return e;
+    const cudaError_t err = dgc_sumsq(fuse.grad, n, const_cast<float*>(fuse.sumsq), stream);
+    if (err != cudaSuccess) return err;
   }
+  cudaError_t e = cudaSuccess;
+  const dim3 block(kThreads);
+  float* const sumsq = fuse.mode == 2 && fuse.clip > 0.f ? const_cast<float*>(fuse.sumsq) : nullptr;
   if (sample_cnt > 0) {
     int64_t sb = (sample_cnt + kThreads - 1) / kThreads;
-    if (sb > kMaxBlocks) sb = kMaxBlocks;
-    sample_round_kernel<0><<<int(sb), kThreads, 0, stream>>>(f, R, n, sample_cnt, unsigned(rank0), seed, s, keys, dst.epoch_dev);
-    sample_round_kernel<1><<<int(sb), kThreads, 0, stream>>>(f, R, n, sample_cnt, unsigned(rank0), seed, s, keys, dst.epoch_dev);
-    sample_round_kernel<2><<<int(sb), kThreads, 0, stream>>>(f, R, n, sample_cnt, unsigned(rank0), seed, s, keys, dst.epoch_dev);
+    if (sb > kMaxSampleBlocks) sb = kMaxSampleBlocks;
+    const dim3 grid = dim3(unsigned(sb));
+    // the first kernel of the chain, unless the gradient's norm was taken before it
+    e = launch_with(sumsq != nullptr, 1, sample_round_kernel<0>, grid, block, 0, stream, f, R, n, sample_cnt,
+                    unsigned(rank0), seed, s, keys, dst.epoch_dev);
+    if (keys != nullptr) {
+      if (e == cudaSuccess)
+        e = launch_after(select_kernel, grid, block, 0, stream, sample_cnt, unsigned(rank0), s, keys, keys + lp.key_capacity);
+    } else {
+      if (e == cudaSuccess)
+        e = launch_after(sample_round_kernel<1>, grid, block, 0, stream, f, R, n, sample_cnt, unsigned(rank0), seed, s, keys,
+                         dst.epoch_dev);
+      if (e == cudaSuccess)
+        e = launch_after(sample_round_kernel<2>, grid, block, 0, stream, f, R, n, sample_cnt, unsigned(rank0), seed, s, keys,
+                         dst.epoch_dev);
+    }
+  } else {
+    e = cudaMemsetAsync(&s->call, 0, sizeof(s->call), stream);   // every non-zero element is a candidate
   }
-  PushTargets hdr = dst;
-  hdr.done = nullptr;
+  if (e != cudaSuccess) return e;
+  const dim3 grid = dim3(unsigned(pl.blocks));
+  float* const u_mask = fuse.mode == 2 ? fuse.u : nullptr;
   if (lists) {
+    PushTargets hdr = dst;
+    hdr.done = nullptr;
     uint8_t* pool_base = static_cast<uint8_t*>(scratch) + lp.pool_offset;
     ListPool pool;
     pool.capacity = static_cast<unsigned int>(lp.pool_blocks);
@@ -1442,35 +1614,31 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
     pool.next = pool.count + lp.pool_blocks;
     pool.entry = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(pool.next + lp.pool_blocks) + 127) & ~uintptr_t(127));
     pool.dense = reinterpret_cast<uint32_t*>(pool.entry + size_t(lp.pool_blocks) * kBlockEntries);
+    pool.dense_cta = reinterpret_cast<uint16_t*>(pool.dense + size_t(lp.pool_blocks) * kBlockEntries);
     const int nlists = pl.blocks * (kThreads / 32);
-    if (fuse.mode == 2) collect_kernel<2><<<pl.blocks, kThreads, 0, stream>>>(f, R, n, pl.chunk, sample_cnt, s, pool);
-    else if (fuse.mode == 1) collect_kernel<1><<<pl.blocks, kThreads, 0, stream>>>(f, R, n, pl.chunk, sample_cnt, s, pool);
-    else collect_kernel<0><<<pl.blocks, kThreads, 0, stream>>>(f, R, n, pl.chunk, sample_cnt, s, pool);
-    {
-      cudaError_t e = cudaFuncSetAttribute(cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kCutSmemKeys * int(sizeof(uint32_t)));
-      if (e != cudaSuccess) return e;
-    }
-    cut_kernel<<<1, kCutThreads, kCutSmemKeys * sizeof(uint32_t), stream>>>(unsigned(expected), s, pool);
-    count_scan_kernel<<<pl.blocks, kThreads, 0, stream>>>(
-        nlists, hdr, s, pool, fuse.mode == 2 && fuse.clip > 0.f ? const_cast<float*>(fuse.sumsq) : nullptr);
-    emit_kernel<<<pl.blocks, kThreads, 0, stream>>>(R, fuse.mode == 2 ? fuse.u : nullptr, nlists, dst, s, pool);
-    return cudaGetLastError();
+    auto collect = fuse.mode == 2 ? collect_kernel<2> : (fuse.mode == 1 ? collect_kernel<1> : collect_kernel<0>);
+    e = launch_after(collect, grid, block, 0, stream, f, R, n, pl.chunk, s, pool);   // lists: there was a sample
+    if (e != cudaSuccess) return e;
+    const bool one = expected <= kCutOneCta;
+    const int ctas = one ? 1 : kCutCluster;
+    const size_t smem = size_t(one ? CutForm<1>::kKeys : CutForm<kCutCluster>::kKeys) * sizeof(uint32_t);
+    auto cut = one ? cut_kernel<1> : cut_kernel<kCutCluster>;
+    e = cudaFuncSetAttribute(cut, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    e = launch_with(true, ctas, cut, dim3(unsigned(ctas)), dim3(kCutThreads), smem, stream, unsigned(expected), pl.blocks, hdr,
+                    s, pool, sumsq);
+    if (e != cudaSuccess) return e;
+    return launch_after(emit_kernel, grid, block, 0, stream, R, u_mask, nlists, dst, static_cast<const SparseScratch*>(s), pool);
   }
   // scan form
-  if (fuse.mode == 2) {
-    dgc_update_kernel<<<pl.blocks, kThreads, 0, stream>>>(f, R, n);
-  }
-  count_kernel<<<pl.blocks, kThreads, 0, stream>>>(fuse.grad, R, n, pl.chunk, sample_cnt, unsigned(rank0),
-                                                   fuse.mode == 1 ? 1 : 0, fuse.zero_grad, s);
-  trim_round_kernel<1><<<pl.blocks, kThreads, 0, stream>>>(R, n, pl.chunk, unsigned(expected), s);
-  trim_round_kernel<2><<<pl.blocks, kThreads, 0, stream>>>(R, n, pl.chunk, unsigned(expected), s);
-  recount_kernel<<<pl.blocks, kThreads, 0, stream>>>(R, n, pl.chunk, unsigned(expected), s);
-  scan_kernel<<<1, 1024, 0, stream>>>(pl.blocks, hdr, s);
-  write_kernel<<<pl.blocks, kThreads, 0, stream>>>(R, fuse.mode == 2 ? fuse.u : nullptr,
-                                                   fuse.mode == 2 && fuse.clip > 0.f ? const_cast<float*>(fuse.sumsq) : nullptr,
-                                                   n, pl.chunk, dst, s);
-  return cudaGetLastError();
+  auto count = fuse.mode == 2 ? count_kernel<2> : (fuse.mode == 1 ? count_kernel<1> : count_kernel<0>);
+  e = launch_with(sample_cnt > 0, 1, count, grid, block, 0, stream, f, R, n, pl.chunk, s);
+  if (e == cudaSuccess)
+    e = launch_after(trim_kernel<0>, grid, block, 0, stream, static_cast<const float*>(R), n, pl.chunk, unsigned(expected), s);
+  if (e == cudaSuccess)
+    e = launch_after(trim_kernel<1>, grid, block, 0, stream, static_cast<const float*>(R), n, pl.chunk, unsigned(expected), s);
+  if (e != cudaSuccess) return e;
+  return launch_after(write_kernel, grid, block, 0, stream, R, u_mask, sumsq, n, pl.chunk, unsigned(expected), dst, s);
 }
 
 cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sample_rate,
@@ -1489,7 +1657,7 @@ cudaError_t sparse_read_stats(const void* scratch, unsigned int* host4, cudaStre
   const auto* s = static_cast<const SparseScratch*>(scratch);
   cudaError_t e = cudaMemcpyAsync(host4 + 0, &s->k, 4, cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(host4 + 1, &s->last_cand, 4, cudaMemcpyDeviceToHost, stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(host4 + 2, &s->thr_key, 4, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host4 + 2, &s->call.thr_key, 4, cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(host4 + 3, &s->dropped, 4, cudaMemcpyDeviceToHost, stream);
   return e;
 }

@@ -177,3 +177,53 @@ def test_ecq_compress_paths(bw, offset):
         ops.ecq_compress(g.cuda(), hg, 1.0, 0.9, bw, seed=4, out=out[offset:offset + ref.numel()])
         assert torch.equal(out[offset:offset + ref.numel()].cpu(), ref), n
         assert torch.equal(hg.cpu(), hc), n
+
+
+# ----------------------------------------------------------------------------- sparse compress
+def compare_sparse(r, rate, keep, seed):
+    rc, rg = r.clone(), r.cuda()
+    ref = ops.dgc_compress(rc, rate, keep, seed)
+    out = ops.dgc_compress(rg, rate, keep, seed)
+    total = int(ref[:4].view(torch.int32))
+    assert torch.equal(out[:total].cpu(), ref[:total]), (rate, keep, seed)
+    assert torch.equal(rg.cpu(), rc), (rate, keep, seed)
+
+
+@pytest.mark.parametrize("n", [4097, 700001, (1 << 22) + 3])
+@pytest.mark.parametrize("keep,rate", [(0.02, 0.01), (0.0625, 0.01), (0.25, 0.01), (0.25, 0.05), (0.9, 0.0)])
+def test_sparse_scan_form(n, keep, rate):
+    r = gauss(n, seed=n)
+    for seed in range(1, 5):     # both sides of the over-selection branch
+        compare_sparse(r, rate, keep, seed)
+
+
+@pytest.mark.parametrize("n", [131072, 6000001])
+@pytest.mark.parametrize("keep", [0.001, 0.0099])
+def test_sparse_list_form_one_and_eight_ctas(n, keep):
+    """The cut over the candidates: one CTA, and (59,400 wanted) a cluster of eight."""
+    r = gauss(n, seed=n)
+    for seed in range(1, 5):
+        compare_sparse(r, 0.01, keep, seed)
+
+
+@pytest.mark.parametrize("keep", [0.004, 0.05])
+def test_sparse_magnitudes_over_many_octaves(keep):
+    """Few samples and magnitudes over 30 octaves: the cut may lie far above the sampled threshold."""
+    n = 300000
+    g = torch.Generator().manual_seed(3)
+    r = torch.randn(n, generator=g) * torch.exp2(-30 * torch.rand(n, generator=g))
+    for seed in range(1, 9):
+        compare_sparse(r, 0.0002, keep, seed)
+
+
+@pytest.mark.parametrize("keep", [0.005, 0.05, 0.3])
+@pytest.mark.parametrize("rate", [0.0, 0.01])
+def test_sparse_many_equal_magnitudes(keep, rate):
+    """Ties by the hundred thousand, at and above the cut, kept from the lower index on."""
+    n = 400000
+    g = torch.Generator().manual_seed(5)
+    level = torch.tensor([0.0, 0.25, 0.5, 1.0])[torch.randint(0, 4, (n,), generator=g)]
+    r = level * torch.where(torch.rand(n, generator=g) < 0.5, -1.0, 1.0)
+    r[torch.rand(n, generator=g) < 0.4] = 0.0
+    for seed in (1, 2, 3):
+        compare_sparse(r, rate, keep, seed)
