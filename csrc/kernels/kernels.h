@@ -337,6 +337,15 @@ cudaError_t psgd_gemm_grouped(int mode, const PsgdGemmItem* items, int count, in
                               int* launches, cudaStream_t stream);
 // In-place modified Gram-Schmidt of the n x r matrix P (r <= 16).
 cudaError_t gram_schmidt(float* P, int64_t n, int r, float eps, cudaStream_t stream);
+// The same, and in the same launch what a projection with P as its operand needs: Xt = P transposed and
+// zero-padded to [16][rows_pad] (null: not wanted), and `zero_count` zeros at `zeros`.
+cudaError_t gram_schmidt_for_projection(float* P, int64_t n, int r, float eps, float* Xt, int64_t rows_pad, float* zeros,
+                                        int64_t zero_count, cudaStream_t stream);
+// Mat[:N] = grad + residual, then P = Mat Q, in one pass: ranks 1, 2, 4, 8, m a multiple of 4, and 16-byte
+// aligned arrays (psgd_add_project_eligible).
+bool psgd_add_project_eligible(const float* grad, const float* residual, const float* Mat, const float* Q, int64_t m, int r);
+cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m,
+                             const float* Q, int r, float* P, cudaStream_t stream);
 // approx = P Q^T.  mode 0 (API parity): Mat = approx; residual = grad - Mat[:N]; grad = Mat[:N].
 // mode 1 (error feedback in place): grad[:N] = post_scale * approx; Mat -= approx.
 cudaError_t psgd_expand_residual(const float* P, const float* Q, int64_t n, int64_t m, int r,

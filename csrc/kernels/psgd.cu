@@ -32,6 +32,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "p2p.cuh"
 #include "unpack_lut.cuh"
 
@@ -179,6 +180,7 @@ __device__ __forceinline__ void psgd_gemm_body(const CUtensorMap* map_a_p, const
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s.tmem_base;
   volatile int* abort = &s.abort;
+  wait_for_previous();   // the set-up above overlaps the end of the kernel that wrote the operands
 
   if (nkb > 0) {
     if (warp == 0 && lane == 0) {
@@ -401,44 +403,145 @@ simt_gemm_q_kernel(const float* __restrict__ Mat, const float* __restrict__ P, i
 // ---------------------------------------------------------------- Gram-Schmidt
 constexpr int kGsThreads = 1024;
 
-__device__ __forceinline__ float block_sum(float v, float* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < kGsThreads / 32 ? sh[lane] : 0.f;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[0] = v;
+// One CTA orthonormalises one n x r matrix in place (modified Gram-Schmidt, columns left to right):
+// col_j /= (|col_j| + eps); col_k -= <col_j, col_k> col_j.  A serial chain of r steps on one SM, bound by
+// the latency of each step's block-wide reduction, so a step has one: |col_j|^2 and the products of the
+// unscaled col_j with all later columns are summed together and scaled afterwards.
+//
+// Factors of up to 1024 * Q rows stay in registers: a thread holds Q rows of the (up to) R columns.  A
+// reduction is then a warp shuffle, one barrier, and a second shuffle over the 32 warps' sums, which every
+// warp does for itself.
+// 4096 x 4 (ncu, cold): 24.9 us with one reduction per column pair and the matrix in memory, 13.8 now.
+template <int R, int Q>
+__device__ __forceinline__ void gs_in_registers(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt,
+                                                int64_t rows_pad, float (*part)[32][16] /* [2] */) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float v[Q][R];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int64_t i = tid + int64_t(q) * kGsThreads;
+#pragma unroll
+    for (int c = 0; c < R; ++c) v[q][c] = (i < n && c < r) ? P[i * r + c] : 0.0f;
   }
-  __syncthreads();
-  return sh[0];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    if (j >= r) break;
+    float sum[R];
+#pragma unroll
+    for (int c = j; c < R; ++c) {
+      sum[c] = 0.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) sum[c] += v[q][j] * v[q][c];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+      if (lane == 0) part[j & 1][warp][c] = sum[c];
+    }
+    __syncthreads();   // the other buffer is written next, this one only after the next barrier
+#pragma unroll
+    for (int c = j; c < R; ++c) {
+      sum[c] = part[j & 1][lane][c];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+    }
+    const float inv = 1.0f / (sqrtf(sum[j]) + eps);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      v[q][j] *= inv;
+#pragma unroll
+      for (int c = j + 1; c < R; ++c) v[q][c] -= sum[c] * inv * v[q][j];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int64_t i = tid + int64_t(q) * kGsThreads;
+    if (i < n) {
+#pragma unroll
+      for (int c = 0; c < R; ++c) {
+        if (c < r) {
+          P[i * r + c] = v[q][c];
+          if (Xt != nullptr) Xt[c * rows_pad + i] = v[q][c];
+        }
+      }
+    }
+  }
 }
 
-// One CTA orthonormalises one n x r matrix in place (modified Gram-Schmidt,
-// columns left to right): col_j /= (|col_j| + eps); col_k -= <col_j, col_k> col_j.
-__global__ void __launch_bounds__(kGsThreads)
-gram_schmidt_kernel(float* __restrict__ P, int64_t n, int r, float eps) {
-  __shared__ float sh[kGsThreads / 32];
+// Larger factors: two passes over the (L2-resident) matrix per column.
+__device__ __forceinline__ void gs_in_memory(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt,
+                                             int64_t rows_pad, float (*part)[32][16]) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int j = 0; j < r; ++j) {
-    float ss = 0.f;
-    for (int64_t i = threadIdx.x; i < n; i += kGsThreads) {
-      const float v = P[i * r + j];
-      ss += v * v;
+    float sum[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) sum[c] = 0.f;
+    for (int64_t i = tid; i < n; i += kGsThreads) {
+      const float x = P[i * r + j];
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        if (c >= j && c < r) sum[c] += x * P[i * r + c];
     }
-    const float norm = sqrtf(block_sum(ss, sh));
-    const float inv = 1.0f / (norm + eps);
-    for (int64_t i = threadIdx.x; i < n; i += kGsThreads) P[i * r + j] *= inv;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      if (c >= j && c < r) {
+        for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+        if (lane == 0) part[j & 1][warp][c] = sum[c];
+      }
+    }
     __syncthreads();
-    for (int c = j + 1; c < r; ++c) {
-      float dot = 0.f;
-      for (int64_t i = threadIdx.x; i < n; i += kGsThreads) dot += P[i * r + j] * P[i * r + c];
-      dot = block_sum(dot, sh);
-      for (int64_t i = threadIdx.x; i < n; i += kGsThreads) P[i * r + c] -= dot * P[i * r + j];
-      __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      if (c >= j && c < r) {
+        sum[c] = part[j & 1][lane][c];
+        for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+      }
+    }
+    float norm2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c)
+      if (c == j) norm2 = sum[c];
+    const float inv = 1.0f / (sqrtf(norm2) + eps);
+    // a thread updates the rows that it reads: no barrier between this pass and the next column's
+    for (int64_t i = tid; i < n; i += kGsThreads) {
+      const float x = P[i * r + j] * inv;
+      P[i * r + j] = x;
+      if (Xt != nullptr) Xt[j * rows_pad + i] = x;
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        if (c > j && c < r) P[i * r + c] -= sum[c] * inv * x;
     }
   }
+}
+
+// Xt: null, or the transposed copy [16][rows_pad] that the next projection reads (its padding is the
+// caller's).
+__device__ __forceinline__ void gram_schmidt_cta(float* P, int64_t n, int r, float eps, float* Xt, int64_t rows_pad) {
+  __shared__ float part[2][32][16];
+  if (r == 1 && n <= 16 * kGsThreads) gs_in_registers<1, 16>(P, n, r, eps, Xt, rows_pad, part);
+  else if (r == 2 && n <= 16 * kGsThreads) gs_in_registers<2, 16>(P, n, r, eps, Xt, rows_pad, part);
+  else if (r <= 4 && n <= 8 * kGsThreads) gs_in_registers<4, 8>(P, n, r, eps, Xt, rows_pad, part);
+  else if (r <= 8 && n <= 4 * kGsThreads) gs_in_registers<8, 4>(P, n, r, eps, Xt, rows_pad, part);
+  else if (r <= 16 && n <= 2 * kGsThreads) gs_in_registers<16, 2>(P, n, r, eps, Xt, rows_pad, part);
+  else gs_in_memory(P, n, r, eps, Xt, rows_pad, part);
+}
+
+// CTA 0 orthonormalises P; the others write what the projection with P wants beside it: the padding of
+// the transposed operand, and zeros where the projection accumulates.  Xt, zeros: null when not wanted.
+__global__ void __launch_bounds__(kGsThreads)
+gram_schmidt_kernel(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt, int64_t rows_pad,
+                    float* __restrict__ zeros, int64_t zero_count) {
+  let_next_start();
+  if (blockIdx.x == 0) {
+    gram_schmidt_cta(P, n, r, eps, Xt, rows_pad);
+    return;
+  }
+  const int64_t stride = int64_t(gridDim.x - 1) * kGsThreads;
+  const int64_t first = int64_t(blockIdx.x - 1) * kGsThreads + threadIdx.x;
+  if (Xt != nullptr) {
+    const int64_t pad = rows_pad - n, pads = pad * r, rest = (kBN - r) * rows_pad;
+    for (int64_t i = first; i < pads; i += stride) Xt[(i / pad) * rows_pad + n + i % pad] = 0.0f;
+    for (int64_t i = first; i < rest; i += stride) Xt[r * rows_pad + i] = 0.0f;
+  }
+  for (int64_t i = first; i < zero_count; i += stride) zeros[i] = 0.0f;
 }
 
 // ---------------------------------------------------------------- expand
@@ -611,6 +714,97 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
   return true;
 }
 
+// ---------------------------------------------------------------- M = grad + residual, P = M Q
+// Both in one pass over the matrix, fp32 throughout.  At ranks up to 8 the products are a few per cent of
+// what the SMs can do in the time the matrix takes to stream, while a second launch reads all of M again
+// (and the tensor cores would round it to tf32).  A CTA owns 32 / R rows; each thread walks its columns
+// four at a time with the Q rows of those columns in registers, used by all rows, and four rows' loads
+// in flight.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across
+// the warps in shared memory.  Few rows are also split by columns; the parts then meet in P by atomics,
+// which the launcher zeroes first.
+// 4096 x 4096, rank 4 (ncu, cold): add 28.9 + zero 2.5 + transpose 3.5 + tensor-core projection
+// 15.2 us before, 32 us now; error of the three stages against 64 bits 8.4e-4 before, 7.3e-4 now.
+template <int R>
+__global__ void __launch_bounds__(256, 2)
+add_project_kernel(const float* __restrict__ grad, const float* __restrict__ residual, int64_t N, float* __restrict__ Mat,
+                   int64_t n, int64_t m, const float* __restrict__ Q, float* __restrict__ P, int64_t cols_per_cta) {
+  constexpr int RB = 32 / R;                    // rows per CTA
+  constexpr int RG = 4;                         // rows whose loads are issued together
+  __shared__ float sums[8][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t i0 = int64_t(blockIdx.x) * RB;
+  const int64_t c_end = min(int64_t(blockIdx.y + 1) * cols_per_cta, m);
+  float acc[32];                                // [row][column of Q]
+#pragma unroll
+  for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+  for (int64_t col = int64_t(blockIdx.y) * cols_per_cta + tid * 4; col < c_end; col += 1024) {
+    float q[4 * R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(Q + col * R) + k);
+      q[4 * k] = t.x; q[4 * k + 1] = t.y; q[4 * k + 2] = t.z; q[4 * k + 3] = t.w;
+    }
+#pragma unroll
+    for (int g0 = 0; g0 < RB; g0 += RG) {
+      float4 a[RG], b[RG];
+#pragma unroll
+      for (int k = 0; k < RG; ++k) {
+        const int64_t e = (i0 + g0 + k) * m + col;
+        a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i0 + g0 + k < n) {
+          if (e + 3 < N) {
+            a[k] = __ldg(reinterpret_cast<const float4*>(grad + e));
+            b[k] = __ldg(reinterpret_cast<const float4*>(residual + e));
+          } else {   // past the gradient the matrix keeps what it holds
+            float* x = reinterpret_cast<float*>(&a[k]);
+            float* y = reinterpret_cast<float*>(&b[k]);
+            for (int j = 0; j < 4; ++j) {
+              if (e + j < N) {
+                x[j] = grad[e + j];
+                y[j] = residual[e + j];
+              } else {
+                x[j] = Mat[e + j];
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < RG; ++k) {
+        const float x[4] = {a[k].x + b[k].x, a[k].y + b[k].y, a[k].z + b[k].z, a[k].w + b[k].w};
+        if (i0 + g0 + k < n)
+          *reinterpret_cast<float4*>(Mat + (i0 + g0 + k) * m + col) = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int c = 0; c < R; ++c) acc[(g0 + k) * R + c] += x[j] * q[j * R + c];
+      }
+    }
+  }
+  // lane L ends up with the warp's sum of acc[L]
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const float keep = upper ? acc[k + o] : acc[k], send = upper ? acc[k] : acc[k + o];
+      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  sums[warp][lane] = acc[0];
+  __syncthreads();
+  if (warp == 0) {
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x += sums[w][lane];
+    if (i0 + lane / R < n) {
+      float* p = P + i0 * R + lane;
+      if (gridDim.y == 1) *p = x;
+      else atomicAdd(p, x);
+    }
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
@@ -673,6 +867,38 @@ OwnerTargets owners_of(const ReduceTargets& red, int64_t rows) {
 }
 
 }  // namespace
+
+bool psgd_add_project_eligible(const float* grad, const float* residual, const float* Mat, const float* Q, int64_t m, int r) {
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(residual) |
+                         reinterpret_cast<uintptr_t>(Mat) | reinterpret_cast<uintptr_t>(Q);
+  return (bits & 15) == 0 && (m & 3) == 0 && (r == 1 || r == 2 || r == 4 || r == 8);
+}
+
+cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m,
+                             const float* Q, int r, float* P, cudaStream_t stream) {
+  if (n < 1 || m < 1 || N < 0 || N > n * m || !psgd_add_project_eligible(grad, residual, Mat, Q, m, r))
+    return cudaErrorInvalidValue;
+  const int64_t row_blocks = (n + 32 / r - 1) / (32 / r);
+  // two resident CTAs per SM; columns in steps of 1,024 (one per thread of a CTA, four wide)
+  const int64_t steps = (m + 1023) / 1024;
+  int64_t splits = (148 * 2 + row_blocks - 1) / row_blocks;
+  if (splits > steps) splits = steps;
+  const int64_t cols = (steps + splits - 1) / splits * 1024;
+  const dim3 grid(unsigned(row_blocks), unsigned((m + cols - 1) / cols));
+  if (grid.y > 1) {
+    const cudaError_t e = cudaMemsetAsync(P, 0, size_t(n) * r * sizeof(float), stream);
+    if (e != cudaSuccess) return e;
+  }
+#define HP_ADD_PROJECT(RR) add_project_kernel<RR><<<grid, 256, 0, stream>>>(grad, residual, N, Mat, n, m, Q, P, cols)
+  switch (r) {
+    case 1: HP_ADD_PROJECT(1); break;
+    case 2: HP_ADD_PROJECT(2); break;
+    case 4: HP_ADD_PROJECT(4); break;
+    default: HP_ADD_PROJECT(8); break;
+  }
+#undef HP_ADD_PROJECT
+  return cudaGetLastError();
+}
 
 int64_t psgd_kpad(int64_t k) { return (k + kKPad - 1) / kKPad * kKPad; }
 
@@ -742,8 +968,9 @@ cudaError_t psgd_gemm(int mode, const float* Mat, int64_t n, int64_t m, const fl
     cudaError_t e = cudaFuncSetAttribute(psgd_gemm_kernel<MODE, BK, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                          int(smem));                                                                 \
     if (e != cudaSuccess) return e;                                                                                  \
-    psgd_gemm_kernel<MODE, BK, ST><<<grid, kGemmThreads, smem, stream>>>(map_a, map_b, Mat, n, m, out_rows, r,        \
-                                                                         total_kb, kbps, out, status);               \
+    e = launch_after(psgd_gemm_kernel<MODE, BK, ST>, grid, dim3(kGemmThreads), smem, stream, map_a, map_b, Mat, n, m,  \
+                     out_rows, r, total_kb, kbps, out, status);                                                      \
+    if (e != cudaSuccess) return e;                                                                                  \
   } while (0)
 #define HP_GEMM_MODE(BK, ST)           \
   do {                                 \
@@ -912,28 +1139,8 @@ struct GsBatch {
 };
 __global__ void __launch_bounds__(kGsThreads)
 gram_schmidt_batched_kernel(GsBatch b) {
-  __shared__ float sh[kGsThreads / 32];
   const PsgdGsItem it = b.item[blockIdx.x];
-  float* P = it.P;
-  const int64_t n = it.n;
-  const int r = it.r;
-  for (int j = 0; j < r; ++j) {
-    float ss = 0.f;
-    for (int64_t i = threadIdx.x; i < n; i += kGsThreads) {
-      const float v = P[i * r + j];
-      ss += v * v;
-    }
-    const float inv = 1.0f / (sqrtf(block_sum(ss, sh)) + b.eps);
-    for (int64_t i = threadIdx.x; i < n; i += kGsThreads) P[i * r + j] *= inv;
-    __syncthreads();
-    for (int c = j + 1; c < r; ++c) {
-      float dot = 0.f;
-      for (int64_t i = threadIdx.x; i < n; i += kGsThreads) dot += P[i * r + j] * P[i * r + c];
-      dot = block_sum(dot, sh);
-      for (int64_t i = threadIdx.x; i < n; i += kGsThreads) P[i * r + c] -= dot * P[i * r + j];
-      __syncthreads();
-    }
-  }
+  gram_schmidt_cta(it.P, it.n, it.r, b.eps, nullptr, 0);
 }
 
 }  // namespace
@@ -992,7 +1199,16 @@ cudaError_t gram_schmidt_batched(const PsgdGsItem* items, int count, float eps, 
 
 cudaError_t gram_schmidt(float* P, int64_t n, int r, float eps, cudaStream_t stream) {
   if (n < 1 || r < 1 || r > kBN) return cudaErrorInvalidValue;
-  gram_schmidt_kernel<<<1, kGsThreads, 0, stream>>>(P, n, r, eps);
+  gram_schmidt_kernel<<<1, kGsThreads, 0, stream>>>(P, n, r, eps, nullptr, 0, nullptr, 0);
+  return cudaGetLastError();
+}
+
+cudaError_t gram_schmidt_for_projection(float* P, int64_t n, int r, float eps, float* Xt, int64_t rows_pad, float* zeros,
+                                        int64_t zero_count, cudaStream_t stream) {
+  if (n < 1 || r < 1 || r > kBN || zero_count < 0 || (Xt != nullptr && rows_pad < n)) return cudaErrorInvalidValue;
+  const int64_t side = std::max<int64_t>(zero_count, Xt != nullptr ? (kBN - r) * rows_pad + (rows_pad - n) * r : 0);
+  const int64_t blocks = std::min<int64_t>((side + 4 * kGsThreads - 1) / (4 * kGsThreads), 147);
+  gram_schmidt_kernel<<<unsigned(1 + blocks), kGsThreads, 0, stream>>>(P, n, r, eps, Xt, rows_pad, zeros, zero_count);
   return cudaGetLastError();
 }
 

@@ -624,6 +624,13 @@ void powersgd_encode1(const torch::Tensor& grad, const torch::Tensor& residual,
   TORCH_CHECK(residual.numel() == N && N <= s.n * s.m, "grad/residual must fit in M");
   if (M.is_cuda()) {
     c10::cuda::CUDAGuard guard(M.device());
+    if (cuda::psgd_add_project_eligible(grad.data_ptr<float>(), residual.data_ptr<float>(), M.data_ptr<float>(),
+                                        Q.data_ptr<float>(), s.m, int(s.r))) {
+      HP_CHECK_CUDA(cuda::psgd_add_project(grad.data_ptr<float>(), residual.data_ptr<float>(), N, M.data_ptr<float>(),
+                                           s.n, s.m, Q.data_ptr<float>(), int(s.r), P.data_ptr<float>(),
+                                           at::cuda::getCurrentCUDAStream()));
+      return;
+    }
     HP_CHECK_CUDA(cuda::add_into(grad.data_ptr<float>(), residual.data_ptr<float>(),
                                  M.data_ptr<float>(), N, at::cuda::getCurrentCUDAStream()));
     P.zero_();
@@ -637,9 +644,19 @@ void powersgd_encode1(const torch::Tensor& grad, const torch::Tensor& residual,
 void powersgd_encode2(torch::Tensor P, const torch::Tensor& M, torch::Tensor Q) {
   const PsgdShape s = psgd_shape(M, P, Q);
   if (M.is_cuda()) {
-    gram_schmidt(P, 1e-8);
-    Q.zero_();
-    psgd_project(1, M, P, {Q}, false);
+    c10::cuda::CUDAGuard guard(M.device());
+    auto stream = at::cuda::getCurrentCUDAStream();
+    const int64_t kp = cuda::psgd_kpad(s.n);
+    torch::Tensor xt;
+    if (cuda::psgd_tensor_core_eligible(M.data_ptr<float>(), s.n, s.m)) xt = torch::empty({16, kp}, M.options());
+    float* xt_ptr = xt.defined() ? xt.data_ptr<float>() : nullptr;
+    HP_CHECK_CUDA(cuda::gram_schmidt_for_projection(P.data_ptr<float>(), s.n, int(s.r), 1e-8f, xt_ptr, kp,
+                                                    Q.data_ptr<float>(), Q.numel(), stream));
+    cuda::ReduceTargets red;
+    red.world = 1;
+    red.dst[0] = Q.data_ptr<float>();
+    HP_CHECK_CUDA(cuda::psgd_gemm(1, M.data_ptr<float>(), s.n, s.m, P.data_ptr<float>(), xt_ptr, int(s.r), red, 0,
+                                  status_word_for(M), stream));
   } else {
     cpu::powersgd_encode2(P.data_ptr<float>(), M.data_ptr<float>(), s.n, s.m, s.r, Q.data_ptr<float>());
   }

@@ -227,3 +227,38 @@ def test_sparse_many_equal_magnitudes(keep, rate):
     r[torch.rand(n, generator=g) < 0.4] = 0.0
     for seed in (1, 2, 3):
         compare_sparse(r, rate, keep, seed)
+
+
+# ----------------------------------------------------------------------------- PowerSGD
+@pytest.mark.parametrize("n,r", [(1, 1), (16384, 1), (16385, 1), (16385, 2), (8192, 4), (8193, 3), (4096, 8), (4097, 8),
+                                 (2048, 16), (2049, 11), (33, 16)])
+def test_gram_schmidt_forms(n, r):
+    """In registers and in memory: columns of unit length, pairwise orthogonal, and the column order of the definition."""
+    P = gauss(n, 1.0, seed=n + r).view(n, 1).repeat(1, r) * 0.5 + gauss(n * r, 1.0, seed=r).view(n, r)
+    want = P.double().clone()
+    for j in range(min(r, n)):
+        want[:, j] /= want[:, j].norm() + 1e-8
+        for c in range(j + 1, r):
+            want[:, c] -= (want[:, j] @ want[:, c]) * want[:, j]
+    got = ops.gram_schmidt(P.cuda().contiguous())
+    cols = min(r, n)
+    # a column keeps about sqrt(1 - overlap^2) >= 0.3 of its length here, so 32-bit rounding shows as a few 1e-6
+    assert (got[:, :cols].double().cpu() - want[:, :cols]).norm() <= 2e-5 * want[:, :cols].norm()
+
+
+@pytest.mark.parametrize("n,m,r", [(1, 4, 1), (7, 1028, 1), (33, 1024, 2), (64, 25088, 4), (9, 4096, 4), (1000, 2052, 4),
+                                   (13, 300, 8), (4096, 512, 8)])
+@pytest.mark.parametrize("short", [0, 3])
+def test_powersgd_encode1_one_pass(n, m, r, short):
+    """short: the gradient ends before the matrix does; what lies behind keeps its value and counts in P."""
+    N = n * m - min(short, n * m - 1)
+    grad, res = gauss(N, 1.0, seed=1), gauss(N, 0.5, seed=2)
+    Q, M0 = gauss(m * r, 1.0, seed=3).view(m, r), gauss(n * m, 1.0, seed=4)
+    want = M0.clone()
+    want[:N] = grad + res
+    M, P = M0.clone().view(n, m).cuda(), torch.full((n, r), 7.0, device="cuda")
+    ops.powersgd_encode1(grad.cuda(), res.cuda(), Q.cuda(), M, P)
+    assert torch.equal(M.cpu().view(-1), want)
+    ref = want.view(n, m).double() @ Q.double()
+    # fp32 products and sums of m terms: sqrt(m) roundings of 2^-24 each, and a wide margin
+    assert (P.cpu().double() - ref).norm() <= 4 * m ** 0.5 * 2 ** -24 * (want.norm() * Q.norm()).double()
