@@ -97,6 +97,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("init",
         [](const std::string& alg, std::unordered_map<std::string, double> params, int device_id,
            int rank_id, int size) {
+          py::gil_scoped_release nogil;   // it may have to wait for workers that let go of Python tensors
           return runtime::TaskRuntime::instance().init(alg, std::move(params), device_id, rank_id, size);
         },
         "init(alg_name, alg_paras, device_id, rank_id, size) -> bool", py::arg("alg_name"),
@@ -105,6 +106,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::gil_scoped_release nogil;
     return runtime::TaskRuntime::instance().end();
   });
+  m.def("_errorMarks", [](int task_id) { return runtime::TaskRuntime::instance().error_marks(task_id); });
+  m.def("_waitResults", [](int task_id, double timeout_s, unsigned long long seen) {
+    return runtime::TaskRuntime::instance().wait_results(task_id, timeout_s, seen);
+  }, py::call_guard<py::gil_scoped_release>());
   m.def("getResults", [](int task_id) { return runtime::TaskRuntime::instance().get_results(task_id); });
   m.def("getErrors", [] { return runtime::TaskRuntime::instance().get_errors(); });
   m.def("numThreads", [] { return runtime::TaskRuntime::instance().num_threads(); });

@@ -52,11 +52,10 @@ bool TaskRuntime::init(const std::string& alg_name, std::unordered_map<std::stri
     std::lock_guard<std::mutex> lk(err_mu_);
     errors_.clear();
   }
-  pool_ = std::make_unique<WorkerPool>(threads, [](int) {});
+  pool_ = std::make_unique<WorkerPool>(threads, [](int) {}, [this](int) { settle(); });
   const double age_limit = params.count("task_age_limit") ? params["task_age_limit"] : 120.0;
   watchdog_ = std::make_unique<AgeWatchdog>(age_limit, [this](const std::string& label, double age) {
-    std::lock_guard<std::mutex> lk(err_mu_);
-    errors_.push_back(label + ": still running after " + std::to_string(age) + " s (task age limit)");
+    add_error(label + ": still running after " + std::to_string(age) + " s (task age limit)");
   });
   return true;
 }
@@ -96,6 +95,29 @@ std::vector<std::string> TaskRuntime::get_results(int task_id) {
     default:
       return {};
   }
+}
+
+std::vector<std::string> TaskRuntime::wait_results(int task_id, double timeout_s, unsigned long long seen) {
+  switch (task_id) {
+    case kCompTask: case kPowerSgdEncode1:
+    case kDecompTask: case kPowerSgdDecode:
+    case kRootDecompCompTask: case kPowerSgdEncode2:
+      return queue_for(task_id).wait_drain(timeout_s, seen);
+    default:
+      return {};
+  }
+}
+
+unsigned long long TaskRuntime::error_marks(int task_id) { return queue_for(task_id).wakes(); }
+
+void TaskRuntime::add_error(std::string text) {
+  {
+    std::lock_guard<std::mutex> lk(err_mu_);
+    errors_.push_back(std::move(text));
+  }
+  comp_.wake();
+  decomp_.wake();
+  root_.wake();
 }
 
 std::vector<std::string> TaskRuntime::get_errors() {
@@ -171,6 +193,44 @@ bool TaskRuntime::submit_powersgd(const std::string& name, torch::Tensor tensor,
   return submit(std::move(t));
 }
 
+namespace {
+// Tasks of this worker whose kernels and copies are queued on its stream.  The worker goes on to its next
+// task instead of waiting for each: a copy of one overlaps the kernels of the next, and the stream is
+// waited for when the queue is empty.
+struct Queued {
+  Task task;   // keeps the tensors
+  std::unique_ptr<at::cuda::CUDAEvent> done;
+};
+std::vector<Queued>& queued() {
+  thread_local std::vector<Queued> q;
+  return q;
+}
+}  // namespace
+
+// A task's tensors are let go before its name is reported: the caller may drop them, and end the runtime,
+// as soon as it knows the name, and the last owner of a Python tensor needs the interpreter lock.
+void TaskRuntime::settle() {
+  std::vector<Queued> batch;
+  batch.swap(queued());
+  for (Queued& q : batch) {
+    const int task_id = q.task.task_id;
+    const std::string name = q.task.tensor_name;
+    const uint64_t serial = q.task.serial;
+    std::string error;
+    try {
+      c10::cuda::CUDAGuard dev(q.task.tensor.device());
+      q.done->synchronize();
+    } catch (const std::exception& e) {
+      error = e.what();
+    }
+    q.task = Task{};
+    q.done.reset();
+    if (error.empty()) queue_for(task_id).push(name);
+    else add_error(name + ": " + error);
+    watchdog_->done(serial);
+  }
+}
+
 bool TaskRuntime::submit(Task t) {
   TORCH_CHECK(pool_ != nullptr && pool_->alive(), "hipress runtime is not initialised (call init first)");
   t.serial = serial_.fetch_add(1);
@@ -196,14 +256,20 @@ bool TaskRuntime::submit(Task t) {
         c10::cuda::CUDAStreamGuard sg(stream);
         ready->block(stream);
         run(t);
-        stream.synchronize();
-      } else {
-        run(t);
+        auto done = std::make_unique<at::cuda::CUDAEvent>();
+        done->record(stream);
+        queued().push_back(Queued{std::move(t), std::move(done)});
+        return;
       }
-      queue_for(t.task_id).push(t.tensor_name);
+      run(t);
+      const int task_id = t.task_id;
+      const std::string name = t.tensor_name;
+      t = Task{};
+      queue_for(task_id).push(name);
     } catch (const std::exception& e) {
-      std::lock_guard<std::mutex> lk(err_mu_);
-      errors_.push_back(t.tensor_name + ": " + e.what());
+      const std::string name = t.tensor_name;
+      t = Task{};
+      add_error(name + ": " + e.what());
     }
     watchdog_->done(serial);
   });

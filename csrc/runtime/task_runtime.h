@@ -72,6 +72,10 @@ class TaskRuntime {
   bool submit_powersgd(const std::string& name, torch::Tensor tensor, torch::Tensor residual,
                        torch::Tensor M, torch::Tensor P, torch::Tensor Q, int task_id);
   std::vector<std::string> get_results(int task_id);
+  // get_results(), after waiting until a task of that kind finishes, an error is recorded, or the time is
+  // up.  seen: error_marks() as read before the caller last looked at get_errors().
+  std::vector<std::string> wait_results(int task_id, double timeout_s, unsigned long long seen);
+  unsigned long long error_marks(int task_id);
   std::vector<std::string> get_errors();
   int num_threads() const { return pool_ ? pool_->size() : 0; }
   const CompAlg& algorithm() const { return alg_; }
@@ -87,6 +91,8 @@ class TaskRuntime {
   void run_root(Task& t);
   void run_powersgd(Task& t);
   FinishQueue& queue_for(int task_id);
+  void add_error(std::string text);
+  void settle();
 
   CompAlg alg_;
   int device_id_ = 0, rank_ = 0, size_ = 1;

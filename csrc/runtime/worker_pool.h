@@ -3,7 +3,9 @@
 // Workers sleep on a condition variable and wake when work arrives (the
 // reference's workers poll their queue on a fixed 500 us cycle,
 // ref hp_cuda.cpp:174-184).  Submission is round-robin over the queues, or to
-// an explicit worker when ordering between tasks matters.  An exception thrown
+// an explicit worker when ordering between tasks matters.  A job may leave work behind that only has
+// to be waited for (copies in flight on a stream): the optional `settle` hook runs in the worker when its
+// queue is empty, or after kMaxUnsettled jobs, and only then do the jobs count as done.  An exception thrown
 // by a task is caught, recorded and reported through `last_error()`; the worker
 // keeps running (in the reference the thread prints and exits, after which
 // every poll hangs: hp_cuda.cpp:805-809).
@@ -28,8 +30,8 @@ class WorkerPool {
 
   // `on_start` runs once in each worker thread before it takes work (device
   // guard, stream creation).
-  WorkerPool(int num_workers, std::function<void(int)> on_start)
-      : workers_(static_cast<size_t>(num_workers)) {
+  WorkerPool(int num_workers, std::function<void(int)> on_start, std::function<void(int)> settle = nullptr)
+      : workers_(static_cast<size_t>(num_workers)), settle_(std::move(settle)) {
     for (int i = 0; i < num_workers; ++i) {
       auto& w = workers_[static_cast<size_t>(i)];
       w = std::make_unique<Worker>();
@@ -119,6 +121,7 @@ class WorkerPool {
       w.started = true;
     }
     w.cv_idle.notify_all();
+    int unsettled = 0;
     for (;;) {
       Job job;
       {
@@ -135,10 +138,27 @@ class WorkerPool {
       } catch (...) {
         record("unknown exception in worker task");
       }
+      ++unsettled;
+      if (settle_) {
+        bool more;
+        {
+          std::lock_guard<std::mutex> lk(w.mu);
+          more = !w.jobs.empty();
+        }
+        if (more && unsettled < kMaxUnsettled) continue;
+        try {
+          settle_(index);
+        } catch (const std::exception& e) {
+          record(e.what());
+        } catch (...) {
+          record("unknown exception in worker task");
+        }
+      }
       {
         std::lock_guard<std::mutex> lk(w.mu);
-        --w.pending;
+        w.pending -= unsettled;
       }
+      unsettled = 0;
       w.cv_idle.notify_all();
     }
   }
@@ -149,7 +169,9 @@ class WorkerPool {
     ++error_count_;
   }
 
+  static constexpr int kMaxUnsettled = 16;
   std::vector<std::unique_ptr<Worker>> workers_;
+  std::function<void(int)> settle_;
   std::atomic<uint64_t> next_{0};
   std::mutex err_mu_;
   std::string last_error_;

@@ -41,25 +41,30 @@ numThreads = _C.numThreads
 
 
 def wait_for(task_id: int, names, timeout_s: float = 60.0) -> List[str]:
-    """Poll ``getResults(task_id)`` until every name in ``names`` has been reported.
+    """Collect ``getResults(task_id)`` until every name in ``names`` has been reported.
 
-    Convenience for callers of the polling API; raises on timeout or on a failed task.
+    Convenience for callers of the polling API; raises on timeout or on a failed task.  The wait between
+    two looks ends as soon as a task of that kind finishes or fails (it used to be a sleep of 200 us,
+    which four 1 MB TBQ tasks spent most of their 560 us in).
     """
     pending = set(names)
     done: List[str] = []
     deadline = time.monotonic() + timeout_s
-    while pending:
-        for key in getResults(task_id):
+    keys = getResults(task_id)
+    while True:
+        for key in keys:
             done.append(key)
             pending.discard(key)
         if not pending:
             break
+        marks = _C._errorMarks(task_id)
         errors = getErrors()
         if errors:
             raise RuntimeError("hipress task failed: " + "; ".join(errors))
-        if time.monotonic() > deadline:
+        left = deadline - time.monotonic()
+        if left < 0:
             raise TimeoutError(f"tasks not finished after {timeout_s}s: {sorted(pending)}")
-        time.sleep(0.0002)
+        keys = _C._waitResults(task_id, min(left, 0.1), marks)
     return done
 
 
