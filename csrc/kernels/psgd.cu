@@ -596,7 +596,32 @@ __device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, co
     for (int c = 0; c < R; ++c) q[j][c] = Q[(col + j) * R + c];
   const int64_t r0 = int64_t(row_block) * rows_per_cta;
   const int64_t r1 = min(r0 + rows_per_cta, n);
-  for (int64_t i = r0; i < r1; ++i) {
+  int64_t i = r0;
+  if (MODE == 0) {
+    // four rows of the gradient in flight: one load at a time per thread left this pass waiting for memory
+    constexpr int U = 4;
+    for (; i + U <= r1 && (i + U - 1) * m + col + 3 < N; i += U) {
+      float4 g[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) g[u] = *reinterpret_cast<const float4*>(grad + (i + u) * m + col);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float a[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float acc = 0.f;
+#pragma unroll
+          for (int c = 0; c < R; ++c) acc += __ldg(P + (i + u) * R + c) * q[j][c];
+          a[j] = acc;
+        }
+        const int64_t e = (i + u) * m + col;
+        *reinterpret_cast<float4*>(Mat + e) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4*>(residual + e) = make_float4(g[u].x - a[0], g[u].y - a[1], g[u].z - a[2], g[u].w - a[3]);
+        *reinterpret_cast<float4*>(grad + e) = make_float4(a[0], a[1], a[2], a[3]);
+      }
+    }
+  }
+  for (; i < r1; ++i) {
     float p[R];
 #pragma unroll
     for (int c = 0; c < R; ++c) p[c] = __ldg(P + i * R + c);
