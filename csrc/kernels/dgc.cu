@@ -7,6 +7,7 @@
 //   * local gradient clipping: g is scaled by min(1, clip / |g|) per bucket
 //     before it enters u (clip already divided by sqrt(world) by the caller)
 // The selector itself is sparse_compress (sparse.cu) run on v.
+#include "adamw.cuh"
 #include "kernels.h"
 #include "launch.cuh"
 #include "p2p.cuh"
@@ -110,47 +111,24 @@ dgc_mask_kernel(const uint8_t* __restrict__ payload, int64_t cap, float* __restr
   }
 }
 
-__device__ __forceinline__ void adamw_one(const AdamWApply& a, float bc1, float rsqrt_bc2, float g,
-                                          float& p, float& m, float& v) {
-  p -= a.lr * a.weight_decay * p;  // decoupled weight decay
-  m = a.beta1 * m + (1.0f - a.beta1) * g;
-  v = a.beta2 * v + (1.0f - a.beta2) * g * g;
-  const float denom = sqrtf(v) * rsqrt_bc2 + a.eps;
-  p -= (a.lr / bc1) * (m / denom);
-}
-
 // VEC: all four arrays 16-byte aligned; four elements per thread and iteration.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
 adamw_kernel(float* __restrict__ grad, float scale, AdamWApply a, int64_t n) {
   // an earlier kernel of the step recorded a failure: leave parameters and moments untouched
   if (a.guard != nullptr && *reinterpret_cast<const volatile int*>(a.guard) != 0) return;
-  const float step = float(a.step_dev != nullptr ? int(*a.step_dev) : a.step);
-  const float bc1 = 1.0f - powf(a.beta1, step);
-  const float rsqrt_bc2 = 1.0f / sqrtf(1.0f - powf(a.beta2, step));
+  float bc1, rsqrt_bc2;
+  adamw_bias(a, bc1, rsqrt_bc2);
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t nv = VEC ? (n >> 2) : 0;
   for (int64_t i = tid; i < nv; i += stride) {
     const float4 g4 = reinterpret_cast<const float4*>(grad)[i];
-    const float4 p4 = reinterpret_cast<const float4*>(a.param)[i];
-    const float4 m4 = reinterpret_cast<const float4*>(a.exp_avg)[i];
-    const float4 v4 = reinterpret_cast<const float4*>(a.exp_avg_sq)[i];
-    float g[4] = {g4.x, g4.y, g4.z, g4.w}, p[4] = {p4.x, p4.y, p4.z, p4.w};
-    float m[4] = {m4.x, m4.y, m4.z, m4.w}, v[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) adamw_one(a, bc1, rsqrt_bc2, g[k] * scale, p[k], m[k], v[k]);
-    reinterpret_cast<float4*>(a.exp_avg)[i] = make_float4(m[0], m[1], m[2], m[3]);
-    reinterpret_cast<float4*>(a.exp_avg_sq)[i] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4*>(a.param)[i] = make_float4(p[0], p[1], p[2], p[3]);
+    adamw_four(a, bc1, rsqrt_bc2, i, make_float4(g4.x * scale, g4.y * scale, g4.z * scale, g4.w * scale));
     if (a.clear_grad) reinterpret_cast<float4*>(grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   for (int64_t i = (nv << 2) + tid; i < n; i += stride) {
-    float p = a.param[i], m = a.exp_avg[i], v = a.exp_avg_sq[i];
-    adamw_one(a, bc1, rsqrt_bc2, grad[i] * scale, p, m, v);
-    a.exp_avg[i] = m;
-    a.exp_avg_sq[i] = v;
-    a.param[i] = p;
+    adamw_at(a, bc1, rsqrt_bc2, i, grad[i] * scale);
     if (a.clear_grad) grad[i] = 0.f;
   }
 }

@@ -173,10 +173,11 @@ cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n,
                                 float post_scale, int* status, cudaStream_t stream,
                                 unsigned int* redo = nullptr);
 
-// out[idx] = 0 for every index of every payload (one launch): after the optimizer has consumed a
-// dense gradient that only held scattered payload entries, this leaves it all zero again
-// without a pass over the whole buffer.
-cudaError_t sparse_clear(const UnpackSources& src, float* out, int64_t n, cudaStream_t stream);
+// Decodes the payloads and applies the optimizer step (exactly one of sgd, adamw) to the parameters in one
+// pass, without a dense gradient.  The indices of each payload must ascend, as the compressor writes them;
+// a payload that does not fit is recorded in *status, and parameters and moments then stay as they are.
+cudaError_t sparse_apply(const UnpackSources& src, int64_t n, float post_scale, const SgdApply* sgd,
+                         const struct AdamWApply* adamw, int* status, cudaStream_t stream);
 
 // ---------------------------------------------------------------- flags
 // Spins (one warp) until flag[r] >= epoch for all r < world, or timeout_ns

@@ -47,9 +47,11 @@
 // list_plan); should it still run out, the candidates that did not fit stay in the residual
 // and are sent in a later step (counted in SparseScratch::dropped).
 #include "../common/codec_math.h"
+#include "adamw.cuh"
 #include "kernels.h"
 #include "launch.cuh"
 #include "p2p.cuh"
+#include "unpack_lut.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1244,38 +1246,6 @@ emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScr
   publish_when_grid_done(dst);
 }
 
-// out[idx] = 0 for every index of every payload: puts a dense buffer that only holds scattered
-// payload entries back to all zeros without a pass over the whole buffer.
-struct ClearSources {
-  const uint8_t* payload[kMaxWorld];
-  int64_t cap[kMaxWorld];
-};
-__global__ void __launch_bounds__(kThreads)
-clear_kernel(ClearSources src, float* __restrict__ out, int64_t n, const uint32_t* epoch_dev, int64_t parity_stride,
-             const int* guard) {
-  if (status_guarded(guard)) return;
-  const uint8_t* payload = src.payload[0];
-  int64_t cap = src.cap[0];
-#pragma unroll
-  for (int r = 1; r < kMaxWorld; ++r) {
-    if (r == int(blockIdx.y)) {
-      payload = src.payload[r];
-      cap = src.cap[r];
-    }
-  }
-  if (epoch_dev != nullptr && (*epoch_dev & 1u)) payload += parity_stride;
-  uint32_t total = 0;
-  for (int k = 0; k < 4; ++k) total |= uint32_t(payload[k]) << (8 * k);
-  if (total < 4 || int64_t(total) > cap) return;   // reported by the scatter kernel
-  const int64_t k = (int64_t(total) - 4) / 8;
-  const uint32_t* idx = reinterpret_cast<const uint32_t*>(payload + 4);
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < k; x += stride) {
-    const uint32_t i = idx[x];
-    if (int64_t(i) < n) out[i] = 0.0f;
-  }
-}
-
 // ================================================================ one-pass decode
 // All payloads into a dense tensor that is written from scratch: a CTA owns a tile of the tensor,
 // adds the payloads' entries of that range to a zeroed tile in shared memory, rank after rank, and
@@ -1349,25 +1319,21 @@ __device__ __forceinline__ uint32_t payload_entries(const uint8_t* payload, int6
   return 0;
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(kThreads, 6)
-dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int tile, float post_scale, int* status,
-                  unsigned int* redo) {
-  __shared__ __align__(16) float buf[kDenseTile];
+// The tile [lo, lo + len) of this CTA, decoded into buf (its float4s are whole).  False in the threads that
+// met an entry which the search put into the wrong tile.  Ends with a barrier.
+__device__ __forceinline__ bool decode_tile(const UnpackSources& src, int64_t n, int tile, int64_t lo, int len,
+                                            float post_scale, int* status, float* buf) {
   __shared__ uint32_t seg_begin[kMaxWorld], seg_end[kMaxWorld], entries[kMaxWorld];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t lo = int64_t(blockIdx.x) * tile;
-  const int len = int(lo + tile < n ? tile : n - lo);
   const bool first = blockIdx.x == 0, last = blockIdx.x == gridDim.x - 1;
-  let_next_start();
   bool bad = false;
   uint32_t k = 0;
   const uint32_t* idx = nullptr;
 #pragma unroll
   for (int r = 0; r < kMaxWorld; ++r) {   // compile-time index into src; one warp per rank
     if (r == warp && r < src.world) {
-      k = payload_entries(src.payload[r], src.payload_bytes[r], status, first && lane == 0);
-      idx = reinterpret_cast<const uint32_t*>(src.payload[r] + 4);
+      k = payload_entries(src.payload[r] + src.parity_off, src.payload_bytes[r], status, first && lane == 0);
+      idx = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
     }
   }
   for (int i = tid; i < (len + 3) / 4; i += kThreads) reinterpret_cast<float4*>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1397,7 +1363,7 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
     if (r < src.world) {
       const uint32_t e = seg_begin[r] + tid;
       if (e < seg_end[r]) {
-        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + 4);
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
         i0[r] = from[e];
         v0[r] = __uint_as_float(from[entries[r] + e]);
       }
@@ -1431,7 +1397,7 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
 #pragma unroll
     for (int r = 0; r < kMaxWorld; ++r) {
       if (r < src.world) {
-        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + 4);
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
         const uint32_t total = entries[r], end = seg_end[r];
         uint32_t e = seg_begin[r] + tid;
         if (e < end) add_entry(i0[r], v0[r]);
@@ -1452,7 +1418,19 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
       }
     }
   }
-  if (bad) *redo = 1u;
+  return !bad;
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads, 6)
+dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int tile, float post_scale, int* status,
+                  unsigned int* redo) {
+  __shared__ __align__(16) float buf[kDenseTile];
+  let_next_start();
+  const int tid = threadIdx.x;
+  const int64_t lo = int64_t(blockIdx.x) * tile;
+  const int len = int(lo + tile < n ? tile : n - lo);
+  if (!decode_tile(src, n, tile, lo, len, post_scale, status, buf)) *redo = 1u;
   float* o = out + lo;
   if (VEC) {
     for (int i = tid; i < (len >> 2); i += kThreads) reinterpret_cast<float4*>(o)[i] = reinterpret_cast<const float4*>(buf)[i];
@@ -1460,6 +1438,63 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
     if (i < len) o[i] = buf[i];
   } else {
     for (int i = tid; i < len; i += kThreads) o[i] = buf[i];
+  }
+}
+
+// ---- decode and optimizer step in one pass
+// When nobody keeps the dense gradient, the tile goes straight into the update of its parameters: the
+// gradient is neither written nor read (4 of AdamW's 28 bytes per element) nor cleared afterwards, and
+// one pass takes the place of a scatter per rank, the dense update and the clearing pass:
+// a BERT-large step (11 buckets, 335 M parameters, one GPU): 19.93 ms with the scatter, the dense
+// update and the clearing pass, 19.66 ms now.
+// An update cannot be taken back, so the payloads are looked at first: sparse_check_kernel records any
+// index that does not ascend or lies outside, and the update kernel returns on a recorded failure, as the
+// dense ones do.  OPT: 0 = SGD with momentum, 1 = AdamW.
+__global__ void __launch_bounds__(kThreads)
+sparse_check_kernel(UnpackSources src, int64_t n, int* status) {
+  let_next_start();
+  if (status_guarded(src.guard)) return;
+  resolve_epoch(src);
+  const int r = blockIdx.y;
+  const uint8_t* payload = select_payload(src, r) + src.parity_off;
+  const uint32_t k = payload_entries(payload, select_payload_bytes(src, r), status, threadIdx.x == 0);
+  const uint32_t* idx = reinterpret_cast<const uint32_t*>(payload + 4);
+  bool bad = false;
+  for (uint32_t e = blockIdx.x * kThreads + threadIdx.x; e < k; e += gridDim.x * kThreads) {
+    const uint32_t i = idx[e];
+    bad = bad || int64_t(i) >= n || (e > 0 && idx[e - 1] >= i);
+  }
+  if (bad) atomicExch(status, int(kPayloadBounds));
+}
+
+template <int OPT>
+__global__ void __launch_bounds__(kThreads, 4)
+sparse_apply_kernel(UnpackSources src, int64_t n, int tile, float post_scale, SgdApply sgd, AdamWApply adamw, int vec,
+                    const int* guard, int* status) {
+  __shared__ __align__(16) float buf[kDenseTile];
+  wait_for_previous();
+  if (status_guarded(guard)) return;
+  resolve_epoch(src);
+  float bc1 = 0.f, rsqrt_bc2 = 0.f;
+  if (OPT == 1) adamw_bias(adamw, bc1, rsqrt_bc2);
+  const int tid = threadIdx.x;
+  const int64_t lo = int64_t(blockIdx.x) * tile;
+  const int len = int(lo + tile < n ? tile : n - lo);
+  decode_tile(src, n, tile, lo, len, post_scale, status, buf);
+  const int quads = vec ? len >> 2 : 0;
+#pragma unroll 2
+  for (int i = tid; i < quads; i += kThreads) {
+    const float4 g = reinterpret_cast<const float4*>(buf)[i];
+    if (OPT == 1) {
+      adamw_four(adamw, bc1, rsqrt_bc2, (lo >> 2) + i, g);
+    } else {
+      const float g4[4] = {g.x, g.y, g.z, g.w};
+      sgd_update4(sgd, lo + 4 * i, g4);
+    }
+  }
+  for (int i = 4 * quads + tid; i < len; i += kThreads) {
+    if (OPT == 1) adamw_at(adamw, bc1, rsqrt_bc2, lo + i, buf[i]);
+    else sgd_update(sgd, lo + i, buf[i]);
   }
 }
 
@@ -1662,21 +1697,41 @@ cudaError_t sparse_read_stats(const void* scratch, unsigned int* host4, cudaStre
   return e;
 }
 
-cudaError_t sparse_clear(const UnpackSources& src, float* out, int64_t n, cudaStream_t stream) {
-  if (n <= 0 || src.world < 1 || src.world > kMaxWorld) return cudaErrorInvalidValue;
-  ClearSources cs{};
+namespace {
+// Tiles of 8,192 elements, smaller ones while they would not cover every SM four times.
+inline int64_t dense_tile_for(int64_t n) {
+  const int64_t tile = (n / (148 * 4) + 1023) / 1024 * 1024;
+  return std::min<int64_t>(std::max<int64_t>(tile, 1024), kDenseTile);
+}
+}  // namespace
+
+cudaError_t sparse_apply(const UnpackSources& src, int64_t n, float post_scale, const SgdApply* sgd,
+                         const AdamWApply* adamw, int* status, cudaStream_t stream) {
+  if (n <= 0 || n > 0x7fffffff || src.world < 1 || src.world > kMaxWorld || status == nullptr ||
+      (sgd != nullptr) == (adamw != nullptr))
+    return cudaErrorInvalidValue;
   int64_t kmax = 1;
   for (int r = 0; r < src.world; ++r) {
-    if (reinterpret_cast<uintptr_t>(src.payload[r]) & 3) return cudaErrorInvalidValue;
-    cs.payload[r] = src.payload[r];
-    cs.cap[r] = src.payload_bytes[r];
+    if ((reinterpret_cast<uintptr_t>(src.payload[r]) | uintptr_t(src.parity_stride)) & 3) return cudaErrorInvalidValue;
     kmax = std::max<int64_t>(kmax, (src.payload_bytes[r] - 4) / 8);
   }
-  int64_t blocks = (kmax + kThreads - 1) / kThreads;
-  if (blocks > 148 * 2) blocks = 148 * 2;
-  clear_kernel<<<dim3(unsigned(blocks), unsigned(src.world), 1), kThreads, 0, stream>>>(cs, out, n, src.epoch_dev,
-                                                                                          src.parity_stride, src.guard);
-  return cudaGetLastError();
+  const int64_t check_blocks = std::min<int64_t>((kmax + kThreads - 1) / kThreads, 148);
+  sparse_check_kernel<<<dim3(unsigned(check_blocks), unsigned(src.world)), kThreads, 0, stream>>>(src, n, status);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  const int64_t tile = dense_tile_for(n);
+  const dim3 grid = dim3(unsigned((n + tile - 1) / tile)), block(kThreads);
+  if (adamw != nullptr) {
+    if (!adamw->param || !adamw->exp_avg || !adamw->exp_avg_sq || adamw->step < 1) return cudaErrorInvalidValue;
+    const int vec = al(adamw->param) && al(adamw->exp_avg) && al(adamw->exp_avg_sq) ? 1 : 0;
+    return launch_after(sparse_apply_kernel<1>, grid, block, 0, stream, src, n, int(tile), post_scale, SgdApply{}, *adamw, vec,
+                        static_cast<const int*>(status), status);
+  }
+  if (!sgd->param || !sgd->momentum) return cudaErrorInvalidValue;
+  const int vec = al(sgd->param) && al(sgd->momentum) ? 1 : 0;
+  return launch_after(sparse_apply_kernel<0>, grid, block, 0, stream, src, n, int(tile), post_scale, *sgd, AdamWApply{}, vec,
+                      static_cast<const int*>(status), status);
 }
 
 cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
@@ -1685,9 +1740,7 @@ cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n,
   if (!add && redo != nullptr && n <= 0x7fffffff && src.epoch_dev == nullptr && src.guard == nullptr) {
     for (int r = 0; r < src.world; ++r)
       if (reinterpret_cast<uintptr_t>(src.payload[r]) & 3) return cudaErrorInvalidValue;
-    // tiles of 8,192 elements, smaller ones while they would not cover every SM four times
-    int64_t tile = (n / (148 * 4) + 1023) / 1024 * 1024;
-    tile = std::min<int64_t>(std::max<int64_t>(tile, 1024), kDenseTile);
+    const int64_t tile = dense_tile_for(n);
     const unsigned blocks = unsigned((n + tile - 1) / tile);
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     if (vec) dense_tile_kernel<true><<<blocks, kThreads, 0, stream>>>(src, out, n, int(tile), post_scale, status, redo);

@@ -383,7 +383,7 @@ cuda::SgdApply DdpEngine::sgd_apply_for(int b) const {
   return apply;
 }
 
-void DdpEngine::issue_adamw(int b, cudaStream_t stream, int clear_grad) {
+cuda::AdamWApply DdpEngine::adamw_apply_for(int b, int clear_grad) const {
   if (!param_ || !momentum_ || !second_) throw std::runtime_error("AdamW needs param and both moment buffers");
   const BucketDesc& B = buckets_[static_cast<size_t>(b)];
   cuda::AdamWApply aw;
@@ -397,9 +397,15 @@ void DdpEngine::issue_adamw(int b, cudaStream_t stream, int clear_grad) {
   aw.weight_decay = wd_;
   aw.step = int(steps_) + 1;
   aw.step_dev = epoch_dev_;   // one epoch per step: the device counter is the 1-based step count
-  aw.clear_grad = clear_grad < 0 ? cfg_.clear_grad : clear_grad;
+  aw.clear_grad = clear_grad;
   aw.guard = status_;
-  check(cuda::adamw_apply_dense(grad_ + B.offset, 1.0f, aw, B.numel, stream), "adamw_apply_dense");
+  return aw;
+}
+
+void DdpEngine::issue_adamw(int b, cudaStream_t stream) {
+  const BucketDesc& B = buckets_[static_cast<size_t>(b)];
+  check(cuda::adamw_apply_dense(grad_ + B.offset, 1.0f, adamw_apply_for(b, cfg_.clear_grad), B.numel, stream),
+        "adamw_apply_dense");
 }
 
 // Phase 1: every shard of the bucket is compressed as a payload of its own and stored into the
@@ -711,6 +717,19 @@ void DdpEngine::issue_recv(int b, int worker) {
       launched += 1;
       break;
     case Codec::kSparse:
+      if (cfg_.clear_grad && (fused_sgd_ || adamw_)) {
+        // nobody keeps the dense gradient: decode and update in one pass (the compressor left zeros in
+        // the bucket, ready for the next backward pass)
+        if (adamw_) {
+          const cuda::AdamWApply aw = adamw_apply_for(b, 0);
+          check(cuda::sparse_apply(src, n, post, nullptr, &aw, status_, w.recv), "sparse_apply");
+        } else {
+          check(cuda::sparse_apply(src, n, post, &apply, nullptr, status_, w.recv), "sparse_apply");
+        }
+        applied = true;
+        launched += 2;
+        break;
+      }
       // the compressor left zeros in the bucket: the payloads are added onto them
       check(cuda::sparse_unpack_accum(src, g, n, 1, post, status_, w.recv), "sparse_unpack");
       launched += cfg_.world;
@@ -731,22 +750,12 @@ void DdpEngine::issue_recv(int b, int worker) {
       break;
     }
   }
-  // Sparse codecs: the dense gradient holds the scattered payload entries and zeros.  Instead of
-  // letting the optimizer kernel write zeros over all of it again, only the scattered positions
-  // are cleared afterwards.
-  const bool sparse_clear = cfg_.codec == Codec::kSparse && cfg_.clear_grad && (fused_sgd_ || adamw_);
   if (fused_sgd_ && !applied) {
-    cuda::SgdApply dense = apply;
-    if (sparse_clear) dense.clear_grad = 0;
-    check(cuda::sgd_apply_dense(g, 1.0f, dense, n, w.recv), "sgd_apply_dense");
+    check(cuda::sgd_apply_dense(g, 1.0f, apply, n, w.recv), "sgd_apply_dense");
     launched += 1;
   }
-  if (adamw_) {
-    issue_adamw(b, w.recv, sparse_clear ? 0 : cfg_.clear_grad);
-    launched += 1;
-  }
-  if (sparse_clear) {
-    check(cuda::sparse_clear(src, g, n, w.recv), "sparse_clear");
+  if (adamw_ && !applied) {
+    issue_adamw(b, w.recv);
     launched += 1;
   }
   stamp(b, kStampDone, w.recv);

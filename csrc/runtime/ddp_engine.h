@@ -200,7 +200,8 @@ class DdpEngine {
   enum Stamp : int { kStampReady = 0, kStampPushed = 1, kStampArrived = 2, kStampDone = 3, kStampCount = 4 };
   void stamp(int b, int which, cudaStream_t stream);
   cuda::SgdApply sgd_apply_for(int b) const;
-  void issue_adamw(int b, cudaStream_t stream, int clear_grad = -1);  // -1: as configured
+  cuda::AdamWApply adamw_apply_for(int b, int clear_grad) const;
+  void issue_adamw(int b, cudaStream_t stream);
   void issue_bucket(int b, int worker);
   void issue_push(int b, int worker);
   void issue_recv(int b, int worker);

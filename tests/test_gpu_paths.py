@@ -262,3 +262,50 @@ def test_powersgd_encode1_one_pass(n, m, r, short):
     ref = want.view(n, m).double() @ Q.double()
     # fp32 products and sums of m terms: sqrt(m) roundings of 2^-24 each, and a wide margin
     assert (P.cpu().double() - ref).norm() <= 4 * m ** 0.5 * 2 ** -24 * (want.norm() * Q.norm()).double()
+
+
+# ----------------------------------------------------------------------------- sparse decode and update in one pass
+@pytest.mark.parametrize("opt", ["sgd", "adamw"])
+@pytest.mark.parametrize("world,n", [(1, 70001), (3, 8192 * 2), (8, 100003)])
+@pytest.mark.parametrize("device_epoch", [0, 1])
+def test_sparse_update_pass_equals_scatter_and_dense_update(opt, world, n, device_epoch):
+    """clear_grad=1 (nobody keeps the gradient) decodes straight into the update; clear_grad=0 scatters first."""
+    import hipress_b200 as hp
+    from hipress_b200.parallel import SymmetricMemory
+    results = []
+    for clear in (0, 1):
+        kw = dict(device_epoch=1, num_workers=0) if device_epoch else {}
+        engines = [hp._C.DdpEngine(dict(rank=r, world=world, device=0, codec="graddrop", seed=3, flag_timeout_s=2.0,
+                                        defer_recv=1, keep_fraction=0.01, sample_rate=0.05, clear_grad=clear, **kw),
+                                   [(0, n, 1)], [0]) for r in range(world)]
+        mems = SymmetricMemory.emulate(engines[0].symmetric_bytes, world)
+        state = []
+        for r, (e, m) in enumerate(zip(engines, mems)):
+            bufs = [gauss(n, seed=10 + r).cuda(), torch.zeros(n, device="cuda"), gauss(n, 1.0, seed=5).cuda(),
+                    torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")]
+            e.set_buffers(bufs[0], bufs[1], bufs[2], bufs[3], None, bufs[4])
+            e.set_symmetric(m.buf)
+            if opt == "adamw":
+                e.set_adamw(0.1, 0.9, 0.999, 1e-8, 0.01)
+            else:
+                e.set_sgd(0.1, 0.9, 0.01, True)
+            state.append(bufs)
+        for step in range(3):
+            for e in engines:
+                e.begin_step()
+            for e in engines:
+                e.bucket_ready(0, 0)
+            for e in engines:
+                e.drain()
+            torch.cuda.synchronize()
+            for e in engines:
+                e.finish_step(0)
+            torch.cuda.synchronize()
+            for r, e in enumerate(engines):
+                assert e.check_status() == 0
+                if clear:
+                    assert float(state[r][0].abs().max()) == 0.0
+                state[r][0].copy_(gauss(n, seed=100 * (step + 1) + r))
+        results.append([t.cpu() for bufs in state for t in bufs[1:]])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
