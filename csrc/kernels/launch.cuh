@@ -24,6 +24,22 @@ __device__ __forceinline__ T* after_wait(T* p) {
   return p;
 }
 
+// A kernel whose CTAs wait for one another: all of them are resident at once, or the launch fails.
+template <typename... Params, typename... Args>
+cudaError_t launch_resident(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // overlap: start while the kernel before is still running.  cluster: CTAs per cluster (1: none).
 template <typename... Params, typename... Args>
 cudaError_t launch_with(bool overlap, int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,

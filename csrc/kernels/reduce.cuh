@@ -17,7 +17,7 @@ constexpr int kReduceMaxBlocks = 1024;
 
 struct MinMaxScratch {
   unsigned int counter;  // zero between launches
-  unsigned int pad;
+  unsigned int left;     // zero between launches
   float mn, mx;    // result
   float inv, gap;  // compress-side scale and decode-side step
   float partial_min[kReduceMaxBlocks];
@@ -55,6 +55,48 @@ __device__ __forceinline__ void block_minmax(float& mn, float& mx) {
     mx = warp_max(mx);
   }
   __syncthreads();
+}
+
+// Extremes over a grid whose CTAs are all resident (launch_resident): every thread of every CTA gets them.
+// The wait is bounded; false when it ran out (a CTA that is resident arrives, so it does not).
+template <int THREADS>
+__device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, float& mx) {
+  __shared__ float res[2];
+  __shared__ bool arrived;
+  block_minmax<THREADS>(mn, mx);
+  if (threadIdx.x == 0) {
+    s->partial_min[blockIdx.x] = mn;
+    s->partial_max[blockIdx.x] = mx;
+    __threadfence();
+    atomicAdd(&s->counter, 1u);
+    arrived = false;
+    for (unsigned int i = 0; i < 40000000u && !arrived; ++i)   // seconds
+      arrived = *reinterpret_cast<volatile unsigned int*>(&s->counter) >= gridDim.x;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!arrived) return false;
+  mn = INFINITY;
+  mx = -INFINITY;
+  for (int i = threadIdx.x; i < int(gridDim.x); i += THREADS) {
+    mn = fminf(mn, __ldcg(&s->partial_min[i]));
+    mx = fmaxf(mx, __ldcg(&s->partial_max[i]));
+  }
+  block_minmax<THREADS>(mn, mx);
+  if (threadIdx.x == 0) {
+    res[0] = mn;
+    res[1] = mx;
+    // the last CTA to have read the partials makes the counters ready for the next launch
+    __threadfence();
+    if (atomicAdd(&s->left, 1u) == gridDim.x - 1) {
+      s->counter = 0u;
+      s->left = 0u;
+    }
+  }
+  __syncthreads();
+  mn = res[0];
+  mx = res[1];
+  return true;
 }
 
 // Returns true in every thread of exactly one CTA: the last to arrive.  Before

@@ -485,6 +485,118 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
   publish_when_grid_done(dst);
 }
 
+// Medium tensors: both passes in one launch that reads the inputs once.  One CTA per SM keeps its part of
+// grad + residual in shared memory (up to 208 KB of it: 30 MB over the chip), the CTAs exchange their
+// extremes through the scratch, and quantise from shared memory.  The two-launch form reads both arrays
+// twice, the second time from L2, and drains and refills the chip in between.  All CTAs have to be resident
+// at once, so this form is for calls that have the GPU to themselves: the exchange engine, whose compressors
+// run beside the backward pass, keeps the two launches.
+// 25 MB with error feedback, 2 bits (ncu, cold): 14.3 + 18.0 us in two launches, 21.6 in one; with the
+// decode of eight payloads 63.4 and 55.4 us, and 9.4 MB at 4 bits 18.4 and 14.4 us.
+constexpr int kHoldThreads = 1024;
+constexpr size_t kHoldBytes = 208 * 1024;    // of grad + residual per CTA
+template <int BW> struct HoldForm {
+  static constexpr int kDpb = 8 / BW;
+  static constexpr int kUnit = Unit<BW>::EPT;
+  // a CTA's part: a multiple of 512 elements, so that the parts' payload bytes start equally far past a
+  // 16-byte boundary (64 bytes at 1 bit) and its units are whole
+  static constexpr int kGrain = 512;
+  static constexpr size_t stage_bytes(int64_t part) { return size_t(part / kDpb) + 32; }
+};
+template <int BW, bool EF>
+__global__ void __launch_bounds__(kHoldThreads, 1)
+tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int64_t part, int random,
+                 uint64_t seed, PushTargets dst, MinMaxScratch* scratch, int shift) {
+  constexpr int DPB = 8 / BW, EPT = Unit<BW>::EPT, BPT = Unit<BW>::BPT;
+  extern __shared__ __align__(16) float hold[];           // [part], then the payload bytes
+  __shared__ float scale[3];
+  uint8_t* const bytes_at = reinterpret_cast<uint8_t*>(hold + part);
+  const int tid = threadIdx.x;
+  const int64_t begin = int64_t(blockIdx.x) * part;       // a multiple of 512
+  const int64_t left = n - begin;
+  const int len = int(left < 0 ? 0 : (left < part ? left : part));
+  const float4* g4 = reinterpret_cast<const float4*>(grad + begin);
+  const float4* r4 = EF ? reinterpret_cast<const float4*>(residual + begin) : nullptr;
+  float mn = INFINITY, mx = -INFINITY;
+  const int quads = len >> 2;
+  auto take = [&](int i, float4 g, float4 r) {
+    if (EF) {
+      g.x = hp_add(g.x, r.x); g.y = hp_add(g.y, r.y);
+      g.z = hp_add(g.z, r.z); g.w = hp_add(g.w, r.w);
+    }
+    mn = fminf(mn, fminf(fminf(g.x, g.y), fminf(g.z, g.w)));
+    mx = fmaxf(mx, fmaxf(fmaxf(g.x, g.y), fmaxf(g.z, g.w)));
+    reinterpret_cast<float4*>(hold)[i] = g;
+  };
+  int q = tid;
+  for (; q + 3 * kHoldThreads < quads; q += 4 * kHoldThreads) {
+    float4 g[4], r[4] = {};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      g[u] = __ldg(g4 + q + u * kHoldThreads);
+      if (EF) r[u] = r4[q + u * kHoldThreads];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) take(q + u * kHoldThreads, g[u], r[u]);
+  }
+  for (; q < quads; q += kHoldThreads) take(q, __ldg(g4 + q), EF ? r4[q] : make_float4(0.f, 0.f, 0.f, 0.f));
+  for (int e = 4 * quads + tid; e < len; e += kHoldThreads) {   // fewer than four
+    const float v = EF ? hp_add(grad[begin + e], residual[begin + e]) : grad[begin + e];
+    mn = fminf(mn, v);
+    mx = fmaxf(mx, v);
+  }
+  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx)) return;
+  const PushCursor cur{nullptr};
+  if (tid == 0) {
+    const float gap = tern_gap(mn, mx, BW);
+    scale[0] = gap;
+    scale[1] = tern_gap_inverse(gap);
+    if (blockIdx.x == 0) put_header(dst, cur, n, BW, mn, mx);
+  }
+  __syncthreads();
+  const float gap = scale[0], inv = scale[1];
+  const int64_t byte0 = begin / DPB;                       // first payload byte of the part
+  const int units = len / EPT;
+  for (int u = tid; u < units; u += kHoldThreads) {
+    float x[EPT], ef[EPT];
+#pragma unroll
+    for (int v = 0; v < EPT / 4; ++v) {
+      const float4 h = reinterpret_cast<const float4*>(hold)[u * (EPT / 4) + v];
+      x[4 * v] = h.x; x[4 * v + 1] = h.y; x[4 * v + 2] = h.z; x[4 * v + 3] = h.w;
+    }
+    const uint32_t b = tern_quant_unit<BW, EF>(x, byte0 + int64_t(u) * BPT, mn, inv, gap, random, seed, ef);
+    if (EF) {
+#pragma unroll
+      for (int v = 0; v < EPT / 4; ++v)
+        reinterpret_cast<float4*>(residual + begin)[u * (EPT / 4) + v] =
+            make_float4(ef[4 * v], ef[4 * v + 1], ef[4 * v + 2], ef[4 * v + 3]);
+    }
+    uint8_t* at = bytes_at + shift + u * BPT;              // shift is even
+    if (BPT == 1) {
+      *at = uint8_t(b);
+    } else {
+#pragma unroll
+      for (int h = 0; h < BPT / 2; ++h) reinterpret_cast<uint16_t*>(at)[h] = uint16_t(b >> (16 * h));
+    }
+  }
+  __syncthreads();
+  // the part's bytes: 16-byte words of the destination, the first and the last one by bytes
+  const int count = units * BPT;
+  const int words = (shift + count) >> 4;                  // words that end inside the part
+  for (int w = tid + (shift != 0 ? 1 : 0); w < words; w += kHoldThreads)
+    put_u128(dst, cur, kTernHeaderBytes + byte0 - shift + 16 * w, reinterpret_cast<const uint4*>(bytes_at)[w]);
+  const int head_end = shift == 0 ? 0 : (16 < shift + count ? 16 : shift + count);
+  const int tail_begin = words * 16 > head_end ? words * 16 : head_end;
+  if (tid < 16) {
+    if (tid >= shift && tid < head_end) put_u8(dst, cur, kTernHeaderBytes + byte0 - shift + tid, bytes_at[tid]);
+  } else if (tid < 32) {
+    const int at = tail_begin + tid - 16;
+    if (at >= shift && at < shift + count) put_u8(dst, cur, kTernHeaderBytes + byte0 - shift + at, bytes_at[at]);
+  } else if (tid == 32 && len > 0 && units * EPT < len) {
+    tern_leftover<BW, EF>(grad, residual, begin + int64_t(units) * EPT, n, mn, inv, gap, random, seed, dst, cur);
+  }
+}
+
 struct TernHeader {
   float mn, gap;
   int bw, ok;
@@ -724,6 +836,42 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
     LAUNCH_BITS(LAUNCH_SMALL);
 #undef LAUNCH_SMALL
     return cudaGetLastError();
+  }
+  // one read of the inputs (see tern_hold_kernel): a destination of this call's own, 16-byte aligned
+  // inputs, and a part per SM that fits its shared memory
+  if (S == 0 && vec && shift >= 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
+      dst.epoch_dev == nullptr && dst.remote == 0 && dst.mc == nullptr) {
+    int device = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    if (sms > kReduceMaxBlocks) sms = kReduceMaxBlocks;
+    const int64_t part = ((n + sms - 1) / sms + 511) / 512 * 512;
+    if (part * int64_t(sizeof(float)) <= int64_t(kHoldBytes)) {
+      const unsigned ctas = unsigned((n + part - 1) / part);
+#define LAUNCH_HOLD_AS(BW, E)                                                                                     \
+  do {                                                                                                            \
+    const size_t smem = size_t(part) * sizeof(float) + HoldForm<BW>::stage_bytes(part);                           \
+    if (smem <= 224 * 1024) {                                                                                     \
+      e = cudaFuncSetAttribute(tern_hold_kernel<BW, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));  \
+      if (e != cudaSuccess) return e;                                                                             \
+      e = launch_resident(tern_hold_kernel<BW, E>, dim3(ctas), dim3(kHoldThreads), smem, stream, grad, residual,  \
+                          n, part, enable_random, seed, dst, s, shift);                                           \
+      if (e != cudaErrorCooperativeLaunchTooLarge) return e;                                                      \
+      cudaGetLastError();   /* fewer SMs than the device has: the two launches below */                           \
+    }                                                                                                             \
+  } while (0)
+#define LAUNCH_HOLD(BW) \
+  if (ef) LAUNCH_HOLD_AS(BW, true); else LAUNCH_HOLD_AS(BW, false)
+      switch (bitwidth) {
+        case 1: LAUNCH_HOLD(1); break;
+        case 2: LAUNCH_HOLD(2); break;
+        case 4: LAUNCH_HOLD(4); break;
+        default: LAUNCH_HOLD(8); break;
+      }
+#undef LAUNCH_HOLD
+#undef LAUNCH_HOLD_AS
+    }
   }
   const int shards = S > 0 ? int((n + S - 1) / S) : 1;
   PushTargets hdr_dst = dst;

@@ -264,6 +264,61 @@ def test_powersgd_encode1_one_pass(n, m, r, short):
     assert (P.cpu().double() - ref).norm() <= 4 * m ** 0.5 * 2 ** -24 * (want.norm() * Q.norm()).double()
 
 
+# ----------------------------------------------------------------------------- one launch, inputs read once
+@pytest.mark.parametrize("bw", [1, 2, 4, 8])
+@pytest.mark.parametrize("feedback", [False, True])
+@pytest.mark.parametrize("offset", [0, 6])
+def test_terngrad_resident_form(bw, feedback, offset):
+    """Ragged last parts (148 parts of a multiple of 512 elements), the largest part and one element beyond it."""
+    largest = 148 * 208 * 256
+    for n in (131073, 148 * 1024 - 1, 148 * 1024 + 1, 2359807) + ((largest, largest + 1) if bw == 2 else ()):
+        g, r = gauss(n, seed=n), gauss(n, 0.004, seed=n + 1)
+        rc = r.clone() if feedback else None
+        rg = r.cuda() if feedback else None
+        ref = ops.terngrad_compress(g, bw, True, seed=7, residual=rc)
+        out = torch.zeros(ref.numel() + offset + 64, dtype=torch.uint8, device="cuda")
+        dev_g = g.cuda()
+        for _ in range(2):      # back to back: the shared state is left ready
+            if feedback:
+                rg.copy_(r)
+            ops.terngrad_compress(dev_g, bw, True, seed=7, residual=rg, out=out[offset:offset + ref.numel()])
+        assert torch.equal(out[offset:offset + ref.numel()].cpu(), ref), n
+        assert int(out[offset + ref.numel():].sum()) == 0, n
+        if feedback:
+            assert torch.equal(rg.cpu(), rc), n
+
+
+@pytest.mark.parametrize("n", [4096, 300007])
+def test_terngrad_one_launch_forms_under_capture(n):
+    g = gauss(n, seed=1).cuda()
+    want = ops.terngrad_compress(g, 2, True, seed=5)
+    out = torch.zeros_like(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.terngrad_compress(g, 2, True, seed=5, out=out)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, want)
+
+
+def test_terngrad_resident_form_on_two_streams():
+    n = 3000001
+    g = [gauss(n, seed=s).cuda() for s in range(2)]
+    want = [ops.terngrad_compress(x, 2, True, seed=5) for x in g]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[torch.zeros_like(w) for _ in range(20)] for w in want]
+    torch.cuda.synchronize()
+    for i in range(20):
+        for s in range(2):
+            with torch.cuda.stream(streams[s]):
+                ops.terngrad_compress(g[s], 2, True, seed=5, out=outs[s][i])
+    torch.cuda.synchronize()
+    for s in range(2):
+        for o in outs[s]:
+            assert torch.equal(o, want[s])
+
+
 # ----------------------------------------------------------------------------- sparse decode and update in one pass
 @pytest.mark.parametrize("opt", ["sgd", "adamw"])
 @pytest.mark.parametrize("world,n", [(1, 70001), (3, 8192 * 2), (8, 100003)])
