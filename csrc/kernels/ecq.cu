@@ -320,7 +320,7 @@ ecq_unpack_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add
 // The byte loop above costs one scalar load per rank and one scalar store per element:
 // 4 bits, four payloads, 25 MB (ncu, cold): 34.9 us before, 14.0 now.
 template <int WORLD>
-__global__ void __launch_bounds__(kIndexThreads, WORLD > 4 ? 2 : 3)
+__global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 ecq_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, float post_scale, int* status, int align) {
   if (status_guarded(src.guard)) return;
   resolve_epoch(src);
@@ -365,8 +365,8 @@ cudaError_t launch_ecq_index(const UnpackSources& src, float* out, int64_t n, fl
     if (e != cudaSuccess) return e;
   }
   // sized by the smallest chunk (4 bits); at 8 bits the loop strides over what there is
-  const int grid = index_grid(n, IndexForm<4>::kChunk, smem);
-  ecq_unpack_index_kernel<WORLD><<<grid, kIndexThreads, smem, stream>>>(src, out, n, post_scale, status,
+  const int grid = index_grid(n, IndexForm<4>::kChunk, WORLD, smem);
+  ecq_unpack_index_kernel<WORLD><<<grid, index_threads(WORLD), smem, stream>>>(src, out, n, post_scale, status,
                                                                         payload_alignment(src, kEcqHeaderBytes));
   return cudaGetLastError();
 }

@@ -1446,7 +1446,7 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
 // gradient is neither written nor read (4 of AdamW's 28 bytes per element) nor cleared afterwards, and
 // one pass takes the place of a scatter per rank, the dense update and the clearing pass:
 // a BERT-large step (11 buckets, 335 M parameters, one GPU): 19.93 ms with the scatter, the dense
-// update and the clearing pass, 19.66 ms now.
+// update and the clearing pass, 19.66 in one pass.
 // An update cannot be taken back, so the payloads are looked at first: sparse_check_kernel records any
 // index that does not ascend or lies outside, and the update kernel returns on a recorded failure, as the
 // dense ones do.  OPT: 0 = SGD with momentum, 1 = AdamW.

@@ -148,7 +148,7 @@ tbq_compress_kernel(const float* __restrict__ grad, float* __restrict__ residual
 
 // Aligned dense arrays: one index table shared by all groups of four ranks (see unpack_lut.cuh).
 template <bool APPLY, int WORLD>
-__global__ void __launch_bounds__(kIndexThreads, WORLD > 4 ? 2 : 3)
+__global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 tbq_unpack_index_kernel(UnpackSources src, float thr, float* __restrict__ out, int64_t n, int add, float post_scale,
                         SgdApply apply, int align) {
   if (unpack_guarded(src)) return;
@@ -187,8 +187,8 @@ cudaError_t launch_tbq_index(const UnpackSources& src, float thr, float* out, in
                              const SgdApply& apply, cudaStream_t stream) {
   using L = IndexLayout<2, WORLD, true, false>;
   static_assert(L::kBytes <= 48 * 1024, "fits the default shared-memory limit");
-  const int grid = index_grid(n, IndexForm<2>::kChunk, L::kBytes);
-  tbq_unpack_index_kernel<APPLY, WORLD><<<grid, kIndexThreads, L::kBytes, stream>>>(
+  const int grid = index_grid(n, IndexForm<2>::kChunk, WORLD, L::kBytes);
+  tbq_unpack_index_kernel<APPLY, WORLD><<<grid, index_threads(WORLD), L::kBytes, stream>>>(
       src, thr, out, n, add, post_scale, apply, payload_alignment(src, 0));
   return cudaGetLastError();
 }

@@ -656,7 +656,7 @@ __device__ __forceinline__ bool read_headers(const UnpackSources& src, int64_t n
 
 // Known bitwidth and 16-byte aligned dense arrays: index tables, or arithmetic at 8 bits.
 template <int BW, bool APPLY, int WORLD>
-__global__ void __launch_bounds__(kIndexThreads, WORLD > 4 ? 2 : 3)
+__global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 tern_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add, float post_scale, SgdApply apply,
                          int* status, int align) {
   if (unpack_guarded(src)) return;
@@ -746,19 +746,19 @@ template <int BW, bool APPLY, int WORLD>
 cudaError_t launch_tern_index(const UnpackSources& src, float* out, int64_t n, int add, float post_scale,
                               const SgdApply& apply, int* status, cudaStream_t stream) {
   const int align = payload_alignment(src, kTernHeaderBytes);
-  int grid = grid_for((n + 3) >> 2, kIndexThreads, 148 * 8);
+  int grid = grid_for((n + 3) >> 2, index_threads(WORLD), 148 * 8);
   size_t smem = 0;
   if constexpr (BW != 8) {
     using L = IndexLayout<BW, WORLD, false, false>;
     smem = L::kBytes;
-    grid = index_grid(n, IndexForm<BW>::kChunk, smem);
+    grid = index_grid(n, IndexForm<BW>::kChunk, WORLD, smem);
     if (smem > 40 * 1024) {   // with the static part, past the default limit; per device, and cheap: set on every launch rather than remembered per process
       const cudaError_t e = cudaFuncSetAttribute(tern_unpack_index_kernel<BW, APPLY, WORLD>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
       if (e != cudaSuccess) return e;
     }
   }
-  tern_unpack_index_kernel<BW, APPLY, WORLD><<<grid, kIndexThreads, smem, stream>>>(src, out, n, add, post_scale, apply,
+  tern_unpack_index_kernel<BW, APPLY, WORLD><<<grid, index_threads(WORLD), smem, stream>>>(src, out, n, add, post_scale, apply,
                                                                                   status, align);
   return cudaGetLastError();
 }

@@ -305,9 +305,14 @@ __device__ __forceinline__ void unpack_nibble_body(const float* lut, uint32_t (&
 // its warp; the lanes read them back so that every dense access is a 512-byte run across the warp.
 // The form before this one read a table entry per pair of ranks and two elements, with bank conflicts,
 // and moved every index word by shuffle:
-// 4 bits, one payload, 2.4 M elements (ncu, cold): 15.8 us before, 6.9 now; 2 bits, eight payloads, 25 MB,
-// compress and decode together: 62.7 us before, 58 now.
-constexpr int kIndexThreads = 256;
+// 4 bits, one payload, 2.4 M elements (ncu, cold): 15.8 us before, 6.4 now; 2 bits, eight payloads, 25 MB: 26.6
+// and 17.3.
+// Threads per CTA and CTAs per SM.  Eight payloads' tables and index buffers take 80 KB: two CTAs of 512
+// threads that share them, because two of 256 leave four warps per scheduler, too few to cover the
+// shared-memory latency (25 MB, compress and decode: 51.2 us against 43.0).  With one group of ranks three
+// CTAs of 256 threads do.
+__host__ __device__ constexpr int index_threads(int world) { return world > 4 ? 512 : 256; }
+__host__ __device__ constexpr int index_ctas(int world) { return world > 4 ? 2 : 3; }
 
 template <int BW>
 struct IndexForm {
@@ -329,7 +334,7 @@ struct IndexLayout {
   static constexpr int kRows = SEQ ? kFull + (WORLD - kFirst) * (1 << BW)
                                    : (SHARED ? kFull : kFull * (kGroups - 1) + rows(kGroups - 1));
   static constexpr int kStage = 32 * F::kElems * kGroups;                    // bytes per warp
-  static constexpr size_t kBytes = size_t(kRows) * 128 + size_t(kIndexThreads / 32) * kStage;
+  static constexpr size_t kBytes = size_t(kRows) * 128 + size_t(index_threads(WORLD) / 32) * kStage;
 };
 
 // value(r, q): decoded value of level q of rank r.
@@ -599,12 +604,12 @@ inline int payload_alignment(const UnpackSources& src, int header_bytes) {
   for (int r = 0; r < src.world; ++r) bits |= reinterpret_cast<uintptr_t>(src.payload[r] + header_bytes);
   return (bits & 3) == 0 ? 4 : ((bits & 1) == 0 ? 2 : 1);
 }
-// Resident CTAs of an index-table kernel: by shared memory, and no more than three per SM by registers.
-inline int index_grid(int64_t n, int chunk, size_t smem_bytes) {
-  const int warps = kIndexThreads / 32;
+// Resident CTAs of an index-table kernel: by shared memory and by registers (index_ctas).
+inline int index_grid(int64_t n, int chunk, int world, size_t smem_bytes) {
+  const int warps = index_threads(world) / 32;
   int64_t blocks = (n / chunk + warps - 1) / warps;
   int per_sm = int((size_t(227) * 1024) / (smem_bytes + 1024));
-  per_sm = per_sm < 1 ? 1 : (per_sm > 3 ? 3 : per_sm);
+  per_sm = per_sm < 1 ? 1 : (per_sm > index_ctas(world) ? index_ctas(world) : per_sm);
   if (blocks > 148 * per_sm) blocks = 148 * per_sm;
   return blocks < 1 ? 1 : int(blocks);
 }
