@@ -17,8 +17,9 @@
 // sit in registers, and four rows are in flight per thread.  The two reductions store one
 // partial result per CTA and channel; a small finalize kernel (32 channels per CTA, 32 warps
 // striding over the partials, added in a fixed order, so results are deterministic) combines
-// them -- the squares about the mean of the whole batch, so no precision is lost to
-// E[x^2] - E[x]^2 -- and writes the coefficients the elementwise kernel needs.  The three kernels of
+// them -- the variance with Chan's parallel update, so no precision is lost to
+// E[x^2] - E[x]^2 over the whole batch -- and writes the coefficients the elementwise kernel
+// needs.  The three kernels of
 // a direction overlap at their ends (launch.cuh).  (A first version let the last CTA to finish combine all partials: one thread per
 // channel walking ~1,200 partials in sequence took 6x longer than reading the activations.)
 //
@@ -81,27 +82,36 @@ bn_stats_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int C, int tx_co
 constexpr int kFinChannels = 32;  // channels per finalize CTA (one per lane)
 constexpr int kFinThreads = 1024;
 constexpr int kFinWarps = kFinThreads / 32;
-constexpr int kFinHeld = 19;      // partials per thread, all requested at once: their load latencies overlap
+constexpr int kFinHeld = 20;      // partials per thread, all requested at once: their load latencies overlap
 static_assert(kFinHeld * kFinWarps >= 148 * 4, "covers the row blocks of nhwc.cuh's geometry");
 
-// Sum over the warps of one value per lane (a channel): every thread returns its lane's total.
-__device__ __forceinline__ float channel_sum(float v, float (*sh)[kFinWarps + 1], float* tot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  static_assert(kFinWarps == kFinChannels, "warp w adds up channel w");
-  sh[lane][warp] = v;
-  __syncthreads();
-  v = sh[warp][lane];
+// Chan et al.: merges the (count, mean, M2) of disjoint sets, one after another, into (cnt, mean, m2).  The
+// weights follow from the counts alone: they are all computed first, so that the chain of dependent
+// operations is a subtraction and a multiply-add per set, and not a divide.  nb[j] <= 0: no such set.
+template <int N>
+__device__ __forceinline__ void chan_merge(float& cnt, float& mean, float& m2, const float (&nb)[N], const float (&mb)[N],
+                                           const float (&m2b)[N]) {
+  float frac[N], before[N];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) tot[warp] = v;
-  __syncthreads();
-  return tot[lane];
+  for (int j = 0; j < N; ++j) {
+    before[j] = cnt;
+    const float tot = cnt + nb[j];
+    frac[j] = __fdividef(nb[j], tot);  // weights of a mean: 2 ulp is plenty, an IEEE divide per step is not free
+    if (nb[j] > 0.f) cnt = tot;
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (nb[j] <= 0.f) continue;
+    const float delta = mb[j] - mean;
+    mean += delta * frac[j];
+    m2 += m2b[j] + delta * delta * (before[j] * frac[j]);
+  }
 }
 
-// grid = C / 32.  Lane = channel, warp w holds the partials of row blocks w, w+32, ... in registers.  A
-// few CTAs with little to do: what counts is the length of the dependent chain, so the mean is taken
-// first (a plain sum) and the squares are then summed about it, both by shuffles, instead of merging
-// partials one after another (each merge a divide and four dependent operations):
+// grid = C / 32.  Lane = channel, warp w merges row blocks w, w+32, ... and the warp results are merged in
+// warp order (always the same order: results are deterministic).  A few CTAs with little to do: what counts
+// is the length of the dependent chain, so all partials of a thread are requested at once, the weights are
+// taken out of the chain, and the kernel starts while the one before it ends:
 // a ResNet-50 step of 64 images takes 8.83 ms with the weights in the chain and plain launches, 8.35
 // to 8.45 now.
 __global__ void __launch_bounds__(kFinThreads)
@@ -110,7 +120,7 @@ bn_stats_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int
                          const float* __restrict__ beta, float* running_mean, float* running_var,
                          long long* num_batches, float momentum, float eps, float* __restrict__ mean_out,
                          float* __restrict__ invstd_out, float2* __restrict__ ab_out) {
-  __shared__ float sh[kFinChannels][kFinWarps + 1], tot[2][kFinChannels];
+  __shared__ float sh[3][kFinWarps][kFinChannels];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * kFinChannels + lane;
   let_next_start();
@@ -125,28 +135,46 @@ bn_stats_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int
     rm_c = running_mean[c];
     rv_c = running_var[c];
   }
-  float2 p[kFinHeld];
+  float cnt = 0.f, mean = 0.f, m2 = 0.f;
+  {
+    float2 p[kFinHeld];
 #pragma unroll
-  for (int j = 0; j < kFinHeld; ++j) {
-    const int y = warp + j * kFinWarps;
-    p[j] = c < C && y < row_blocks ? __ldcg(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
+    for (int j = 0; j < kFinHeld; ++j) {
+      const int y = warp + j * kFinWarps;
+      p[j] = c < C && y < row_blocks ? __ldcg(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
+    }
+    const int full_blocks = int(M / rows_per_block), blocks = c < C ? row_blocks : 0;
+    const float full_rows = float(rows_per_block), last_rows = float(M % rows_per_block);
+#pragma unroll
+    for (int j0 = 0; j0 < kFinHeld; j0 += 5) {
+      float nb[5], mb[5], m2b[5];
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const int y = warp + (j0 + j) * kFinWarps;
+        nb[j] = y < blocks ? (y < full_blocks ? full_rows : last_rows) : 0.f;
+        mb[j] = p[j0 + j].x;
+        m2b[j] = p[j0 + j].y;
+      }
+      chan_merge<5>(cnt, mean, m2, nb, mb, m2b);
+    }
   }
-  const int full_blocks = int(M / rows_per_block);
-  const float full_rows = float(rows_per_block), last_rows = float(M % rows_per_block);
-  auto rows_of = [&](int y) { return y < full_blocks ? full_rows : (y == full_blocks ? last_rows : 0.f); };
-  const float cnt = float(M);
-  float s = 0.f;
-#pragma unroll
-  for (int j = 0; j < kFinHeld; ++j) s += rows_of(warp + j * kFinWarps) * p[j].x;
-  const float mean = channel_sum(s, sh, tot[0]) / cnt;
-  float q = 0.f;
-#pragma unroll
-  for (int j = 0; j < kFinHeld; ++j) {
-    const float d = p[j].x - mean;
-    q += p[j].y + rows_of(warp + j * kFinWarps) * d * d;
-  }
-  const float m2 = channel_sum(q, sh, tot[1]);
+  sh[0][warp][lane] = cnt;
+  sh[1][warp][lane] = mean;
+  sh[2][warp][lane] = m2;
+  __syncthreads();
   if (warp != 0 || c >= C) return;
+#pragma unroll
+  for (int w0 = 1; w0 < kFinWarps; w0 += 8) {
+    float nb[8], mb[8], m2b[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int w = w0 + j;
+      nb[j] = w < kFinWarps ? sh[0][w][lane] : 0.f;
+      mb[j] = w < kFinWarps ? sh[1][w][lane] : 0.f;
+      m2b[j] = w < kFinWarps ? sh[2][w][lane] : 0.f;
+    }
+    chan_merge<8>(cnt, mean, m2, nb, mb, m2b);
+  }
   const float var = m2 / cnt;
   const float invstd = rsqrtf(var + eps);
   mean_out[c] = mean;
@@ -266,7 +294,7 @@ bn_bwd_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int64
                        const float* __restrict__ mean, const float* __restrict__ invstd,
                        const float* __restrict__ gamma, float* __restrict__ dgamma,
                        float* __restrict__ dbeta, float4* __restrict__ coef) {
-  __shared__ float sh[kFinChannels][kFinWarps + 1], tot[2][kFinChannels];
+  __shared__ float sh[2][kFinWarps][kFinChannels];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * kFinChannels + lane;
   let_next_start();
@@ -289,9 +317,15 @@ bn_bwd_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int64
     t1 += p[j].x;
     t2 += p[j].y;
   }
-  t1 = channel_sum(t1, sh, tot[0]);
-  t2 = channel_sum(t2, sh, tot[1]);
+  sh[0][warp][lane] = t1;
+  sh[1][warp][lane] = t2;
+  __syncthreads();
   if (warp != 0 || c >= C) return;
+#pragma unroll 8
+  for (int w = 1; w < kFinWarps; ++w) {
+    t1 += sh[0][w][lane];
+    t2 += sh[1][w][lane];
+  }
   if (dbeta) dbeta[c] = t1;
   if (dgamma) dgamma[c] = t2 * is;
   // dx = a*(dy' - mean(dy') - xhat*mean(dy'*xhat)),  xhat = (x - m)*is,  a = w*is

@@ -319,6 +319,21 @@ def test_terngrad_resident_form_on_two_streams():
             assert torch.equal(o, want[s])
 
 
+# ----------------------------------------------------------------------------- batch norm
+@pytest.mark.parametrize("n,c,h", [(2, 64, 9), (3, 8, 1), (4, 256, 14), (16, 2048, 7), (1, 512, 33)])
+def test_bn_statistics_against_64_bits(n, c, h):
+    from hipress_b200 import _C
+    torch.manual_seed(c)
+    x = (torch.randn(n, c, h, h, device="cuda") * 2 + 0.5).bfloat16().contiguous(memory_format=torch.channels_last)
+    _, stats = _C.bn_forward(x, None, None, None, None, None, None, 0.1, 1e-5, True)
+    xd = x.double().permute(0, 2, 3, 1).reshape(-1, c)
+    # a few roundings of 2^-24, on values of order one
+    assert (stats[0].double() - xd.mean(0)).abs().max() <= 4e-6
+    if xd.shape[0] > 1:
+        var = xd.var(0, unbiased=False)
+        assert ((stats[1].double() - (var + 1e-5).rsqrt()) * (var + 1e-5).sqrt()).abs().max() <= 4e-6
+
+
 # ----------------------------------------------------------------------------- sparse decode and update in one pass
 @pytest.mark.parametrize("opt", ["sgd", "adamw"])
 @pytest.mark.parametrize("world,n", [(1, 70001), (3, 8192 * 2), (8, 100003)])
