@@ -78,13 +78,15 @@ void cpu_accumulate(size_t world, int64_t n, float* out, bool add, double post_s
 }
 
 // Places in a stream's scratch (see scratch_for): the min/max state of the quantisers at 0, the
-// sum of squares of DGC's clipping, the words of the sparse decode, and from 16,384 the sparse state.
-constexpr size_t kSumsqOffset = 12288, kRedoOffset = 12352, kSparseOffset = 16384;
+// sum of squares of DGC's clipping, and from 16,384 the sparse state.
+constexpr size_t kSumsqOffset = 12288, kSparseOffset = 16384;
 
 struct DeviceState {
   std::map<std::pair<int, cudaStream_t>, torch::Tensor> scratch;
   std::map<int, torch::Tensor> status;
+  std::map<std::pair<int, cudaStream_t>, torch::Tensor> redo;
   std::mutex mu;
+  std::mutex decode;   // held while the launches of one sparse decode are queued
 };
 DeviceState& state() {
   static DeviceState* s = new DeviceState();  // leaked on purpose: outlives static destruction order
@@ -106,6 +108,19 @@ void* scratch_for(const torch::Tensor& like, size_t bytes) {
     it = st.scratch.insert_or_assign(key, t).first;
   }
   return it->second.data_ptr();
+}
+
+// The words of the sparse decode: zero between its calls, never moved while the process lives (the scratch
+// is replaced when a call needs a larger one, which calls of another thread on the stream may not expect).
+static unsigned int* redo_words_for(const torch::Tensor& like) {
+  auto& st = state();
+  const int dev = like.get_device();
+  const auto key = std::make_pair(dev, at::cuda::getCurrentCUDAStream(dev).stream());
+  std::lock_guard<std::mutex> lk(st.mu);
+  auto it = st.redo.find(key);
+  if (it == st.redo.end())
+    it = st.redo.emplace(key, torch::zeros({2}, torch::dtype(torch::kInt32).device(like.device()))).first;
+  return reinterpret_cast<unsigned int*>(it->second.data_ptr<int>());
 }
 
 int* status_word_for(const torch::Tensor& like) {
@@ -321,13 +336,12 @@ void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor
   if (out.is_cuda()) {
     c10::cuda::CUDAGuard guard(out.device());
     auto stream = at::cuda::getCurrentCUDAStream();
-    // The one-pass decode needs two words of the stream's scratch.  A captured graph may outlive
-    // that scratch, or run beside later calls on the stream, and takes the form without them.
+    // The one-pass decode shares two words with the stream's other decodes: its launches must not mix with
+    // theirs.  A captured graph may run beside later calls on the stream, and takes the form without them.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     HP_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
-    unsigned int* redo = nullptr;
-    if (!add && capture == cudaStreamCaptureStatusNone)
-      redo = reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(scratch_for(out, kSparseOffset)) + kRedoOffset);
+    unsigned int* redo = !add && capture == cudaStreamCaptureStatusNone ? redo_words_for(out) : nullptr;
+    std::lock_guard<std::mutex> one_at_a_time(state().decode);
     HP_CHECK_CUDA(cuda::sparse_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
                                             add ? 1 : 0, float(post_scale), status_word_for(out), stream, redo));
   } else {

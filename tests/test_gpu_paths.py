@@ -379,3 +379,29 @@ def test_sparse_update_pass_equals_scatter_and_dense_update(opt, world, n, devic
         results.append([t.cpu() for bufs in state for t in bufs[1:]])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+def test_sparse_decode_from_two_threads_on_one_stream():
+    """Decodes of ordered and unordered payloads queued by two threads on the default stream do not disturb each other."""
+    import threading
+    n, k = 200000, 3000
+    jobs = []
+    for t, order in enumerate(("ascending", "random")):
+        p = random_payload(n, k, 40 + t, order)
+        ref = torch.empty(n)
+        ops.sparse_decompress(p, ref)
+        jobs.append((p.cuda(), ref, [torch.empty(n, device="cuda") for _ in range(100)]))
+
+    def work(p, outs):
+        for o in outs:
+            ops.sparse_decompress(p, o)
+
+    threads = [threading.Thread(target=work, args=(p, outs)) for p, _, outs in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for _, ref, outs in jobs:
+        for o in outs:
+            assert torch.equal(o.cpu(), ref)
