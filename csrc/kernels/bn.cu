@@ -16,12 +16,12 @@
 // adjacent channels (one 16-byte load per row) for the whole kernel, so per-channel constants
 // sit in registers, and four rows are in flight per thread.  The two reductions store one
 // partial result per CTA and channel; a small finalize kernel (32 channels per CTA, 32 warps
-// striding over the partials, added in a fixed order, so results are deterministic) combines
+// striding over the partials, merged in a fixed order, so results are deterministic) combines
 // them -- the variance with Chan's parallel update, so no precision is lost to
 // E[x^2] - E[x]^2 over the whole batch -- and writes the coefficients the elementwise kernel
-// needs.  The three kernels of
-// a direction overlap at their ends (launch.cuh).  (A first version let the last CTA to finish combine all partials: one thread per
-// channel walking ~1,200 partials in sequence took 6x longer than reading the activations.)
+// needs.  The three kernels of a direction overlap at their ends (launch.cuh).  (A first version
+// let the last CTA to finish combine all partials: one thread per channel walking ~1,200 partials
+// in sequence took 6x longer than reading the activations.)
 //
 // The reference has no model code; this belongs to the model zoo built around its codecs.
 #include <cuda_bf16.h>

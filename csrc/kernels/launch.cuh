@@ -3,13 +3,13 @@
 // of one and the ramp-up of the next.
 //
 // Rules the kernels here follow.  A kernel launched by launch_after() calls wait_for_previous()
-// before it touches memory; the wait covers the whole kernel before it, so a chain is ordered
-// exactly as plain launches are.  Pointers that are read through the read-only path afterwards are
-// passed through after_wait(), so that no such load can be moved above the wait.  The kernel before
-// it calls let_next_start() (its result is only about when the next one is brought in, never about
+// before it touches what the kernel before it wrote; the wait covers that whole kernel, so a chain is
+// ordered exactly as plain launches are.  What a kernel reads through the read-only path (__ldg, const
+// __restrict__) was complete before the chain began: such a load may be moved above the wait.  The kernel
+// before it calls let_next_start() (its result is only about when the next one is brought in, never about
 // what it may read), and a long one only when its work is nearly done: CTAs that wait hold registers and
-// shared memory which kernels of other streams, the backward pass above all, could use.  The first kernel of a chain is launched plainly: its inputs come from kernels
-// of the caller, which know nothing of this.
+// shared memory which kernels of other streams, the backward pass above all, could use.  The first kernel
+// of a chain is launched plainly: its inputs come from kernels of the caller, which know nothing of this.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -18,12 +18,6 @@ namespace cuda {
 
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename T>
-__device__ __forceinline__ T* after_wait(T* p) {
-  asm volatile("" : "+l"(p)::"memory");
-  return p;
-}
-
 // A kernel whose CTAs wait for one another: all of them are resident at once, or the launch fails.
 template <typename... Params, typename... Args>
 cudaError_t launch_resident(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

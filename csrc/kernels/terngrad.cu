@@ -752,7 +752,9 @@ cudaError_t launch_tern_index(const UnpackSources& src, float* out, int64_t n, i
     using L = IndexLayout<BW, WORLD, false, false>;
     smem = L::kBytes;
     grid = index_grid(n, IndexForm<BW>::kChunk, WORLD, smem);
-    if (smem > 40 * 1024) {   // with the static part, past the default limit; per device, and cheap: set on every launch rather than remembered per process
+    // with the static part, past the default limit; per device, and cheap: set on every launch rather than
+    // remembered per process
+    if (smem > 40 * 1024) {
       const cudaError_t e = cudaFuncSetAttribute(tern_unpack_index_kernel<BW, APPLY, WORLD>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
       if (e != cudaSuccess) return e;

@@ -616,8 +616,9 @@ inline int index_grid(int64_t n, int chunk, int world, size_t smem_bytes) {
 
 // ---------------------------------------------------------------- concatenated shards, 2 bits
 // Sharded exchange, last phase: payload[j] encodes shard j alone.  nib: [world or 1][16][2]
-// nibble tables (rank j's at nib + j*32 floats; one table when SHARED).  Lane L
-// decodes payload byte j*32 + L (j = 0..3) of the warp's 128-byte chunk; a 512-element chunk never straddles two shards (shard_elems % 2048 == 0).
+// nibble tables (rank j's at nib + j*32 floats; one table when SHARED).  Lane L decodes payload byte
+// j*32 + L (j = 0..3) of the warp's 128-byte chunk; a 512-element chunk never straddles two shards
+// (shard_elems % 2048 == 0).
 // header_bytes + slot_shift: where the packed data starts inside payload[j].
 template <bool APPLY, bool SHARED>
 __device__ __forceinline__ void unpack_concat_body(const float* nib, const UnpackSources& src, int64_t data_offset,
