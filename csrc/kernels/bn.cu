@@ -141,7 +141,7 @@ bn_stats_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int
 #pragma unroll
     for (int j = 0; j < kFinHeld; ++j) {
       const int y = warp + j * kFinWarps;
-      p[j] = c < C && y < row_blocks ? __ldcg(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
+      p[j] = c < C && y < row_blocks ? load_written(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
     }
     const int full_blocks = int(M / rows_per_block), blocks = c < C ? row_blocks : 0;
     const float full_rows = float(rows_per_block), last_rows = float(M % rows_per_block);
@@ -309,7 +309,7 @@ bn_bwd_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int64
 #pragma unroll
   for (int j = 0; j < kFinHeld; ++j) {
     const int y = warp + j * kFinWarps;
-    p[j] = c < C && y < row_blocks ? __ldcg(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
+    p[j] = c < C && y < row_blocks ? load_written(&partial[int64_t(y) * C + c]) : make_float2(0.f, 0.f);
   }
   float t1 = 0.f, t2 = 0.f;
 #pragma unroll

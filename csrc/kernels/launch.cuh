@@ -18,6 +18,24 @@ namespace cuda {
 
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Loads past L1 of what another CTA or the kernel before has just written.  Unlike __ldcg, which the
+// compiler may move freely, these keep their place behind the wait, the flag or the counter that they follow.
+__device__ __forceinline__ float2 load_written(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_written(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned int load_written(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // A kernel whose CTAs wait for one another: all of them are resident at once, or the launch fails.
 template <typename... Params, typename... Args>
 cudaError_t launch_resident(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace hipress {
 namespace cuda {
 
@@ -79,8 +81,8 @@ __device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, flo
   mn = INFINITY;
   mx = -INFINITY;
   for (int i = threadIdx.x; i < int(gridDim.x); i += THREADS) {
-    mn = fminf(mn, __ldcg(&s->partial_min[i]));
-    mx = fmaxf(mx, __ldcg(&s->partial_max[i]));
+    mn = fminf(mn, load_written(&s->partial_min[i]));
+    mx = fmaxf(mx, load_written(&s->partial_max[i]));
   }
   block_minmax<THREADS>(mn, mx);
   if (threadIdx.x == 0) {

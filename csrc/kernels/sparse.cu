@@ -342,7 +342,7 @@ select_kernel(int64_t sample_cnt, unsigned int rank0, SparseScratch* s, const ui
     for (int i = threadIdx.x; i < kBins; i += kThreads) sh[i] = 0;
     __syncthreads();
     for (unsigned int i = threadIdx.x; i < count; i += kThreads) {
-      const uint32_t key = __ldcg(kept + i);
+      const uint32_t key = load_written(kept + i);
       if (prefix_matches(key, round, prefix)) atomicAdd(&sh[digit_of(key, round)], 1u);
     }
     __syncthreads();
