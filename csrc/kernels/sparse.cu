@@ -334,6 +334,7 @@ select_kernel(int64_t sample_cnt, unsigned int rank0, SparseScratch* s, const ui
     if (threadIdx.x == 0 && held != 0) place = atomicAdd(&s->s_kept, held);   // one per CTA, not one per warp
     __syncthreads();
     if (threadIdx.x < held) kept[place + threadIdx.x] = mine[threadIdx.x];
+    __syncthreads();   // the next step of a large sample resets `held`
   }
   if (!last_cta(&s->s_done)) return;
   const unsigned int count = *reinterpret_cast<volatile unsigned int*>(&s->s_kept);

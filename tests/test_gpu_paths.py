@@ -229,6 +229,20 @@ def test_sparse_many_equal_magnitudes(keep, rate):
         compare_sparse(r, rate, keep, seed)
 
 
+@pytest.mark.parametrize("keep", [0.001, 0.25])
+@pytest.mark.parametrize("few_magnitudes", [False, True])
+def test_sparse_samples_of_several_steps(keep, few_magnitudes):
+    """From 15.2 M elements on, a CTA of the selection takes more than 256 sampled keys, in steps: a quarter kept puts
+    up to 30 of each 256 into the threshold's bin, few magnitudes all of them."""
+    n = (1 << 24) + 3
+    r = gauss(n, seed=11)
+    if few_magnitudes:
+        i = torch.arange(n)
+        r = torch.sign(r) * torch.where(i % 2000 == 0, 1.0, torch.tensor([0.5, 0.5, 0.25, 0.25, 0.25] + 5 * [0.0])[i % 10])
+    for seed in (1, 2, 3):
+        compare_sparse(r, 0.01, keep, seed)
+
+
 # ----------------------------------------------------------------------------- PowerSGD
 @pytest.mark.parametrize("n,r", [(1, 1), (16384, 1), (16385, 1), (16385, 2), (8192, 4), (8193, 3), (4096, 8), (4097, 8),
                                  (2048, 16), (2049, 11), (33, 16)])
