@@ -1377,7 +1377,7 @@ __device__ __forceinline__ bool decode_tile(const UnpackSources& src, int64_t n,
     if (at >= 0 && at < len) {
       if (post_scale != 1.0f) v = hp_mul(v, post_scale);
       buf[at] = hp_add(buf[at], v);   // indices are unique inside one payload
-    } else if (last && int64_t(i) >= n) {
+    } else if (int64_t(i) >= n) {   // every entry is seen by some tile, wherever it stands in the payload
       if (status != nullptr) atomicExch(status, int(kPayloadBounds));
     } else {
       bad = true;

@@ -66,6 +66,26 @@ def test_sparse_decode_reports_indices_past_the_end():
     assert torch.equal(out.cpu(), ref)
 
 
+@pytest.mark.parametrize("order", ["ascending", "random"])
+@pytest.mark.parametrize("world", [1, 3])
+@pytest.mark.parametrize("at", [0, 1234, 4999])
+@pytest.mark.parametrize("bad", [400000, 0xffffffff])
+def test_sparse_decode_reports_one_index_past_the_end(order, world, at, bad):
+    """Wherever it stands in the payload; the other entries are decoded all the same."""
+    n, k = 400000, 5000
+    payloads = [random_payload(n, k, s, order) for s in range(world)]
+    idx = payloads[-1][4:4 + 4 * k].view(torch.int32).long()
+    val = payloads[-1][4 + 4 * k:].view(torch.float32)
+    others = torch.arange(k) != at
+    ref = torch.empty(n)
+    ops.sparse_decompress(payloads[:-1] + [sparse_payload(idx[others], val[others])], ref)
+    idx[at] = bad
+    out = torch.full((n,), 7.0, device="cuda")
+    ops.sparse_decompress([p.cuda() for p in payloads[:-1] + [sparse_payload(idx, val)]], out)
+    assert ops.read_status(out) == 2
+    assert torch.equal(out.cpu(), ref)
+
+
 def test_sparse_decode_under_capture():
     n = 100000
     p = [random_payload(n, 500, s).cuda() for s in range(2)]
