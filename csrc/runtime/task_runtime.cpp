@@ -18,9 +18,25 @@ TaskRuntime& TaskRuntime::instance() {
   return *rt;
 }
 
+// Nobody waits for the lock with the interpreter lock in hand: whoever holds it may be waiting for workers,
+// and they need the interpreter lock to let go of Python tensors.
+std::unique_lock<std::mutex> TaskRuntime::life_lock() {
+  std::unique_lock<std::mutex> lk(life_mu_, std::try_to_lock);
+  if (!lk.owns_lock()) {
+    if (PyGILState_Check()) {
+      py::gil_scoped_release nogil;
+      lk.lock();
+    } else {
+      lk.lock();
+    }
+  }
+  return lk;
+}
+
 bool TaskRuntime::init(const std::string& alg_name, std::unordered_map<std::string, double> params,
                        int device_id, int rank_id, int size) {
-  if (pool_) end();
+  const auto life = life_lock();
+  if (pool_) end_locked();
   CompAlg alg;
   alg.name = alg_name;
   int threads = kBackThreads;
@@ -61,6 +77,12 @@ bool TaskRuntime::init(const std::string& alg_name, std::unordered_map<std::stri
 }
 
 bool TaskRuntime::end() {
+  const auto life = life_lock();
+  end_locked();
+  return true;
+}
+
+void TaskRuntime::end_locked() {
   if (pool_) {
     pool_->drain();
     pool_->shutdown();
@@ -69,7 +91,11 @@ bool TaskRuntime::end() {
   watchdog_.reset();
   std::lock_guard<std::mutex> lk(map_mu_);
   gathered_.clear();
-  return true;
+}
+
+int TaskRuntime::num_threads() {
+  const auto life = life_lock();
+  return pool_ ? pool_->size() : 0;
 }
 
 int64_t TaskRuntime::graddrop_staging_bytes(int64_t n) const {
@@ -232,6 +258,7 @@ void TaskRuntime::settle() {
 }
 
 bool TaskRuntime::submit(Task t) {
+  const auto life = life_lock();
   TORCH_CHECK(pool_ != nullptr && pool_->alive(), "hipress runtime is not initialised (call init first)");
   t.serial = serial_.fetch_add(1);
   // order the worker's stream after whatever the caller has queued so far

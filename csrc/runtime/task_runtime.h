@@ -63,8 +63,6 @@ class TaskRuntime {
   bool init(const std::string& alg_name, std::unordered_map<std::string, double> params,
             int device_id, int rank_id, int size);
   bool end();
-  bool running() const { return pool_ != nullptr; }
-
   bool submit_without_residual(const std::string& name, torch::Tensor tensor, torch::Tensor B,
                                torch::Tensor C, int is_root, int task_id);
   bool submit_with_residual(const std::string& name, torch::Tensor tensor, torch::Tensor residual,
@@ -77,13 +75,15 @@ class TaskRuntime {
   std::vector<std::string> wait_results(int task_id, double timeout_s, unsigned long long seen);
   unsigned long long error_marks(int task_id);
   std::vector<std::string> get_errors();
-  int num_threads() const { return pool_ ? pool_->size() : 0; }
+  int num_threads();
   const CompAlg& algorithm() const { return alg_; }
   // fixed staging size of a GradDrop payload (ref hp_cuda.cpp:230)
   int64_t graddrop_staging_bytes(int64_t n) const;
 
  private:
   TaskRuntime() = default;
+  std::unique_lock<std::mutex> life_lock();
+  void end_locked();
   bool submit(Task t);
   void run(Task& t);
   void run_compress(Task& t);
@@ -94,6 +94,9 @@ class TaskRuntime {
   void add_error(std::string text);
   void settle();
 
+  // Held while the runtime is started or ended and while a task is handed to it: pool_, watchdog_ and alg_
+  // change under it only, and only when no worker runs.  See life_lock().
+  std::mutex life_mu_;
   CompAlg alg_;
   int device_id_ = 0, rank_ = 0, size_ = 1;
   std::unique_ptr<WorkerPool> pool_;

@@ -1,5 +1,8 @@
 """Waiting for tasks: the wait ends with the task, and the runtime can be restarted the moment a name is known."""
+import subprocess
+import sys
 import time
+from pathlib import Path
 
 import pytest
 import torch
@@ -39,3 +42,45 @@ def test_wait_ends_on_error_and_on_timeout():
         hp_cuda.wait_for(hp_cuda.COMP_TASK, ["never"], timeout_s=0.3)
     assert 0.2 < time.monotonic() - t0 < 10
     hp_cuda.end()
+
+
+RESTART_BESIDE_SUBMIT = """
+import sys, threading, time
+import torch
+from hipress_b200 import hp_cuda, ops
+
+n, size = 64, ops.tbq_payload_bytes(64)
+stop = time.monotonic() + 3.0
+failures = []
+
+def submit(k):
+    try:
+        while time.monotonic() < stop:
+            t = (torch.randn(n) * 1e-3, torch.zeros(n), torch.zeros(size, dtype=torch.uint8),
+                 torch.zeros(size, dtype=torch.uint8))
+            assert hp_cuda.submit_task(f"t{k}", *t, 0, hp_cuda.COMP_TASK)
+            hp_cuda.getResults(hp_cuda.COMP_TASK)
+            hp_cuda.numThreads()
+    except Exception as e:
+        failures.append(repr(e))
+
+assert hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+threads = [threading.Thread(target=submit, args=(k,)) for k in range(2)]
+for t in threads:
+    t.start()
+while time.monotonic() < stop:
+    assert hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+for t in threads:
+    t.join()
+assert not failures and not hp_cuda.getErrors(), failures
+hp_cuda.end()
+print("ended")
+"""
+
+
+@pytest.mark.timeout(90)
+def test_restart_beside_submitting_threads():
+    """Two threads hand in tasks while a third restarts the runtime; in a process of its own, whose end is looked at."""
+    root = Path(__file__).resolve().parent.parent
+    done = subprocess.run([sys.executable, "-c", RESTART_BESIDE_SUBMIT], cwd=root, capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0 and "ended" in done.stdout, (done.returncode, done.stderr[-2000:])
