@@ -97,20 +97,44 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("init",
         [](const std::string& alg, std::unordered_map<std::string, double> params, int device_id,
            int rank_id, int size) {
-          py::gil_scoped_release nogil;   // it may have to wait for workers that let go of Python tensors
-          return runtime::TaskRuntime::instance().init(alg, std::move(params), device_id, rank_id, size);
+          auto& rt = runtime::TaskRuntime::instance();
+          bool ok;
+          {
+            py::gil_scoped_release nogil;   // it may have to wait for workers, and they for the interpreter lock
+            ok = rt.init(alg, std::move(params), device_id, rank_id, size);
+          }
+          rt.release_spent();
+          return ok;
         },
         "init(alg_name, alg_paras, device_id, rank_id, size) -> bool", py::arg("alg_name"),
         py::arg("alg_paras"), py::arg("device_id"), py::arg("rank_id"), py::arg("size"));
   m.def("end", [] {
-    py::gil_scoped_release nogil;
-    return runtime::TaskRuntime::instance().end();
+    auto& rt = runtime::TaskRuntime::instance();
+    bool ok;
+    {
+      py::gil_scoped_release nogil;
+      ok = rt.end();
+    }
+    rt.release_spent();
+    return ok;
   });
   m.def("_errorMarks", [](int task_id) { return runtime::TaskRuntime::instance().error_marks(task_id); });
   m.def("_waitResults", [](int task_id, double timeout_s, unsigned long long seen) {
-    return runtime::TaskRuntime::instance().wait_results(task_id, timeout_s, seen);
-  }, py::call_guard<py::gil_scoped_release>());
-  m.def("getResults", [](int task_id) { return runtime::TaskRuntime::instance().get_results(task_id); });
+    auto& rt = runtime::TaskRuntime::instance();
+    std::vector<std::string> names;
+    {
+      py::gil_scoped_release nogil;
+      names = rt.wait_results(task_id, timeout_s, seen);
+    }
+    rt.release_spent();
+    return names;
+  });
+  m.def("getResults", [](int task_id) {
+    auto& rt = runtime::TaskRuntime::instance();
+    auto names = rt.get_results(task_id);
+    rt.release_spent();
+    return names;
+  });
   m.def("getErrors", [] { return runtime::TaskRuntime::instance().get_errors(); });
   m.def("numThreads", [] { return runtime::TaskRuntime::instance().num_threads(); });
   m.def("submit_task",

@@ -6,6 +6,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <cmath>
+#include <deque>
 
 #include "../common/host_utils.h"
 #include "../ops/ops.h"
@@ -68,7 +69,7 @@ bool TaskRuntime::init(const std::string& alg_name, std::unordered_map<std::stri
     std::lock_guard<std::mutex> lk(err_mu_);
     errors_.clear();
   }
-  pool_ = std::make_unique<WorkerPool>(threads, [](int) {}, [this](int) { settle(); });
+  pool_ = std::make_unique<WorkerPool>(threads, [](int) {}, [this](int, bool wait) { return settle(wait); });
   const double age_limit = params.count("task_age_limit") ? params["task_age_limit"] : 120.0;
   watchdog_ = std::make_unique<AgeWatchdog>(age_limit, [this](const std::string& label, double age) {
     add_error(label + ": still running after " + std::to_string(age) + " s (task age limit)");
@@ -220,44 +221,60 @@ bool TaskRuntime::submit_powersgd(const std::string& name, torch::Tensor tensor,
 }
 
 namespace {
-// Tasks of this worker whose kernels and copies are queued on its stream.  The worker goes on to its next
-// task instead of waiting for each: a copy of one overlaps the kernels of the next, and the stream is
-// waited for when the queue is empty.
+// Tasks of this worker whose kernels and copies are queued on its stream, oldest first.  The worker goes on
+// to its next task instead of waiting for each: a copy of one overlaps the kernels of the next.
 struct Queued {
   Task task;   // keeps the tensors
   std::unique_ptr<at::cuda::CUDAEvent> done;
 };
-std::vector<Queued>& queued() {
-  thread_local std::vector<Queued> q;
+std::deque<Queued>& queued() {
+  thread_local std::deque<Queued> q;
   return q;
 }
 }  // namespace
 
-// A task's tensors are let go before its name is reported: the caller may drop them, and end the runtime,
-// as soon as it knows the name, and the last owner of a Python tensor needs the interpreter lock.
-void TaskRuntime::settle() {
-  std::vector<Queued> batch;
-  batch.swap(queued());
-  for (Queued& q : batch) {
-    const int task_id = q.task.task_id;
-    const std::string name = q.task.tensor_name;
-    const uint64_t serial = q.task.serial;
+// The last owner of a Python tensor needs the interpreter lock, which a worker would have to wait for with
+// the next tasks behind it.  The tensors go back to the callers, who hold that lock, before the name is out.
+void TaskRuntime::report(Task& t, const std::string& error) {
+  const int task_id = t.task_id;
+  const std::string name = t.tensor_name;
+  watchdog_->done(t.serial);
+  {
+    std::lock_guard<std::mutex> lk(spent_mu_);
+    spent_.push_back(std::move(t));
+  }
+  if (error.empty()) queue_for(task_id).push(name);
+  else add_error(name + ": " + error);
+}
+
+void TaskRuntime::release_spent() {
+  std::vector<Task> spent;
+  std::lock_guard<std::mutex> lk(spent_mu_);
+  spent.swap(spent_);
+}
+
+// Reports the tasks of this worker that are done: after every task those that the device has finished by
+// then, and with `wait` all of them, one by one.  Returns how many are left.
+int TaskRuntime::settle(bool wait) {
+  std::deque<Queued>& q = queued();
+  while (!q.empty()) {
+    Queued& first = q.front();
     std::string error;
     try {
-      c10::cuda::CUDAGuard dev(q.task.tensor.device());
-      q.done->synchronize();
+      c10::cuda::CUDAGuard dev(first.task.tensor.device());
+      if (wait) first.done->synchronize();
+      else if (!first.done->query()) break;
     } catch (const std::exception& e) {
       error = e.what();
     }
-    q.task = Task{};
-    q.done.reset();
-    if (error.empty()) queue_for(task_id).push(name);
-    else add_error(name + ": " + error);
-    watchdog_->done(serial);
+    report(first.task, error);
+    q.pop_front();
   }
+  return int(q.size());
 }
 
 bool TaskRuntime::submit(Task t) {
+  release_spent();
   const auto life = life_lock();
   TORCH_CHECK(pool_ != nullptr && pool_->alive(), "hipress runtime is not initialised (call init first)");
   t.serial = serial_.fetch_add(1);
@@ -267,9 +284,9 @@ bool TaskRuntime::submit(Task t) {
     ready = std::make_shared<at::cuda::CUDAEvent>();
     ready->record(at::cuda::getCurrentCUDAStream(t.tensor.get_device()));
   }
-  const uint64_t serial = t.serial;
-  watchdog_->track(serial, t.tensor_name + " (task " + std::to_string(t.task_id) + ")");
-  pool_->submit([this, t, ready, serial](int) mutable {
+  watchdog_->track(t.serial, t.tensor_name + " (task " + std::to_string(t.task_id) + ")");
+  pool_->submit([this, t, ready](int) mutable {
+    std::string error;
     try {
       if (t.tensor.is_cuda()) {
         c10::cuda::CUDAGuard dev(t.tensor.device());
@@ -282,23 +299,27 @@ bool TaskRuntime::submit(Task t) {
         c10::cuda::CUDAStream stream = it->second;
         c10::cuda::CUDAStreamGuard sg(stream);
         ready->block(stream);
+        // a copy from or to pageable memory holds the worker up: the names before it go out first, and the
+        // wait for its own costs nothing
+        const bool blocking = t.C.defined() && !t.C.is_cuda() && !t.C.is_pinned();
+        if (blocking) settle(true);
         run(t);
-        auto done = std::make_unique<at::cuda::CUDAEvent>();
-        done->record(stream);
-        queued().push_back(Queued{std::move(t), std::move(done)});
-        return;
+        if (blocking) {
+          stream.synchronize();
+        } else {
+          auto done = std::make_unique<at::cuda::CUDAEvent>();
+          done->record(stream);
+          queued().push_back(Queued{std::move(t), std::move(done)});
+          return;
+        }
+      } else {
+        settle(true);   // the CPU codec takes its time: the names before it go out first
+        run(t);
       }
-      run(t);
-      const int task_id = t.task_id;
-      const std::string name = t.tensor_name;
-      t = Task{};
-      queue_for(task_id).push(name);
     } catch (const std::exception& e) {
-      const std::string name = t.tensor_name;
-      t = Task{};
-      add_error(name + ": " + e.what());
+      error = e.what();
     }
-    watchdog_->done(serial);
+    report(t, error);
   });
   return true;
 }

@@ -76,6 +76,8 @@ class TaskRuntime {
   unsigned long long error_marks(int task_id);
   std::vector<std::string> get_errors();
   int num_threads();
+  // Lets go of the tensors of finished tasks; called with the interpreter lock in hand.
+  void release_spent();
   const CompAlg& algorithm() const { return alg_; }
   // fixed staging size of a GradDrop payload (ref hp_cuda.cpp:230)
   int64_t graddrop_staging_bytes(int64_t n) const;
@@ -92,7 +94,8 @@ class TaskRuntime {
   void run_powersgd(Task& t);
   FinishQueue& queue_for(int task_id);
   void add_error(std::string text);
-  void settle();
+  int settle(bool wait);
+  void report(Task& t, const std::string& error);
 
   // Held while the runtime is started or ended and while a task is handed to it: pool_, watchdog_ and alg_
   // change under it only, and only when no worker runs.  See life_lock().
@@ -102,6 +105,8 @@ class TaskRuntime {
   std::unique_ptr<WorkerPool> pool_;
   std::unique_ptr<AgeWatchdog> watchdog_;
   FinishQueue comp_, decomp_, root_;
+  std::mutex spent_mu_;
+  std::vector<Task> spent_;   // finished, their tensors not yet let go
   std::mutex err_mu_;
   std::vector<std::string> errors_;
   std::mutex map_mu_;

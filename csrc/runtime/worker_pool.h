@@ -4,8 +4,9 @@
 // reference's workers poll their queue on a fixed 500 us cycle,
 // ref hp_cuda.cpp:174-184).  Submission is round-robin over the queues, or to
 // an explicit worker when ordering between tasks matters.  A job may leave work behind that only has
-// to be waited for (copies in flight on a stream): the optional `settle` hook runs in the worker when its
-// queue is empty, or after kMaxUnsettled jobs, and only then do the jobs count as done.  An exception thrown
+// to be waited for (copies in flight on a stream): the optional `settle` hook runs in the worker after every
+// job and returns how many jobs are still unsettled.  It is told to wait for all of them when the queue is
+// empty, or when kMaxUnsettled are, and only settled jobs count as done.  An exception thrown
 // by a task is caught, recorded and reported through `last_error()`; the worker
 // keeps running (in the reference the thread prints and exits, after which
 // every poll hangs: hp_cuda.cpp:805-809).
@@ -27,10 +28,11 @@ namespace runtime {
 class WorkerPool {
  public:
   using Job = std::function<void(int /*worker index*/)>;
+  using Settle = std::function<int(int /*worker index*/, bool /*wait*/)>;
 
   // `on_start` runs once in each worker thread before it takes work (device
   // guard, stream creation).
-  WorkerPool(int num_workers, std::function<void(int)> on_start, std::function<void(int)> settle = nullptr)
+  WorkerPool(int num_workers, std::function<void(int)> on_start, Settle settle = nullptr)
       : workers_(static_cast<size_t>(num_workers)), settle_(std::move(settle)) {
     for (int i = 0; i < num_workers; ++i) {
       auto& w = workers_[static_cast<size_t>(i)];
@@ -139,15 +141,17 @@ class WorkerPool {
         record("unknown exception in worker task");
       }
       ++unsettled;
+      int left = 0;
       if (settle_) {
         bool more;
         {
           std::lock_guard<std::mutex> lk(w.mu);
           more = !w.jobs.empty();
         }
-        if (more && unsettled < kMaxUnsettled) continue;
+        const bool wait = !more || unsettled >= kMaxUnsettled;
+        left = wait ? 0 : unsettled;   // should the hook throw
         try {
-          settle_(index);
+          left = settle_(index, wait);
         } catch (const std::exception& e) {
           record(e.what());
         } catch (...) {
@@ -156,9 +160,9 @@ class WorkerPool {
       }
       {
         std::lock_guard<std::mutex> lk(w.mu);
-        w.pending -= unsettled;
+        w.pending -= unsettled - left;
       }
-      unsettled = 0;
+      unsettled = left;
       w.cv_idle.notify_all();
     }
   }
@@ -171,7 +175,7 @@ class WorkerPool {
 
   static constexpr int kMaxUnsettled = 16;
   std::vector<std::unique_ptr<Worker>> workers_;
-  std::function<void(int)> settle_;
+  Settle settle_;
   std::atomic<uint64_t> next_{0};
   std::mutex err_mu_;
   std::string last_error_;

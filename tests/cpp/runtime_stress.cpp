@@ -4,9 +4,11 @@
 // The reference's equivalents carry known races -- one static stream shared by its five
 // threads (ref hp_cuda.cpp:789), an unsynchronised round-robin counter (ref hp_cuda.cpp:930) --
 // which is why these paths are exercised from several submitting threads at once.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <deque>
 #include <set>
 #include <stdexcept>
 #include <string>
@@ -82,6 +84,45 @@ static void pool_and_queue() {
   }
 }
 
+// Jobs that leave work behind: settled after each job where it is done, waited for when the queue is empty
+// or too much has piled up, and drain() returns only when all of it is settled.
+static void settling() {
+  struct Pending {
+    std::deque<int> ids;   // of one worker
+    int most = 0;
+  };
+  constexpr int kWorkers = 3, kJobs = 5000;
+  std::vector<Pending> pending(kWorkers);
+  std::atomic<int> settled{0};
+  std::atomic<int> ready{0};   // ids below this are done
+  WorkerPool pool(kWorkers, nullptr, [&](int w, bool wait) {
+    Pending& p = pending[size_t(w)];
+    p.most = std::max(p.most, int(p.ids.size()));
+    while (!p.ids.empty() && (wait || p.ids.front() < ready.load())) {
+      p.ids.pop_front();
+      ++settled;
+    }
+    if (p.ids.size() == 7) throw std::runtime_error("injected failure of the hook");
+    return int(p.ids.size());
+  });
+  for (int round = 0; round < 3; ++round) {
+    std::vector<std::thread> submitters;
+    for (int s = 0; s < 2; ++s)
+      submitters.emplace_back([&] {
+        for (int i = 0; i < kJobs; ++i) {
+          pool.submit([&, i](int w) {
+            pending[size_t(w)].ids.push_back(i);
+            if (i % 5 == 0) ready = i;
+          });
+        }
+      });
+    for (auto& t : submitters) t.join();
+    pool.drain();
+    CHECK(settled.load() == (round + 1) * 2 * kJobs);
+  }
+  for (auto& p : pending) CHECK(p.ids.empty());
+}
+
 static void watchdog() {
   std::mutex mu;
   std::vector<std::string> overdue;
@@ -117,6 +158,7 @@ static void watchdog() {
 
 int main() {
   pool_and_queue();
+  settling();
   watchdog();
   std::puts("runtime_stress: ok");
   return 0;

@@ -1,6 +1,7 @@
 """The reference's module API (init / submit_task / getResults / end) on CUDA tensors with the
 CPU staging buffer ``C`` of the original contract."""
 import struct
+import time
 
 import pytest
 import torch
@@ -109,3 +110,27 @@ def test_powersgd_tasks_on_gpu(runtime):
     torch.testing.assert_close(grad, approx, atol=1e-3, rtol=1e-3)
     torch.testing.assert_close(resid, g0 - approx, atol=1e-3, rtol=1e-3)
     assert runtime.getErrors() == []
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("task", ["compress", "decompress"])
+def test_names_of_a_backlog_come_one_by_one(runtime, pinned, task):
+    """One worker and a backlog: a name is out when its task is done, and not together with those behind it."""
+    n, count = 1 << 26, 20
+    runtime.init("tbq", {"threshold": 0.02}, 0, 0, 1)
+    size = ops.tbq_payload_bytes(n)
+    x, r = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    B = torch.zeros(size, dtype=torch.uint8, device="cuda")
+    C = torch.zeros(size, dtype=torch.uint8)
+    C = C.pin_memory() if pinned else C
+    kind = runtime.COMP_TASK if task == "compress" else runtime.DECOMP_TASK
+    for warm in (True, False):
+        torch.cuda.synchronize()
+        t0, came = time.monotonic(), []
+        for i in range(count):
+            runtime.submit_task(f"t{i}", x, r, B, C, 0, kind)
+        while len(came) < count and time.monotonic() < t0 + 30:
+            came += [(k, time.monotonic() - t0) for k in runtime.getResults(kind)]
+    assert [k for k, _ in came] == [f"t{i}" for i in range(count)]
+    when = [t for _, t in came]
+    assert when[9] - when[0] > 0.25 * (when[-1] - when[0]), when   # 9 of 19 steps if all take the same time

@@ -44,6 +44,48 @@ def test_wait_ends_on_error_and_on_timeout():
     hp_cuda.end()
 
 
+@pytest.mark.timeout(60)
+def test_names_do_not_wait_for_the_interpreter():
+    """A name is out when its task is done, also while some Python code keeps the interpreter lock."""
+    hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+    n, names = 64, {"a", "b", "c"}
+    size = ops.tbq_payload_bytes(n)
+    tensors = [(name, torch.randn(n) * 1e-3, torch.zeros(n), torch.zeros(size, dtype=torch.uint8),
+                torch.zeros(size, dtype=torch.uint8)) for name in sorted(names)]
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(20.0)
+    try:
+        for t in tensors:
+            hp_cuda.submit_task(*t, 0, hp_cuda.COMP_TASK)
+        seen, t0 = set(), time.monotonic()
+        while seen < names and time.monotonic() < t0 + 5:
+            seen.update(hp_cuda.getResults(hp_cuda.COMP_TASK))
+    finally:
+        sys.setswitchinterval(interval)
+    assert seen == names
+    hp_cuda.end()
+
+
+EXIT_AFTER_NAME = """
+import torch
+from hipress_b200 import hp_cuda, ops
+size = ops.tbq_payload_bytes(64)
+assert hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+for i in range(200):
+    hp_cuda.submit_task("x", torch.zeros(64), torch.zeros(64), torch.zeros(size, dtype=torch.uint8),
+                        torch.zeros(size, dtype=torch.uint8), 0, hp_cuda.COMP_TASK)
+hp_cuda.wait_for(hp_cuda.COMP_TASK, ["x"])
+"""
+
+
+@pytest.mark.timeout(90)
+def test_exit_with_tasks_in_the_workers():
+    """The program ends without end(), while workers still finish tasks that own the last reference to their tensors."""
+    root = Path(__file__).resolve().parent.parent
+    done = subprocess.run([sys.executable, "-c", EXIT_AFTER_NAME], cwd=root, capture_output=True, text=True, timeout=60)
+    assert done.returncode == 0, (done.returncode, done.stderr[-2000:])
+
+
 RESTART_BESIDE_SUBMIT = """
 import sys, threading, time
 import torch
