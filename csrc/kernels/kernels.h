@@ -113,9 +113,11 @@ size_t minmax_scratch_bytes();
 // residual may be null.  With a residual, the tensor quantised is grad+residual
 // and residual receives the quantisation error.  scratch must be zero before
 // its first use and is left ready for the next call.
+// whole_gpu: the call may be launched with CTAs that fill every SM at once (see tern_hold_kernel); not for
+// callers that run beside other work.
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
-                              void* scratch, cudaStream_t stream);
+                              void* scratch, cudaStream_t stream, bool whole_gpu = false);
 // Element count per payload is taken from its header and must equal n; all
 // payloads must carry the same bitwidth (kBadHeader otherwise).  bitwidth_hint
 // (0 = unknown) lets the launcher size the decode table for that bitwidth; a

@@ -489,8 +489,10 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
 // grad + residual in shared memory (up to 208 KB of it: 30 MB over the chip), the CTAs exchange their
 // extremes through the scratch, and quantise from shared memory.  The two-launch form reads both arrays
 // twice, the second time from L2, and drains and refills the chip in between.  All CTAs have to be resident
-// at once, so this form is for calls that have the GPU to themselves: the exchange engine, whose compressors
-// run beside the backward pass, keeps the two launches.
+// at once and each needs an SM to itself, so this form is for callers that say the GPU is theirs (whole_gpu):
+// the exchange engine and the task API, whose compressors run beside the backward pass, keep the two launches.
+// Beside a chain of 16384^3 matrix products a 4 MB task takes 850 us in this form (it waits for SMs to fall
+// free) and 260 in two launches; on an idle GPU 64 and 71 us.
 // 25 MB with error feedback, 2 bits (ncu, cold): 14.3 + 18.0 us in two launches, 21.6 in one; with the
 // decode of eight payloads 63.4 and 55.4 us, and 9.4 MB at 4 bits 18.4 and 14.4 us.
 constexpr int kHoldThreads = 1024;
@@ -809,7 +811,7 @@ size_t minmax_scratch_bytes() { return sizeof(MinMaxScratch); }
 
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
-                              void* scratch, cudaStream_t stream) {
+                              void* scratch, cudaStream_t stream, bool whole_gpu) {
   if (n <= 0 || !tern_bitwidth_ok(bitwidth) || scratch == nullptr) return cudaErrorInvalidValue;
   auto* s = static_cast<MinMaxScratch*>(scratch);
   const bool ef = residual != nullptr;
@@ -839,9 +841,9 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
 #undef LAUNCH_SMALL
     return cudaGetLastError();
   }
-  // one read of the inputs (see tern_hold_kernel): a destination of this call's own, 16-byte aligned
-  // inputs, and a part per SM that fits its shared memory
-  if (S == 0 && vec && shift >= 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
+  // one read of the inputs (see tern_hold_kernel): a caller that says so, a destination of this call's own,
+  // 16-byte aligned inputs, and a part per SM that fits its shared memory
+  if (whole_gpu && S == 0 && vec && shift >= 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
       dst.epoch_dev == nullptr && dst.remote == 0 && dst.mc == nullptr) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);

@@ -208,8 +208,8 @@ void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
 }
 
 // ------------------------------------------------------------------ TernGrad
-void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
-                       bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual) {
+static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
+                              int64_t seed, c10::optional<torch::Tensor> residual, bool whole_gpu) {
   check_f32(grad, "grad");
   check_u8(out, "out");
   check_same_device(grad, out);
@@ -230,13 +230,23 @@ void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bit
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
     HP_CHECK_CUDA(cuda::terngrad_compress(grad.data_ptr<float>(), res, n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed), local_target(out),
-                                          scratch, at::cuda::getCurrentCUDAStream()));
+                                          scratch, at::cuda::getCurrentCUDAStream(), whole_gpu));
   } else {
     const int rc = cpu::terngrad_compress(grad.data_ptr<float>(), n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed),
                                           out.data_ptr<uint8_t>(), out.numel(), res);
     TORCH_CHECK(rc == 0, "terngrad_compress failed");
   }
+}
+
+void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
+                       bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual) {
+  terngrad_compress(grad, out, bitwidth, enable_random, seed, residual, /*whole_gpu=*/true);
+}
+
+void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
+                              int64_t seed) {
+  terngrad_compress(grad, out, bitwidth, enable_random, seed, c10::nullopt, /*whole_gpu=*/false);
 }
 
 void terngrad_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,

@@ -29,6 +29,9 @@ void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
 
 void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
                        bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual);
+// The same for a stream beside which the caller's own work runs: it does not ask for all SMs at once.
+void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
+                              int64_t seed);
 // bitwidth: 0 = read it from the payload headers on the device; a known bitwidth selects a kernel
 // compiled for it (payloads with another bitwidth are then rejected through the status word).
 void terngrad_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,

@@ -349,8 +349,7 @@ void TaskRuntime::run_compress(Task& t) {
   const auto& a = alg_;
   auto g = t.tensor.view(-1);
   if (a.name == "terngrad") {
-    ops::terngrad_compress(g, t.B, a.bitwidth, a.enable_random != 0, int64_t(task_seed(a, t)),
-                           c10::nullopt);
+    ops::terngrad_compress_beside(g, t.B, a.bitwidth, a.enable_random != 0, int64_t(task_seed(a, t)));
   } else if (a.name == "tbq") {
     ops::tbq_compress(g, t.residual.view(-1), t.B, a.threshold);
   } else if (a.name == "graddrop") {
