@@ -373,20 +373,17 @@ tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
 // quantising pass starts from the registers.  At these sizes a launch costs more than the work: eight
 // SMs take the tensor in and quantise it in less time than the second launch and its ramp-up need.
 // 256 KB, compress and decode of two payloads: 16.4 us in three launches, 14.3 in two.
+// A cluster starts when eight neighbouring SMs have room for 1,024 threads each, so this form is for callers
+// that say the GPU is theirs (whole_gpu): beside 16384^3 matrix products a 256 KB task takes 560 us in it
+// and 153 in two launches; beside a chain of 4096^3 ones the op takes 96 and 55 us.
 constexpr int kSmallCtas = 8, kSmallThreads = 1024, kSmallPerThread = 16;
 constexpr int64_t kSmallElems = int64_t(kSmallCtas) * kSmallThreads * kSmallPerThread;
 template <int BW, bool VEC, bool EF>
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
 tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int random, uint64_t seed,
                   PushTargets dst) {
-  // The CTAs may read the guard at different times and must not part before they have met: each tells
-  // the others what it saw.
-  const bool skip = push_guarded(dst);
-  resolve_epoch(dst);
-  if (dst.epoch_dev != nullptr) seed += uint64_t(dst.epoch) * kEpochSeedStride;
   constexpr int EPT = Unit<BW>::EPT, BPT = Unit<BW>::BPT, UPT = kSmallPerThread / EPT;
   __shared__ float ext_mn[kSmallCtas], ext_mx[kSmallCtas], scale[4];
-  __shared__ int ext_skip[kSmallCtas];
   const cg::cluster_group cluster = cg::this_cluster();
   const int64_t units = n / EPT;
   const int64_t tid = int64_t(blockIdx.x) * kSmallThreads + threadIdx.x;
@@ -433,14 +430,9 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
     for (int c = 0; c < kSmallCtas; ++c) {
       cluster.map_shared_rank(ext_mn, c)[blockIdx.x] = mn;
       cluster.map_shared_rank(ext_mx, c)[blockIdx.x] = mx;
-      cluster.map_shared_rank(ext_skip, c)[blockIdx.x] = skip ? 1 : 0;
     }
   }
   cluster.sync();
-  int any_skip = 0;
-#pragma unroll
-  for (int c = 0; c < kSmallCtas; ++c) any_skip |= ext_skip[c];
-  if (any_skip) return;   // the whole cluster
   PushCursor cur{nullptr};
   if (threadIdx.x == 0) {
     mn = ext_mn[0];
@@ -482,15 +474,14 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
   }
   if (tid == 0 && units * EPT < n)
     tern_leftover<BW, EF>(grad, residual, units * EPT, n, mn, inv, gap, random, seed, dst, cur);
-  publish_when_grid_done(dst);
 }
 
 // Medium tensors: both passes in one launch that reads the inputs once.  One CTA per SM keeps its part of
 // grad + residual in shared memory (up to 208 KB of it: 30 MB over the chip), the CTAs exchange their
 // extremes through the scratch, and quantise from shared memory.  The two-launch form reads both arrays
 // twice, the second time from L2, and drains and refills the chip in between.  All CTAs have to be resident
-// at once and each needs an SM to itself, so this form is for callers that say the GPU is theirs (whole_gpu):
-// the exchange engine and the task API, whose compressors run beside the backward pass, keep the two launches.
+// at once and each needs an SM to itself, so this form too is for callers that say the GPU is theirs: the
+// exchange engine and the task API, whose compressors run beside the backward pass, keep the two launches.
 // Beside a chain of 16384^3 matrix products a 4 MB task takes 850 us in this form (it waits for SMs to fall
 // free) and 260 in two launches; on an idle GPU 64 and 71 us.
 // 25 MB with error feedback, 2 bits (ncu, cold): 14.3 + 18.0 us in two launches, 21.6 in one; with the
@@ -834,17 +825,19 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
     case 4: LAUNCH_FORMS(LAUNCH, 4); break;   \
     default: LAUNCH_FORMS(LAUNCH, 8); break;  \
   }
-  if (S == 0 && n <= kSmallElems) {
+  // a caller that has the GPU to itself, and a destination of this call's own: one launch where the tensor
+  // fits (see tern_small_kernel and tern_hold_kernel)
+  const bool own = whole_gpu && S == 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
+                   dst.epoch_dev == nullptr && dst.remote == 0 && dst.mc == nullptr;
+  if (own && n <= kSmallElems) {
 #define LAUNCH_SMALL(BW, V, E) \
   tern_small_kernel<BW, V, E><<<kSmallCtas, kSmallThreads, 0, stream>>>(grad, residual, n, enable_random, seed, dst)
     LAUNCH_BITS(LAUNCH_SMALL);
 #undef LAUNCH_SMALL
     return cudaGetLastError();
   }
-  // one read of the inputs (see tern_hold_kernel): a caller that says so, a destination of this call's own,
   // 16-byte aligned inputs, and a part per SM that fits its shared memory
-  if (whole_gpu && S == 0 && vec && shift >= 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
-      dst.epoch_dev == nullptr && dst.remote == 0 && dst.mc == nullptr) {
+  if (own && vec && shift >= 0) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);

@@ -136,10 +136,10 @@ def test_names_of_a_backlog_come_one_by_one(runtime, pinned, task):
     assert when[9] - when[0] > 0.25 * (when[-1] - when[0]), when   # 9 of 19 steps if all take the same time
 
 
-def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime):
+@pytest.mark.parametrize("n", [65536, 1 << 20])
+def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime, n):
     """Beside matrix products that fill the chip, a task starts on what is left of it (about a third of the time of the
-    form that wants every SM at once, which the op takes)."""
-    n = 1 << 20
+    forms that want eight or all SMs at once, which the op takes)."""
     runtime.init("terngrad", {"enable_random": 0, "bitwidth": 2}, 0, 0, 1)
     g = gauss(n).cuda()
     B = torch.zeros(ops.terngrad_payload_bytes(n, 2), dtype=torch.uint8, device="cuda")
