@@ -338,8 +338,8 @@ void dgc_momentum_compress(torch::Tensor grad, torch::Tensor u, torch::Tensor v,
                                             local_target(out), base + kSparseOffset, at::cuda::getCurrentCUDAStream()));
 }
 
-void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,
-                       double post_scale) {
+static void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add, double post_scale,
+                              bool tiles) {
   check_f32(out, "out");
   const int64_t n = out.numel();
   TORCH_CHECK(n > 0, "empty tensor");
@@ -350,7 +350,7 @@ void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor
     // theirs.  A captured graph may run beside later calls on the stream, and takes the form without them.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     HP_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
-    unsigned int* redo = !add && capture == cudaStreamCaptureStatusNone ? redo_words_for(out) : nullptr;
+    unsigned int* redo = tiles && !add && capture == cudaStreamCaptureStatusNone ? redo_words_for(out) : nullptr;
     std::lock_guard<std::mutex> one_at_a_time(state().decode);
     HP_CHECK_CUDA(cuda::sparse_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
                                             add ? 1 : 0, float(post_scale), status_word_for(out), stream, redo));
@@ -376,6 +376,14 @@ void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor
       }
     }
   }
+}
+
+void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add, double post_scale) {
+  sparse_decompress(payloads, out, add, post_scale, /*tiles=*/true);
+}
+
+void sparse_decompress_beside(const torch::Tensor& payload, torch::Tensor out, bool add) {
+  sparse_decompress({payload}, out, add, 1.0, /*tiles=*/false);
 }
 
 // ------------------------------------------------------------------ ECQ

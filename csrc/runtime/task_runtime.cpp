@@ -373,7 +373,7 @@ void TaskRuntime::run_decompress(Task& t) {
   } else if (a.name == "tbq") {
     ops::tbq_decompress({t.B}, out, a.threshold, add, 1.0);
   } else if (a.name == "graddrop") {
-    ops::sparse_decompress({t.B.slice(0, 0, bytes)}, out, add, 1.0);
+    ops::sparse_decompress_beside(t.B.slice(0, 0, bytes), out, add);
   } else {
     TORCH_CHECK(false, "task ", t.task_id, " is not valid for algorithm ", a.name);
   }
@@ -409,7 +409,7 @@ void TaskRuntime::run_root(Task& t) {
     const bool add_to = add || i > 0;
     if (a.name == "terngrad") ops::terngrad_decompress({peers[i]}, out, add_to, 1.0, alg_.bitwidth);
     else if (a.name == "tbq") ops::tbq_decompress({peers[i]}, out, a.threshold, add_to, 1.0);
-    else if (a.name == "graddrop") ops::sparse_decompress({peers[i]}, out, add_to, 1.0);
+    else if (a.name == "graddrop") ops::sparse_decompress_beside(peers[i], out, add_to);
     else TORCH_CHECK(false, "task 30 is not valid for algorithm ", a.name);
   }
   run_compress(t);

@@ -136,30 +136,13 @@ def test_names_of_a_backlog_come_one_by_one(runtime, pinned, task):
     assert when[9] - when[0] > 0.25 * (when[-1] - when[0]), when   # 9 of 19 steps if all take the same time
 
 
-@pytest.mark.parametrize("n", [65536, 1 << 20])
-def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime, n):
-    """Beside matrix products that fill the chip, a task starts on what is left of it (about a third of the time of the
-    forms that want eight or all SMs at once, which the op takes)."""
-    runtime.init("terngrad", {"enable_random": 0, "bitwidth": 2}, 0, 0, 1)
-    g = gauss(n).cuda()
-    B = torch.zeros(ops.terngrad_payload_bytes(n, 2), dtype=torch.uint8, device="cuda")
-    C = torch.zeros(B.numel(), dtype=torch.uint8).pin_memory()
+def medians_beside_matrix_products(*calls):
+    """Median time of each call, started while products that fill the chip run on another stream."""
     a = torch.randn(16384, 16384, device="cuda").bfloat16()
     c = torch.empty_like(a)
-    side, high = torch.cuda.Stream(), torch.cuda.Stream(priority=-1)
-
-    def task():
-        runtime.submit_task("t", g, B, C, 0, runtime.COMP_TASK)
-        runtime.wait_for(runtime.COMP_TASK, ["t"])
-
-    def op():
-        with torch.cuda.stream(high):
-            ops.terngrad_compress(g, 2, False, out=B)
-            C.copy_(B, non_blocking=True)
-        high.synchronize()
-
-    median = {}
-    for call in (task, op):
+    side = torch.cuda.Stream()
+    medians = []
+    for call in calls:
         call()
         times = []
         for _ in range(9):
@@ -171,5 +154,56 @@ def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime, n):
             t = time.monotonic()
             call()
             times.append(time.monotonic() - t)
-        median[call] = sorted(times)[4]
-    assert median[task] < 0.75 * median[op], median
+        medians.append(sorted(times)[4])
+    return medians
+
+
+@pytest.mark.parametrize("n", [65536, 1 << 20])
+def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime, n):
+    """Beside matrix products that fill the chip, a task starts on what is left of it (about a third of the time of the
+    forms that want eight or all SMs at once, which the op takes)."""
+    runtime.init("terngrad", {"enable_random": 0, "bitwidth": 2}, 0, 0, 1)
+    g = gauss(n).cuda()
+    B = torch.zeros(ops.terngrad_payload_bytes(n, 2), dtype=torch.uint8, device="cuda")
+    C = torch.zeros(B.numel(), dtype=torch.uint8).pin_memory()
+    high = torch.cuda.Stream(priority=-1)
+
+    def task():
+        runtime.submit_task("t", g, B, C, 0, runtime.COMP_TASK)
+        runtime.wait_for(runtime.COMP_TASK, ["t"])
+
+    def op():
+        with torch.cuda.stream(high):
+            ops.terngrad_compress(g, 2, False, out=B)
+            C.copy_(B, non_blocking=True)
+        high.synchronize()
+
+    of_task, of_op = medians_beside_matrix_products(task, op)
+    assert of_task < 0.75 * of_op
+
+
+def test_graddrop_decode_tasks_do_not_wait_for_a_free_gpu(runtime):
+    """The same for the sparse decode, whose op works in tiles."""
+    n, drop = 1 << 20, 0.999
+    runtime.init("graddrop", {"drop_ratio": drop, "sample_rate": 0.01, "seed": 3}, 0, 0, 1)
+    r = gauss(n, seed=1).cuda()
+    B = ops.graddrop_compress(torch.zeros_like(r), r, 0.01, drop, 3)
+    C = torch.zeros(B.numel(), dtype=torch.uint8).pin_memory()
+    C.copy_(B)
+    out, want = torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+    high = torch.cuda.Stream(priority=-1)
+    torch.cuda.synchronize()
+
+    def task():
+        runtime.submit_task("t", out, r, B, C, 0, runtime.DECOMP_TASK)
+        runtime.wait_for(runtime.DECOMP_TASK, ["t"])
+
+    def op():
+        with torch.cuda.stream(high):
+            B.copy_(C, non_blocking=True)
+            ops.sparse_decompress(B, want)
+        high.synchronize()
+
+    of_task, of_op = medians_beside_matrix_products(task, op)
+    assert torch.equal(out, want)
+    assert of_task < 0.75 * of_op
