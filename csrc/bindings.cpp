@@ -174,6 +174,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("terngrad_compress", &ops::terngrad_compress, py::arg("grad"), py::arg("out"),
         py::arg("bitwidth"), py::arg("enable_random"), py::arg("seed"),
         py::arg("residual") = py::none());
+  m.def("_terngrad_resident_wait", &ops::terngrad_resident_wait);
   m.def("terngrad_decompress", &ops::terngrad_decompress, py::arg("payloads"), py::arg("out"),
         py::arg("add") = false, py::arg("post_scale") = 1.0, py::arg("bitwidth") = 0);
   m.def("dgc_momentum_compress", &ops::dgc_momentum_compress, py::arg("grad"), py::arg("u"), py::arg("v"),

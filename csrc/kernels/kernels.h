@@ -96,7 +96,9 @@ enum Status : int {
   kFlagTimeout = 1,    // a peer's flag did not reach the epoch in time
   kPayloadBounds = 2,  // a header describes more bytes / elements than the slot holds
   kBadHeader = 3,
+  kGridWait = 4,       // CTAs of one launch did not all get to run in time; what the call wrote is incomplete
 };
+constexpr uint64_t kGridWaitNs = 2000000000ull;   // of a wait of CTAs for one another
 
 // ---------------------------------------------------------------- TBQ
 // grad and residual hold n floats; each payload destination ceil(n/4) bytes.
@@ -113,11 +115,13 @@ size_t minmax_scratch_bytes();
 // residual may be null.  With a residual, the tensor quantised is grad+residual
 // and residual receives the quantisation error.  scratch must be zero before
 // its first use and is left ready for the next call.
-// whole_gpu: the call may be launched with CTAs that fill every SM at once (see tern_hold_kernel); not for
-// callers that run beside other work.
+// whole_gpu: the call may be launched with CTAs that fill every SM at once (see tern_hold_kernel), which wait
+// for one another; not for callers that run beside other work.  status: where such a wait that runs out
+// after grid_wait_ns is recorded (kGridWait); without it the call does not take that form.
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
-                              void* scratch, cudaStream_t stream, bool whole_gpu = false);
+                              void* scratch, cudaStream_t stream, bool whole_gpu = false, int* status = nullptr,
+                              uint64_t grid_wait_ns = kGridWaitNs);
 // Element count per payload is taken from its header and must equal n; all
 // payloads must carry the same bitwidth (kBadHeader otherwise).  bitwidth_hint
 // (0 = unknown) lets the launcher size the decode table for that bitwidth; a

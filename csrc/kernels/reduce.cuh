@@ -10,7 +10,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
 #include "launch.cuh"
+#include "p2p.cuh"
 
 namespace hipress {
 namespace cuda {
@@ -60,9 +62,11 @@ __device__ __forceinline__ void block_minmax(float& mn, float& mx) {
 }
 
 // Extremes over a grid whose CTAs are all resident (launch_resident): every thread of every CTA gets them.
-// The wait is bounded; false when it ran out (a CTA that is resident arrives, so it does not).
+// The wait is bounded; when it runs out (a CTA that is resident arrives, so it does not) the CTA returns false
+// after recording it in *status.  Every CTA arrives once and leaves once, whatever it saw, and the last one to
+// leave makes both counters ready for the next launch.
 template <int THREADS>
-__device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, float& mx) {
+__device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, float& mx, uint64_t wait_ns, int* status) {
   __shared__ float res[2];
   __shared__ bool arrived;
   block_minmax<THREADS>(mn, mx);
@@ -71,24 +75,30 @@ __device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, flo
     s->partial_max[blockIdx.x] = mx;
     __threadfence();
     atomicAdd(&s->counter, 1u);
-    arrived = false;
-    for (unsigned int i = 0; i < 40000000u && !arrived; ++i)   // seconds
-      arrived = *reinterpret_cast<volatile unsigned int*>(&s->counter) >= gridDim.x;
+    const uint64_t t0 = globaltimer_ns();
+    bool all = false;
+    for (unsigned int i = 1; !all; ++i) {
+      all = *reinterpret_cast<volatile unsigned int*>(&s->counter) >= gridDim.x;
+      if ((i & 255u) == 0 && globaltimer_ns() - t0 > wait_ns) break;
+    }
     __threadfence();
+    if (!all) atomicExch(status, int(kGridWait));
+    arrived = all;
   }
   __syncthreads();
-  if (!arrived) return false;
-  mn = INFINITY;
-  mx = -INFINITY;
-  for (int i = threadIdx.x; i < int(gridDim.x); i += THREADS) {
-    mn = fminf(mn, load_written(&s->partial_min[i]));
-    mx = fmaxf(mx, load_written(&s->partial_max[i]));
+  const bool ok = arrived;
+  if (ok) {
+    mn = INFINITY;
+    mx = -INFINITY;
+    for (int i = threadIdx.x; i < int(gridDim.x); i += THREADS) {
+      mn = fminf(mn, load_written(&s->partial_min[i]));
+      mx = fmaxf(mx, load_written(&s->partial_max[i]));
+    }
+    block_minmax<THREADS>(mn, mx);
   }
-  block_minmax<THREADS>(mn, mx);
   if (threadIdx.x == 0) {
     res[0] = mn;
     res[1] = mx;
-    // the last CTA to have read the partials makes the counters ready for the next launch
     __threadfence();
     if (atomicAdd(&s->left, 1u) == gridDim.x - 1) {
       s->counter = 0u;
@@ -98,7 +108,7 @@ __device__ __forceinline__ bool grid_minmax_all(MinMaxScratch* s, float& mn, flo
   __syncthreads();
   mn = res[0];
   mx = res[1];
-  return true;
+  return ok;
 }
 
 // Returns true in every thread of exactly one CTA: the last to arrive.  Before

@@ -499,7 +499,7 @@ template <int BW> struct HoldForm {
 template <int BW, bool EF>
 __global__ void __launch_bounds__(kHoldThreads, 1)
 tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int64_t part, int random,
-                 uint64_t seed, PushTargets dst, MinMaxScratch* scratch, int shift) {
+                 uint64_t seed, PushTargets dst, MinMaxScratch* scratch, int shift, uint64_t wait_ns, int* status) {
   constexpr int DPB = 8 / BW, EPT = Unit<BW>::EPT, BPT = Unit<BW>::BPT;
   extern __shared__ __align__(16) float hold[];           // [part], then the payload bytes
   __shared__ float scale[3];
@@ -538,7 +538,7 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
     mn = fminf(mn, v);
     mx = fmaxf(mx, v);
   }
-  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx)) return;
+  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status)) return;
   const PushCursor cur{nullptr};
   if (tid == 0) {
     const float gap = tern_gap(mn, mx, BW);
@@ -802,7 +802,7 @@ size_t minmax_scratch_bytes() { return sizeof(MinMaxScratch); }
 
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
-                              void* scratch, cudaStream_t stream, bool whole_gpu) {
+                              void* scratch, cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns) {
   if (n <= 0 || !tern_bitwidth_ok(bitwidth) || scratch == nullptr) return cudaErrorInvalidValue;
   auto* s = static_cast<MinMaxScratch*>(scratch);
   const bool ef = residual != nullptr;
@@ -837,7 +837,7 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
     return cudaGetLastError();
   }
   // 16-byte aligned inputs, and a part per SM that fits its shared memory
-  if (own && vec && shift >= 0) {
+  if (own && status != nullptr && vec && shift >= 0) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -853,7 +853,7 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
       e = cudaFuncSetAttribute(tern_hold_kernel<BW, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));  \
       if (e != cudaSuccess) return e;                                                                             \
       e = launch_resident(tern_hold_kernel<BW, E>, dim3(ctas), dim3(kHoldThreads), smem, stream, grad, residual,  \
-                          n, part, enable_random, seed, dst, s, shift);                                           \
+                          n, part, enable_random, seed, dst, s, shift, grid_wait_ns, status);                     \
       if (e != cudaErrorCooperativeLaunchTooLarge) return e;                                                      \
       cudaGetLastError();   /* fewer SMs than the device has: the two launches below */                           \
     }                                                                                                             \

@@ -230,7 +230,8 @@ static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int6
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
     HP_CHECK_CUDA(cuda::terngrad_compress(grad.data_ptr<float>(), res, n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed), local_target(out),
-                                          scratch, at::cuda::getCurrentCUDAStream(), whole_gpu));
+                                          scratch, at::cuda::getCurrentCUDAStream(), whole_gpu,
+                                          whole_gpu ? status_word_for(grad) : nullptr));
   } else {
     const int rc = cpu::terngrad_compress(grad.data_ptr<float>(), n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed),
@@ -242,6 +243,17 @@ static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int6
 void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
                        bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual) {
   terngrad_compress(grad, out, bitwidth, enable_random, seed, residual, /*whole_gpu=*/true);
+}
+
+int64_t terngrad_resident_wait(const torch::Tensor& grad, torch::Tensor out, torch::Tensor scratch, int64_t wait_us) {
+  TORCH_CHECK(grad.is_cuda() && scratch.is_cuda() && size_t(scratch.nbytes()) >= cuda::minmax_scratch_bytes(), "scratch too small");
+  TORCH_CHECK(out.numel() == tern_payload_bytes(grad.numel(), 2), "out must have the payload's size");
+  c10::cuda::CUDAGuard guard(grad.device());
+  auto status = torch::zeros({1}, grad.options().dtype(torch::kInt32));
+  HP_CHECK_CUDA(cuda::terngrad_compress(grad.data_ptr<float>(), nullptr, grad.numel(), 2, 0, 0, local_target(out),
+                                        scratch.data_ptr(), at::cuda::getCurrentCUDAStream(), true,
+                                        status.data_ptr<int>(), uint64_t(wait_us) * 1000));
+  return status.item<int>();
 }
 
 void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,

@@ -29,6 +29,9 @@ void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
 
 void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
                        bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual);
+// For tests: a 2-bit payload by the form whose CTAs wait for one another, at most wait_us microseconds, with
+// scratch state of the caller's; returns the status word.
+int64_t terngrad_resident_wait(const torch::Tensor& grad, torch::Tensor out, torch::Tensor scratch, int64_t wait_us);
 // The same for a stream beside which the caller's own work runs: it does not ask for all SMs at once.
 void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
                               int64_t seed);

@@ -316,7 +316,7 @@ class CompressedDataParallel(nn.Module):
         status = self.engine.check_status()
         if status != 0:
             names = {1: "a peer's flag was not published in time", 2: "payload exceeds its slot",
-                     3: "malformed payload header"}
+                     3: "malformed payload header", 4: "CTAs of one launch waited too long for one another"}
             raise RuntimeError(f"hipress engine: {names.get(status, status)}")
 
     # ------------------------------------------------------------------ state

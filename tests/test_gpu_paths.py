@@ -322,6 +322,23 @@ def test_terngrad_resident_form(bw, feedback, offset):
             assert torch.equal(rg.cpu(), rc), n
 
 
+def test_terngrad_resident_form_when_its_wait_runs_out():
+    """A counter that starts one short: no CTA ever sees all others arrive.  The wait ends, the status word says so, and
+    the next call finds its state ready."""
+    from hipress_b200 import _C
+    n = 300007
+    g = gauss(n, seed=1).cuda()
+    want = ops.terngrad_compress(g, 2, False)
+    scratch = torch.zeros(1 << 14, dtype=torch.uint8, device="cuda")
+    scratch[:4] = 255
+    out = torch.full_like(want, 7)
+    assert _C._terngrad_resident_wait(g, out, scratch, 20000) == 4
+    assert int((out != 7).sum()) == 0
+    assert int(scratch[:8].sum()) == 0
+    assert _C._terngrad_resident_wait(g, out, scratch, 2000000) == 0
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("n", [4096, 300007])
 def test_terngrad_one_launch_forms_under_capture(n):
     g = gauss(n, seed=1).cuda()
