@@ -143,7 +143,7 @@ size_t sparse_scratch_bytes(int64_t n);
 // Each destination needs 4 + 8*ceil(n*keep_fraction) bytes.
 cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sample_rate,
                             double keep_fraction, uint64_t seed, int accumulate,
-                            const PushTargets& dst, void* scratch, cudaStream_t stream);
+                            const PushTargets& dst, void* scratch, cudaStream_t stream, int* status = nullptr);
 // The same compressor with the codec's state update fused into its one pass over the tensor.
 //   mode 0  plain: select from R as it is (DGC without momentum correction)
 //   mode 1  GradDrop: R += grad, then select from R
@@ -154,7 +154,8 @@ cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sampl
 //           payloads afterwards, which saves the separate clearing pass.
 // For keep fractions up to 1 % the tensor is read once ("list form", see sparse.cu); otherwise,
 // or when the scratch cannot hold the expected candidates, the multi-pass scan form runs.
-// scratch: sparse_scratch_bytes(n) bytes, zero before its first use.
+// scratch: sparse_scratch_bytes(n) bytes, zero before its first use.  status: where a wait between CTAs that
+// runs out is recorded (kGridWait).
 struct SparseFuse {
   int mode = 0;
   const float* grad = nullptr;
@@ -165,7 +166,7 @@ struct SparseFuse {
 };
 cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, double sample_rate,
                                   double keep_fraction, uint64_t seed, const PushTargets& dst, void* scratch,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, int* status = nullptr);
 // {elements emitted, candidates over the sampled threshold (list form), threshold as float bits,
 // candidates dropped so far for lack of pool space} of the last call on `scratch`; asynchronous
 // copies to host4 on `stream`.

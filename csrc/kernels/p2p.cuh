@@ -200,8 +200,9 @@ inline int chunk_shift(const PushTargets& t, int data_off) {
 // is bumped; the last CTA fences again after observing every other CTA's bump
 // and only then releases the flags.  With a single local destination the
 // consumer is on this GPU and device scope is enough.  The counter is left at
-// zero for the next launch.
-__device__ __forceinline__ void publish_when_grid_done(const PushTargets& t) {
+// zero for the next launch.  failed: a word that a CTA sets, before it gets here,
+// when the payload will not be whole; the flag is then not published.
+__device__ __forceinline__ void publish_when_grid_done(const PushTargets& t, const unsigned int* failed = nullptr) {
   if (t.done == nullptr) return;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -212,6 +213,7 @@ __device__ __forceinline__ void publish_when_grid_done(const PushTargets& t) {
     if (prev == total - 1) {
       if (remote) __threadfence_system(); else __threadfence();
       *t.done = 0u;
+      if (failed != nullptr && *reinterpret_cast<const volatile unsigned int*>(failed) != 0u) return;
 #pragma unroll
       for (int p = 0; p < kMaxWorld; ++p)
         if (p < t.world && t.flag[p] != nullptr) st_release_sys(t.flag[p], t.epoch);

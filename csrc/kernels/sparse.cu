@@ -86,6 +86,7 @@ struct SparseScratch {
     unsigned int exact[kExactBins];    // keys inside the bin that holds the cut
     unsigned long long agg[kMaxBlocks];  // write kernel: what each chunk keeps, once known
     unsigned int ticket;               // write kernel: chunks handed out
+    unsigned int gave_up;              // a wait of the write kernel ran out (see there)
     unsigned int trim_done[2];         // CTA arrivals of the trim kernels
     unsigned int t_prefix, t_rank;     // progress of the trim digits
     unsigned int clipped;              // the cut lies in the last fine bin
@@ -101,7 +102,6 @@ struct SparseScratch {
   unsigned int k;                       // elements emitted
   unsigned int dropped;                 // candidates that found no block (cumulative)
   unsigned int last_cand;               // candidates seen by the last call (metrics)
-  unsigned int gave_up;                 // waits of the write kernel that ran out (never, see there)
   unsigned int off_gt[kMaxBlocks], off_eq[kMaxBlocks];
   unsigned int list_head[kMaxLists];    // first block of each warp's list, kNoBlock when empty
 };
@@ -540,25 +540,27 @@ trim_kernel(const float* R, int64_t n, int64_t chunk, unsigned int expected, Spa
 // min(ties kept, elements equal to the cut before it).  A chunk's starting counts are what the chunks
 // before it keep: every CTA publishes its own counts as soon as it has them and adds up those of its
 // predecessors.  Chunks are handed out by a ticket, so the ones waited for belong to CTAs that already
-// run, and each publishes before it waits: the wait ends.  (It is bounded all the same.)
+// run, and each publishes before it waits: the wait ends.  It is bounded all the same; a CTA whose wait runs
+// out records kGridWait, delivers nothing and clears nothing, and the payload's flag is not published.
 // Inside the CTA each warp owns a contiguous part of the chunk: a first walk counts what the warp will
 // emit, one barrier turns the counts into per-warp offsets, and a second walk (its data now in L1 / L2)
 // emits with warp-level ballots only.
 // 25 MB, 6.25 % kept (ncu, cold): 50 us when every lane stored its own entries, 28 now.
 constexpr unsigned long long kAggReady = 1ull << 62;
-constexpr uint64_t kAggWaitNs = 2000000000ull;
 __global__ void __launch_bounds__(kThreads)
 write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t chunk, unsigned int expected,
-             PushTargets dst, SparseScratch* s) {
+             PushTargets dst, SparseScratch* s, int* status) {
   wait_for_previous();
   resolve_epoch(dst);
   constexpr int kWarps = kThreads / 32;
   __shared__ unsigned int warp_gt[kWarps], warp_eq[kWarps], before_gt, before_eq;
+  __shared__ bool gave_up;
   __shared__ uint2 packs[kWarps][512];
   __shared__ int ticket;
   if (threadIdx.x == 0) {
     ticket = int(atomicAdd(&s->call.ticket, 1u));
     before_gt = before_eq = 0;
+    gave_up = false;
   }
   const uint32_t cut = s->call.cut_key;
   const unsigned int ties = s->call.ties_kept;
@@ -652,8 +654,8 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
   for (int b = threadIdx.x; b < block; b += kThreads) {
     unsigned long long v;
     while (((v = *reinterpret_cast<volatile unsigned long long*>(&s->call.agg[b])) & kAggReady) == 0) {
-      if (globaltimer_ns() - t0 > kAggWaitNs) {
-        s->gave_up = 1u;
+      if (globaltimer_ns() - t0 > kGridWaitNs) {
+        gave_up = true;
         break;
       }
     }
@@ -670,6 +672,14 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
     atomicAdd(&before_eq, add_eq);
   }
   __syncthreads();
+  if (gave_up) {
+    if (threadIdx.x == 0) {
+      s->call.gave_up = 1u;
+      if (status != nullptr) atomicExch(status, int(kGridWait));
+    }
+    publish_when_grid_done(dst, &s->call.gave_up);
+    return;
+  }
   unsigned int run_gt = before_gt, run_eq = before_eq;
   for (int w = 0; w < warp; ++w) {
     run_gt += warp_gt[w];
@@ -748,7 +758,7 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
       run_kept += held;
     }
   }
-  publish_when_grid_done(dst);
+  publish_when_grid_done(dst, &s->call.gave_up);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -1582,7 +1592,7 @@ size_t sparse_scratch_bytes(int64_t n) { return list_plan(n < 1 ? 1 : n).total_b
 
 cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, double sample_rate,
                                   double keep_fraction, uint64_t seed, const PushTargets& dst, void* scratch,
-                                  cudaStream_t stream) {
+                                  cudaStream_t stream, int* status) {
   if (n <= 0 || n > 0x7fffffff || scratch == nullptr || R == nullptr) return cudaErrorInvalidValue;
   if (fuse.mode < 0 || fuse.mode > 2 || (fuse.mode >= 1 && fuse.grad == nullptr) || (fuse.mode == 2 && fuse.u == nullptr))
     return cudaErrorInvalidValue;
@@ -1674,16 +1684,17 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
   if (e == cudaSuccess)
     e = launch_after(trim_kernel<1>, grid, block, 0, stream, static_cast<const float*>(R), n, pl.chunk, unsigned(expected), s);
   if (e != cudaSuccess) return e;
-  return launch_after(write_kernel, grid, block, 0, stream, R, u_mask, sumsq, n, pl.chunk, unsigned(expected), dst, s);
+  return launch_after(write_kernel, grid, block, 0, stream, R, u_mask, sumsq, n, pl.chunk, unsigned(expected), dst, s,
+                      status);
 }
 
 cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sample_rate,
                             double keep_fraction, uint64_t seed, int accumulate,
-                            const PushTargets& dst, void* scratch, cudaStream_t stream) {
+                            const PushTargets& dst, void* scratch, cudaStream_t stream, int* status) {
   SparseFuse fuse;
   fuse.mode = accumulate ? 1 : 0;
   fuse.grad = accumulate ? grad : nullptr;
-  return sparse_compress_fused(fuse, R, n, sample_rate, keep_fraction, seed, dst, scratch, stream);
+  return sparse_compress_fused(fuse, R, n, sample_rate, keep_fraction, seed, dst, scratch, stream, status);
 }
 
 // Counters of the last compress call that used `scratch`: {elements emitted, candidates over the

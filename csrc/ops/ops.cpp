@@ -311,7 +311,7 @@ void sparse_compress(const c10::optional<torch::Tensor>& grad, torch::Tensor R, 
     void* scratch = static_cast<uint8_t*>(scratch_for(R, kSparseOffset + cuda::sparse_scratch_bytes(n))) + kSparseOffset;
     HP_CHECK_CUDA(cuda::sparse_compress(g, R.data_ptr<float>(), n, sample_rate, keep_fraction,
                                         uint64_t(seed), accumulate ? 1 : 0, local_target(out),
-                                        scratch, at::cuda::getCurrentCUDAStream()));
+                                        scratch, at::cuda::getCurrentCUDAStream(), status_word_for(R)));
   } else {
     const int64_t rc = cpu::sparse_compress(g, R.data_ptr<float>(), n, sample_rate, keep_fraction,
                                             uint64_t(seed), accumulate ? 1 : 0,
@@ -347,7 +347,8 @@ void dgc_momentum_compress(torch::Tensor grad, torch::Tensor u, torch::Tensor v,
   fuse.sumsq = reinterpret_cast<float*>(base + kSumsqOffset);
   fuse.zero_grad = zero_grad ? 1 : 0;
   HP_CHECK_CUDA(cuda::sparse_compress_fused(fuse, v.data_ptr<float>(), n, sample_rate, keep_fraction, uint64_t(seed),
-                                            local_target(out), base + kSparseOffset, at::cuda::getCurrentCUDAStream()));
+                                            local_target(out), base + kSparseOffset, at::cuda::getCurrentCUDAStream(),
+                                            status_word_for(v)));
 }
 
 static void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add, double post_scale,
