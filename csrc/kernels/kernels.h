@@ -155,7 +155,7 @@ cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sampl
 // For keep fractions up to 1 % the tensor is read once ("list form", see sparse.cu); otherwise,
 // or when the scratch cannot hold the expected candidates, the multi-pass scan form runs.
 // scratch: sparse_scratch_bytes(n) bytes, zero before its first use.  status: where a wait between CTAs that
-// runs out is recorded (kGridWait).
+// runs out is recorded (kGridWait).  launches: the kernels launched are added to it.
 struct SparseFuse {
   int mode = 0;
   const float* grad = nullptr;
@@ -166,7 +166,7 @@ struct SparseFuse {
 };
 cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, double sample_rate,
                                   double keep_fraction, uint64_t seed, const PushTargets& dst, void* scratch,
-                                  cudaStream_t stream, int* status = nullptr);
+                                  cudaStream_t stream, int* status = nullptr, int* launches = nullptr);
 // {elements emitted, candidates over the sampled threshold (list form), threshold as float bits,
 // candidates dropped so far for lack of pool space} of the last call on `scratch`; asynchronous
 // copies to host4 on `stream`.

@@ -1592,7 +1592,7 @@ size_t sparse_scratch_bytes(int64_t n) { return list_plan(n < 1 ? 1 : n).total_b
 
 cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, double sample_rate,
                                   double keep_fraction, uint64_t seed, const PushTargets& dst, void* scratch,
-                                  cudaStream_t stream, int* status) {
+                                  cudaStream_t stream, int* status, int* launches) {
   if (n <= 0 || n > 0x7fffffff || scratch == nullptr || R == nullptr) return cudaErrorInvalidValue;
   if (fuse.mode < 0 || fuse.mode > 2 || (fuse.mode >= 1 && fuse.grad == nullptr) || (fuse.mode == 2 && fuse.u == nullptr))
     return cudaErrorInvalidValue;
@@ -1648,6 +1648,8 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
     e = cudaMemsetAsync(&s->call, 0, sizeof(s->call), stream);   // every non-zero element is a candidate
   }
   if (e != cudaSuccess) return e;
+  if (launches != nullptr)   // the norm; the sample and its selection; the list form's kernels or the scan form's
+    *launches += (sumsq != nullptr ? 1 : 0) + (sample_cnt > 0 ? (keys != nullptr ? 2 : 3) : 0) + (lists ? 3 : 4);
   const dim3 grid = dim3(unsigned(pl.blocks));
   float* const u_mask = fuse.mode == 2 ? fuse.u : nullptr;
   if (lists) {

@@ -646,9 +646,8 @@ void DdpEngine::issue_push(int b, int worker) {
       }
       void* sparse_scratch = static_cast<uint8_t*>(w.scratch) + 16384;
       check(cuda::sparse_compress_fused(fuse, res, n, cfg_.sample_rate, keep_fraction_, seed, dst, sparse_scratch,
-                                        w.push, status_),
+                                        w.push, status_, &launched),
             "sparse_compress");
-      launched += (keep_fraction_ <= 0.01 ? 5 : 6) + (fuse.mode == 2 && fuse.clip > 0.f ? 1 : 0);
       if (sparse_stats_host_)
         check(cuda::sparse_read_stats(sparse_scratch, sparse_stats_host_ + 4 * b, w.push), "sparse stats");
       break;

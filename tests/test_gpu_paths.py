@@ -456,3 +456,62 @@ def test_sparse_decode_from_two_threads_on_one_stream():
     for _, ref, outs in jobs:
         for o in outs:
             assert torch.equal(o.cpu(), ref)
+
+
+# ----------------------------------------------------------------------------- launch counts
+def kernels_of(call):
+    """Kernels that a call launches: the kernel nodes of its captured graph."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()               # the stream's scratch exists from here on
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    raw = runtime.cudaGraph_t(init_value=graph.raw_cuda_graph())
+    _, _, count = runtime.cudaGraphGetNodes(raw)
+    _, nodes, count = runtime.cudaGraphGetNodes(raw, count)
+    return sum(runtime.cudaGraphNodeGetType(x)[1] == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in nodes[:count])
+
+
+@pytest.mark.parametrize("codec,n,kw", [
+    ("terngrad", 65536, {}), ("terngrad", 300000, {}), ("graddrop", 400000, dict(keep_fraction=0.001, sample_rate=0.01)),
+    ("graddrop", 400000, dict(keep_fraction=0.02, sample_rate=0.01)),
+    ("graddrop", 400000, dict(keep_fraction=0.02, sample_rate=0.05)),
+    ("graddrop", 400000, dict(keep_fraction=0.02, sample_rate=0.0)),
+    ("graddrop", 400000, dict(keep_fraction=0.02, sample_rate=0.01, momentum_correction=1, dgc_clip=1.0))])
+def test_engine_counts_the_kernels_it_launches(codec, n, kw):
+    """Push half of one rank's bucket, against the kernels of the same compression captured on its own."""
+    import hipress_b200 as hp
+    from hipress_b200.parallel import SymmetricMemory
+    grad, res, aux = (gauss(n, seed=s).cuda() for s in range(3))
+
+    def push_launches(codec, **kw):
+        e = hp._C.DdpEngine(dict(rank=0, world=1, device=0, codec=codec, seed=3, flag_timeout_s=2.0, defer_recv=1, **kw),
+                            [(0, n, 1)], [0])
+        m = SymmetricMemory.emulate(e.symmetric_bytes, 1)[0]
+        e.set_buffers(grad, res, None, None, aux)
+        e.set_symmetric(m.buf)
+        e.set_sgd(0.0, 0.0, 0.0, False)
+        e.begin_step()
+        before = e.launches
+        e.bucket_ready(0, 0)
+        e.drain()
+        count = e.launches - before
+        torch.cuda.synchronize()
+        e.finish_step(0)
+        torch.cuda.synchronize()
+        assert e.check_status() == 0
+        return count
+
+    if codec == "terngrad":
+        want = 2     # one launch is for callers that have the GPU to themselves
+    elif kw.get("momentum_correction"):
+        out = torch.zeros(ops.sparse_payload_bytes(n, kw["keep_fraction"]), dtype=torch.uint8, device="cuda")
+        want = kernels_of(lambda: ops.dgc_momentum_compress(grad, aux, res, kw["sample_rate"], kw["keep_fraction"], 3,
+                                                            momentum=0.9, clip=1.0, out=out))
+    else:
+        out = torch.zeros(ops.sparse_payload_bytes(n, 1 - (1 - kw["keep_fraction"])), dtype=torch.uint8, device="cuda")
+        want = kernels_of(lambda: ops.graddrop_compress(grad, res, kw["sample_rate"], 1 - kw["keep_fraction"], 3, out=out))
+    assert push_launches(codec, **kw) == want
