@@ -291,13 +291,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
 
   // number of raw values in [start, start + count*stride) for which the reciprocal-multiply
-  // form of the unit draw differs from the reference's division form (expected: 0)
+  // form of the unit draw, or the form that the device uses, differs from the reference's division
+  // form (expected: 0)
   m.def("lcg_unit_mismatches", [](uint64_t start, uint64_t count, uint64_t stride) {
     uint64_t bad = 0;
     for (uint64_t i = 0; i < count; ++i) {
       const uint32_t raw = uint32_t(start + i * stride);
-      const float a = Lcg32::unit_from_raw(raw), b = Lcg32::unit_from_raw_by_division(raw);
-      bad += std::memcmp(&a, &b, 4) != 0;
+      const float a = Lcg32::unit_from_raw_in_double(raw), b = Lcg32::unit_from_raw_by_division(raw);
+      const float c = Lcg32::unit_from_raw_in_single(raw);
+      bad += std::memcmp(&a, &b, 4) != 0 || std::memcmp(&c, &b, 4) != 0;
     }
     return bad;
   });

@@ -22,20 +22,27 @@ struct Lcg32 {
   // rounds to float, float(double(raw) / 4294967295.0), so the top 129 raw
   // values come out as exactly 1.0f (naive_random.hpp:53-69 with bounds (0,1)).
   // Multiplying by the double reciprocal instead gives the same float for every
-  // one of the 2^32 raw values (checked exhaustively) and costs one double
-  // multiply where the division costs a long instruction sequence on the GPU.
+  // one of the 2^32 raw values and costs one double multiply where the division
+  // costs a long instruction sequence on the GPU.
   HP_HD float next_unit() { return unit_from_raw(next()); }
-  //
-  // On the device the multiply goes through conversions to and from double, which run at an eighth of
-  // the rate of the rest.  raw / (2^32 - 1) is raw * 2^-32 plus a little less than one unit of the last
-  // integer place, so it rounds to 24 bits like the integer with its lowest bit set, as long as two bits
-  // or more are dropped (raw >= 2^25); next to 2^32 the product's own rounding to double shows, and both
-  // ends take the formula (checked exhaustively too).
   HP_HD static float unit_from_raw(uint32_t raw) {
 #if defined(__CUDA_ARCH__)
-    if (raw - 0x02000000u < 0xfdfffc00u) return __fmul_rn(__uint2float_rn(raw | 1u), 2.3283064365386963e-10f);
+    return unit_from_raw_in_single(raw);
+#else
+    return unit_from_raw_in_double(raw);
 #endif
+  }
+  HP_HD static float unit_from_raw_in_double(uint32_t raw) {
     return static_cast<float>(hp_dmul(static_cast<double>(raw), 1.0 / 4294967295.0));
+  }
+  // For the device, where conversions to and from double run at an eighth of the rate of the rest.
+  // raw / (2^32 - 1) is raw * 2^-32 plus a little less than one unit of the last integer place, so it
+  // rounds to 24 bits like the integer with its lowest bit set, as long as two bits or more are dropped
+  // (raw >= 2^25); next to 2^32 the product's own rounding to double shows, and both ends take the formula.
+  // The conversion rounds to nearest and the multiplication is exact.
+  HP_HD static float unit_from_raw_in_single(uint32_t raw) {
+    if (raw - 0x02000000u < 0xfdfffc00u) return static_cast<float>(raw | 1u) * 2.3283064365386963e-10f;
+    return unit_from_raw_in_double(raw);
   }
   HP_HD static float unit_from_raw_by_division(uint32_t raw) {
     return static_cast<float>(hp_ddiv(static_cast<double>(raw), 4294967295.0));

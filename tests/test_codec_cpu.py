@@ -38,6 +38,17 @@ def test_lcg_unit_draw_multiply_equals_division():
     assert C.lcg_unit_mismatches((1 << 31) - (1 << 15), 1 << 16, 1) == 0
 
 
+def test_lcg_unit_draw_of_the_device_where_its_form_changes():
+    # the device converts in single precision between 2^25 and 2^32 - 2^10 and in double outside; the counter looks at
+    # both forms (all 2^32 values: 0 mismatches, 10 s)
+    C = hp._C
+    for edge in (1 << 25, (1 << 32) - (1 << 10) - (1 << 15)):
+        assert C.lcg_unit_mismatches(edge - (1 << 15), 1 << 16, 1) == 0
+    for power in range(1, 32):      # where the number of dropped bits changes
+        assert C.lcg_unit_mismatches(max(0, (1 << power) - 512), 1024, 1) == 0
+    assert C.lcg_unit_mismatches(12345, 1 << 24, 255) == 0
+
+
 # ----------------------------------------------------------------------------- TBQ
 def test_tbq_hand_vector():
     # g[i] = (i-5)*0.004, t = 0.01, N = 10 -> bytes 40 55 5a (hand-derived from tbq_body.h:70-87)
