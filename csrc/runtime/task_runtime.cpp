@@ -5,8 +5,10 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <chrono>
 #include <cmath>
 #include <deque>
+#include <thread>
 
 #include "../common/host_utils.h"
 #include "../ops/ops.h"
@@ -130,7 +132,8 @@ std::vector<std::string> TaskRuntime::wait_results(int task_id, double timeout_s
     case kDecompTask: case kPowerSgdDecode:
     case kRootDecompCompTask: case kPowerSgdEncode2:
       return queue_for(task_id).wait_drain(timeout_s, seen);
-    default:
+    default:   // no task has such an id: nothing will come
+      std::this_thread::sleep_for(std::chrono::duration<double>(timeout_s));
       return {};
   }
 }

@@ -45,6 +45,16 @@ def test_wait_ends_on_error_and_on_timeout():
 
 
 @pytest.mark.timeout(60)
+def test_wait_for_an_unknown_kind_of_task_sleeps():
+    hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+    cpu = time.process_time()
+    with pytest.raises(TimeoutError):
+        hp_cuda.wait_for(99, ["never"], timeout_s=1.0)
+    assert time.process_time() - cpu < 0.5
+    hp_cuda.end()
+
+
+@pytest.mark.timeout(60)
 def test_names_do_not_wait_for_the_interpreter():
     """A name is out when its task is done, also while some Python code keeps the interpreter lock."""
     hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
