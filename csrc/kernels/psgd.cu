@@ -411,7 +411,7 @@ constexpr int kGsThreads = 1024;
 // Factors of up to 1024 * Q rows stay in registers: a thread holds Q rows of the (up to) R columns.  A
 // reduction is then a warp shuffle, one barrier, and a second shuffle over the 32 warps' sums, which every
 // warp does for itself.
-// 4096 x 4 (ncu, cold): 24.9 us with one reduction per column pair and the matrix in memory, 13.8 now.
+// 4096 x 4 (ncu, cold): 13.8 us; 24.9 with one reduction per column pair and the matrix in memory.
 template <int R, int Q>
 __device__ __forceinline__ void gs_in_registers(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt,
                                                 int64_t rows_pad, float (*part)[32][16] /* [2] */) {
@@ -747,8 +747,8 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
 // in flight.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across
 // the warps in shared memory.  Few rows are also split by columns; the parts then meet in P by atomics,
 // which the launcher zeroes first.
-// 4096 x 4096, rank 4 (ncu, cold): add 28.9 + zero 2.5 + transpose 3.5 + tensor-core projection
-// 15.2 us before, 32 us now; error of the three stages against 64 bits 8.4e-4 before, 7.3e-4 now.
+// 4096 x 4096, rank 4 (ncu, cold): 32 us; as add 28.9, zero 2.5, transpose 3.5 and tensor-core projection
+// 15.2.  Error of the three stages against 64 bits 7.4e-4, and 8.4e-4 with the projection in tf32.
 template <int R>
 __global__ void __launch_bounds__(256, 2)
 add_project_kernel(const float* __restrict__ grad, const float* __restrict__ residual, int64_t N, float* __restrict__ Mat,

@@ -39,12 +39,12 @@
 //
 // The kernels of a call overlap at their ends (launch.cuh): at 25 MB none but the pass over the tensor
 // takes longer than the gap between two plain launches.
-// 64 MB, GradDrop at 0.1 %, compress and decode: 129 us with eight plain launches, 112 now;
-// 25 MB, DGC: 102 and 81 us.
+// Compress and decode, 64 MB, GradDrop at 0.1 %, four payloads: 112 us, and 129 as eight plain launches (the
+// same decode); 25 MB, DGC, eight payloads: 82 and 102.
 //
 // A sample of more than a hundredth of the elements does not fit the key array; its keys are then drawn
-// again in each of three rounds, one per digit.  The pool is sized for many times the expected number of candidates (see
-// list_plan); should it still run out, the candidates that did not fit stay in the residual
+// again in each of three rounds, one per digit.  The pool is sized for many times the expected number of
+// candidates (see list_plan); should it still run out, the candidates that did not fit stay in the residual
 // and are sent in a later step (counted in SparseScratch::dropped).
 #include "../common/codec_math.h"
 #include "adamw.cuh"
@@ -545,7 +545,7 @@ trim_kernel(const float* R, int64_t n, int64_t chunk, unsigned int expected, Spa
 // Inside the CTA each warp owns a contiguous part of the chunk: a first walk counts what the warp will
 // emit, one barrier turns the counts into per-warp offsets, and a second walk (its data now in L1 / L2)
 // emits with warp-level ballots only.
-// 25 MB, 6.25 % kept (ncu, cold): 50 us when every lane stored its own entries, 28 now.
+// 25 MB, 6.25 % kept (ncu, cold): 28 us; 50 when every lane stores its own entries.
 constexpr unsigned long long kAggReady = 1ull << 62;
 __global__ void __launch_bounds__(kThreads)
 write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t chunk, unsigned int expected,
@@ -792,7 +792,7 @@ scatter_kernel(const uint8_t* __restrict__ payload, int64_t cap, float* __restri
 
 // ================================================================ list form
 // Pool of list blocks, behind the sample keys in the scratch: block b holds count[b] (index,
-// value bits) pairs in entry[b * 16 ..] and continues in block next[b].  
+// value bits) pairs in entry[b * 16 ..] and continues in block next[b].
 struct ListPool {
   unsigned int* count;
   unsigned int* next;
@@ -1004,7 +1004,7 @@ collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScr
 // Two digits of the distance from the threshold (2,048 bins of 4,096 keys: one octave above it, then the
 // keys of one bin) find the cut of ordinary data, and they spread: the leading bits of the keys themselves
 // are nearly all the same, which costs either colliding atomics or a match instruction per warp (38 us for
-// the 17,000 candidates of a 64 MB tensor, 21 us now).  Only when the cut lies in the last bin are the
+// the 17,000 candidates of a 64 MB tensor; 21 us by distance).  Only when the cut lies in the last bin are the
 // three digits of the keys counted.
 constexpr int kCutThreads = 1024;
 constexpr int kCutCluster = 8;
@@ -1265,13 +1265,14 @@ emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScr
 //
 // What bounds it: the dense store, and below a few MB the chain header -> search -> entries (about
 // 2 us).  It replaces a memset and one scatter per rank, which cost a launch each and, from a
-// thousandth of the elements up, a read and a write of the same 32-byte sectors per rank:
-// 25 MB of eight payloads at 0.1 %, compress and decode together: 120 us with the scatters, 102 us in one pass.
+// thousandth of the elements up, a read and a write of the same 32-byte sectors per rank: 25 MB at 0.1 %, one
+// call waited for: eight payloads 37 us, 72 with the scatters; one payload 31 and 30.
 //
 // A payload whose indices do not ascend is still decoded: the segments that the searches return for
 // neighbouring tiles share their ends, so they cut the payload into consecutive pieces, and an entry
 // outside its tile's range is seen by the tile that got it.  That tile raises `redo`, and the kernel
-// behind decodes everything again without assuming an order.
+// behind decodes everything again without assuming an order.  An index past the end is reported by the tile
+// that meets it.
 constexpr int kDenseTile = 8192;   // elements: 32 KB, six CTAs per SM
 
 // For both x: the first position in idx[0, k) whose value is not below it, for ascending idx below n; for
@@ -1455,9 +1456,9 @@ dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int til
 // ---- decode and optimizer step in one pass
 // When nobody keeps the dense gradient, the tile goes straight into the update of its parameters: the
 // gradient is neither written nor read (4 of AdamW's 28 bytes per element) nor cleared afterwards, and
-// one pass takes the place of a scatter per rank, the dense update and the clearing pass:
-// a BERT-large step (11 buckets, 335 M parameters, one GPU): 19.93 ms with the scatter, the dense
-// update and the clearing pass, 19.66 in one pass.
+// one pass takes the place of a scatter per rank, the dense update and the clearing pass.
+// Receive half of a 128 MB bucket at 0.1 %, by the host's clock: AdamW with eight payloads 204 us, 249 with the
+// scatters, the dense update and the clearing pass; with one payload 187 and 192.  SGD: 135 and 220, 121 and 165.
 // An update cannot be taken back, so the payloads are looked at first: sparse_check_kernel records any
 // index that does not ascend or lies outside, and the update kernel returns on a recorded failure, as the
 // dense ones do.  OPT: 0 = SGD with momentum, 1 = AdamW.

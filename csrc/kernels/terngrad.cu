@@ -210,9 +210,8 @@ __device__ __forceinline__ void tern_leftover(const float* grad, float* residual
 // destination, against the 32 bytes per warp of the word path, which is what NVLink peer stores need
 // to run near link speed, and half the instructions.  The rest of the tensor (less than one chunk)
 // takes the word path.  A payload at the start of a tensor has its packed data 10 bytes past a
-// boundary:
-// compress and decode of 9.4 MB at 4 bits 20.5 us with 2-byte stores, 18.4 now; of 25 MB
-// with ECQ 56.8 and 52.6 us (both with the cheaper draws of Lcg32::unit_from_raw).
+// boundary: against 2-byte stores, and together with the cheaper draws of Lcg32::unit_from_raw, chunks save 2 us of
+// compressing 9.4 MB at 4 bits in two launches and 4 us of 25 MB with ECQ.
 template <int BW, bool VEC, bool EF>
 __global__ void __launch_bounds__(kThreads)
 tern_quant_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n,
@@ -484,8 +483,8 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
 // exchange engine and the task API, whose compressors run beside the backward pass, keep the two launches.
 // Beside a chain of 16384^3 matrix products a 4 MB task takes 850 us in this form (it waits for SMs to fall
 // free) and 260 in two launches; on an idle GPU 64 and 71 us.
-// 25 MB with error feedback, 2 bits (ncu, cold): 14.3 + 18.0 us in two launches, 21.6 in one; with the
-// decode of eight payloads 63.4 and 55.4 us, and 9.4 MB at 4 bits 18.4 and 14.4 us.
+// 25 MB with error feedback, 2 bits (ncu, cold): 21.3 us; 14.3 + 18.0 in two launches.  9.4 MB at 4 bits, compress
+// and decode: 14.4 and 18.4.
 constexpr int kHoldThreads = 1024;
 constexpr size_t kHoldBytes = 208 * 1024;    // of grad + residual per CTA
 template <int BW> struct HoldForm {
@@ -836,7 +835,7 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
 #undef LAUNCH_SMALL
     return cudaGetLastError();
   }
-  // 16-byte aligned inputs, and a part per SM that fits its shared memory
+  // 16-byte aligned inputs, and a part per SM that fits its shared memory: one read of them
   if (own && status != nullptr && vec && shift >= 0) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);

@@ -303,10 +303,9 @@ __device__ __forceinline__ void unpack_nibble_body(const float* lut, uint32_t (&
 // A lane loads 32 payload bits of each rank, turns the words of a group into one index byte per element
 // (a shift and a bit select per field, then a byte transposition), and writes those bytes to a buffer of
 // its warp; the lanes read them back so that every dense access is a 512-byte run across the warp.
-// The form before this one read a table entry per pair of ranks and two elements, with bank conflicts,
-// and moved every index word by shuffle:
-// 4 bits, one payload, 2.4 M elements (ncu, cold): 15.8 us before, 6.4 now; 2 bits, eight payloads, 25 MB: 26.6
-// and 17.3.
+// A table entry per pair of ranks and two elements, with bank conflicts and every index word moved by shuffle,
+// is the alternative.  2 bits, eight payloads, 25 MB (ncu, cold): 17.3 us, and 26.6 by pairs; 4 bits, one
+// payload, 2.4 M elements: 6.4, and 15.8 by nibble tables.
 // Threads per CTA and CTAs per SM.  Eight payloads' tables and index buffers take 80 KB: two CTAs of 512
 // threads that share them, because two of 256 leave four warps per scheduler, too few to cover the
 // shared-memory latency (25 MB, compress and decode: 51.2 us against 43.0).  With one group of ranks three
