@@ -178,6 +178,8 @@ def test_terngrad_tasks_do_not_wait_for_a_free_gpu(runtime, n):
             C.copy_(B, non_blocking=True)
         high.synchronize()
 
+    task()
+    assert torch.equal(C, ops.terngrad_compress(g.cpu(), 2, False))
     of_task, of_op = medians_beside_matrix_products(task, op)
     assert of_task < 0.75 * of_op
 

@@ -82,6 +82,32 @@ def test_noalloc_without_residual_and_with_4_byte_aligned_buffers():
             assert torch.equal(r_new, r_ref)
 
 
+@pytest.mark.parametrize("bw", [1, 2, 4, 8])
+@pytest.mark.parametrize("feedback", [False, True])
+@pytest.mark.parametrize("offset", [0, 1, 2, 6, 8])
+def test_two_launches_against_the_cpu_codec(bw, feedback, offset):
+    """This entry takes the two-launch form at every size, as the exchange engine and the task API do: both sides of the
+    chunked path (296 chunks of 512 payload bytes), with packed data at every kind of distance from a 16-byte boundary."""
+    from hipress_b200 import ops
+    lib, fn = _lib()
+    stream = torch.cuda.current_stream().cuda_stream
+    chunked = 296 * 512 * 8 // bw
+    for n in (1, 4099, 131072, chunked - 1, chunked, chunked + 777):
+        gen = torch.Generator().manual_seed(n)
+        g, r = torch.randn(n, generator=gen) * 0.01, torch.randn(n, generator=gen) * 0.004
+        rc, rg = r.clone(), r.cuda()
+        ref = ops.terngrad_compress(g, bw, True, 7, residual=rc if feedback else None)
+        size = ref.numel()
+        out = torch.zeros(size + offset + 64, dtype=torch.uint8, device="cuda")
+        dev = g.cuda()
+        assert fn(dev.data_ptr(), rg.data_ptr() if feedback else None, n, bw, 1, 7, out.data_ptr() + offset, size, stream) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out[offset:offset + size].cpu(), ref), n
+        assert int(out[:offset].sum()) == 0 and int(out[offset + size:].sum()) == 0, n
+        if feedback:
+            assert torch.equal(rg.cpu(), rc), n
+
+
 def test_noalloc_rejects_bad_sizes():
     lib, fn = _lib()
     g = torch.zeros(16, device="cuda")
