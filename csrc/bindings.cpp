@@ -135,7 +135,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     rt.release_spent();
     return names;
   });
-  m.def("getErrors", [] { return runtime::TaskRuntime::instance().get_errors(); });
+  m.def("getErrors", [] {
+    auto& rt = runtime::TaskRuntime::instance();
+    auto errors = rt.get_errors();
+    rt.release_spent();
+    return errors;
+  });
   m.def("numThreads", [] { return runtime::TaskRuntime::instance().num_threads(); });
   m.def("submit_task",
         [](const std::string& name, torch::Tensor tensor, torch::Tensor B, torch::Tensor C, int is_root,

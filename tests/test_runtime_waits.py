@@ -2,6 +2,7 @@
 import subprocess
 import sys
 import time
+import weakref
 from pathlib import Path
 
 import pytest
@@ -73,6 +74,35 @@ def test_names_do_not_wait_for_the_interpreter():
     finally:
         sys.setswitchinterval(interval)
     assert seen == names
+    hp_cuda.end()
+
+
+@pytest.mark.timeout(60)
+@pytest.mark.parametrize("collect", ["getResults", "getErrors", "submit_task", "end"])
+def test_tensors_are_let_go_with_the_next_call(collect):
+    """Of a task that worked and of one that failed."""
+    hp_cuda.init("tbq", {"threshold": 2e-3}, 0, 0, 1)
+    size = ops.tbq_payload_bytes(64)
+
+    def submit(dtype):
+        t = (torch.zeros(64, dtype=dtype), torch.zeros(64), torch.zeros(size, dtype=torch.uint8),
+             torch.zeros(size, dtype=torch.uint8))
+        hp_cuda.submit_task("x", *t, 0, hp_cuda.COMP_TASK)
+        return [weakref.ref(x) for x in t]
+
+    held = submit(torch.float32) + submit(torch.float64)
+    deadline = time.monotonic() + 20
+    while any(x() is not None for x in held) and time.monotonic() < deadline:
+        time.sleep(0.01)
+        if collect == "getResults":
+            hp_cuda.getResults(hp_cuda.COMP_TASK)
+        elif collect == "getErrors":
+            hp_cuda.getErrors()
+        elif collect == "submit_task":
+            submit(torch.float32)
+        else:
+            hp_cuda.end()
+    assert all(x() is None for x in held)
     hp_cuda.end()
 
 
