@@ -1258,43 +1258,60 @@ emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScr
 }
 
 // ================================================================ one-pass decode
-// All payloads into a dense tensor that is written from scratch: a CTA owns a tile of the tensor,
-// adds the payloads' entries of that range to a zeroed tile in shared memory, rank after rank, and
-// stores the tile once.  The indices of a payload ascend (the content rule above), so a tile's
-// entries are found by a search: one warp per rank, two or three dependent loads.
+// All payloads into a dense tensor that is written from scratch: a CTA owns a tile of the tensor and adds the
+// payloads' entries of that range, rank after rank, in shared memory.  The indices of a payload ascend (the
+// content rule above), so a tile's entries are found by a search: one warp per rank.
 //
-// What bounds it: the dense store, and below a few MB the chain header -> search -> entries (about
-// 2 us).  It replaces a memset and one scatter per rank, which cost a launch each and, from a
-// thousandth of the elements up, a read and a write of the same 32-byte sectors per rank: 25 MB at 0.1 %, one
-// call waited for: eight payloads 37 us, 72 with the scatters; one payload 31 and 30.
+// What bounds it: the dense store, and a chain of dependent loads.  The chain is two long: the payload's
+// header together with the probes of the search, whose places follow from the slot's size; then the entries
+// of a window that certainly holds the tile's and a few of its neighbours', which are passed over.  Searching
+// on until the tile's ends are known exactly costs one to three loads more.  Where a tile holds few entries its
+// zeros are stored before the search ends, and the few sums afterwards, so that the store and the chain overlap
+// (SPARSE).
+// 25 MB at 0.1 %, eight payloads, in a chain of calls: 10.0 us, 17.4 with exact ends and the tile stored at the
+// end; 64 MB, four payloads: 18.4 and 25.9.
 //
-// A payload whose indices do not ascend is still decoded: the segments that the searches return for
-// neighbouring tiles share their ends, so they cut the payload into consecutive pieces, and an entry
-// outside its tile's range is seen by the tile that got it.  That tile raises `redo`, and the kernel
-// behind decodes everything again without assuming an order.  An index past the end is reported by the tile
-// that meets it.
+// A payload whose indices do not ascend is still decoded: the tiles' windows begin where a boundary's search
+// ended, the same place for the tile before, so the pieces from one beginning to the next cover the payload;
+// each tile compares the neighbouring indices of its piece.  One that finds a descent raises `redo`, and the
+// kernel behind decodes everything again without assuming an order.  Where there is none, every probe said the
+// truth and the windows are right.  An index past the end is reported by the tile whose piece holds it.
 constexpr int kDenseTile = 8192;   // elements: 32 KB, six CTAs per SM
+constexpr int kBriefWindow = 64;   // entries of a rank that its warp holds in registers, two per lane
+constexpr double kSparseTile = 24; // evenly spread entries of a tile up to which SPARSE is taken
 
-// For both x: the first position in idx[0, k) whose value is not below it, for ascending idx below n; for
-// any other idx some position in [0, k], the same one for every caller.  Whole warp.  The first 32 probes
-// sit around the place that evenly spread indices would give, two square roots of k to either side; what is
-// left is searched 32 ways.  The two searches share their rounds: a round is a dependent load.
-__device__ __forceinline__ void warp_lower_bounds(const uint32_t* __restrict__ idx, uint32_t k, int64_t n,
-                                                  const int64_t (&x)[2], int lane, uint32_t (&found)[2]) {
-  uint32_t a[2] = {0, 0}, len[2] = {k, k};
-  const int64_t step0 = 1 + int64_t(sqrtf(float(k)) * 0.125f);
-  bool below[2];
-  int64_t p0[2];
+// The window of a tile in one rank's payload: entries outside [begin, end) lie outside the tile, and
+// [begin, own_end) is the piece whose order this tile checks.
+struct TileWindow {
+  uint32_t begin, own_end, end;
+};
+// The first probes of a search for both ends of a tile: positions around the place that evenly spread indices
+// would give, two square roots of the expected count to either side, and what was read there.
+struct TileProbes {
+  int64_t at[2];
+  uint32_t found[2];
+};
+__device__ __forceinline__ int64_t probe_step(uint32_t guess) { return 1 + int64_t(sqrtf(float(guess)) * 0.125f); }
+// guess: entries that fit the slot; no position from there on is read, whatever the header will say.
+__device__ __forceinline__ void first_probes(const uint32_t* __restrict__ idx, uint32_t guess, float inv_n,
+                                             const int64_t (&x)[2], int lane, TileProbes& p) {
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    p0[t] = int64_t(double(x[t]) / double(n) * double(k)) + int64_t(lane - 16) * step0;
-    below[t] = p0[t] < 0;
-    if (p0[t] >= 0 && p0[t] < int64_t(k)) below[t] = int64_t(idx[p0[t]]) < x[t];
+    p.at[t] = int64_t(float(x[t]) * inv_n * float(guess)) + int64_t(lane - 16) * probe_step(guess);
+    p.found[t] = p.at[t] >= 0 && p.at[t] < int64_t(guess) ? idx[p.at[t]] : 0u;
   }
+}
+// Whole warp.  For each end x the first position whose index is not below it lies between two places that
+// depend on x, k and the payload alone; they are brought within `slack` of one another, 32 ways at a time.
+__device__ __forceinline__ TileWindow tile_window(const uint32_t* __restrict__ idx, uint32_t k, uint32_t guess,
+                                                  const TileProbes& p, const int64_t (&x)[2], uint32_t slack, int lane) {
+  uint32_t a[2], len[2];
+  const int64_t step0 = probe_step(guess);
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int hits = __popc(__ballot_sync(0xffffffffu, below[t]));
-    const int64_t lowest = __shfl_sync(0xffffffffu, p0[t], 0);
+    const bool below = p.at[t] < 0 || (p.at[t] < int64_t(k) && int64_t(p.found[t]) < x[t]);
+    const int hits = __popc(__ballot_sync(0xffffffffu, below));
+    const int64_t lowest = __shfl_sync(0xffffffffu, p.at[t], 0);
     int64_t lo = hits == 0 ? 0 : lowest + int64_t(hits - 1) * step0 + 1;   // past the last probe below x
     int64_t hi = hits == 32 ? int64_t(k) : lowest + int64_t(hits) * step0; // the first one that is not
     lo = lo < 0 ? 0 : (lo > int64_t(k) ? int64_t(k) : lo);
@@ -1302,25 +1319,25 @@ __device__ __forceinline__ void warp_lower_bounds(const uint32_t* __restrict__ i
     a[t] = uint32_t(lo);
     len[t] = uint32_t(hi - lo);
   }
-  while ((len[0] | len[1]) != 0) {
+  while (len[0] > slack || len[1] > slack) {
     uint32_t step[2];
+    bool below[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       step[t] = (len[t] + 31) / 32;
-      const uint64_t p = uint64_t(a[t]) + uint64_t(lane + 1) * step[t] - 1;
-      below[t] = len[t] != 0 && p < uint64_t(a[t]) + len[t] && int64_t(idx[p]) < x[t];
+      const uint64_t at = uint64_t(a[t]) + uint64_t(lane + 1) * step[t] - 1;
+      below[t] = len[t] > slack && at < uint64_t(a[t]) + len[t] && int64_t(idx[at]) < x[t];
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const uint32_t hits = uint32_t(__popc(__ballot_sync(0xffffffffu, below[t])));
-      if (len[t] == 0) continue;
+      if (len[t] <= slack) continue;
       const uint32_t rest = len[t] - hits * step[t];   // hits * step <= len: every hit lies inside
       a[t] += hits * step[t];
       len[t] = rest < step[t] - 1 ? rest : step[t] - 1;   // the probe after the last hit is not below x
     }
   }
-  found[0] = a[0];
-  found[1] = a[1];
+  return {a[0], a[1], a[1] + len[1]};
 }
 
 // Entries of a payload, 0 with the status word set when the header does not fit the slot.
@@ -1331,126 +1348,166 @@ __device__ __forceinline__ uint32_t payload_entries(const uint8_t* payload, int6
   return 0;
 }
 
-// The tile [lo, lo + len) of this CTA, decoded into buf (its float4s are whole).  False in the threads that
-// met an entry which the search put into the wrong tile.  Ends with a barrier.
-__device__ __forceinline__ bool decode_tile(const UnpackSources& src, int64_t n, int tile, int64_t lo, int len,
-                                            float post_scale, int* status, float* buf) {
-  __shared__ uint32_t seg_begin[kMaxWorld], seg_end[kMaxWorld], entries[kMaxWorld];
+struct TilePlan {
+  int tile;         // elements
+  uint32_t slack;   // see tile_window
+  float inv_n;
+};
+
+// The tile [lo, lo + len) of this CTA, decoded into buf (its float4s are whole), or with SPARSE into memory at
+// o; vec: o is 16-byte aligned.  False in the threads that saw a descent.  Ends with a barrier, except where it
+// has stored everything itself.
+template <bool SPARSE>
+__device__ __forceinline__ bool decode_tile(const UnpackSources& src, int64_t n, const TilePlan& plan, int64_t lo, int len,
+                                            float post_scale, int* status, float* buf, float* o, bool vec) {
+  __shared__ TileWindow windows[kMaxWorld];
+  __shared__ uint32_t entries[kMaxWorld];
+  __shared__ int list_at[kMaxWorld][kBriefWindow];     // place in the tile, or negative
+  __shared__ float list_value[kMaxWorld][kBriefWindow];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool first = blockIdx.x == 0, last = blockIdx.x == gridDim.x - 1;
+  const int64_t ends[2] = {lo, lo + plan.tile};
   bool bad = false;
-  uint32_t k = 0;
+  uint32_t k = 0, guess = 0;
   const uint32_t* idx = nullptr;
+  TileProbes probes{};
 #pragma unroll
   for (int r = 0; r < kMaxWorld; ++r) {   // compile-time index into src; one warp per rank
     if (r == warp && r < src.world) {
-      k = payload_entries(src.payload[r] + src.parity_off, src.payload_bytes[r], status, first && lane == 0);
-      idx = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
+      const uint8_t* payload = src.payload[r] + src.parity_off;
+      const int64_t fit = (src.payload_bytes[r] - 4) / 8;
+      guess = uint32_t(fit < 0 ? 0 : fit);
+      idx = reinterpret_cast<const uint32_t*>(payload + 4);
+      first_probes(idx, guess, plan.inv_n, ends, lane, probes);
+      k = payload_entries(payload, src.payload_bytes[r], status, first && lane == 0);
     }
   }
-  for (int i = tid; i < (len + 3) / 4; i += kThreads) reinterpret_cast<float4*>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto clear_buf = [&]() {
+    for (int i = tid; i < (len + 3) / 4; i += kThreads) reinterpret_cast<float4*>(buf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (SPARSE) {
+    const int quads = vec ? len >> 2 : 0;
+    for (int i = tid; i < quads; i += kThreads) reinterpret_cast<float4*>(o)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 4 * quads + tid; i < len; i += kThreads) o[i] = 0.f;
+  } else {
+    clear_buf();
+  }
+  // An entry that was read at e: its place in the tile, or negative.
+  auto place = [&](uint32_t i, uint32_t next, uint32_t e, uint32_t total, const TileWindow& w) -> int {
+    if (e < w.own_end) {
+      if (e + 1 < total && next < i) bad = true;
+      if (int64_t(i) >= n && status != nullptr) atomicExch(status, int(kPayloadBounds));
+    }
+    const int64_t at = int64_t(i) - lo;
+    return at >= 0 && at < len ? int(at) : -1;
+  };
+  auto scaled = [&](float v) { return post_scale != 1.0f ? hp_mul(v, post_scale) : v; };
+  int at[2] = {-1, -1};
+  bool brief = true;
   if (warp < src.world) {
-    const int64_t ends[2] = {lo, lo + tile};
-    uint32_t at[2];
-    warp_lower_bounds(idx, k, n, ends, lane, at);
-    if (first) at[0] = 0;
-    if (last) at[1] = k;
-    if (at[0] > at[1]) {
-      bad = true;
-      at[1] = at[0];
+    TileWindow w = tile_window(idx, k, guess, probes, ends, plan.slack, lane);
+    if (first) w.begin = 0;
+    if (last) w.own_end = w.end = k;
+    brief = w.end <= w.begin || w.end - w.begin <= kBriefWindow;
+    if (brief) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t e = w.begin + lane + 32 * q;
+        float v = 0.f;
+        if (e < w.end) {
+          const uint32_t i = idx[e], next = e + 1 < k ? idx[e + 1] : 0u;
+          v = __uint_as_float(idx[k + e]);
+          at[q] = place(i, next, e, k, w);
+        }
+        if (SPARSE && at[q] >= 0) buf[at[q]] = 0.f;
+        list_at[warp][lane + 32 * q] = at[q];
+        list_value[warp][lane + 32 * q] = scaled(v);
+      }
     }
     if (lane == 0) {
-      seg_begin[warp] = at[0];
-      seg_end[warp] = at[1];
+      windows[warp] = w;
       entries[warp] = k;
     }
   }
-  __syncthreads();
-  // the first entry of every rank is requested before any is added: at a thousandth of the elements
-  // a tile holds eight of each rank
-  uint32_t i0[kMaxWorld];
-  float v0[kMaxWorld];
-#pragma unroll
-  for (int r = 0; r < kMaxWorld; ++r) {
-    if (r < src.world) {
-      const uint32_t e = seg_begin[r] + tid;
-      if (e < seg_end[r]) {
-        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
-        i0[r] = from[e];
-        v0[r] = __uint_as_float(from[entries[r] + e]);
-      }
-    }
-  }
-  bool brief = true;   // no rank has more than a warp's worth here
-  for (int r = 0; r < src.world; ++r) brief = brief && seg_end[r] - seg_begin[r] <= 32;
-  auto add_entry = [&](uint32_t i, float v) {
-    const int64_t at = int64_t(i) - lo;
-    if (at >= 0 && at < len) {
-      if (post_scale != 1.0f) v = hp_mul(v, post_scale);
-      buf[at] = hp_add(buf[at], v);   // indices are unique inside one payload
-    } else if (int64_t(i) >= n) {   // every entry is seen by some tile, wherever it stands in the payload
-      if (status != nullptr) atomicExch(status, int(kPayloadBounds));
-    } else {
-      bad = true;
-    }
-  };
-  if (brief) {
+  if (__syncthreads_and(brief)) {
     if (warp == 0) {
+      // ranks one after another, the indices inside a payload are unique
 #pragma unroll
       for (int r = 0; r < kMaxWorld; ++r) {
         if (r < src.world) {
-          if (seg_begin[r] + lane < seg_end[r]) add_entry(i0[r], v0[r]);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int here = list_at[r][lane + 32 * q];
+            if (here >= 0) buf[here] = hp_add(buf[here], list_value[r][lane + 32 * q]);
+          }
           __syncwarp();
         }
       }
     }
     __syncthreads();
-  } else {
+    if (SPARSE) {   // over the zeros stored before the barriers
 #pragma unroll
-    for (int r = 0; r < kMaxWorld; ++r) {
-      if (r < src.world) {
-        const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
-        const uint32_t total = entries[r], end = seg_end[r];
-        uint32_t e = seg_begin[r] + tid;
-        if (e < end) add_entry(i0[r], v0[r]);
-        // four entries in flight per thread: at a quarter of the elements a tile holds 2,048 per rank
-        for (e += kThreads; e + 3 * kThreads < end; e += 4 * kThreads) {
-          uint32_t i[4];
-          float v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            i[u] = from[e + u * kThreads];
-            v[u] = __uint_as_float(from[total + e + u * kThreads]);
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) add_entry(i[u], v[u]);
-        }
-        for (; e < end; e += kThreads) add_entry(from[e], __uint_as_float(from[total + e]));
-        __syncthreads();
-      }
+      for (int q = 0; q < 2; ++q)
+        if (at[q] >= 0) o[at[q]] = buf[at[q]];
     }
+    return !bad;
+  }
+  if (SPARSE) {   // more entries than expected: the tile is put together here and stored over the zeros
+    clear_buf();
+    __syncthreads();
+  }
+#pragma unroll
+  for (int r = 0; r < kMaxWorld; ++r) {
+    if (r < src.world) {
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(src.payload[r] + src.parity_off + 4);
+      const uint32_t total = entries[r];
+      const TileWindow w = windows[r];
+      auto add_entry = [&](uint32_t i, uint32_t next, float v, uint32_t e) {
+        const int here = place(i, next, e, total, w);
+        if (here >= 0) buf[here] = hp_add(buf[here], scaled(v));
+      };
+      // four entries in flight per thread: at a quarter of the elements a tile holds 2,048 per rank
+      uint32_t e = w.begin + tid;
+      for (; int64_t(e) + 3 * kThreads < int64_t(w.end); e += 4 * kThreads) {
+        uint32_t i[4], next[4];
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t x = e + u * kThreads;
+          i[u] = from[x];
+          next[u] = x + 1 < total ? from[x + 1] : 0u;
+          v[u] = __uint_as_float(from[total + x]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add_entry(i[u], next[u], v[u], e + u * kThreads);
+      }
+      for (; e < w.end; e += kThreads) add_entry(from[e], e + 1 < total ? from[e + 1] : 0u, __uint_as_float(from[total + e]), e);
+      __syncthreads();
+    }
+  }
+  if (SPARSE) {
+    const int quads = vec ? len >> 2 : 0;
+    for (int i = tid; i < quads; i += kThreads) reinterpret_cast<float4*>(o)[i] = reinterpret_cast<const float4*>(buf)[i];
+    for (int i = 4 * quads + tid; i < len; i += kThreads) o[i] = buf[i];
   }
   return !bad;
 }
 
-template <bool VEC>
+template <bool SPARSE, bool VEC>
 __global__ void __launch_bounds__(kThreads, 6)
-dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int tile, float post_scale, int* status,
+dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, TilePlan plan, float post_scale, int* status,
                   unsigned int* redo) {
   __shared__ __align__(16) float buf[kDenseTile];
   let_next_start();
   const int tid = threadIdx.x;
-  const int64_t lo = int64_t(blockIdx.x) * tile;
-  const int len = int(lo + tile < n ? tile : n - lo);
-  if (!decode_tile(src, n, tile, lo, len, post_scale, status, buf)) *redo = 1u;
+  const int64_t lo = int64_t(blockIdx.x) * plan.tile;
+  const int len = int(lo + plan.tile < n ? plan.tile : n - lo);
   float* o = out + lo;
-  if (VEC) {
-    for (int i = tid; i < (len >> 2); i += kThreads) reinterpret_cast<float4*>(o)[i] = reinterpret_cast<const float4*>(buf)[i];
-    const int i = (len & ~3) + tid;
-    if (i < len) o[i] = buf[i];
-  } else {
-    for (int i = tid; i < len; i += kThreads) o[i] = buf[i];
-  }
+  if (!decode_tile<SPARSE>(src, n, plan, lo, len, post_scale, status, buf, o, VEC)) *redo = 1u;
+  if (SPARSE) return;
+  const int quads = VEC ? len >> 2 : 0;
+  for (int i = tid; i < quads; i += kThreads) reinterpret_cast<float4*>(o)[i] = reinterpret_cast<const float4*>(buf)[i];
+  for (int i = 4 * quads + tid; i < len; i += kThreads) o[i] = buf[i];
 }
 
 // ---- decode and optimizer step in one pass
@@ -1481,7 +1538,7 @@ sparse_check_kernel(UnpackSources src, int64_t n, int* status) {
 
 template <int OPT>
 __global__ void __launch_bounds__(kThreads, 4)
-sparse_apply_kernel(UnpackSources src, int64_t n, int tile, float post_scale, SgdApply sgd, AdamWApply adamw, int vec,
+sparse_apply_kernel(UnpackSources src, int64_t n, TilePlan plan, float post_scale, SgdApply sgd, AdamWApply adamw, int vec,
                     const int* guard, int* status) {
   __shared__ __align__(16) float buf[kDenseTile];
   wait_for_previous();
@@ -1490,9 +1547,9 @@ sparse_apply_kernel(UnpackSources src, int64_t n, int tile, float post_scale, Sg
   float bc1 = 0.f, rsqrt_bc2 = 0.f;
   if (OPT == 1) adamw_bias(adamw, bc1, rsqrt_bc2);
   const int tid = threadIdx.x;
-  const int64_t lo = int64_t(blockIdx.x) * tile;
-  const int len = int(lo + tile < n ? tile : n - lo);
-  decode_tile(src, n, tile, lo, len, post_scale, status, buf);
+  const int64_t lo = int64_t(blockIdx.x) * plan.tile;
+  const int len = int(lo + plan.tile < n ? plan.tile : n - lo);
+  decode_tile<false>(src, n, plan, lo, len, post_scale, status, buf, nullptr, false);
   const int quads = vec ? len >> 2 : 0;
 #pragma unroll 2
   for (int i = tid; i < quads; i += kThreads) {
@@ -1713,10 +1770,15 @@ cudaError_t sparse_read_stats(const void* scratch, unsigned int* host4, cudaStre
 }
 
 namespace {
-// Tiles of 8,192 elements, smaller ones while they would not cover every SM four times.
-inline int64_t dense_tile_for(int64_t n) {
-  const int64_t tile = (n / (148 * 4) + 1023) / 1024 * 1024;
-  return std::min<int64_t>(std::max<int64_t>(tile, 1024), kDenseTile);
+// Tiles of 8,192 elements, smaller ones while they would not cover every SM four times.  per_tile: entries of
+// the fullest slot that a tile would hold if they were evenly spread.
+inline TilePlan tile_plan(const UnpackSources& src, int64_t n, double& per_tile) {
+  const int64_t tile = std::min<int64_t>(std::max<int64_t>((n / (148 * 4) + 1023) / 1024 * 1024, 1024), kDenseTile);
+  int64_t fit = 0;
+  for (int r = 0; r < src.world; ++r) fit = std::max<int64_t>(fit, (src.payload_bytes[r] - 4) / 8);
+  per_tile = double(fit) * double(tile) / double(n);
+  // a window may be that much longer than the tile's entries at either end
+  return {int(tile), uint32_t(16 + std::min(per_tile, double(tile)) / 4), 1.0f / float(n)};
 }
 }  // namespace
 
@@ -1735,17 +1797,18 @@ cudaError_t sparse_apply(const UnpackSources& src, int64_t n, float post_scale, 
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  const int64_t tile = dense_tile_for(n);
-  const dim3 grid = dim3(unsigned((n + tile - 1) / tile)), block(kThreads);
+  double per_tile;
+  const TilePlan plan = tile_plan(src, n, per_tile);
+  const dim3 grid = dim3(unsigned((n + plan.tile - 1) / plan.tile)), block(kThreads);
   if (adamw != nullptr) {
     if (!adamw->param || !adamw->exp_avg || !adamw->exp_avg_sq || adamw->step < 1) return cudaErrorInvalidValue;
     const int vec = al(adamw->param) && al(adamw->exp_avg) && al(adamw->exp_avg_sq) ? 1 : 0;
-    return launch_after(sparse_apply_kernel<1>, grid, block, 0, stream, src, n, int(tile), post_scale, SgdApply{}, *adamw, vec,
+    return launch_after(sparse_apply_kernel<1>, grid, block, 0, stream, src, n, plan, post_scale, SgdApply{}, *adamw, vec,
                         static_cast<const int*>(status), status);
   }
   if (!sgd->param || !sgd->momentum) return cudaErrorInvalidValue;
   const int vec = al(sgd->param) && al(sgd->momentum) ? 1 : 0;
-  return launch_after(sparse_apply_kernel<0>, grid, block, 0, stream, src, n, int(tile), post_scale, *sgd, AdamWApply{}, vec,
+  return launch_after(sparse_apply_kernel<0>, grid, block, 0, stream, src, n, plan, post_scale, *sgd, AdamWApply{}, vec,
                       static_cast<const int*>(status), status);
 }
 
@@ -1755,11 +1818,15 @@ cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n,
   if (!add && redo != nullptr && n <= 0x7fffffff && src.epoch_dev == nullptr && src.guard == nullptr) {
     for (int r = 0; r < src.world; ++r)
       if (reinterpret_cast<uintptr_t>(src.payload[r]) & 3) return cudaErrorInvalidValue;
-    const int64_t tile = dense_tile_for(n);
-    const unsigned blocks = unsigned((n + tile - 1) / tile);
+    double per_tile;
+    const TilePlan plan = tile_plan(src, n, per_tile);
+    const unsigned blocks = unsigned((n + plan.tile - 1) / plan.tile);
     const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    if (vec) dense_tile_kernel<true><<<blocks, kThreads, 0, stream>>>(src, out, n, int(tile), post_scale, status, redo);
-    else dense_tile_kernel<false><<<blocks, kThreads, 0, stream>>>(src, out, n, int(tile), post_scale, status, redo);
+    // few entries: the window of nearly every tile fits a warp's registers (see decode_tile)
+    const bool sparse = per_tile <= kSparseTile;
+    auto kernel = sparse ? (vec ? dense_tile_kernel<true, true> : dense_tile_kernel<true, false>)
+                         : (vec ? dense_tile_kernel<false, true> : dense_tile_kernel<false, false>);
+    kernel<<<blocks, kThreads, 0, stream>>>(src, out, n, plan, post_scale, status, redo);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_after(dense_redo_kernel, dim3(148), dim3(kRedoThreads), 0, stream, src, out, n, post_scale, redo);

@@ -40,6 +40,34 @@ def test_sparse_decode_tiles(n, k, world, offset):
     assert ops.read_status(out) == 0
 
 
+@pytest.mark.parametrize("n,k", [(300007, 40), (5000011, 5000), (5000011, 60000)])
+@pytest.mark.parametrize("spread", ["even", "one_tile", "ends"])
+@pytest.mark.parametrize("room", [0, 1, 3])
+def test_sparse_decode_windows(n, k, spread, room):
+    """Where the first probes of the search miss: entries crowded into a few tiles, slots with room for more entries
+    than they hold.  Then a single descent, which only the tile that compares these two neighbours can see."""
+    g = torch.Generator().manual_seed(k)
+    payloads = []
+    for r in range(3):
+        if spread == "even":
+            idx = torch.randperm(n, generator=g)[:k]
+        else:
+            near = torch.randperm(n // 3, generator=g)[:k] if k > 8000 else 8192 + torch.randperm(8192, generator=g)[:k]
+            idx = near if spread == "one_tile" else torch.cat([near[:k // 2] % 8192, n - 1 - near[:k // 2] % 8192]).unique()
+        p = sparse_payload(idx.sort().values, torch.randn(idx.numel(), generator=g))
+        payloads.append(torch.cat([p, torch.full((8 * k * room,), 0x01, dtype=torch.uint8)]))
+    for swap in (None, 0, k // 3):
+        if swap is not None and spread != "ends":
+            idx = payloads[1][4:4 + 4 * k].view(torch.int32)
+            idx[swap], idx[swap + 1] = int(idx[swap + 1]), int(idx[swap])
+        ref = torch.empty(n)
+        ops.sparse_decompress(payloads, ref, post_scale=0.25)
+        out = torch.full((n,), 7.0, device="cuda")
+        ops.sparse_decompress([p.cuda() for p in payloads], out, post_scale=0.25)
+        assert torch.equal(out.cpu(), ref), swap
+    assert ops.read_status(out) == 0
+
+
 @pytest.mark.parametrize("world", [1, 3])
 def test_sparse_decode_of_unordered_payloads(world):
     """Order is a property of this library's compressor, not of the format: any order decodes, and the calls after
