@@ -186,7 +186,11 @@ template <bool APPLY, int WORLD>
 cudaError_t launch_tbq_index(const UnpackSources& src, float thr, float* out, int64_t n, int add, float post_scale,
                              const SgdApply& apply, cudaStream_t stream) {
   using L = IndexLayout<2, WORLD, true, false>;
-  static_assert(L::kBytes <= 48 * 1024, "fits the default shared-memory limit");
+  if (L::kBytes > 40 * 1024) {   // past the default limit; set on every launch rather than remembered per process
+    const cudaError_t e = cudaFuncSetAttribute(tbq_unpack_index_kernel<APPLY, WORLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(L::kBytes));
+    if (e != cudaSuccess) return e;
+  }
   const int grid = index_grid(n, IndexForm<2>::kChunk, WORLD, L::kBytes);
   tbq_unpack_index_kernel<APPLY, WORLD><<<grid, index_threads(WORLD), L::kBytes, stream>>>(
       src, thr, out, n, add, post_scale, apply, payload_alignment(src, 0));

@@ -619,25 +619,25 @@ __device__ __forceinline__ bool read_headers(const UnpackSources& src, int64_t n
   __shared__ int all_ok;
   if (threadIdx.x == 0) all_ok = 1;
   __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kMaxWorld; ++r) {   // thread r reads header r; compile-time index into src
-    if (int(threadIdx.x) == r && r < src.world) {
-      const int64_t count = concat ? shard_count(n, src.shard_elems, r) : n;
-      if (count > 0) {
-        hdr[r] = read_header(src.payload[r] + src.parity_off, src.payload_bytes[r], count);
-        if (!hdr[r].ok) all_ok = 0;
-      } else {
-        hdr[r].ok = 1; hdr[r].bw = 0; hdr[r].mn = 0.f; hdr[r].gap = 0.f;
-      }
+  // Thread r reads header r.  The payload is selected and not branched to: a branch per rank would have the
+  // ranks' loads, each a miss of every cache, wait for one another.
+  const int r = int(threadIdx.x);
+  if (r < src.world) {
+    const int64_t count = concat ? shard_count(n, src.shard_elems, r) : n;
+    if (count > 0) {
+      hdr[r] = read_header(select_payload(src, r) + src.parity_off, select_payload_bytes(src, r), count);
+      if (!hdr[r].ok) all_ok = 0;
+    } else {
+      hdr[r].ok = 1; hdr[r].bw = 0; hdr[r].mn = 0.f; hdr[r].gap = 0.f;
     }
   }
   __syncthreads();
   bw = BW;
   if (all_ok) {
-    for (int r = 0; r < src.world; ++r) {  // every thread computes the same verdict
-      if (hdr[r].bw == 0) continue;        // empty shard
-      if (bw == 0) bw = hdr[r].bw;
-      if (hdr[r].bw != bw) all_ok = 0;
+    for (int q = 0; q < src.world; ++q) {  // every thread computes the same verdict
+      if (hdr[q].bw == 0) continue;        // empty shard
+      if (bw == 0) bw = hdr[q].bw;
+      if (hdr[q].bw != bw) all_ok = 0;
     }
   }
   __syncthreads();

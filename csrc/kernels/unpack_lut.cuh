@@ -301,11 +301,13 @@ __device__ __forceinline__ void unpack_nibble_body(const float* lut, uint32_t (&
 // of the few resident CTAs.
 //
 // A lane loads 32 payload bits of each rank, turns the words of a group into one index byte per element
-// (a shift and a bit select per field, then a byte transposition), and writes those bytes to a buffer of
+// (fields are exchanged between words, then bytes transposed), and writes those bytes to a buffer of
 // its warp; the lanes read them back so that every dense access is a 512-byte run across the warp.
+// The tables of two groups share rows of 256 bytes, 128 each: the address of an entry is then the index
+// byte above the lane's column, which one byte permutation puts together.
 // A table entry per pair of ranks and two elements, with bank conflicts and every index word moved by shuffle,
-// is the alternative.  2 bits, eight payloads, 25 MB (ncu, cold): 17.3 us, and 26.6 by pairs; 4 bits, one
-// payload, 2.4 M elements: 6.4, and 15.8 by nibble tables.
+// is the alternative.  2 bits, eight payloads, 25 MB, in a chain of calls: 12.3 us; 17.2 with rows of 128 bytes, the
+// fields moved one by one and the headers read one after another; (ncu, cold) 17.3 so, and 26.6 by pairs.
 // Threads per CTA and CTAs per SM.  Eight payloads' tables and index buffers take 80 KB: two CTAs of 512
 // threads that share them, because two of 256 leave four warps per scheduler, too few to cover the
 // shared-memory latency (25 MB, compress and decode: 51.2 us against 43.0).  With one group of ranks three
@@ -321,19 +323,26 @@ struct IndexForm {
   static constexpr int kDpb = 8 / BW;
 };
 // Sequential sums (the order of the ECQ codec: ascending ranks, one by one) read the first group's sum
-// from its table and every later rank from a table of its own.
+// from its table and every later rank from a table of its own, all of them in the other half of its rows.
 template <int BW, int WORLD, bool SHARED, bool SEQ>
 struct IndexLayout {
   using F = IndexForm<BW>;
   static constexpr int kGroups = (WORLD + F::kRanks - 1) / F::kRanks;
   static constexpr int kFirst = WORLD < F::kRanks ? WORLD : F::kRanks;      // ranks of the first group
   static constexpr int kLast = WORLD - (kGroups - 1) * F::kRanks;            // ranks of the last one
-  static constexpr int rows(int g) { return 1 << (BW * (g + 1 < kGroups || SHARED ? kFirst : kLast)); }
-  static constexpr int kFull = 1 << (BW * kFirst);                           // rows before group 1
-  static constexpr int kRows = SEQ ? kFull + (WORLD - kFirst) * (1 << BW)
-                                   : (SHARED ? kFull : kFull * (kGroups - 1) + rows(kGroups - 1));
+  static constexpr int kFull = 1 << (BW * kFirst);                           // rows of a group but the last
+  static constexpr int kTables = SHARED || SEQ ? 1 : kGroups;                // groups with a table of their own
+  __host__ __device__ static constexpr int rows(int g) { return SHARED || g + 1 < kGroups ? kFull : 1 << (BW * kLast); }
+  // bytes from row to row: the last of an odd number of groups has nothing to share its rows with
+  __host__ __device__ static constexpr int stride(int g) { return kTables > 1 && g + 1 == kTables && g % 2 == 0 ? 128 : 256; }
+  __host__ __device__ static constexpr int offset(int g) { return (g / 2) * kFull * 256 + (g % 2) * 128; }
+  // SEQ: the tables of rank kFirst and on
+  static constexpr int kSingles = SEQ ? (WORLD - kFirst) * (1 << BW) : 0;
+  static_assert(kSingles <= kFull, "the other half of the rows holds them");
+  __host__ __device__ static constexpr int single(int r) { return ((r - kFirst) << BW) * 256 + 128; }
+  static constexpr int kTableBytes = offset(kTables - kTables % 2) + (kTables % 2) * rows(kTables - 1) * stride(kTables - 1);
   static constexpr int kStage = 32 * F::kElems * kGroups;                    // bytes per warp
-  static constexpr size_t kBytes = size_t(kRows) * 128 + size_t(index_threads(WORLD) / 32) * kStage;
+  static constexpr size_t kBytes = size_t(kTableBytes) + size_t(index_threads(WORLD) / 32) * kStage;
 };
 
 // value(r, q): decoded value of level q of rank r.
@@ -342,47 +351,57 @@ __device__ __forceinline__ void build_index_tables(float* tables, Value value) {
   using L = IndexLayout<BW, WORLD, SHARED, SEQ>;
   constexpr int R = IndexForm<BW>::kRanks;
   constexpr uint32_t mask = (1u << BW) - 1u;
-  for (int i = threadIdx.x; i < L::kRows; i += blockDim.x) {
-    float x;
-    if (SEQ && i >= L::kFull) {
-      const int at = i - L::kFull;
-      x = value(L::kFirst + (at >> BW), uint32_t(at) & mask);
-    } else {
-      const int g = SHARED || SEQ ? 0 : i / L::kFull;
-      const uint32_t byte = uint32_t(i - g * L::kFull);
-      float v[R];
-#pragma unroll
-      for (int p = 0; p < R; ++p) v[p] = g * R + p < WORLD ? value(g * R + p, (byte >> (BW * p)) & mask) : 0.0f;
-      const int ranks = WORLD - g * R < R ? WORLD - g * R : R;
-      if (SEQ) {
-        x = v[0];
-#pragma unroll
-        for (int p = 1; p < R; ++p)
-          if (p < ranks) x = hp_add(x, v[p]);
-      } else {
-        x = tree_sum(v, ranks);
-      }
-    }
-    // 32 copies; the lanes start at different columns, so that the stores spread over the banks
-    float4* row = reinterpret_cast<float4*>(tables + i * 32);
+  // 32 copies; the lanes start at different columns, so that the stores spread over the banks
+  auto put = [&](int at, float x) {
+    float4* row = reinterpret_cast<float4*>(reinterpret_cast<char*>(tables) + at);
 #pragma unroll
     for (int c = 0; c < 8; ++c) row[(c + threadIdx.x) & 7] = make_float4(x, x, x, x);
+  };
+#pragma unroll
+  for (int g = 0; g < L::kTables; ++g) {
+    const int ranks = WORLD - g * R < R ? WORLD - g * R : R;
+    for (int i = threadIdx.x; i < L::rows(g); i += blockDim.x) {
+      float v[R];
+#pragma unroll
+      for (int p = 0; p < R; ++p) v[p] = g * R + p < WORLD ? value(g * R + p, (uint32_t(i) >> (BW * p)) & mask) : 0.0f;
+      if (SEQ) {
+#pragma unroll
+        for (int p = 1; p < R; ++p)
+          if (p < ranks) v[0] = hp_add(v[0], v[p]);
+      } else {
+        tree_sum(v, ranks);
+      }
+      put(L::offset(g) + i * L::stride(g), v[0]);
+    }
   }
+  for (int i = threadIdx.x; i < L::kSingles; i += blockDim.x)
+    put(L::single(L::kFirst) + i * 256, value(L::kFirst + (i >> BW), uint32_t(i) & mask));
 }
 
 // Index bytes of one group: u[] holds them in element order.  w: the payload words of the group's ranks.
 template <int BW, int N>
 __device__ __forceinline__ void index_bytes(const uint32_t (&w)[N], uint32_t (&u)[IndexForm<BW>::kElems / 4]) {
   constexpr int D = IndexForm<BW>::kDpb;
-  constexpr uint32_t field = BW == 4 ? 0x0f0f0f0fu : (BW == 2 ? 0x03030303u : 0x01010101u);
   uint32_t t[D];   // t[j], byte b: index of element b * D + j
+  if constexpr (BW == 2 && N >= 3) {
+    // the four words' fields as a 4 x 4 matrix in each byte, transposed in two steps of exchanges
+    const uint32_t w3 = N == 4 ? w[N - 1] : 0u;
+    const uint32_t a0 = (w[0] & 0x33333333u) | ((w[1] << 2) & 0xccccccccu), a1 = ((w[0] >> 2) & 0x33333333u) | (w[1] & 0xccccccccu);
+    const uint32_t a2 = (w[2] & 0x33333333u) | ((w3 << 2) & 0xccccccccu), a3 = ((w[2] >> 2) & 0x33333333u) | (w3 & 0xccccccccu);
+    t[0] = (a0 & 0x0f0f0f0fu) | ((a2 << 4) & 0xf0f0f0f0u);
+    t[1] = (a1 & 0x0f0f0f0fu) | ((a3 << 4) & 0xf0f0f0f0u);
+    t[2] = ((a0 >> 4) & 0x0f0f0f0fu) | (a2 & 0xf0f0f0f0u);
+    t[3] = ((a1 >> 4) & 0x0f0f0f0fu) | (a3 & 0xf0f0f0f0u);
+  } else {
+    constexpr uint32_t field = BW == 4 ? 0x0f0f0f0fu : (BW == 2 ? 0x03030303u : 0x01010101u);
 #pragma unroll
-  for (int j = 0; j < D; ++j) {
-    t[j] = 0;
+    for (int j = 0; j < D; ++j) {
+      t[j] = 0;
 #pragma unroll
-    for (int p = 0; p < N; ++p) {
-      const uint32_t moved = j >= p ? w[p] >> (BW * (j - p)) : w[p] << (BW * (p - j));
-      t[j] |= moved & (field << (BW * p));
+      for (int p = 0; p < N; ++p) {
+        const uint32_t moved = j >= p ? w[p] >> (BW * (j - p)) : w[p] << (BW * (p - j));
+        t[j] |= moved & (field << (BW * p));
+      }
     }
   }
   if constexpr (D == 2) {
@@ -463,19 +482,30 @@ __device__ __forceinline__ void unpack_index_body(float* smem, PayloadWords<WORL
   constexpr int R = F::kRanks, G = L::kGroups, V = F::kElems / 4;
   constexpr uint32_t mask = (1u << BW) - 1u;
   const int lane = threadIdx.x & 31;
-  uint32_t* stage = reinterpret_cast<uint32_t*>(smem + L::kRows * 32) + (threadIdx.x >> 5) * (L::kStage / 4);
-  const float* table = smem + lane;
-  auto sum_of = [&](const uint32_t (&byte)[G]) -> float {
+  uint32_t* stage = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(smem) + L::kTableBytes) + (threadIdx.x >> 5) * (L::kStage / 4);
+  const char* const table = reinterpret_cast<const char*>(smem);
+  const uint32_t column = lane * 4;
+  // four: per group, the index bytes of four elements; k: the element
+  auto sum_of = [&](const uint32_t (&four)[G], int k) -> float {
+    auto entry = [&](int g, int at) -> float {
+      uint32_t off;
+      if (L::stride(at) == 256) off = __byte_perm(four[g], column, 0x5504 | (k << 4));   // byte k, then the column
+      else off = ((k == 0 ? four[g] << 7 : four[g] >> (8 * k - 7)) & 0x7f80u) | column;
+      return *reinterpret_cast<const float*>(table + L::offset(at) + off);
+    };
     if constexpr (SEQ) {
-      float x = table[byte[0] * 32];
+      float x = entry(0, 0);
 #pragma unroll
-      for (int r = L::kFirst; r < WORLD; ++r)
-        x = hp_add(x, table[(L::kFull + ((r - L::kFirst) << BW) + ((byte[r / R] >> (BW * (r % R))) & mask)) * 32]);
+      for (int r = L::kFirst; r < WORLD; ++r) {
+        const int bit = 8 * k + BW * (r % R);   // of the rank's level, which goes to bit 8
+        const uint32_t off = ((bit < 8 ? four[r / R] << (8 - bit) : four[r / R] >> (bit - 8)) & (mask << 8)) | column;
+        x = hp_add(x, *reinterpret_cast<const float*>(table + L::single(r) + off));
+      }
       return x;
     } else {
       float v[G];
 #pragma unroll
-      for (int g = 0; g < G; ++g) v[g] = table[((SHARED ? 0 : g * L::kFull) + byte[g]) * 32];
+      for (int g = 0; g < G; ++g) v[g] = entry(g, SHARED ? 0 : g);
       return tree_sum(v, G);
     }
   };
@@ -516,12 +546,7 @@ __device__ __forceinline__ void unpack_index_body(float* smem, PayloadWords<WORL
       for (int g = 0; g < G; ++g) four[g] = stage[g * (8 * F::kElems) + j * 32 + lane];
       float acc[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        uint32_t byte[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) byte[g] = (four[g] >> (8 * k)) & 255u;
-        acc[k] = sum_of(byte);
-      }
+      for (int k = 0; k < 4; ++k) acc[k] = sum_of(four, k);
       unpack_finish4<APPLY>(acc, o, j * 128, add, post_scale, apply, c * F::kChunk + lane * 4 + j * 128);
     }
     __syncwarp();
@@ -543,7 +568,7 @@ __device__ __forceinline__ void unpack_index_body(float* smem, PayloadWords<WORL
           byte[g] |= q << (BW * p);
         }
       }
-      unpack_finish1<APPLY>(sum_of(byte), out, e, add, post_scale, apply);
+      unpack_finish1<APPLY>(sum_of(byte, 0), out, e, add, post_scale, apply);
     }
   }
 }
