@@ -11,8 +11,10 @@
 // quantise / update H / pack / store to every destination / publish flag.  Both read
 // with 16-byte loads when the arrays are aligned, take the step's epoch (flag value, slot
 // parity, rounding seed) from the device when asked to, and return at once when an earlier
-// kernel of the step recorded a failure.
+// kernel of the step recorded a failure.  Callers that have the GPU to themselves get both in one launch where
+// the tensor fits the chip (ecq_hold_kernel).
 #include "../common/codec_math.h"
+#include "hold.cuh"
 #include "kernels.h"
 #include "launch.cuh"
 #include "p2p.cuh"
@@ -33,6 +35,53 @@ inline int grid_for(int64_t items, int threads, int max_blocks) {
   if (blocks < 1) blocks = 1;
   if (blocks > max_blocks) blocks = max_blocks;
   return int(blocks);
+}
+
+struct EcqScale {
+  float mx, gap, inv;
+  bool zero;   // nothing to send: every level is 0
+};
+__device__ __forceinline__ EcqScale ecq_scale(float absmax, int bw) {
+  EcqScale s;
+  s.zero = absmax < kEcqZeroCutoff;
+  s.mx = s.zero ? 0.0f : absmax;
+  s.gap = s.zero ? 0.0f : ecq_gap(absmax, bw);
+  s.inv = s.zero ? 0.0f : ecq_gap_inverse(s.gap);
+  return s;
+}
+__device__ __forceinline__ void ecq_put_header(const PushTargets& dst, int64_t n, int bw, float mx) {
+  const int dpb = 8 / bw;
+  const int64_t M = (n + dpb - 1) / dpb;
+  const uint32_t total = uint32_t(kEcqHeaderBytes + M);
+  const uint32_t mb = __float_as_uint(mx);
+  uint8_t header[kEcqHeaderBytes];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    header[k] = uint8_t(total >> (8 * k));
+    header[4 + k] = uint8_t(mb >> (8 * k));
+  }
+  header[8] = uint8_t(bw);
+  header[9] = uint8_t(M * dpb - n);
+  push_bytes(dst, 0, header, kEcqHeaderBytes);
+}
+
+// `count` elements of one payload byte: v = g + alpha * h in, h takes the new history; returns the byte.
+template <int BW>
+__device__ __forceinline__ uint32_t ecq_quant_byte(const float* v, float* h, int count, float beta, const EcqScale& s, uint64_t seed,
+                                                   int64_t byte_index) {
+  uint8_t q = 0;
+  Lcg32 rng(tern_byte_seed(seed, byte_index));
+#pragma unroll
+  for (int j = 0; j < 8 / BW; ++j) {
+    if (j < count) {
+      uint8_t t = 0;
+      if (!s.zero) t = ecq_quant(v[j], s.mx, s.inv, rng.next_unit());
+      q = uint8_t(q | (int(t) << (BW * j)));
+      const uint32_t kept = uint32_t(t) & ((1u << BW) - 1u);
+      h[j] = ecq_history(h[j], beta, v[j], ecq_dequant(kept, s.gap, s.mx));
+    }
+  }
+  return q;
 }
 
 template <bool VEC>
@@ -68,26 +117,12 @@ ecq_absmax_header_kernel(const float* __restrict__ grad, const float* __restrict
   float gmn, gmx;
   if (!grid_minmax_last_block<kThreads>(scratch, unused, mx, gmn, gmx)) return;
   if (threadIdx.x == 0) {
-    const bool zero = gmx < kEcqZeroCutoff;
-    const float hmx = zero ? 0.0f : gmx;
-    const float gap = zero ? 0.0f : ecq_gap(gmx, bw);
-    scratch->mx = hmx;
-    scratch->mn = zero ? 1.0f : 0.0f;  // "zero tensor" marker for kernel 2
-    scratch->gap = gap;
-    scratch->inv = zero ? 0.0f : ecq_gap_inverse(gap);
-    const int dpb = 8 / bw;
-    const int64_t M = (n + dpb - 1) / dpb;
-    const uint32_t total = uint32_t(kEcqHeaderBytes + M);
-    const uint32_t mb = __float_as_uint(hmx);
-    uint8_t header[kEcqHeaderBytes];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      header[k] = uint8_t(total >> (8 * k));
-      header[4 + k] = uint8_t(mb >> (8 * k));
-    }
-    header[8] = uint8_t(bw);
-    header[9] = uint8_t(M * dpb - n);
-    push_bytes(dst, 0, header, kEcqHeaderBytes);
+    const EcqScale scale = ecq_scale(gmx, bw);
+    scratch->mx = scale.mx;
+    scratch->mn = scale.zero ? 1.0f : 0.0f;  // for kernel 2
+    scratch->gap = scale.gap;
+    scratch->inv = scale.inv;
+    ecq_put_header(dst, n, bw, scale.mx);
   }
 }
 
@@ -109,23 +144,12 @@ ecq_quant_kernel(const float* __restrict__ grad, float* __restrict__ hist, int64
   if (dst.epoch_dev != nullptr) seed += uint64_t(dst.epoch) * kEpochSeedStride;
   constexpr int DPB = 8 / BW;
   constexpr int BPT = 4 / DPB;  // bytes per thread: 1, 2, 4
-  const float mx = scratch->mx, inv = scratch->inv, gap = scratch->gap;
-  const bool zero = scratch->mn != 0.0f;
+  const EcqScale scale{scratch->mx, scratch->gap, scratch->inv, scratch->mn != 0.0f};
   auto quant_byte = [&](const float* g, float* h, int count, int64_t byte_index) -> uint32_t {
-    uint8_t q = 0;
-    Lcg32 rng(tern_byte_seed(seed, byte_index));
+    float v[DPB];
 #pragma unroll
-    for (int j = 0; j < DPB; ++j) {
-      if (j < count) {
-        const float v = ecq_compensated(g[j], h[j], alpha);
-        uint8_t t = 0;
-        if (!zero) t = ecq_quant(v, mx, inv, rng.next_unit());
-        q = uint8_t(q | (int(t) << (BW * j)));
-        const uint32_t kept = uint32_t(t) & ((1u << BW) - 1u);
-        h[j] = ecq_history(h[j], beta, v, ecq_dequant(kept, gap, mx));
-      }
-    }
-    return q;
+    for (int j = 0; j < DPB; ++j) v[j] = j < count ? ecq_compensated(g[j], h[j], alpha) : 0.0f;
+    return ecq_quant_byte<BW>(v, h, count, beta, scale, seed, byte_index);
   };
   int64_t unit0 = 0;   // first unit of the rest
   if (VEC && shift >= 0) {
@@ -243,6 +267,92 @@ ecq_quant_kernel(const float* __restrict__ grad, float* __restrict__ hist, int64
     }
   }
   publish_when_grid_done(dst);
+}
+
+// Medium tensors, callers that have the GPU to themselves: both passes in one launch that reads the gradient
+// once.  What a CTA keeps in shared memory is v = g + alpha * h; the history itself is read again, from L2,
+// where it and the gradient (two tensors of 30 MB at most) still are.  All CTAs have to be resident at once, each
+// with an SM to itself: the exchange engine, whose compressor runs beside the backward pass, keeps the two launches.
+// 25 MB, 4 bits, in a chain of calls: 26.5 us; 28.4 in two launches.  256 KB: 6.4 and 8.1.
+constexpr int kHoldAhead = 4;   // history words of a thread in flight
+template <int BW>
+__global__ void __launch_bounds__(kHoldThreads, 1)
+ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t part, float alpha, float beta, uint64_t seed,
+                PushTargets dst, MinMaxScratch* scratch, int shift, uint64_t wait_ns, int* status) {
+  constexpr int DPB = 8 / BW, BPT = 4 / DPB;
+  extern __shared__ __align__(16) float hold[];           // [part], then the payload bytes
+  __shared__ EcqScale shared_scale;
+  uint8_t* const bytes_at = reinterpret_cast<uint8_t*>(hold + part);
+  const int tid = threadIdx.x;
+  const int64_t begin = int64_t(blockIdx.x) * part;       // a multiple of 512
+  const int64_t left = n - begin;
+  const int len = int(left < 0 ? 0 : (left < part ? left : part));
+  const float4* g4 = reinterpret_cast<const float4*>(grad + begin);
+  float4* h4 = reinterpret_cast<float4*>(hist + begin);
+  float mn = 0.0f, mx = 0.0f;
+  const int quads = len >> 2;
+  auto take = [&](int i, float4 g, float4 h) {
+    const float4 v = make_float4(ecq_compensated(g.x, h.x, alpha), ecq_compensated(g.y, h.y, alpha),
+                                 ecq_compensated(g.z, h.z, alpha), ecq_compensated(g.w, h.w, alpha));
+    mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    reinterpret_cast<float4*>(hold)[i] = v;
+  };
+  int q = tid;
+  for (; q + (kHoldAhead - 1) * kHoldThreads < quads; q += kHoldAhead * kHoldThreads) {
+    float4 g[kHoldAhead], h[kHoldAhead];
+#pragma unroll
+    for (int u = 0; u < kHoldAhead; ++u) {
+      g[u] = __ldg(g4 + q + u * kHoldThreads);
+      h[u] = h4[q + u * kHoldThreads];
+    }
+#pragma unroll
+    for (int u = 0; u < kHoldAhead; ++u) take(q + u * kHoldThreads, g[u], h[u]);
+  }
+  for (; q < quads; q += kHoldThreads) take(q, __ldg(g4 + q), h4[q]);
+  for (int e = 4 * quads + tid; e < len; e += kHoldThreads)   // fewer than four
+    mx = fmaxf(mx, fabsf(ecq_compensated(grad[begin + e], hist[begin + e], alpha)));
+  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status)) return;
+  if (tid == 0) {
+    shared_scale = ecq_scale(mx, BW);
+    if (blockIdx.x == 0) ecq_put_header(dst, n, BW, shared_scale.mx);
+  }
+  __syncthreads();
+  const EcqScale scale = shared_scale;
+  const int64_t byte0 = begin / DPB;                       // first payload byte of the part
+  auto quantise = [&](int u, float4 old) {
+    const float4 held = reinterpret_cast<const float4*>(hold)[u];
+    const float v[4] = {held.x, held.y, held.z, held.w};
+    float h[4] = {old.x, old.y, old.z, old.w};
+    uint32_t bytes = 0;
+#pragma unroll
+    for (int b = 0; b < BPT; ++b)
+      bytes |= ecq_quant_byte<BW>(v + b * DPB, h + b * DPB, DPB, beta, scale, seed, byte0 + int64_t(u) * BPT + b) << (8 * b);
+    h4[u] = make_float4(h[0], h[1], h[2], h[3]);
+    hold_unit_bytes<BPT>(bytes_at + shift + u * BPT, bytes);   // shift is even
+  };
+  int u = tid;
+  for (; u + (kHoldAhead - 1) * kHoldThreads < quads; u += kHoldAhead * kHoldThreads) {
+    float4 h[kHoldAhead];
+#pragma unroll
+    for (int k = 0; k < kHoldAhead; ++k) h[k] = h4[u + k * kHoldThreads];
+#pragma unroll
+    for (int k = 0; k < kHoldAhead; ++k) quantise(u + k * kHoldThreads, h[k]);
+  }
+  for (; u < quads; u += kHoldThreads) quantise(u, h4[u]);
+  __syncthreads();
+  hold_put(dst, kEcqHeaderBytes, byte0, bytes_at, shift, quads * BPT);
+  if (tid == 32) {   // fewer than four leftover elements
+    for (int e = 4 * quads; e < len; e += DPB) {
+      const int count = len - e < DPB ? len - e : DPB;
+      float v[DPB], h[DPB];
+      for (int j = 0; j < count; ++j) {
+        h[j] = hist[begin + e + j];
+        v[j] = ecq_compensated(grad[begin + e + j], h[j], alpha);
+      }
+      push_u8(dst, kEcqHeaderBytes + byte0 + e / DPB, uint8_t(ecq_quant_byte<BW>(v, h, count, beta, scale, seed, byte0 + e / DPB)));
+      for (int j = 0; j < count; ++j) hist[begin + e + j] = h[j];
+    }
+  }
 }
 
 // Headers of all payloads -> mx, gap, bw (shared memory); false, with the status word set, when one of
@@ -374,17 +484,31 @@ cudaError_t launch_ecq_index(const UnpackSources& src, float* out, int64_t n, fl
 
 cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alpha, float beta,
                          int bitwidth, uint64_t seed, const PushTargets& dst, void* scratch,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns) {
   if (n <= 0 || !ecq_bitwidth_ok(bitwidth) || scratch == nullptr) return cudaErrorInvalidValue;
   auto* s = static_cast<MinMaxScratch*>(scratch);
   PushTargets hdr_dst = dst;
   hdr_dst.done = nullptr;
   const bool vec = aligned16(grad) && aligned16(history);
+  const int shift = chunk_shift(dst, kEcqHeaderBytes);
+  if (hold_alone(whole_gpu, dst) && status != nullptr && vec && shift >= 0) {
+    HoldPlan hold;
+    cudaError_t e = hold_plan(n, bitwidth, hold);
+    if (e != cudaSuccess) return e;
+    if (hold.part > 0) {
+      auto kernel = bitwidth == 2 ? ecq_hold_kernel<2> : (bitwidth == 4 ? ecq_hold_kernel<4> : ecq_hold_kernel<8>);
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hold.smem));
+      if (e != cudaSuccess) return e;
+      e = launch_resident(kernel, dim3(hold.ctas), dim3(kHoldThreads), hold.smem, stream, grad, history, n, hold.part, alpha, beta,
+                          seed, dst, s, shift, grid_wait_ns, status);
+      if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+      cudaGetLastError();   // fewer SMs than the device has: the two launches below
+    }
+  }
   const int hgrid = grid_for((n + 3) >> 2, kThreads, 148 * 4);
   if (vec) ecq_absmax_header_kernel<true><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
   else ecq_absmax_header_kernel<false><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
   // chunked path once there is a chunk per warp of a half-filled GPU
-  const int shift = chunk_shift(dst, kEcqHeaderBytes);
   const int64_t chunks = n / (int64_t(kStageBytes) * (8 / bitwidth));
   const bool wide = vec && shift >= 0 && chunks >= 148 * 2;
   const int threads = wide ? 128 : kThreads;

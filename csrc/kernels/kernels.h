@@ -133,7 +133,8 @@ cudaError_t terngrad_unpack_accum(const UnpackSources& src, float* out, int64_t 
 // ---------------------------------------------------------------- ECQ
 cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alpha, float beta,
                          int bitwidth, uint64_t seed, const PushTargets& dst, void* scratch,
-                         cudaStream_t stream);
+                         cudaStream_t stream, bool whole_gpu = false, int* status = nullptr,
+                         uint64_t grid_wait_ns = kGridWaitNs);   // the last three: see terngrad_compress
 cudaError_t ecq_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
                              float post_scale, int* status, cudaStream_t stream);
 

@@ -15,6 +15,7 @@
 // Unpack-accumulate decodes the payloads of all ranks in one pass, each with
 // its own header, in ascending rank order.
 #include "../common/codec_math.h"
+#include "hold.cuh"
 #include "kernels.h"
 #include "launch.cuh"
 #include "p2p.cuh"
@@ -485,16 +486,6 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
 // free) and 260 in two launches; on an idle GPU 64 and 71 us.
 // 25 MB with error feedback, 2 bits (ncu, cold): 21.3 us; 14.3 + 18.0 in two launches.  9.4 MB at 4 bits, compress
 // and decode: 14.4 and 18.4.
-constexpr int kHoldThreads = 1024;
-constexpr size_t kHoldBytes = 208 * 1024;    // of grad + residual per CTA
-template <int BW> struct HoldForm {
-  static constexpr int kDpb = 8 / BW;
-  static constexpr int kUnit = Unit<BW>::EPT;
-  // a CTA's part: a multiple of 512 elements, so that the parts' payload bytes start equally far past a
-  // 16-byte boundary (64 bytes at 1 bit) and its units are whole
-  static constexpr int kGrain = 512;
-  static constexpr size_t stage_bytes(int64_t part) { return size_t(part / kDpb) + 32; }
-};
 template <int BW, bool EF>
 __global__ void __launch_bounds__(kHoldThreads, 1)
 tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int64_t part, int random,
@@ -563,30 +554,12 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
         reinterpret_cast<float4*>(residual + begin)[u * (EPT / 4) + v] =
             make_float4(ef[4 * v], ef[4 * v + 1], ef[4 * v + 2], ef[4 * v + 3]);
     }
-    uint8_t* at = bytes_at + shift + u * BPT;              // shift is even
-    if (BPT == 1) {
-      *at = uint8_t(b);
-    } else {
-#pragma unroll
-      for (int h = 0; h < BPT / 2; ++h) reinterpret_cast<uint16_t*>(at)[h] = uint16_t(b >> (16 * h));
-    }
+    hold_unit_bytes<BPT>(bytes_at + shift + u * BPT, b);   // shift is even
   }
   __syncthreads();
-  // the part's bytes: 16-byte words of the destination, the first and the last one by bytes
-  const int count = units * BPT;
-  const int words = (shift + count) >> 4;                  // words that end inside the part
-  for (int w = tid + (shift != 0 ? 1 : 0); w < words; w += kHoldThreads)
-    put_u128(dst, cur, kTernHeaderBytes + byte0 - shift + 16 * w, reinterpret_cast<const uint4*>(bytes_at)[w]);
-  const int head_end = shift == 0 ? 0 : (16 < shift + count ? 16 : shift + count);
-  const int tail_begin = words * 16 > head_end ? words * 16 : head_end;
-  if (tid < 16) {
-    if (tid >= shift && tid < head_end) put_u8(dst, cur, kTernHeaderBytes + byte0 - shift + tid, bytes_at[tid]);
-  } else if (tid < 32) {
-    const int at = tail_begin + tid - 16;
-    if (at >= shift && at < shift + count) put_u8(dst, cur, kTernHeaderBytes + byte0 - shift + at, bytes_at[at]);
-  } else if (tid == 32 && len > 0 && units * EPT < len) {
+  hold_put(dst, kTernHeaderBytes, byte0, bytes_at, shift, units * BPT);
+  if (tid == 32 && len > 0 && units * EPT < len)
     tern_leftover<BW, EF>(grad, residual, begin + int64_t(units) * EPT, n, mn, inv, gap, random, seed, dst, cur);
-  }
 }
 
 struct TernHeader {
@@ -826,8 +799,7 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
   }
   // a caller that has the GPU to itself, and a destination of this call's own: one launch where the tensor
   // fits (see tern_small_kernel and tern_hold_kernel)
-  const bool own = whole_gpu && S == 0 && dst.world == 1 && dst.done == nullptr && dst.guard == nullptr &&
-                   dst.epoch_dev == nullptr && dst.remote == 0 && dst.mc == nullptr;
+  const bool own = hold_alone(whole_gpu, dst);
   if (own && n <= kSmallElems) {
 #define LAUNCH_SMALL(BW, V, E) \
   tern_small_kernel<BW, V, E><<<kSmallCtas, kSmallThreads, 0, stream>>>(grad, residual, n, enable_random, seed, dst)
@@ -837,25 +809,18 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
   }
   // 16-byte aligned inputs, and a part per SM that fits its shared memory: one read of them
   if (own && status != nullptr && vec && shift >= 0) {
-    int device = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    HoldPlan hold;
+    cudaError_t e = hold_plan(n, bitwidth, hold);
     if (e != cudaSuccess) return e;
-    if (sms > kReduceMaxBlocks) sms = kReduceMaxBlocks;
-    const int64_t part = ((n + sms - 1) / sms + 511) / 512 * 512;
-    if (part * int64_t(sizeof(float)) <= int64_t(kHoldBytes)) {
-      const unsigned ctas = unsigned((n + part - 1) / part);
-#define LAUNCH_HOLD_AS(BW, E)                                                                                     \
-  do {                                                                                                            \
-    const size_t smem = size_t(part) * sizeof(float) + HoldForm<BW>::stage_bytes(part);                           \
-    if (smem <= 224 * 1024) {                                                                                     \
-      e = cudaFuncSetAttribute(tern_hold_kernel<BW, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));  \
-      if (e != cudaSuccess) return e;                                                                             \
-      e = launch_resident(tern_hold_kernel<BW, E>, dim3(ctas), dim3(kHoldThreads), smem, stream, grad, residual,  \
-                          n, part, enable_random, seed, dst, s, shift, grid_wait_ns, status);                     \
-      if (e != cudaErrorCooperativeLaunchTooLarge) return e;                                                      \
-      cudaGetLastError();   /* fewer SMs than the device has: the two launches below */                           \
-    }                                                                                                             \
+    if (hold.part > 0) {
+#define LAUNCH_HOLD_AS(BW, E)                                                                                       \
+  do {                                                                                                              \
+    e = cudaFuncSetAttribute(tern_hold_kernel<BW, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(hold.smem)); \
+    if (e != cudaSuccess) return e;                                                                                 \
+    e = launch_resident(tern_hold_kernel<BW, E>, dim3(hold.ctas), dim3(kHoldThreads), hold.smem, stream, grad,      \
+                        residual, n, hold.part, enable_random, seed, dst, s, shift, grid_wait_ns, status);          \
+    if (e != cudaErrorCooperativeLaunchTooLarge) return e;                                                          \
+    cudaGetLastError();   /* fewer SMs than the device has: the two launches below */                               \
   } while (0)
 #define LAUNCH_HOLD(BW) \
   if (ef) LAUNCH_HOLD_AS(BW, true); else LAUNCH_HOLD_AS(BW, false)

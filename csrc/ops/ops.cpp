@@ -418,7 +418,8 @@ void ecq_compress(const torch::Tensor& grad, torch::Tensor history, torch::Tenso
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
     HP_CHECK_CUDA(cuda::ecq_compress(grad.data_ptr<float>(), history.data_ptr<float>(), n,
                                      float(alpha), float(beta), int(bitwidth), uint64_t(seed),
-                                     local_target(out), scratch, at::cuda::getCurrentCUDAStream()));
+                                     local_target(out), scratch, at::cuda::getCurrentCUDAStream(),
+                                     /*whole_gpu=*/true, status_word_for(grad)));
   } else {
     const int rc = cpu::ecq_compress(grad.data_ptr<float>(), history.data_ptr<float>(), n,
                                      float(alpha), float(beta), int(bitwidth), uint64_t(seed),

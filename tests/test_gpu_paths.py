@@ -350,6 +350,26 @@ def test_terngrad_resident_form(bw, feedback, offset):
             assert torch.equal(rg.cpu(), rc), n
 
 
+@pytest.mark.parametrize("bw", [2, 4, 8])
+@pytest.mark.parametrize("offset", [0, 6])
+def test_ecq_resident_form(bw, offset):
+    """One element, ragged last parts, the largest part and one element beyond it; a tensor of zeros."""
+    largest = 148 * 208 * 256
+    for n in (1, 511, 513, 148 * 1024 - 1, 148 * 1024 + 1, 2359807) + ((largest, largest + 1) if bw == 2 else ()):
+        for std in (0.01, 0.0):
+            g, h = gauss(n, std, seed=n), gauss(n, 0.4 * std, seed=n + 1)
+            hc, hg = h.clone(), h.cuda()
+            ref = ops.ecq_compress(g, hc, 1.0, 0.9, bw, 7)
+            out = torch.zeros(ref.numel() + offset + 64, dtype=torch.uint8, device="cuda")
+            dev_g = g.cuda()
+            for _ in range(2):      # back to back: the shared state is left ready
+                hg.copy_(h)
+                ops.ecq_compress(dev_g, hg, 1.0, 0.9, bw, 7, out=out[offset:offset + ref.numel()])
+            assert torch.equal(out[offset:offset + ref.numel()].cpu(), ref), n
+            assert int(out[offset + ref.numel():].sum()) == 0, n
+            assert torch.equal(hg.cpu(), hc), n
+
+
 def test_terngrad_resident_form_when_its_wait_runs_out():
     """A counter that starts one short: no CTA ever sees all others arrive.  The wait ends, the status word says so, and
     the next call finds its state ready."""
