@@ -742,91 +742,96 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
 // ---------------------------------------------------------------- M = grad + residual, P = M Q
 // Both in one pass over the matrix, fp32 throughout.  At ranks up to 8 the products are a few per cent of
 // what the SMs can do in the time the matrix takes to stream, while a second launch reads all of M again
-// (and the tensor cores would round it to tf32).  A CTA owns 32 / R rows; each thread walks its columns
-// four at a time with the Q rows of those columns in registers, used by all rows, and four rows' loads
-// in flight.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across
+// (and the tensor cores would round it to tf32).  A CTA owns a range of rows and takes up to 32 / R of them at a
+// time; each thread walks its columns four at a time with the Q rows of those columns in registers, used by all of
+// these rows, and four rows' loads in flight.  Two CTAs fit an SM, and the rows are shared out evenly over that many.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across
 // the warps in shared memory.  Few rows are also split by columns; the parts then meet in P by atomics,
 // which the launcher zeroes first.
-// 4096 x 4096, rank 4 (ncu, cold): 32 us; as add 28.9, zero 2.5, transpose 3.5 and tensor-core projection
+// 4096 x 4096, rank 4, in a chain of calls: 37.8 us, 38.4 as 512 CTAs of eight rows.  (ncu, cold) 32 us so; as add 28.9, zero 2.5, transpose 3.5 and tensor-core projection
 // 15.2.  Error of the three stages against 64 bits 7.4e-4, and 8.4e-4 with the projection in tf32.
 template <int R>
 __global__ void __launch_bounds__(256, 2)
 add_project_kernel(const float* __restrict__ grad, const float* __restrict__ residual, int64_t N, float* __restrict__ Mat,
-                   int64_t n, int64_t m, const float* __restrict__ Q, float* __restrict__ P, int64_t cols_per_cta) {
-  constexpr int RB = 32 / R;                    // rows per CTA
+                   int64_t n, int64_t m, const float* __restrict__ Q, float* __restrict__ P, int64_t cols_per_cta,
+                   int64_t rows_per_cta, int rows_at_once) {
+  constexpr int RB = 32 / R;                    // rows at once, at most
   constexpr int RG = 4;                         // rows whose loads are issued together
   __shared__ float sums[8][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t i0 = int64_t(blockIdx.x) * RB;
   const int64_t c_end = min(int64_t(blockIdx.y + 1) * cols_per_cta, m);
-  float acc[32];                                // [row][column of Q]
+  const int64_t r_end = min(int64_t(blockIdx.x + 1) * rows_per_cta, n);
+  for (int64_t i0 = int64_t(blockIdx.x) * rows_per_cta; i0 < r_end; i0 += rows_at_once) {
+    const int rows = int(min(int64_t(rows_at_once), r_end - i0));
+    float acc[32];                                // [row][column of Q]
 #pragma unroll
-  for (int k = 0; k < 32; ++k) acc[k] = 0.f;
-  for (int64_t col = int64_t(blockIdx.y) * cols_per_cta + tid * 4; col < c_end; col += 1024) {
-    float q[4 * R];
+    for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+    for (int64_t col = int64_t(blockIdx.y) * cols_per_cta + tid * 4; col < c_end; col += 1024) {
+      float q[4 * R];
 #pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(Q + col * R) + k);
-      q[4 * k] = t.x; q[4 * k + 1] = t.y; q[4 * k + 2] = t.z; q[4 * k + 3] = t.w;
-    }
+      for (int k = 0; k < R; ++k) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(Q + col * R) + k);
+        q[4 * k] = t.x; q[4 * k + 1] = t.y; q[4 * k + 2] = t.z; q[4 * k + 3] = t.w;
+      }
 #pragma unroll
-    for (int g0 = 0; g0 < RB; g0 += RG) {
-      float4 a[RG], b[RG];
+      for (int g0 = 0; g0 < RB; g0 += RG) {
+        float4 a[RG], b[RG];
 #pragma unroll
-      for (int k = 0; k < RG; ++k) {
-        const int64_t e = (i0 + g0 + k) * m + col;
-        a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i0 + g0 + k < n) {
-          if (e + 3 < N) {
-            a[k] = __ldg(reinterpret_cast<const float4*>(grad + e));
-            b[k] = __ldg(reinterpret_cast<const float4*>(residual + e));
-          } else {   // past the gradient the matrix keeps what it holds
-            float* x = reinterpret_cast<float*>(&a[k]);
-            float* y = reinterpret_cast<float*>(&b[k]);
-            for (int j = 0; j < 4; ++j) {
-              if (e + j < N) {
-                x[j] = grad[e + j];
-                y[j] = residual[e + j];
-              } else {
-                x[j] = Mat[e + j];
+        for (int k = 0; k < RG; ++k) {
+          const int64_t e = (i0 + g0 + k) * m + col;
+          a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (g0 + k < rows) {
+            if (e + 3 < N) {
+              a[k] = __ldg(reinterpret_cast<const float4*>(grad + e));
+              b[k] = __ldg(reinterpret_cast<const float4*>(residual + e));
+            } else {   // past the gradient the matrix keeps what it holds
+              float* x = reinterpret_cast<float*>(&a[k]);
+              float* y = reinterpret_cast<float*>(&b[k]);
+              for (int j = 0; j < 4; ++j) {
+                if (e + j < N) {
+                  x[j] = grad[e + j];
+                  y[j] = residual[e + j];
+                } else {
+                  x[j] = Mat[e + j];
+                }
               }
             }
           }
         }
+#pragma unroll
+        for (int k = 0; k < RG; ++k) {
+          const float x[4] = {a[k].x + b[k].x, a[k].y + b[k].y, a[k].z + b[k].z, a[k].w + b[k].w};
+          if (g0 + k < rows)
+            *reinterpret_cast<float4*>(Mat + (i0 + g0 + k) * m + col) = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int c = 0; c < R; ++c) acc[(g0 + k) * R + c] += x[j] * q[j * R + c];
+        }
       }
+    }
+    // lane L ends up with the warp's sum of acc[L]
 #pragma unroll
-      for (int k = 0; k < RG; ++k) {
-        const float x[4] = {a[k].x + b[k].x, a[k].y + b[k].y, a[k].z + b[k].z, a[k].w + b[k].w};
-        if (i0 + g0 + k < n)
-          *reinterpret_cast<float4*>(Mat + (i0 + g0 + k) * m + col) = make_float4(x[0], x[1], x[2], x[3]);
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool upper = (lane & o) != 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int c = 0; c < R; ++c) acc[(g0 + k) * R + c] += x[j] * q[j * R + c];
+      for (int k = 0; k < o; ++k) {
+        const float keep = upper ? acc[k + o] : acc[k], send = upper ? acc[k] : acc[k + o];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
       }
     }
-  }
-  // lane L ends up with the warp's sum of acc[L]
+    sums[warp][lane] = acc[0];
+    __syncthreads();
+    if (warp == 0) {
+      float x = 0.f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool upper = (lane & o) != 0;
-#pragma unroll
-    for (int k = 0; k < o; ++k) {
-      const float keep = upper ? acc[k + o] : acc[k], send = upper ? acc[k] : acc[k + o];
-      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      for (int w = 0; w < 8; ++w) x += sums[w][lane];
+      if (lane / R < rows) {
+        float* p = P + i0 * R + lane;
+        if (gridDim.y == 1) *p = x;
+        else atomicAdd(p, x);
+      }
     }
-  }
-  sums[warp][lane] = acc[0];
-  __syncthreads();
-  if (warp == 0) {
-    float x = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) x += sums[w][lane];
-    if (i0 + lane / R < n) {
-      float* p = P + i0 * R + lane;
-      if (gridDim.y == 1) *p = x;
-      else atomicAdd(p, x);
-    }
+    __syncthreads();   // the sums are written again
   }
 }
 
@@ -903,10 +908,13 @@ cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N
                              const float* Q, int r, float* P, cudaStream_t stream) {
   if (n < 1 || m < 1 || N < 0 || N > n * m || !psgd_add_project_eligible(grad, residual, Mat, Q, m, r))
     return cudaErrorInvalidValue;
-  const int64_t row_blocks = (n + 32 / r - 1) / (32 / r);
   // two resident CTAs per SM; columns in steps of 1,024 (one per thread of a CTA, four wide)
+  constexpr int64_t resident = 148 * 2;
+  const int64_t most = 32 / r, rows_per = std::max<int64_t>(most, (n + resident - 1) / resident);
+  const int64_t turns = (rows_per + most - 1) / most, at_once = (rows_per + turns - 1) / turns;
+  const int64_t row_blocks = (n + rows_per - 1) / rows_per;
   const int64_t steps = (m + 1023) / 1024;
-  int64_t splits = (148 * 2 + row_blocks - 1) / row_blocks;
+  int64_t splits = rows_per > most ? 1 : (resident + row_blocks - 1) / row_blocks;
   if (splits > steps) splits = steps;
   const int64_t cols = (steps + splits - 1) / splits * 1024;
   const dim3 grid(unsigned(row_blocks), unsigned((m + cols - 1) / cols));
@@ -914,7 +922,8 @@ cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N
     const cudaError_t e = cudaMemsetAsync(P, 0, size_t(n) * r * sizeof(float), stream);
     if (e != cudaSuccess) return e;
   }
-#define HP_ADD_PROJECT(RR) add_project_kernel<RR><<<grid, 256, 0, stream>>>(grad, residual, N, Mat, n, m, Q, P, cols)
+#define HP_ADD_PROJECT(RR) \
+  add_project_kernel<RR><<<grid, 256, 0, stream>>>(grad, residual, N, Mat, n, m, Q, P, cols, rows_per, int(at_once))
   switch (r) {
     case 1: HP_ADD_PROJECT(1); break;
     case 2: HP_ADD_PROJECT(2); break;
