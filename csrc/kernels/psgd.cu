@@ -411,17 +411,28 @@ constexpr int kGsThreads = 1024;
 // Factors of up to 1024 * Q rows stay in registers: a thread holds Q rows of the (up to) R columns.  A
 // reduction is then a warp shuffle, one barrier, and a second shuffle over the 32 warps' sums, which every
 // warp does for itself.
-// 4096 x 4 (ncu, cold): 13.8 us; 24.9 with one reduction per column pair and the matrix in memory.
+// 4096 x 4, in a chain of calls: 8.1 us; 13.0 with the rows read and written value by value (a store of one column
+// touches 16 sectors: half of the kernel's time).  (ncu, cold) 13.8 so; 24.9 with one reduction per column pair and the matrix in memory.
 template <int R, int Q>
 __device__ __forceinline__ void gs_in_registers(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt,
                                                 int64_t rows_pad, float (*part)[32][16] /* [2] */) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float v[Q][R];
+  // a row is one or more 16-byte words when the columns are as many as compiled for
+  const bool words = R % 4 == 0 && r == R && (reinterpret_cast<uintptr_t>(P) & 15) == 0;
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int64_t i = tid + int64_t(q) * kGsThreads;
+    if (words) {
 #pragma unroll
-    for (int c = 0; c < R; ++c) v[q][c] = (i < n && c < r) ? P[i * r + c] : 0.0f;
+      for (int c = 0; c + 3 < R; c += 4) {
+        const float4 x = i < n ? *reinterpret_cast<const float4*>(P + i * R + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[q][c] = x.x; v[q][c + 1] = x.y; v[q][c + 2] = x.z; v[q][c + 3] = x.w;
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < R; ++c) v[q][c] = (i < n && c < r) ? P[i * r + c] : 0.0f;
+    }
   }
 #pragma unroll
   for (int j = 0; j < R; ++j) {
@@ -455,10 +466,15 @@ __device__ __forceinline__ void gs_in_registers(float* __restrict__ P, int64_t n
   for (int q = 0; q < Q; ++q) {
     const int64_t i = tid + int64_t(q) * kGsThreads;
     if (i < n) {
+      if (words) {
+#pragma unroll
+        for (int c = 0; c + 3 < R; c += 4)
+          *reinterpret_cast<float4*>(P + i * R + c) = make_float4(v[q][c], v[q][c + 1], v[q][c + 2], v[q][c + 3]);
+      }
 #pragma unroll
       for (int c = 0; c < R; ++c) {
         if (c < r) {
-          P[i * r + c] = v[q][c];
+          if (!words) P[i * r + c] = v[q][c];
           if (Xt != nullptr) Xt[c * rows_pad + i] = v[q][c];
         }
       }
@@ -518,6 +534,7 @@ __device__ __forceinline__ void gram_schmidt_cta(float* P, int64_t n, int r, flo
   __shared__ float part[2][32][16];
   if (r == 1 && n <= 16 * kGsThreads) gs_in_registers<1, 16>(P, n, r, eps, Xt, rows_pad, part);
   else if (r == 2 && n <= 16 * kGsThreads) gs_in_registers<2, 16>(P, n, r, eps, Xt, rows_pad, part);
+  else if (r <= 4 && n <= 4 * kGsThreads) gs_in_registers<4, 4>(P, n, r, eps, Xt, rows_pad, part);
   else if (r <= 4 && n <= 8 * kGsThreads) gs_in_registers<4, 8>(P, n, r, eps, Xt, rows_pad, part);
   else if (r <= 8 && n <= 4 * kGsThreads) gs_in_registers<8, 4>(P, n, r, eps, Xt, rows_pad, part);
   else if (r <= 16 && n <= 2 * kGsThreads) gs_in_registers<16, 2>(P, n, r, eps, Xt, rows_pad, part);

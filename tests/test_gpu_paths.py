@@ -308,6 +308,16 @@ def test_gram_schmidt_forms(n, r):
     assert (got[:, :cols].double().cpu() - want[:, :cols]).norm() <= 2e-5 * want[:, :cols].norm()
 
 
+@pytest.mark.parametrize("n,r", [(3, 4), (4096, 4), (4097, 4), (1025, 8), (2048, 16)])
+def test_gram_schmidt_of_rows_off_a_word(n, r):
+    """Rows that are whole 16-byte words, at an address that is none: value by value, with the same result."""
+    P = gauss(n * r, 1.0, seed=n).view(n, r)
+    buf = torch.zeros(n * r + 1, device="cuda")
+    buf[1:] = P.view(-1).cuda()
+    off = ops.gram_schmidt(buf[1:].view(n, r))
+    assert torch.equal(off, ops.gram_schmidt(P.cuda())) and float(buf[0]) == 0.0
+
+
 @pytest.mark.parametrize("n,m,r", [(1, 4, 1), (7, 1028, 1), (33, 1024, 2), (64, 25088, 4), (9, 4096, 4), (1000, 2052, 4),
                                    (13, 300, 8), (4096, 512, 8)])
 @pytest.mark.parametrize("short", [0, 3])
