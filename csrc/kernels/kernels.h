@@ -153,7 +153,7 @@ cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sampl
 //           the bucket's gradient to norm `clip` (> 0; sumsq: one float of scratch, zero on entry,
 //           left zero).  zero_grad leaves zeros in grad: the dense gradient is rebuilt from the
 //           payloads afterwards, which saves the separate clearing pass.
-// For keep fractions up to 1 % the tensor is read once ("list form", see sparse.cu); otherwise,
+// For small keep fractions (kListMaxKeep in sparse.cu) the tensor is read once ("list form", see sparse.cu); otherwise,
 // or when the scratch cannot hold the expected candidates, the multi-pass scan form runs.
 // scratch: sparse_scratch_bytes(n) bytes, zero before its first use.  status: where a wait between CTAs that
 // runs out is recorded (kGridWait).  launches: the kernels launched are added to it.

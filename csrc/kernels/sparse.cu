@@ -14,7 +14,7 @@
 //   trim x2     Only when more than ceil(N*keep) candidates qualified (decided on the device; otherwise
 //               the kernels return at once): the exact cut.  One pass over R; the second kernel only
 //               has work when the cut lies more than a factor of two above the threshold.
-//   write       Ordered compaction: indices ascending, values, residual zeroing, stored into every
+//   write       Ordered compaction in one pass: indices ascending, values, residual zeroing, stored into every
 //               destination (local and NVLink peers), then the completion flag.
 //
 // Content rule (identical to the CPU codec): keep |R[i]| > threshold in
@@ -22,7 +22,7 @@
 // toward the lower index.
 //
 // Two forms of everything after the sampling.  The passes above ("scan form") read the whole
-// tensor three or four times.  For keep fractions up to 1 % the "list form" reads it ONCE:
+// tensor two or three times.  For small keep fractions (kListMaxKeep) the "list form" reads it ONCE:
 //
 //   count+collect  the one pass over the tensor.  It applies the codec's state update (R += G
 //               for GradDrop; u = m*u + s*g, v += u and g = 0 for DGC with momentum correction;
@@ -30,17 +30,17 @@
 //               (index, value), to a per-warp list in index order.  A warp owns a contiguous
 //               part of its CTA's chunk, so the lists, taken in order, are sorted by index.
 //               Lists grow in blocks of 16 entries taken from a pool with one atomic.
-//   cut         One CTA (eight for large selections): when more than ceil(N*keep) candidates qualified,
-//               their keys (35 K for a 128 MB bucket at 0.1 %) are gathered into shared memory with
-//               batched loads and the exact cut is found by a radix select there.  It then counts what
-//               each CTA's lists keep and turns the counts into offsets, k and the header.
-//   emit        One warp per list: indices and values to every destination, residual (and
-//               DGC's momentum u) cleared at the emitted positions, then the completion flag.
+//   cut         One CTA (eight for large selections): when more than ceil(N*keep) candidates qualified, the
+//               exact cut, from counts that the collect pass has made of the candidates' magnitudes and
+//               from the candidates themselves in the one bin that holds it.
+//   emit        One warp per list: what each CTA's lists keep, where that starts (kept_before), then indices
+//               and values to every destination, residual (and DGC's momentum u) cleared at the emitted
+//               positions, and the completion flag.
 //
 // The kernels of a call overlap at their ends (launch.cuh): at 25 MB none but the pass over the tensor
 // takes longer than the gap between two plain launches.
-// Compress and decode, 64 MB, GradDrop at 0.1 %, four payloads: 112 us, and 129 as eight plain launches (the
-// same decode); 25 MB, DGC, eight payloads: 82 and 102.
+// Compress and decode, with the decode of that time, 64 MB, GradDrop at 0.1 %, four payloads: 112 us, and 129 as eight
+// plain launches; 25 MB, DGC, eight payloads: 82 and 102.
 //
 // A sample of more than a hundredth of the elements does not fit the key array; its keys are then drawn
 // again in each of three rounds, one per digit.  The pool is sized for many times the expected number of
@@ -72,7 +72,11 @@ constexpr int kTile = kThreads * 4;  // elements per CTA iteration
 constexpr int kMaxLists = kMaxBlocks * (kThreads / 32);
 constexpr int kBlockEntries = 16;
 constexpr unsigned int kNoBlock = 0xffffffffu;
-constexpr double kListMaxKeep = 0.01;   // the list form serves keep fractions up to this
+// The list form serves keep fractions up to these, for tensors up to a size and larger ones.  Lists against scan,
+// compress and decode: 1 M elements at 1 %, 55 us and 59; 6.5 M at 0.4 %, 68 and 82, at 1 %, 87 and 77; 33 M at 0.4 %, 248
+// and 283, at 1 %, 360 and 274.  (The first has room for 1 % as one minus a drop ratio.)
+constexpr double kListMaxKeepSmall = 0.0101, kListMaxKeep = 0.005;
+constexpr int64_t kListSmall = int64_t(2) << 20;
 
 constexpr int kFineBins = 512, kFineShift = 14;       // histogram above the threshold: one octave
 constexpr int kExactBins = 1 << kFineShift;           // the keys of one of its bins
@@ -82,11 +86,10 @@ struct SparseScratch {
   // Cleared by the first kernel of a call (clear_call_state).
   struct Call {
     unsigned int fine[kFineBins];      // candidates by (key - threshold) >> kFineShift; the last bin: all above
-    unsigned int thist[3][kBins];      // digits of the candidates in that last bin
+    unsigned int thist[3][kBins];      // digits of the candidates in that last bin; list form: [0], see far_bin
     unsigned int exact[kExactBins];    // keys inside the bin that holds the cut
-    unsigned long long agg[kMaxBlocks];  // write kernel: what each chunk keeps, once known
-    unsigned int ticket;               // write kernel: chunks handed out
-    unsigned int gave_up;              // a wait of the write kernel ran out (see there)
+    unsigned int ticket;               // write and emit kernels: chunks handed out
+    unsigned int gave_up;              // a wait of theirs ran out (see kept_before)
     unsigned int trim_done[2];         // CTA arrivals of the trim kernels
     unsigned int t_prefix, t_rank;     // progress of the trim digits
     unsigned int clipped;              // the cut lies in the last fine bin
@@ -102,7 +105,6 @@ struct SparseScratch {
   unsigned int k;                       // elements emitted
   unsigned int dropped;                 // candidates that found no block (cumulative)
   unsigned int last_cand;               // candidates seen by the last call (metrics)
-  unsigned int off_gt[kMaxBlocks], off_eq[kMaxBlocks];
   unsigned int list_head[kMaxLists];    // first block of each warp's list, kNoBlock when empty
 };
 
@@ -359,6 +361,8 @@ select_kernel(int64_t sample_cnt, unsigned int rank0, SparseScratch* s, const ui
   for (int i = threadIdx.x; i < kBins; i += kThreads) s->shist[0][i] = 0u;
 }
 
+constexpr int kWriteChunk = 4096;   // elements a CTA of write_kernel takes
+
 // ---- scan form: the pass that updates the state, counts the candidates and files them by magnitude
 // MODE = fuse.mode as a template parameter.  Candidates are filed by their distance from the threshold:
 // the cut, when one is needed, lies a few per cent above the threshold, and its bin of this histogram
@@ -366,8 +370,10 @@ select_kernel(int64_t sample_cnt, unsigned int rank0, SparseScratch* s, const ui
 // above is filed by its first digit as well.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 4)
-count_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s) {
+count_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s, unsigned long long* state) {
   wait_for_previous();
+  for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i * kWriteChunk < n; i += int64_t(gridDim.x) * kThreads)
+    state[i] = 0ull;   // of the write kernel
   constexpr int U = MODE == 2 ? 2 : 4;   // 16-byte loads of each array in flight per thread
   __shared__ unsigned int fine[kFineBins], coarse[kBins];
   __shared__ unsigned int blk_cnt;
@@ -464,6 +470,58 @@ count_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScrat
   if (threadIdx.x == 0) atomicAdd(&s->call.cand, blk_cnt);
 }
 
+// ---- where a chunk's entries start in the payload
+// What each chunk keeps (elements above and at the cut) is published as soon as its CTA knows it, and what all
+// chunks up to it keep once the CTA has added that up: a warp looks at the 32 chunks before, then at the 32 before
+// those, until one has its sum.  (256 or 768 at a time are fewer steps, but what all CTAs poll slows the publishing:
+// the write kernel's 18.1 us at 25 MB and 6.25 % are 20.2 and 22.6 so.)  Chunks are handed out by a ticket, so the ones waited for belong to
+// CTAs that already run, and each publishes before it waits: the wait ends.  It is bounded all the same; a CTA
+// whose wait runs out gets false, and must deliver and clear nothing.
+// state: a word per chunk, zero before; the one word is the whole message.  Whole CTA of kThreads; every thread
+// passes the chunk's own counts and gets those before it.
+constexpr unsigned long long kCountReady = 1ull << 62, kSumReady = 2ull << 62, kReadyMask = 3ull << 62;
+__device__ __forceinline__ unsigned long long pack_counts(unsigned int gt, unsigned int eq) {
+  return (static_cast<unsigned long long>(gt) << 31) | eq;   // both below 2^31
+}
+__device__ __forceinline__ bool kept_before(unsigned long long* state, int block, unsigned int& gt, unsigned int& eq) {
+  __shared__ unsigned int sum_gt, sum_eq;
+  __shared__ bool in_time;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    if (lane == 0) atomicExch(&state[block], (block == 0 ? kSumReady : kCountReady) | pack_counts(gt, eq));
+    unsigned int before_gt = 0, before_eq = 0;
+    bool late = false;
+    const uint64_t t0 = globaltimer_ns();
+    for (int end = block; end > 0;) {   // lane L looks at chunk end - 1 - L
+      const int b = end - 1 - lane;
+      const unsigned long long w = b >= 0 ? *reinterpret_cast<volatile unsigned long long*>(&state[b]) : 0ull + kSumReady;
+      const unsigned int sums = __ballot_sync(0xffffffffu, (w & kReadyMask) == kSumReady);
+      const unsigned int missing = __ballot_sync(0xffffffffu, (w & kReadyMask) == 0ull);
+      const unsigned int upto = sums == 0 ? 0xffffffffu : (2u << (__ffs(sums) - 1)) - 1u;   // lanes that count
+      if ((missing & upto) != 0) {
+        late = __any_sync(0xffffffffu, globaltimer_ns() - t0 > kGridWaitNs);   // the lanes need not agree on the time
+        if (late) break;
+        continue;
+      }
+      const bool counts = ((upto >> lane) & 1u) != 0;
+      before_gt += __reduce_add_sync(0xffffffffu, counts ? unsigned((w & ~kReadyMask) >> 31) : 0u);
+      before_eq += __reduce_add_sync(0xffffffffu, counts ? unsigned(w & 0x7fffffffull) : 0u);
+      if (sums != 0) break;
+      end -= 32;
+    }
+    if (lane == 0) {
+      if (block != 0 && !late) atomicExch(&state[block], kSumReady | pack_counts(before_gt + gt, before_eq + eq));
+      sum_gt = before_gt;
+      sum_eq = before_eq;
+      in_time = !late;
+    }
+  }
+  __syncthreads();
+  gt = sum_gt;
+  eq = sum_eq;
+  return in_time;
+}
+
 // ---- the exact cut (returns at once when not over-selected)
 // ROUND 0: the keys in the cut's bin of the fine histogram, counted one by one; the last CTA has the cut.
 // Should the cut lie in the histogram's last bin, this round counts the second digit of the keys there,
@@ -537,31 +595,30 @@ trim_kernel(const float* R, int64_t n, int64_t chunk, unsigned int expected, Spa
 
 // ---- ordered compaction and delivery
 // Output order is index order; position of an element = (elements above the cut before it) +
-// min(ties kept, elements equal to the cut before it).  A chunk's starting counts are what the chunks
-// before it keep: every CTA publishes its own counts as soon as it has them and adds up those of its
-// predecessors.  Chunks are handed out by a ticket, so the ones waited for belong to CTAs that already
-// run, and each publishes before it waits: the wait ends.  It is bounded all the same; a CTA whose wait runs
-// out records kGridWait, delivers nothing and clears nothing, and the payload's flag is not published.
-// Inside the CTA each warp owns a contiguous part of the chunk: a first walk counts what the warp will
-// emit, one barrier turns the counts into per-warp offsets, and a second walk (its data now in L1 / L2)
-// emits with warp-level ballots only.
-// 25 MB, 6.25 % kept (ncu, cold): 28 us; 50 when every lane stores its own entries.
-constexpr unsigned long long kAggReady = 1ull << 62;
+// min(ties kept, elements equal to the cut before it).  A CTA takes a chunk of 4,096 elements, counts what it
+// keeps, and gets its starting place from kept_before; a CTA whose wait there runs out records kGridWait, delivers
+// nothing and clears nothing, and the payload's flag is not published.
+// What bounds it is instructions, not memory: a test, a position and two clearing stores for each of the 16
+// elements of a lane are a thousand of them a warp.  A lane therefore holds its elements' tests as the bits of a mask
+// and their values in shared memory; one scan over the warp places all of them, and the few that are kept are
+// listed there in order, so that the stores to the payload (which loop over the destinations) and the clearing
+// ones are made by full warps.
+// 25 MB, 6.25 % kept, in a chain of calls: 18.1 us; 28.4 with a position and stores of its own for each element,
+// chunks too large for the registers, which are walked twice, and starting places added up over all chunks.
 __global__ void __launch_bounds__(kThreads)
-write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t chunk, unsigned int expected,
-             PushTargets dst, SparseScratch* s, int* status) {
+write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, unsigned int expected, PushTargets dst, SparseScratch* s,
+             unsigned long long* state, int* status) {
   wait_for_previous();
   resolve_epoch(dst);
   constexpr int kWarps = kThreads / 32;
-  __shared__ unsigned int warp_gt[kWarps], warp_eq[kWarps], before_gt, before_eq;
-  __shared__ bool gave_up;
-  __shared__ uint2 packs[kWarps][512];
+  constexpr int kSteps = 4;                        // 16-byte words of a lane: element j * 128 + lane * 4 + i of the warp
+  constexpr int kWarpElems = kSteps * 128;
+  static_assert(kWarps * kWarpElems == kWriteChunk, "one chunk per CTA");
+  __shared__ unsigned int warp_gt[kWarps], warp_eq[kWarps];
+  __shared__ __align__(16) float values[kWarps][kWarpElems];
+  __shared__ uint16_t kept[kWarps][kWarpElems];    // places among the warp's elements
   __shared__ int ticket;
-  if (threadIdx.x == 0) {
-    ticket = int(atomicAdd(&s->call.ticket, 1u));
-    before_gt = before_eq = 0;
-    gave_up = false;
-  }
+  if (threadIdx.x == 0) ticket = int(atomicAdd(&s->call.ticket, 1u));
   const uint32_t cut = s->call.cut_key;
   const unsigned int ties = s->call.ties_kept;
   const unsigned int cand = s->call.cand;
@@ -569,8 +626,6 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __syncthreads();
   const int block = ticket;
-  const int64_t begin = int64_t(block) * chunk;
-  const int64_t end = begin + chunk < n ? begin + chunk : n;
   if (block == 0 && threadIdx.x == 0) {
     s->k = k_total;
     s->last_cand = cand;
@@ -580,99 +635,50 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
     push_bytes(dst, 0, header, 4);
     if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
   }
-  // warp ranges: multiples of 128 elements so that every step is 32 lanes x 4 elements
-  int64_t wlen = (end - begin + kWarps - 1) / kWarps;
-  wlen = (wlen + 127) / 128 * 128;
-  const int64_t wbegin = begin + warp * wlen < end ? begin + warp * wlen : end;
-  const int64_t wend = wbegin + wlen < end ? wbegin + wlen : end;
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(R) & 15) == 0 && (begin & 3) == 0;
-
-  auto load4 = [&](int64_t e0, float (&v)[4], uint32_t (&key)[4]) {
-    if (vec_ok && e0 + 3 < wend) {
-      const float4 q = *reinterpret_cast<const float4*>(R + e0);
-      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  const int64_t wbegin = int64_t(block) * kWriteChunk + warp * kWarpElems;   // the warp's elements, clipped at n
+  float v[kSteps][4];
+  if ((reinterpret_cast<uintptr_t>(R) & 15) == 0 && wbegin + kWarpElems <= n) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) key[j] = abs_key(v[j]);
-    } else {
+    for (int j = 0; j < kSteps; ++j) {
+      const float4 q = *reinterpret_cast<const float4*>(R + wbegin + j * 128 + lane * 4);
+      v[j][0] = q.x; v[j][1] = q.y; v[j][2] = q.z; v[j][3] = q.w;
+    }
+  } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[j] = (e0 + j < wend) ? R[e0 + j] : 0.0f;
-        key[j] = (e0 + j < wend) ? abs_key(v[j]) : 0u;   // key 0 is below any cut that selects
+    for (int j = 0; j < kSteps; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t e = wbegin + j * 128 + lane * 4 + i;
+        v[j][i] = e < n ? R[e] : 0.0f;
       }
-    }
-  };
-
-  // ---- first walk: how many elements above / at the cut does this warp hold
-  unsigned int my_gt = 0, my_eq = 0;
-  int64_t base = wbegin;
-  if (vec_ok) {
-    // four steps per iteration with their loads issued together: one load in flight per lane
-    // left this walk waiting on DRAM latency
-    for (; base + 512 <= wend; base += 512) {
-      float4 q[4];
+  }
+  // Bit 4 * j + i: the element is above the cut, or at it.  A place past the end holds zero, whose key is above no cut;
+  // it equals the cut only where the cut is zero, and then nothing at the cut is kept: a candidate is above a
+  // threshold that is not negative.
+  uint32_t above = 0, at_cut = 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) q[u] = *reinterpret_cast<const float4*>(R + base + u * 128 + lane * 4);
+  for (int j = 0; j < kSteps; ++j) {
+    *reinterpret_cast<float4*>(&values[warp][j * 128 + lane * 4]) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t k0 = abs_key(q[u].x), k1 = abs_key(q[u].y), k2 = abs_key(q[u].z), k3 = abs_key(q[u].w);
-        my_gt += (k0 > cut) + (k1 > cut) + (k2 > cut) + (k3 > cut);
-        my_eq += (k0 == cut) + (k1 == cut) + (k2 == cut) + (k3 == cut);
-      }
+    for (int i = 0; i < 4; ++i) {
+      above |= abs_key(v[j][i]) > cut ? 1u << (4 * j + i) : 0u;
+      at_cut |= abs_key(v[j][i]) == cut ? 1u << (4 * j + i) : 0u;
     }
   }
-  for (; base < wend; base += 128) {
-    float v[4];
-    uint32_t key[4];
-    load4(base + lane * 4, v, key);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const bool in = base + lane * 4 + j < wend;
-      my_gt += in && key[j] > cut;
-      my_eq += in && key[j] == cut;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    my_gt += __shfl_xor_sync(0xffffffffu, my_gt, o);
-    my_eq += __shfl_xor_sync(0xffffffffu, my_eq, o);
-  }
+  const unsigned int my_gt = __reduce_add_sync(0xffffffffu, unsigned(__popc(above)));
+  const unsigned int my_eq = __reduce_add_sync(0xffffffffu, unsigned(__popc(at_cut)));
   if (lane == 0) {
     warp_gt[warp] = my_gt;
     warp_eq[warp] = my_eq;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long g = 0, q = 0;
-    for (int w = 0; w < kWarps; ++w) {
-      g += warp_gt[w];
-      q += warp_eq[w];
-    }
-    atomicExch(&s->call.agg[block], kAggReady | (g << 31) | q);   // the one word is the whole message
-  }
-  unsigned int add_gt = 0, add_eq = 0;
-  const uint64_t t0 = globaltimer_ns();
-  for (int b = threadIdx.x; b < block; b += kThreads) {
-    unsigned long long v;
-    while (((v = *reinterpret_cast<volatile unsigned long long*>(&s->call.agg[b])) & kAggReady) == 0) {
-      if (globaltimer_ns() - t0 > kGridWaitNs) {
-        gave_up = true;
-        break;
-      }
-    }
-    add_gt += unsigned((v & ~kAggReady) >> 31);
-    add_eq += unsigned(v & 0x7fffffffull);
-  }
+  unsigned int run_gt = 0, run_eq = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    add_gt += __shfl_xor_sync(0xffffffffu, add_gt, o);
-    add_eq += __shfl_xor_sync(0xffffffffu, add_eq, o);
+  for (int w = 0; w < kWarps; ++w) {
+    run_gt += warp_gt[w];
+    run_eq += warp_eq[w];
   }
-  if (lane == 0 && (add_gt | add_eq) != 0) {
-    atomicAdd(&before_gt, add_gt);
-    atomicAdd(&before_eq, add_eq);
-  }
-  __syncthreads();
-  if (gave_up) {
+  if (!kept_before(state, block, run_gt, run_eq)) {
     if (threadIdx.x == 0) {
       s->call.gave_up = 1u;
       if (status != nullptr) atomicExch(status, int(kGridWait));
@@ -680,82 +686,64 @@ write_kernel(float* R, float* u_mask, float* sumsq_to_clear, int64_t n, int64_t 
     publish_when_grid_done(dst, &s->call.gave_up);
     return;
   }
-  unsigned int run_gt = before_gt, run_eq = before_eq;
   for (int w = 0; w < warp; ++w) {
     run_gt += warp_gt[w];
     run_eq += warp_eq[w];
   }
-
-  // ---- second walk: emit
-  // 512 elements at a time: what is kept is packed in shared memory first, so that the stores to the
-  // payload (which loop over the destinations) are made by full warps of neighbouring entries.
-  if (my_gt != 0 || (ties > 0 && my_eq != 0)) {
-    uint2* const packed = packs[warp];
+  // Of a mask, per step: how many bits the steps and lanes before this lane's hold.  A byte per step (128 at most).
+  auto bits_before = [&](uint32_t mask, unsigned int (&before)[kSteps]) {
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < kSteps; ++j) mine |= unsigned(__popc((mask >> (4 * j)) & 15u)) << (8 * j);
+    uint32_t inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    const uint32_t totals = __shfl_sync(0xffffffffu, inc, 31);
+    unsigned int run = 0;
+#pragma unroll
+    for (int j = 0; j < kSteps; ++j) {
+      before[j] = run + (((inc - mine) >> (8 * j)) & 255u);
+      run += (totals >> (8 * j)) & 255u;
+    }
+    return run;
+  };
+  if (my_gt != 0 || (ties > run_eq && my_eq != 0)) {
     unsigned int run_kept = run_gt + (run_eq < ties ? run_eq : ties);
-    const unsigned int lt = (1u << lane) - 1u;
-    for (int64_t base2 = wbegin; base2 < wend; base2 += 512) {
-      float v[4][4];
-      uint32_t key[4][4];
+    uint32_t keep = above;
+    unsigned int before[kSteps];
+    if (my_eq != 0 && run_eq < ties) {   // ties are kept from the lower index on
+      bits_before(at_cut, before);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) load4(base2 + u * 128 + lane * 4, v[u], key[u]);
-      unsigned int held = 0;
+      for (int j = 0; j < kSteps; ++j) {
+        unsigned int rank = run_eq + before[j];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t e0 = base2 + u * 128 + lane * 4;
-        bool keep[4], at_cut = false;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          keep[j] = e0 + j < wend && key[u][j] > cut;
-          at_cut = at_cut || (e0 + j < wend && key[u][j] == cut);
-        }
-        if (ties > 0 && __any_sync(0xffffffffu, at_cut)) {
-          // ties are kept from the lower index on: element order is lane by lane
-          unsigned int before = run_eq, total = 0;
-          unsigned int at[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            at[j] = __ballot_sync(0xffffffffu, e0 + j < wend && key[u][j] == cut);
-            before += __popc(at[j] & lt);
-            total += __popc(at[j]);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if ((at[j] >> lane) & 1u) {
-              keep[j] = before < ties;
-              ++before;
-            }
-          }
-          run_eq += total;
-        }
-        unsigned int at_pos = held;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const unsigned int m = __ballot_sync(0xffffffffu, keep[j]);
-          at_pos += __popc(m & lt);
-          held += __popc(m);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (keep[j]) {
-            packed[at_pos] = make_uint2(uint32_t(e0 + j), __float_as_uint(v[u][j]));
-            if (run_kept + at_pos < k_total) {
-              R[e0 + j] = 0.0f;
-              if (u_mask != nullptr) u_mask[e0 + j] = 0.0f;   // DGC's momentum factor masking
-            }
-            ++at_pos;
-          }
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t bit = at_cut & (1u << (4 * j + i));
+          if (bit != 0 && rank++ < ties) keep |= bit;
         }
       }
-      __syncwarp();
-      for (unsigned int i = lane; i < held; i += 32) {
-        const unsigned int pos = run_kept + i;
-        if (pos < k_total) {
-          push_u32(dst, 4 + 4 * int64_t(pos), packed[i].x);
-          push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), packed[i].y);
-        }
+    }
+    const unsigned int held = bits_before(keep, before);
+#pragma unroll
+    for (int j = 0; j < kSteps; ++j) {
+      unsigned int at = before[j];
+      for (uint32_t bits = (keep >> (4 * j)) & 15u; bits != 0; bits &= bits - 1)
+        kept[warp][at++] = uint16_t(j * 128 + lane * 4 + __ffs(bits) - 1);
+    }
+    __syncwarp();
+    for (unsigned int i = lane; i < held; i += 32) {
+      const unsigned int pos = run_kept + i;
+      if (pos < k_total) {
+        const int place = kept[warp][i];
+        const int64_t e = wbegin + place;
+        push_u32(dst, 4 + 4 * int64_t(pos), uint32_t(e));
+        push_u32(dst, 4 + 4 * int64_t(k_total) + 4 * int64_t(pos), __float_as_uint(values[warp][place]));
+        R[e] = 0.0f;
+        if (u_mask != nullptr) u_mask[e] = 0.0f;   // DGC's momentum factor masking
       }
-      __syncwarp();
-      run_kept += held;
     }
   }
   publish_when_grid_done(dst, &s->call.gave_up);
@@ -797,23 +785,31 @@ struct ListPool {
   unsigned int* count;
   unsigned int* next;
   uint2* entry;
-  uint32_t* dense;        // the candidates' keys once more, densely packed in no particular order,
-  uint16_t* dense_cta;    // and the CTA that found each
+  uint32_t* dense;        // the candidates' keys once more, densely packed in no particular order
   unsigned int capacity;  // blocks
 };
 
-// Cursor of a warp's list; only lane 0's copy is used.
+// Cursor of a warp's list; only lane 0's copy is used, but for the last two.
 struct ListCursor {
   unsigned int block = kNoBlock, fill = 0, lost = 0, total = 0;
   bool exhausted = false;
+  unsigned int seen = 0;   // candidates, the same in all lanes
+  uint32_t key = 0;        // of candidate number `lane`
 };
+// Bin of a candidate by its distance from the threshold: 2,048 bins of 4,096 keys, one octave, the last bin
+// for all above.
+constexpr int kFar = 12;   // log2 of the keys per bin
+__device__ __forceinline__ int far_bin(uint32_t key, uint32_t thr_key) {
+  const uint32_t d = (key - thr_key) >> kFar;
+  return int(d < kBins - 1 ? d : kBins - 1);
+}
 
 // Appends this step's candidates of the calling warp to the warp's list, in lane order and,
 // within a lane, element order.  count: candidates of this lane (0..4); idx / val: their
 // indices and values.  Candidates are rare (0.1 % of the elements), so the entries are handed
 // to lane 0 by shuffle and appended one at a time; a list grows by one block of the pool when
-// its last block is full.
-__device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& pool, int list, int lane,
+// its last block is full.  Each is counted in the bin that the cut is looked for in.
+__device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& pool, int list, int lane, uint32_t thr_key,
                                             unsigned int count, const uint32_t (&idx)[4], const float (&val)[4],
                                             ListCursor& cur) {
   unsigned int mask = __ballot_sync(0xffffffffu, count != 0);
@@ -825,6 +821,7 @@ __device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& po
     for (int j = 0; j < 4; ++j) {
       const uint32_t i = __shfl_sync(0xffffffffu, idx[j], src);
       const float v = __shfl_sync(0xffffffffu, val[j], src);
+      if (j < int(c) && cur.seen++ == unsigned(lane)) cur.key = abs_key(v);
       if (lane != 0 || j >= int(c)) continue;
       if (cur.exhausted) {
         ++cur.lost;
@@ -846,6 +843,7 @@ __device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& po
       }
       pool.entry[size_t(cur.block) * kBlockEntries + cur.fill] = make_uint2(i, __float_as_uint(v));
       pool.count[cur.block] = ++cur.fill;
+      atomicAdd(&s->call.thist[0][far_bin(abs_key(v), thr_key)], 1u);
       ++cur.total;
     }
   }
@@ -856,8 +854,10 @@ __device__ __forceinline__ void list_append(SparseScratch* s, const ListPool& po
 // CTAs per SM, so that the whole grid of 4 x 148 CTAs is resident at once.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 4)
-collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s, ListPool pool) {
+collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScratch* s, ListPool pool,
+               unsigned long long* state) {
   wait_for_previous();
+  if (threadIdx.x == 0) state[blockIdx.x] = 0ull;   // of the emit kernel
   fuse.mode = MODE;
   constexpr int kWarps = kThreads / 32;
   constexpr int U = MODE == 2 ? 2 : 4;   // steps whose loads are issued together
@@ -936,7 +936,7 @@ collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScr
         uint32_t idx[4] = {0u, 0u, 0u, 0u};
         float val[4] = {0.f, 0.f, 0.f, 0.f};
         const unsigned int count = step4(base + q * 128 + lane * 4, r4[q], g4[MODE >= 1 ? q : 0], u4[MODE == 2 ? q : 0], idx, val);
-        if (__ballot_sync(0xffffffffu, count != 0) != 0) list_append(s, pool, list, lane, count, idx, val, cur);
+        if (__ballot_sync(0xffffffffu, count != 0) != 0) list_append(s, pool, list, lane, thr_key, count, idx, val, cur);
       }
     }
   }
@@ -973,46 +973,46 @@ collect_kernel(SparseFuseDev fuse, float* R, int64_t n, int64_t chunk, SparseScr
         }
       }
     }
-    if (__ballot_sync(0xffffffffu, count != 0) != 0) list_append(s, pool, list, lane, count, idx, val, cur);
+    if (__ballot_sync(0xffffffffu, count != 0) != 0) list_append(s, pool, list, lane, thr_key, count, idx, val, cur);
   }
   let_next_start();
-  // The cut kernel wants all candidate keys in one flat array (it is one CTA, or eight: a sweep over
-  // the half-empty list blocks cost a single one 70 us).  Each warp copies the keys of its own list, which
-  // it has just written, to a range it reserves with one atomic.
+  // The cut kernel wants all candidate keys in one flat array (a sweep over the half-empty list blocks cost it
+  // 70 us).  Each warp copies its own to a range that it reserves with one atomic: the lanes hold the first 32, and
+  // the rest is read back from the list.
   if (lane == 0 && cur.lost != 0) atomicAdd(&s->dropped, cur.lost);
   const unsigned int total = __shfl_sync(0xffffffffu, cur.total, 0);
   if (total != 0) {
     unsigned int base = 0;
     if (lane == 0) base = atomicAdd(&s->call.cand, total);
     base = __shfl_sync(0xffffffffu, base, 0);
+    if (total <= 32u) {   // the first `total` candidates found room, any others none
+      if (lane < int(total)) pool.dense[base + lane] = cur.key;
+      return;
+    }
     __syncwarp();   // lane 0's list writes are visible to the other lanes
     unsigned int done = 0;
     for (unsigned int b = s->list_head[list]; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
       const unsigned int c = pool.count[b];
-      if (lane < int(c)) {
-        pool.dense[base + done + lane] = pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu;
-        pool.dense_cta[base + done + lane] = uint16_t(blockIdx.x);
-      }
+      if (lane < int(c)) pool.dense[base + done + lane] = pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu;
       done += c;
     }
   }
 }
 
-// ---- the exact cut among the candidates, and where every CTA's lists go in the payload
-// CTAS = 1, or a cluster of eight that share the candidates: each counts its share of a digit, the
-// counts are added through distributed shared memory, and every CTA picks the same bin.
-// Two digits of the distance from the threshold (2,048 bins of 4,096 keys: one octave above it, then the
-// keys of one bin) find the cut of ordinary data, and they spread: the leading bits of the keys themselves
-// are nearly all the same, which costs either colliding atomics or a match instruction per warp (38 us for
-// the 17,000 candidates of a 64 MB tensor; 21 us by distance).  Only when the cut lies in the last bin are the
-// three digits of the keys counted.
+// ---- the exact cut among the candidates
+// The collect pass has counted the candidates by their distance from the threshold, in bins of 4,096 keys.  The
+// bin that holds the cut follows from those counts, and one pass over the candidates counts the keys of that bin one
+// by one: on ordinary data some hundred of 17,000.  The leading bits of the keys themselves are nearly all the same,
+// which costs either colliding atomics or a match instruction per warp; their three digits are counted only
+// when the cut lies in the last bin, more than an octave above the threshold.
+// CTAS = 1, or a cluster of eight that share the candidates and count in the first CTA's memory.
+// The kernel behind starts at once: its walk over the lists needs nothing from here.
+// 17,000 candidates of 64 MB: 5 us behind the collect pass; 15 with all keys brought to shared memory, three rounds of counting, and a
+// count of what each CTA's lists keep.
 constexpr int kCutThreads = 1024;
 constexpr int kCutCluster = 8;
-template <int CTAS> struct CutForm {
-  static constexpr int kKeys = CTAS == 1 ? 48 * 1024 : 24 * 1024;   // keys a CTA holds in shared memory
-};
-constexpr int64_t kCutOneCta = 40 * 1024;   // selections up to this leave a single CTA's array room for the surplus
-static_assert(kMaxBlocks <= kCutThreads, "one thread scans one CTA's total");
+constexpr int kCutBins = 1 << kFar;
+constexpr int64_t kCutOneCta = 40 * 1024;   // selections up to this are one CTA's work
 
 // Exclusive scan over kCutThreads values, one per thread; total: their sum.  ws: 33 words of shared memory.
 __device__ __forceinline__ unsigned int exclusive_scan_1024(unsigned int v, unsigned int* ws, unsigned int& total) {
@@ -1042,203 +1042,201 @@ __device__ __forceinline__ unsigned int exclusive_scan_1024(unsigned int v, unsi
   return ws[warp] + inc - v;
 }
 
+// The bin that holds the element of 0-indexed `rank` from the top, and the rank inside it.  c: this thread's PER
+// bins, highest first; thread t has those from (1,024 - t) * PER - 1 down.  Whole CTA.
+template <int PER>
+__device__ __forceinline__ uint32_t cut_pick(const unsigned int (&c)[PER], unsigned int& rank, unsigned int* ws, unsigned int* res) {
+  unsigned int mine = 0, unused;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) mine += c[j];
+  const unsigned int before = exclusive_scan_1024(mine, ws, unused);
+  if (rank >= before && rank - before < mine) {
+    unsigned int run = before;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      if (rank >= run && rank - run < c[j]) {
+        res[0] = unsigned((kCutThreads - int(threadIdx.x)) * PER - 1 - j);
+        res[1] = rank - run;
+      }
+      run += c[j];
+    }
+  }
+  __syncthreads();
+  const uint32_t bin = res[0];
+  rank = res[1];
+  __syncthreads();
+  return bin;
+}
+
 template <int CTAS>
-__global__ void __launch_bounds__(kCutThreads)
-cut_kernel(unsigned int expected, int blocks, PushTargets dst, SparseScratch* s, ListPool pool, float* sumsq_to_clear) {
+__global__ void __launch_bounds__(kCutThreads, 1)
+cut_kernel(unsigned int expected, PushTargets dst, SparseScratch* s, ListPool pool, float* sumsq_to_clear) {
   wait_for_previous();
+  let_next_start();   // behind the wait: what the collect pass wrote is complete
   resolve_epoch(dst);
-  extern __shared__ uint32_t keys[];   // CutForm<CTAS>::kKeys
-  __shared__ unsigned int sh[kBins];   // this CTA's counts
-  __shared__ unsigned int all[CTAS > 1 ? kBins : 1];   // the cluster's
-  __shared__ unsigned int kept_gt[kMaxBlocks], kept_eq[kMaxBlocks];
+  constexpr int kAhead = 8;             // keys of a thread in flight
+  __shared__ unsigned int sh[kCutBins];
   __shared__ unsigned int ws[33], res[2];
-  const int t = threadIdx.x, lane = t & 31;
+  const int t = threadIdx.x;
   const int part = CTAS > 1 ? int(blockIdx.x) : 0;
+  uint32_t key[kAhead];
+  if (CTAS == 1) {   // the first ones, whether or not there are that many: the array is longer
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) key[u] = pool.dense[u * kCutThreads + t];
+  }
+  const uint2 top = *reinterpret_cast<const uint2*>(&s->call.thist[0][kBins - 2 - 2 * t]);
   const unsigned int cand = s->call.cand;
+  const uint32_t thr = s->call.thr_key;
   const unsigned int share = (cand + CTAS - 1) / CTAS;
   const unsigned int first = share * part < cand ? share * part : cand;
   const unsigned int count = first + share < cand ? share : cand - first;
-  for (int i = t; i < kMaxBlocks; i += kCutThreads) kept_gt[i] = kept_eq[i] = 0;
-  const bool in_smem = count <= unsigned(CutForm<CTAS>::kKeys);
-  if (in_smem) {
-    // eight independent loads per thread and iteration
-    for (unsigned int base = 0; base < count; base += kCutThreads * 8) {
-      uint32_t k[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const unsigned int i = base + u * kCutThreads + t;
-        k[u] = i < count ? pool.dense[first + i] : 0u;
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const unsigned int i = base + u * kCutThreads + t;
-        if (i < count) keys[i] = k[u];
-      }
-    }
-  }
-  auto key_at = [&](unsigned int i) { return in_smem ? keys[i] : pool.dense[first + i]; };   // else from L2
-  uint32_t cut = s->call.thr_key;
+  for (int i = t; i < kCutBins; i += kCutThreads) sh[i] = 0;
+  if (t == 0) res[0] = res[1] = 0;
+  uint32_t cut = thr;
   unsigned int ties = 0;
   if (cand > expected) {   // the same in every CTA
-    const uint32_t thr = cut;
     unsigned int rank = expected - 1;   // 0-based from the top
-    // one digit: bin(key) below kBins, or negative for a key that does not count
-    auto find = [&](bool collide, auto bin_of) -> uint32_t {
-      for (int i = t; i < kBins; i += kCutThreads) sh[i] = 0;
-      if (t == 0) res[0] = res[1] = 0;
-      __syncthreads();
-      if (collide) {
-        const unsigned int count_padded = (count + 31u) & ~31u;   // whole warps iterate together
-        for (unsigned int i = t; i < count_padded; i += kCutThreads) count_digit(sh, i < count ? bin_of(key_at(i)) : -1);
-      } else {
-        for (unsigned int i = t; i < count; i += kCutThreads) {
-          const int bin = bin_of(key_at(i));
-          if (bin >= 0) atomicAdd(&sh[bin], 1u);
-        }
-      }
-      const unsigned int* hist = sh;
-      if constexpr (CTAS > 1) {
-        const cg::cluster_group cluster = cg::this_cluster();
-        cluster.sync();
-        constexpr int kMine = kBins / CTAS;   // bins that this CTA adds up for all
-        if (t < kMine) {
-          const int bin = part * kMine + t;
-          unsigned int sum = 0;
-#pragma unroll
-          for (int c = 0; c < CTAS; ++c) sum += cluster.map_shared_rank(sh, c)[bin];
-#pragma unroll
-          for (int c = 0; c < CTAS; ++c) cluster.map_shared_rank(all, c)[bin] = sum;
-        }
-        cluster.sync();   // also: nobody clears sh while another CTA still reads it
-        hist = all;
-      } else {
-        __syncthreads();
-      }
-      // bin holding the element of that rank, from the top: two bins per thread
-      const int hi = kBins - 1 - 2 * t;
-      const unsigned int a = hist[hi], b = hist[hi - 1];
-      unsigned int unused;
-      const unsigned int before = exclusive_scan_1024(a + b, ws, unused);
-      if (rank >= before && rank - before < a + b) {
-        const bool upper = rank - before < a;
-        res[0] = upper ? hi : hi - 1;
-        res[1] = upper ? rank - before : rank - before - a;
-      }
-      __syncthreads();
-      const uint32_t bin = res[0];
-      rank = res[1];
-      __syncthreads();
-      return bin;
-    };
-    constexpr int kFar = 12;   // log2 of the keys per bin of the first digit
-    const uint32_t far = find(false, [&](uint32_t key) {
-      const uint32_t d = (key - thr) >> kFar;
-      return int(d < kBins - 1 ? d : kBins - 1);
-    });
+    const unsigned int far_counts[2] = {top.y, top.x};
+    const uint32_t far = cut_pick<2>(far_counts, rank, ws, res);
+    unsigned int* counts = sh;          // the cluster counts in its first CTA
+    if constexpr (CTAS > 1) {
+      cg::this_cluster().sync();        // cleared
+      counts = cg::this_cluster().map_shared_rank(sh, 0);
+    }
     if (far < kBins - 1) {
-      // the bin's 4,096 keys in two steps of the same kind: pairs of keys, then the one of the pair
       const uint32_t base = thr + (far << kFar);
-      const uint32_t pair = find(false, [&](uint32_t key) { return key - base < (1u << kFar) ? int((key - base) >> 1) : -1; });
-      const uint32_t last = find(false, [&](uint32_t key) { return (key - base) >> 1 == pair ? int((key - base) & 1u) : -1; });
-      cut = base + 2 * pair + last;
+      for (unsigned int i0 = 0; i0 < count; i0 += kCutThreads * kAhead) {
+        if (CTAS > 1 || i0 != 0) {
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            const unsigned int i = i0 + u * kCutThreads + t;
+            key[u] = i < count ? pool.dense[first + i] : 0u;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if (i0 + u * kCutThreads + t < count && key[u] - base < unsigned(kCutBins)) atomicAdd(&counts[key[u] - base], 1u);
+      }
+      if constexpr (CTAS > 1) cg::this_cluster().sync();
+      else __syncthreads();
+      if (part == 0) {
+        unsigned int c[kCutBins / kCutThreads];
+        const int hi = (kCutThreads - t) * (kCutBins / kCutThreads) - 1;
+#pragma unroll
+        for (int j = 0; j < kCutBins / kCutThreads; ++j) c[j] = sh[hi - j];
+        cut = base + cut_pick<kCutBins / kCutThreads>(c, rank, ws, res);
+      }
     } else {
       rank = expected - 1;
       uint32_t prefix = 0;
       for (int round = 0; round < 3; ++round) {
-        const uint32_t bin = find(true, [&](uint32_t key) { return prefix_matches(key, round, prefix) ? digit_of(key, round) : -1; });
+        const unsigned int count_padded = (count + 31u) & ~31u;   // whole warps iterate together
+        for (unsigned int i = t; i < count_padded; i += kCutThreads) {
+          const uint32_t k = i < count ? pool.dense[first + i] : 0u;
+          count_digit(counts, i < count && prefix_matches(k, round, prefix) ? digit_of(k, round) : -1);
+        }
+        if constexpr (CTAS > 1) cg::this_cluster().sync();
+        else __syncthreads();
+        const unsigned int c[2] = {counts[kBins - 1 - 2 * t], counts[kBins - 2 - 2 * t]};
+        const uint32_t bin = cut_pick<2>(c, rank, ws, res);
         prefix = extend_prefix(prefix, round, bin);
+        if constexpr (CTAS > 1) cg::this_cluster().sync();   // read by every CTA
+        if (part == 0)
+          for (int i = t; i < kBins; i += kCutThreads) sh[i] = 0;
+        if (t == 0) res[0] = res[1] = 0;
+        if constexpr (CTAS > 1) cg::this_cluster().sync();
+        else __syncthreads();
       }
       cut = prefix;
     }
     ties = rank + 1;
-  } else {
-    __syncthreads();
   }
-  for (unsigned int i = t; i < count; i += kCutThreads) {
-    const uint32_t key = key_at(i);
-    if (key >= cut) {
-      const int cta = pool.dense_cta[first + i];
-      if (key > cut) atomicAdd(&kept_gt[cta], 1u);
-      else if (ties != 0) atomicAdd(&kept_eq[cta], 1u);
-    }
+  if (part == 0 && t == 0) {
+    const unsigned int k = cand < expected ? cand : expected;
+    s->call.cut_key = cut;
+    s->call.ties_kept = ties;
+    s->k = k;
+    s->last_cand = cand;
+    const uint32_t total = 4u + 8u * k;
+    uint8_t header[4];
+    for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
+    push_bytes(dst, 0, header, 4);
+    if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
   }
-  __syncthreads();
-  if constexpr (CTAS > 1) cg::this_cluster().sync();
-  if (part == 0) {
-    unsigned int gt = 0, eq = 0;
-    if (t < blocks) {
-      if constexpr (CTAS > 1) {
-        const cg::cluster_group cluster = cg::this_cluster();
-#pragma unroll
-        for (int c = 0; c < CTAS; ++c) {
-          gt += cluster.map_shared_rank(kept_gt, c)[t];
-          eq += cluster.map_shared_rank(kept_eq, c)[t];
-        }
-      } else {
-        gt = kept_gt[t];
-        eq = kept_eq[t];
-      }
-    }
-    unsigned int total_gt, total_eq;
-    const unsigned int before_gt = exclusive_scan_1024(gt, ws, total_gt);
-    const unsigned int before_eq = exclusive_scan_1024(eq, ws, total_eq);
-    if (t < blocks) {
-      s->off_gt[t] = before_gt;
-      s->off_eq[t] = before_eq;
-    }
-    if (t == 0) {
-      const unsigned int k = total_gt + (total_eq < ties ? total_eq : ties);
-      s->call.cut_key = cut;
-      s->call.ties_kept = ties;
-      s->k = k;
-      s->last_cand = cand;
-      const uint32_t total = 4u + 8u * k;
-      uint8_t header[4];
-      for (int i = 0; i < 4; ++i) header[i] = uint8_t(total >> (8 * i));
-      push_bytes(dst, 0, header, 4);
-      if (sumsq_to_clear != nullptr) *sumsq_to_clear = 0.f;
-    }
-  }
-  if constexpr (CTAS > 1) cg::this_cluster().sync();   // the counts were read from every CTA
+  if constexpr (CTAS > 1) cg::this_cluster().sync();   // nobody leaves while its memory is used
 }
 
 // ---- one warp per list: deliver, clear the emitted positions, publish
+// A CTA takes the eight lists of one CTA of the collect pass, in the order of their indices (see kept_before).
+// The lists were complete before the kernel before this one began to look at them, and are brought in while it
+// works; only the cut is waited for.
 __global__ void __launch_bounds__(kThreads)
-emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScratch* s, ListPool pool) {
-  wait_for_previous();
-  resolve_epoch(dst);
+emit_kernel(float* R, float* u_mask, unsigned int expected, PushTargets dst, SparseScratch* s, ListPool pool,
+            unsigned long long* state, int* status) {
   constexpr int kWarps = kThreads / 32;
   __shared__ unsigned int w_gt[kWarps], w_eq[kWarps];
+  __shared__ int ticket;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int list = blockIdx.x * kWarps + warp;
-  const uint32_t cut = s->call.cut_key;
-  const unsigned int ties = s->call.ties_kept, k_total = s->k;
-  const unsigned int head = list < lists ? s->list_head[list] : kNoBlock;
-  // first walk: what this list keeps
-  unsigned int gt = 0, eq = 0;
-  for (unsigned int b = head; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
-    const unsigned int c = pool.count[b];
-    const uint32_t key = lane < int(c) ? (pool.entry[size_t(b) * kBlockEntries + lane].y & 0x7fffffffu) : 0u;
-    gt += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key > cut));
-    eq += __popc(__ballot_sync(0xffffffffu, lane < int(c) && key == cut));
+  if (threadIdx.x == 0) ticket = int(atomicAdd(&s->call.ticket, 1u));
+  __syncthreads();
+  const int block = ticket;
+  const unsigned int head = s->list_head[block * kWarps + warp];
+  // the list's first block; most lists have one
+  unsigned int first_count = 0, first_next = kNoBlock;
+  uint2 first_entry = make_uint2(0u, 0u);
+  if (head < pool.capacity) {   // kNoBlock is not
+    first_count = pool.count[head];
+    first_next = pool.next[head];
+    if (lane < kBlockEntries) first_entry = pool.entry[size_t(head) * kBlockEntries + lane];
   }
+  wait_for_previous();
+  resolve_epoch(dst);
+  const uint32_t cut = s->call.cut_key;
+  const unsigned int ties = s->call.ties_kept, cand = s->call.cand;
+  const unsigned int k_total = cand < expected ? cand : expected;
+  // calls f(entry, whether this lane has one) for the list's entries, a block at a time
+  auto walk = [&](auto f) {
+    if (head >= pool.capacity) return;
+    f(first_entry, lane < int(first_count));
+    for (unsigned int b = first_next; b < pool.capacity; b = pool.next[b]) {
+      const unsigned int c = pool.count[b];
+      uint2 en = make_uint2(0u, 0u);
+      if (lane < int(c)) en = pool.entry[size_t(b) * kBlockEntries + lane];
+      f(en, lane < int(c));
+    }
+  };
+  unsigned int gt = 0, eq = 0;
+  walk([&](uint2 en, bool has) {
+    const uint32_t key = en.y & 0x7fffffffu;
+    gt += __popc(__ballot_sync(0xffffffffu, has && key > cut));
+    eq += __popc(__ballot_sync(0xffffffffu, has && key == cut));
+  });
   if (lane == 0) {
     w_gt[warp] = gt;
     w_eq[warp] = eq;
   }
   __syncthreads();
-  // what the lists before this one keep: the CTA's offset plus the earlier warps of the CTA
-  unsigned int run_gt = s->off_gt[blockIdx.x], run_eq = s->off_eq[blockIdx.x];
+  unsigned int run_gt = 0, run_eq = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    run_gt += w_gt[w];
+    run_eq += w_eq[w];
+  }
+  if (!kept_before(state, block, run_gt, run_eq)) {
+    if (threadIdx.x == 0) {
+      s->call.gave_up = 1u;
+      if (status != nullptr) atomicExch(status, int(kGridWait));
+    }
+    publish_when_grid_done(dst, &s->call.gave_up);
+    return;
+  }
   for (int w = 0; w < warp; ++w) {
     run_gt += w_gt[w];
     run_eq += w_eq[w];
   }
-  for (unsigned int b = head; b != kNoBlock && b < pool.capacity; b = pool.next[b]) {
-    const unsigned int c = pool.count[b];
-    uint2 en = make_uint2(0u, 0u);
-    if (lane < int(c)) en = pool.entry[size_t(b) * kBlockEntries + lane];
+  walk([&](uint2 en, bool has) {
     const uint32_t key = en.y & 0x7fffffffu;
-    const bool above = lane < int(c) && key > cut, at = lane < int(c) && key == cut;
+    const bool above = has && key > cut, at = has && key == cut;
     const unsigned int ma = __ballot_sync(0xffffffffu, above), me = __ballot_sync(0xffffffffu, at);
     const unsigned int lt = (1u << lane) - 1u;
     const unsigned int gt_before = run_gt + __popc(ma & lt), eq_before = run_eq + __popc(me & lt);
@@ -1253,8 +1251,8 @@ emit_kernel(float* R, float* u_mask, int lists, PushTargets dst, const SparseScr
     }
     run_gt += __popc(ma);
     run_eq += __popc(me);
-  }
-  publish_when_grid_done(dst);
+  });
+  publish_when_grid_done(dst, &s->call.gave_up);
 }
 
 // ================================================================ one-pass decode
@@ -1621,14 +1619,14 @@ inline Plan plan_for(int64_t n) {
 
 namespace {
 
-// Layout of the scratch behind SparseScratch: sample keys, then the pool of list blocks.  Both
+// Layout of the scratch behind SparseScratch: sample keys, the pool of list blocks, the states of kept_before.  All
 // are sized from n alone, so that one allocation serves every keep fraction and sample rate a
 // caller may pick later; a call whose sample or expected candidate count does not fit takes the
 // scan form, which needs neither.
 struct ListPlan {
   int64_t key_capacity;    // sample keys, and as many places for the ones select_kernel keeps
   int64_t pool_blocks;
-  size_t keys_offset, pool_offset, total_bytes;
+  size_t keys_offset, pool_offset, state_offset, total_bytes;
 };
 inline ListPlan list_plan(int64_t n) {
   ListPlan p;
@@ -1639,8 +1637,9 @@ inline ListPlan list_plan(int64_t n) {
   p.pool_blocks = entries / kBlockEntries + kMaxLists;
   p.keys_offset = (sizeof(SparseScratch) + 255) / 256 * 256;
   p.pool_offset = (p.keys_offset + size_t(p.key_capacity) * 8 + 255) / 256 * 256;
-  // count[blocks], next[blocks], entry[blocks][16], dense[blocks * 16], dense_cta[blocks * 16]
-  p.total_bytes = p.pool_offset + size_t(p.pool_blocks) * (8 + kBlockEntries * (sizeof(uint2) + 6)) + 512;
+  // count[blocks], next[blocks], entry[blocks][16], dense[blocks * 16]
+  p.state_offset = (p.pool_offset + size_t(p.pool_blocks) * (8 + kBlockEntries * (sizeof(uint2) + 4)) + 512 + 7) / 8 * 8;
+  p.total_bytes = p.state_offset + size_t((n + kWriteChunk - 1) / kWriteChunk + kMaxBlocks) * 8;   // kept_before's states
   return p;
 }
 
@@ -1667,10 +1666,10 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
   SparseFuseDev f{fuse.grad, fuse.u, fuse.momentum, fuse.clip, fuse.sumsq, fuse.zero_grad, fuse.mode};
   uint32_t* keys = sample_cnt <= lp.key_capacity
                        ? reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + lp.keys_offset) : nullptr;
-  // the list form: keep fractions up to 1 %, and a pool that holds the candidates with a wide
+  // the list form: small keep fractions, and a pool that holds the candidates with a wide
   // margin: their number is about n (rank0+1) / (samples+1) with a relative spread of
   // 1 / sqrt(rank0+1); without sampling every non-zero element is a candidate
-  bool lists = keep_fraction <= kListMaxKeep && sample_cnt > 0;
+  bool lists = keep_fraction <= (n <= kListSmall ? kListMaxKeepSmall : kListMaxKeep) && sample_cnt > 0;
   if (lists) {
     const double mean = double(n) * double(rank0 + 1) / double(sample_cnt + 1);
     const double need = mean * (1.0 + 40.0 / std::sqrt(double(rank0 + 1)));
@@ -1710,6 +1709,7 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
     *launches += (sumsq != nullptr ? 1 : 0) + (sample_cnt > 0 ? (keys != nullptr ? 2 : 3) : 0) + (lists ? 3 : 4);
   const dim3 grid = dim3(unsigned(pl.blocks));
   float* const u_mask = fuse.mode == 2 ? fuse.u : nullptr;
+  auto* state = reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(scratch) + lp.state_offset);
   if (lists) {
     PushTargets hdr = dst;
     hdr.done = nullptr;
@@ -1720,32 +1720,26 @@ cudaError_t sparse_compress_fused(const SparseFuse& fuse, float* R, int64_t n, d
     pool.next = pool.count + lp.pool_blocks;
     pool.entry = reinterpret_cast<uint2*>((reinterpret_cast<uintptr_t>(pool.next + lp.pool_blocks) + 127) & ~uintptr_t(127));
     pool.dense = reinterpret_cast<uint32_t*>(pool.entry + size_t(lp.pool_blocks) * kBlockEntries);
-    pool.dense_cta = reinterpret_cast<uint16_t*>(pool.dense + size_t(lp.pool_blocks) * kBlockEntries);
-    const int nlists = pl.blocks * (kThreads / 32);
     auto collect = fuse.mode == 2 ? collect_kernel<2> : (fuse.mode == 1 ? collect_kernel<1> : collect_kernel<0>);
-    e = launch_after(collect, grid, block, 0, stream, f, R, n, pl.chunk, s, pool);   // lists: there was a sample
+    e = launch_after(collect, grid, block, 0, stream, f, R, n, pl.chunk, s, pool, state);   // lists: there was a sample
     if (e != cudaSuccess) return e;
     const bool one = expected <= kCutOneCta;
     const int ctas = one ? 1 : kCutCluster;
-    const size_t smem = size_t(one ? CutForm<1>::kKeys : CutForm<kCutCluster>::kKeys) * sizeof(uint32_t);
-    auto cut = one ? cut_kernel<1> : cut_kernel<kCutCluster>;
-    e = cudaFuncSetAttribute(cut, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    e = launch_with(true, ctas, one ? cut_kernel<1> : cut_kernel<kCutCluster>, dim3(unsigned(ctas)), dim3(kCutThreads), 0, stream,
+                    unsigned(expected), hdr, s, pool, sumsq);
     if (e != cudaSuccess) return e;
-    e = launch_with(true, ctas, cut, dim3(unsigned(ctas)), dim3(kCutThreads), smem, stream, unsigned(expected), pl.blocks, hdr,
-                    s, pool, sumsq);
-    if (e != cudaSuccess) return e;
-    return launch_after(emit_kernel, grid, block, 0, stream, R, u_mask, nlists, dst, static_cast<const SparseScratch*>(s), pool);
+    return launch_after(emit_kernel, grid, block, 0, stream, R, u_mask, unsigned(expected), dst, s, pool, state, status);
   }
   // scan form
   auto count = fuse.mode == 2 ? count_kernel<2> : (fuse.mode == 1 ? count_kernel<1> : count_kernel<0>);
-  e = launch_with(sample_cnt > 0, 1, count, grid, block, 0, stream, f, R, n, pl.chunk, s);
+  e = launch_with(sample_cnt > 0, 1, count, grid, block, 0, stream, f, R, n, pl.chunk, s, state);
   if (e == cudaSuccess)
     e = launch_after(trim_kernel<0>, grid, block, 0, stream, static_cast<const float*>(R), n, pl.chunk, unsigned(expected), s);
   if (e == cudaSuccess)
     e = launch_after(trim_kernel<1>, grid, block, 0, stream, static_cast<const float*>(R), n, pl.chunk, unsigned(expected), s);
   if (e != cudaSuccess) return e;
-  return launch_after(write_kernel, grid, block, 0, stream, R, u_mask, sumsq, n, pl.chunk, unsigned(expected), dst, s,
-                      status);
+  return launch_after(write_kernel, dim3(unsigned((n + kWriteChunk - 1) / kWriteChunk)), block, 0, stream, R, u_mask, sumsq,
+                      n, unsigned(expected), dst, s, state, status);
 }
 
 cudaError_t sparse_compress(const float* grad, float* R, int64_t n, double sample_rate,

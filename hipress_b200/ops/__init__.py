@@ -151,7 +151,7 @@ def dgc_momentum_compress(grad: torch.Tensor, u: torch.Tensor, v: torch.Tensor, 
     """DGC with momentum correction as one fused pipeline (CUDA tensors): ``u = momentum*u + s*grad``,
     ``v += u``, sampled-threshold top-k of ``v`` into the payload, ``u`` and ``v`` cleared at the
     sent positions (momentum factor masking).  ``s = min(1, clip / |grad|)`` when ``clip > 0``.
-    For keep fractions up to 1 % the three tensors are read once.  (Momentum correction, clipping
+    For keep fractions up to half a per cent the three tensors are read once.  (Momentum correction, clipping
     and masking are not in the reference, whose dgc_body.h is the selector alone.)"""
     if out is None:
         out = _u8(sparse_payload_bytes(v.numel(), keep_fraction), v)

@@ -254,6 +254,48 @@ def test_sparse_list_form_one_and_eight_ctas(n, keep):
         compare_sparse(r, 0.01, keep, seed)
 
 
+@pytest.mark.parametrize("n", [1, 511, 513, 4095, 4097, 8191, 12289, (1 << 21) + 4099])
+@pytest.mark.parametrize("few_magnitudes", [False, True])
+def test_sparse_write_chunks(n, few_magnitudes):
+    """Edges of a warp's 512 elements and a CTA's 4,096, and more chunks than one step of the look-back; with few
+    magnitudes most of what lies at the cut is left behind, lane by lane."""
+    r = gauss(n, seed=n)
+    if few_magnitudes:
+        r = torch.sign(r) * torch.tensor([1.0, 0.5, 0.5, 0.25])[torch.randint(4, (n,), generator=torch.Generator().manual_seed(n))]
+    for keep in (0.03, 0.6):
+        for rate in (0.0, 0.02):
+            compare_sparse(r, rate, keep, 3)
+
+
+@pytest.mark.parametrize("n", [(2 << 20) - 1, 2 << 20, (2 << 20) + 1])
+@pytest.mark.parametrize("keep", [0.005, 0.0051, 0.01, 0.0102])
+def test_sparse_where_lists_end(n, keep):
+    """Both sides of the line between the forms, which must not show."""
+    for seed in (1, 2):
+        compare_sparse(gauss(n, seed=9), 0.01, keep, seed)
+
+
+@pytest.mark.parametrize("octaves", [0, 30])
+def test_sparse_cut_by_a_cluster(octaves):
+    """45,000 wanted: eight CTAs share the candidates.  Over 30 octaves the cut lies in the last of the bins counted by
+    distance, and is found by the keys' digits."""
+    n = 9000001
+    g = torch.Generator().manual_seed(8)
+    r = torch.randn(n, generator=g) * torch.exp2(-octaves * torch.rand(n, generator=g))
+    for seed in range(1, 5):
+        compare_sparse(r, 0.00002 if octaves else 0.01, 0.005, seed)
+
+
+def test_sparse_lists_longer_than_a_warp():
+    """A warp of the collect pass holds the keys of its first 32 candidates; here some have hundreds, others none."""
+    n = 3000001
+    r = gauss(n, 1e-3, seed=5)
+    r[700000:706000] = gauss(6000, 1.0, seed=6)
+    for keep in (0.001, 0.004):
+        for seed in (1, 2, 3):
+            compare_sparse(r, 0.01, keep, seed)
+
+
 @pytest.mark.parametrize("keep", [0.004, 0.05])
 def test_sparse_magnitudes_over_many_octaves(keep):
     """Few samples and magnitudes over 30 octaves: the cut may lie far above the sampled threshold."""
