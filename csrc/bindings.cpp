@@ -213,6 +213,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bias_relu_forward", &ops::bias_relu_forward, py::arg("x"), py::arg("bias"), py::arg("pool"));
   m.def("bias_relu_backward", &ops::bias_relu_backward, py::arg("dy"), py::arg("y"), py::arg("idx"),
         py::arg("pool"));
+  m.def("gelu_supported", &ops::gelu_supported, py::arg("x"));
+  m.def("gelu_forward", &ops::gelu_forward, py::arg("x"));
+  m.def("gelu_backward", &ops::gelu_backward, py::arg("dy"), py::arg("x"));
   m.def("add_ln_supported", &ops::add_ln_supported, py::arg("x"));
   m.def("add_ln_forward", &ops::add_ln_forward, py::arg("x"), py::arg("delta"), py::arg("weight"), py::arg("bias"),
         py::arg("eps"));

@@ -292,6 +292,10 @@ cudaError_t bias_relu_backward(const void* dy, const void* y, const uint8_t* idx
 //             mean / rstd: one fp32 value per row, for backward.
 //   backward: dz (= gradient of x and of delta), dgamma, dbeta; partial = add_ln_partial_elems floats.
 bool add_ln_supported(int64_t rows, int hidden);
+// GELU of n bf16 values, all pointers 16-byte aligned: y = x * Phi(x), dx = dy * (Phi(x) + x * Phi'(x)).
+cudaError_t gelu_forward(const void* x, void* y, int64_t n, cudaStream_t stream);
+cudaError_t gelu_backward(const void* dy, const void* x, void* dx, int64_t n, cudaStream_t stream);
+
 int64_t add_ln_partial_elems(int64_t rows, int hidden);
 cudaError_t add_ln_forward(const void* x, const void* delta, const float* gamma, const float* beta, void* y,
                            void* z, float* mean, float* rstd, int64_t rows, int hidden, float eps,

@@ -227,6 +227,28 @@ int64_t ln_rows(const torch::Tensor& t, const char* name) {
 }
 }  // namespace
 
+bool gelu_supported(const torch::Tensor& x) {
+  return x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.numel() > 0 &&
+         (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0;
+}
+
+torch::Tensor gelu_forward(const torch::Tensor& x) {
+  TORCH_CHECK(gelu_supported(x), "gelu: unsupported input");
+  c10::cuda::CUDAGuard guard(x.device());
+  auto y = torch::empty_like(x);
+  HP_BN_CHECK(cuda::gelu_forward(x.data_ptr(), y.data_ptr(), x.numel(), at::cuda::getCurrentCUDAStream()));
+  return y;
+}
+
+torch::Tensor gelu_backward(const torch::Tensor& dy, const torch::Tensor& x) {
+  TORCH_CHECK(gelu_supported(dy) && gelu_supported(x) && dy.sizes() == x.sizes() && dy.device() == x.device(),
+              "gelu: unsupported gradient");
+  c10::cuda::CUDAGuard guard(x.device());
+  auto dx = torch::empty_like(x);
+  HP_BN_CHECK(cuda::gelu_backward(dy.data_ptr(), x.data_ptr(), dx.data_ptr(), x.numel(), at::cuda::getCurrentCUDAStream()));
+  return dx;
+}
+
 bool add_ln_supported(const torch::Tensor& x) {
   return x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() >= 1 &&
          x.numel() > 0 && cuda::add_ln_supported(x.numel() / x.size(-1), int(x.size(-1)));

@@ -146,6 +146,9 @@ torch::Tensor colsum(const torch::Tensor& dy);
 
 // y = LayerNorm(x + delta) over the last dimension of contiguous bf16 tensors (delta optional).
 // forward -> {y, z = bf16(x + delta) (x itself without delta), stats}; backward -> {dz, dweight, dbias}.
+bool gelu_supported(const torch::Tensor& x);
+torch::Tensor gelu_forward(const torch::Tensor& x);
+torch::Tensor gelu_backward(const torch::Tensor& dy, const torch::Tensor& x);
 bool add_ln_supported(const torch::Tensor& x);
 std::vector<torch::Tensor> add_ln_forward(const torch::Tensor& x, const c10::optional<torch::Tensor>& delta,
                                           const torch::Tensor& weight, const torch::Tensor& bias, double eps);

@@ -8,7 +8,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .layers import FusedAddLayerNorm, FusedLinear
+from .layers import FusedAddLayerNorm, FusedLinear, fused_gelu
 
 
 class BertLayer(nn.Module):
@@ -39,7 +39,7 @@ class BertLayer(nn.Module):
         a = F.scaled_dot_product_attention(q, k, v)
         a = a.transpose(1, 2).reshape(b, s, h)
         x = self.ln1(x, self.drop(self.out(a)))
-        return self.ln2(x, self.drop(self.fc2(F.gelu(self.fc1(x)))))
+        return self.ln2(x, self.drop(self.fc2(fused_gelu(self.fc1(x)))))
 
 
 class BertForMaskedLM(nn.Module):
@@ -74,7 +74,7 @@ class BertForMaskedLM(nn.Module):
         for layer in self.layers:
             x = layer(x)
         if labels is None:
-            h = self.head_ln(F.gelu(self.head_dense(x)))
+            h = self.head_ln(fused_gelu(self.head_dense(x)))
             return F.linear(h, self.tok.weight, self.head_bias)
         # score only the masked positions (labels == -100 elsewhere)
         flat = labels.view(-1)
@@ -90,7 +90,7 @@ class BertForMaskedLM(nn.Module):
             sel = flat >= 0
             h = x.view(b * s, -1)[sel]
             target = flat[sel]
-        h = self.head_ln(F.gelu(self.head_dense(h)))
+        h = self.head_ln(fused_gelu(self.head_dense(h)))
         logits = F.linear(h, self.tok.weight, self.head_bias)
         return F.cross_entropy(logits.float(), target, ignore_index=-100)
 

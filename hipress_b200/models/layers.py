@@ -3,6 +3,7 @@
 ``MaxPool3x3s2`` is the ResNet stem's pooling layer on a gather-style kernel pair.
 ``FusedBiasReLU`` is the epilogue of VGG's convolutions: bias + ReLU (+ 2x2 max pooling).
 ``FusedAddLayerNorm`` is BERT's residual add + LayerNorm on a bf16 residual stream.
+``fused_gelu`` is ``F.gelu`` at memory speed.
 ``FusedLinear`` is ``nn.Linear`` whose backward yields fp32 weight gradients from the GEMM and the
 bias gradient from a two-stage column sum.
 
@@ -168,6 +169,29 @@ class FusedAddLayerNorm(nn.LayerNorm):
                 return _AddLayerNormFunction.apply(xc, None if delta is None else delta.contiguous(),
                                                    self.weight, self.bias, float(self.eps))
         return super().forward(x if delta is None else x + delta)
+
+
+class _GeluFunction(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        ctx.save_for_backward(x)
+        return _C.gelu_forward(x)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (x,) = ctx.saved_tensors
+        dy = dy.contiguous()
+        if torch.is_grad_enabled() or not _C.gelu_supported(dy):   # a gradient of the gradient is wanted
+            return torch.ops.aten.gelu_backward(dy, x)
+        return _C.gelu_backward(dy, x)
+
+
+def fused_gelu(x: torch.Tensor) -> torch.Tensor:
+    """``F.gelu(x)``; bf16 CUDA activations under autocast, where the linear layers on either side run as
+    autograd functions too, take the kernels of ``csrc/kernels/gelu.cu``."""
+    if _C is not None and x.is_cuda and torch.is_autocast_enabled() and _C.gelu_supported(x):
+        return _GeluFunction.apply(x)
+    return F.gelu(x)
 
 
 _MM_FP32_OUT = None   # whether torch.mm(bf16, bf16, out_dtype=float32) works here; probed on first use

@@ -221,6 +221,40 @@ def test_add_layer_norm_matches_fp32_reference(shape, with_delta):
     torch.testing.assert_close(layer.bias.grad, br.grad, atol=2e-3 * rows ** 0.5 + 1e-3, rtol=1e-3)
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 4095, 4096, 4097, 1 << 20])
+@pytest.mark.parametrize("std", [0.1, 1.0, 4.0])
+def test_gelu_error_against_64_bits(n, std):
+    """No further off than the stock kernels: half a unit in the last place of bf16 is up to 2^-8 of a value, and what the
+    kernels add to the rounding is a few 1e-7."""
+    from hipress_b200.models.layers import fused_gelu
+    g = torch.Generator().manual_seed(n)
+    x = (torch.randn(n, generator=g) * std).to(torch.bfloat16).cuda()
+    dy = torch.randn(n, generator=g).to(torch.bfloat16).cuda()
+
+    def run(f, x, dy):
+        x = x.clone().requires_grad_(True)
+        y = f(x)
+        y.backward(dy)
+        return y.detach().double(), x.grad.double()
+
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        ours, stock = run(fused_gelu, x, dy), run(F.gelu, x, dy)
+    exact = run(F.gelu, x.double(), dy.double())
+    for a, b, e in zip(ours, stock, exact):
+        assert n < 4095 or (a - e).norm() <= 1.001 * (b - e).norm() + 1e-9
+        assert ((a - e).abs() <= 2.0 ** -8 * e.abs() * 1.001 + 1e-6).all()
+
+
+def test_gelu_of_infinities_and_nan():
+    from hipress_b200.models.layers import fused_gelu
+    x = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0, -0.0, 3e38, -3e38] * 3, device="cuda").to(torch.bfloat16)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        got = fused_gelu(x)
+    assert torch.equal(got.isnan(), F.gelu(x).isnan())
+    ok = ~got.isnan()
+    assert torch.equal(got[ok], F.gelu(x)[ok])
+
+
 def test_add_layer_norm_stock_path_for_fp32():
     from hipress_b200.models.layers import FusedAddLayerNorm
     layer = FusedAddLayerNorm(48).cuda()
