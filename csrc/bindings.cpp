@@ -202,9 +202,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bn_supported", &ops::bn_supported, py::arg("x"));
   m.def("bn_forward", &ops::bn_forward, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("bias"),
         py::arg("running_mean"), py::arg("running_var"), py::arg("num_batches"), py::arg("momentum"),
-        py::arg("eps"), py::arg("relu"));
+        py::arg("eps"), py::arg("relu"), py::arg("mask") = py::none());
   m.def("bn_backward", &ops::bn_backward, py::arg("dy"), py::arg("x"), py::arg("y"), py::arg("weight"),
-        py::arg("stats"), py::arg("relu"), py::arg("want_dres"));
+        py::arg("stats"), py::arg("relu"), py::arg("want_dres"), py::arg("mask") = py::none());
   m.def("maxpool_supported", &ops::maxpool_supported, py::arg("x"));
   m.def("maxpool3x3s2_forward", &ops::maxpool3x3s2_forward, py::arg("x"));
   m.def("maxpool3x3s2_backward", &ops::maxpool3x3s2_backward, py::arg("dy"), py::arg("idx"), py::arg("h"),

@@ -11,6 +11,10 @@
 //   backward  reduce: sums of dy' and dy'*(x - mean), dy' = dy * (y > 0)
 //             elemt:  dx = dy'*a + x*k2 + k3 [, dres = dy']
 //
+// What the backward pass wants of y is a bit per element.  The apply kernel can leave those (a byte for a thread's
+// eight channels), and both backward kernels then read a sixteenth of what y is: with activations of 103 MB they take
+// 43 and 70 us, and 57 and 86 with y.
+//
 // Every kernel uses the same geometry: a CTA owns a tile of up to 256 channels and a contiguous
 // range of rows (row = one pixel of one image, C contiguous bf16 values).  A thread owns 8
 // adjacent channels (one 16-byte load per row) for the whole kernel, so per-channel constants
@@ -188,11 +192,18 @@ bn_stats_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int
 }
 
 // ---------------------------------------------------------------- forward: apply
+// Bit k: the value that store8 writes for v[k], rounded, is positive.
+__device__ __forceinline__ uint8_t positive8(const float (&v)[kBnVec]) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < kBnVec; ++k) bits |= __bfloat162float(__float2bfloat16_rn(v[k])) > 0.f ? 1u << k : 0u;
+  return uint8_t(bits);
+}
 template <bool RELU, bool ADD>
 __global__ void __launch_bounds__(kBnThreads)
 bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                __nv_bfloat16* __restrict__ y, int64_t M, int C, int tx_count, int64_t rows_per_block,
-                const float2* ab) {
+                __nv_bfloat16* __restrict__ y, uint8_t* __restrict__ mask, int64_t M, int C, int tx_count,
+                int64_t rows_per_block, const float2* ab) {
   wait_for_previous();
   const Lane l = lane_of(tx_count, M, rows_per_block);
   float a[kBnVec], b[kBnVec];
@@ -219,6 +230,7 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         v[u][k] = RELU ? fmaxf(o, 0.f) : o;
       }
       store8(y + (r + u * l.TY) * C + l.c0, v[u]);
+      if (RELU && mask != nullptr) mask[((r + u * l.TY) * C + l.c0) / kBnVec] = positive8(v[u]);
     }
   }
   for (; r < l.r_end; r += l.TY) {
@@ -232,14 +244,27 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
       v[k] = RELU ? fmaxf(o, 0.f) : o;
     }
     store8(y + r * C + l.c0, v);
+    if (RELU && mask != nullptr) mask[(r * C + l.c0) / kBnVec] = positive8(v);
   }
 }
 
+// Where the gradient passes the ReLU: everywhere, where y is positive, or where the apply kernel left a bit.
+enum Gate { kOpen = 0, kOutput = 1, kMask = 2 };
+template <int GATE>
+__device__ __forceinline__ void load_gate(const __nv_bfloat16* y, const uint8_t* mask, int64_t at, float (&o)[kBnVec], uint32_t& bits) {
+  if (GATE == kOutput) load8(y + at, o);
+  if (GATE == kMask) bits = mask[at / kBnVec];
+}
+template <int GATE>
+__device__ __forceinline__ bool passes(const float (&o)[kBnVec], uint32_t bits, int k) {
+  return GATE == kOpen || (GATE == kOutput ? o[k] > 0.f : ((bits >> k) & 1u) != 0);
+}
+
 // ---------------------------------------------------------------- backward: reductions
-template <bool RELU>
+template <int GATE>
 __global__ void __launch_bounds__(kBnThreads)
 bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                     const __nv_bfloat16* __restrict__ y, int64_t M, int C, int tx_count,
+                     const __nv_bfloat16* __restrict__ y, const uint8_t* __restrict__ mask, int64_t M, int C, int tx_count,
                      int64_t rows_per_block, const float* __restrict__ mean, float2* __restrict__ partial) {
   __shared__ float sh[2 * kBnThreads * kBnVec];
   const Lane l = lane_of(tx_count, M, rows_per_block);
@@ -252,29 +277,31 @@ bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   int64_t r = l.r_begin + l.ty;
   for (; r + 1 * l.TY < l.r_end; r += 2 * l.TY) {
     float g[2][kBnVec], v[2][kBnVec], o[2][kBnVec];
+    uint32_t bits[2] = {};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       load8(dy + (r + u * l.TY) * C + l.c0, g[u]);
       load8(x + (r + u * l.TY) * C + l.c0, v[u]);
-      if (RELU) load8(y + (r + u * l.TY) * C + l.c0, o[u]);
+      load_gate<GATE>(y, mask, (r + u * l.TY) * C + l.c0, o[u], bits[u]);
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int k = 0; k < kBnVec; ++k) {
-        const float d = (!RELU || o[u][k] > 0.f) ? g[u][k] : 0.f;
+        const float d = passes<GATE>(o[u], bits[u], k) ? g[u][k] : 0.f;
         s1[k] += d;
         s2[k] += d * (v[u][k] - mu[k]);
       }
   }
   for (; r < l.r_end; r += l.TY) {
     float g[kBnVec], v[kBnVec], o[kBnVec];
+    uint32_t bits = 0;
     load8(dy + r * C + l.c0, g);
     load8(x + r * C + l.c0, v);
-    if (RELU) load8(y + r * C + l.c0, o);
+    load_gate<GATE>(y, mask, r * C + l.c0, o, bits);
 #pragma unroll
     for (int k = 0; k < kBnVec; ++k) {
-      const float d = (!RELU || o[k] > 0.f) ? g[k] : 0.f;
+      const float d = passes<GATE>(o, bits, k) ? g[k] : 0.f;
       s1[k] += d;
       s2[k] += d * (v[k] - mu[k]);
     }
@@ -336,10 +363,10 @@ bn_bwd_finalize_kernel(const float2* __restrict__ partial, int row_blocks, int64
 }
 
 // ---------------------------------------------------------------- backward: elementwise
-template <bool RELU, bool ADD>
+template <int GATE, bool ADD>
 __global__ void __launch_bounds__(kBnThreads)
 bn_bwd_elemt_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                    const __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ dx,
+                    const __nv_bfloat16* __restrict__ y, const uint8_t* __restrict__ mask, __nv_bfloat16* __restrict__ dx,
                     __nv_bfloat16* __restrict__ dres, int64_t M, int C, int tx_count,
                     int64_t rows_per_block, const float4* coef) {
   wait_for_previous();
@@ -355,17 +382,18 @@ bn_bwd_elemt_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
   int64_t r = l.r_begin + l.ty;
   for (; r + 1 * l.TY < l.r_end; r += 2 * l.TY) {
     float g[2][kBnVec], v[2][kBnVec], o[2][kBnVec];
+    uint32_t bits[2] = {};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       load8(dy + (r + u * l.TY) * C + l.c0, g[u]);
       load8(x + (r + u * l.TY) * C + l.c0, v[u]);
-      if (RELU) load8(y + (r + u * l.TY) * C + l.c0, o[u]);
+      load_gate<GATE>(y, mask, (r + u * l.TY) * C + l.c0, o[u], bits[u]);
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
 #pragma unroll
       for (int k = 0; k < kBnVec; ++k) {
-        const float d = (!RELU || o[u][k] > 0.f) ? g[u][k] : 0.f;
+        const float d = passes<GATE>(o[u], bits[u], k) ? g[u][k] : 0.f;
         g[u][k] = d;
         v[u][k] = fmaf(d, a[k], fmaf(v[u][k], k2[k], k3[k]));
       }
@@ -375,12 +403,13 @@ bn_bwd_elemt_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* _
   }
   for (; r < l.r_end; r += l.TY) {
     float g[kBnVec], v[kBnVec], o[kBnVec];
+    uint32_t bits = 0;
     load8(dy + r * C + l.c0, g);
     load8(x + r * C + l.c0, v);
-    if (RELU) load8(y + r * C + l.c0, o);
+    load_gate<GATE>(y, mask, r * C + l.c0, o, bits);
 #pragma unroll
     for (int k = 0; k < kBnVec; ++k) {
-      const float d = (!RELU || o[k] > 0.f) ? g[k] : 0.f;
+      const float d = passes<GATE>(o, bits, k) ? g[k] : 0.f;
       g[k] = d;
       v[k] = fmaf(d, a[k], fmaf(v[k], k2[k], k3[k]));
     }
@@ -405,7 +434,7 @@ int64_t bn_partial_elems(int64_t rows, int channels) {
 cudaError_t bn_forward(const void* x, const void* residual, void* y, int64_t rows, int channels,
                        const float* gamma, const float* beta, float* running_mean, float* running_var,
                        long long* num_batches, float momentum, float eps, int relu, float* mean,
-                       float* invstd, float* ab, float* partial, cudaStream_t stream) {
+                       float* invstd, float* ab, float* partial, cudaStream_t stream, uint8_t* mask) {
   Geom g;
   if (!geometry(rows, channels, &g) || !x || !y || !mean || !invstd || !ab || !partial)
     return cudaErrorInvalidValue;
@@ -424,7 +453,7 @@ cudaError_t bn_forward(const void* x, const void* residual, void* y, int64_t row
   if (e != cudaSuccess) return e;
   const float2* abp = reinterpret_cast<const float2*>(ab);
 #define HP_BN_APPLY(R, A)                                                                                          \
-  e = launch_after(bn_apply_kernel<R, A>, grid, dim3(kBnThreads), 0, stream, xb, rb, yb, rows, channels, g.tx,     \
+  e = launch_after(bn_apply_kernel<R, A>, grid, dim3(kBnThreads), 0, stream, xb, rb, yb, mask, rows, channels, g.tx, \
                    g.rows_per_block, abp)
   if (relu && rb) HP_BN_APPLY(true, true);
   else if (relu) HP_BN_APPLY(true, false);
@@ -437,10 +466,10 @@ cudaError_t bn_forward(const void* x, const void* residual, void* y, int64_t row
 cudaError_t bn_backward(const void* dy, const void* x, const void* y, void* dx, void* dres, int64_t rows,
                         int channels, const float* gamma, const float* mean, const float* invstd,
                         int relu, float* dgamma, float* dbeta, float* coef, float* partial,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, const uint8_t* mask) {
   Geom g;
   if (!geometry(rows, channels, &g) || !dy || !x || !dx || !mean || !invstd || !coef || !partial ||
-      (relu && !y))
+      (relu && !y && !mask))
     return cudaErrorInvalidValue;
   const dim3 grid(static_cast<unsigned>(g.tiles), static_cast<unsigned>(g.row_blocks), 1);
   const int fin_grid = (channels + kFinChannels - 1) / kFinChannels;
@@ -451,24 +480,20 @@ cudaError_t bn_backward(const void* dy, const void* x, const void* y, void* dx, 
   auto* drb = static_cast<__nv_bfloat16*>(dres);
   auto* part = reinterpret_cast<float2*>(partial);
   auto* cf = reinterpret_cast<float4*>(coef);
-  if (relu)
-    bn_bwd_reduce_kernel<true><<<grid, kBnThreads, 0, stream>>>(gb, xb, yb, rows, channels, g.tx, g.rows_per_block,
-                                                                mean, part);
-  else
-    bn_bwd_reduce_kernel<false><<<grid, kBnThreads, 0, stream>>>(gb, xb, yb, rows, channels, g.tx, g.rows_per_block,
-                                                                 mean, part);
+  const int gate = !relu ? kOpen : (mask != nullptr ? kMask : kOutput);
+  (gate == kMask ? bn_bwd_reduce_kernel<kMask> : (gate == kOutput ? bn_bwd_reduce_kernel<kOutput> : bn_bwd_reduce_kernel<kOpen>))
+      <<<grid, kBnThreads, 0, stream>>>(gb, xb, yb, mask, rows, channels, g.tx, g.rows_per_block, mean, part);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   e = launch_after(bn_bwd_finalize_kernel, dim3(fin_grid), dim3(kFinThreads), 0, stream, part, g.row_blocks, rows, channels,
                    mean, invstd, gamma, dgamma, dbeta, cf);
   if (e != cudaSuccess) return e;
-#define HP_BN_ELEMT(R, A)                                                                                          \
-  e = launch_after(bn_bwd_elemt_kernel<R, A>, grid, dim3(kBnThreads), 0, stream, gb, xb, yb, dxb, drb, rows,       \
-                   channels, g.tx, g.rows_per_block, cf)
-  if (relu && drb) HP_BN_ELEMT(true, true);
-  else if (relu) HP_BN_ELEMT(true, false);
-  else if (drb) HP_BN_ELEMT(false, true);
-  else HP_BN_ELEMT(false, false);
+#define HP_BN_ELEMT(G)                                                                                             \
+  e = launch_after(drb ? bn_bwd_elemt_kernel<G, true> : bn_bwd_elemt_kernel<G, false>, grid, dim3(kBnThreads), 0,  \
+                   stream, gb, xb, yb, mask, dxb, drb, rows, channels, g.tx, g.rows_per_block, cf)
+  if (gate == kMask) HP_BN_ELEMT(kMask);
+  else if (gate == kOutput) HP_BN_ELEMT(kOutput);
+  else HP_BN_ELEMT(kOpen);
 #undef HP_BN_ELEMT
   return e;
 }

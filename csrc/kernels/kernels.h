@@ -258,16 +258,17 @@ bool bn_supported(int64_t rows, int channels);
 int64_t bn_partial_elems(int64_t rows, int channels);
 // y = act(bn(x) [+ residual]); writes mean, invstd, ab = (gamma*invstd, beta - mean*gamma*invstd)
 // per channel and updates the running statistics (unbiased variance) when given.
+// mask (rows * channels / 8 bytes, with relu): where y is positive, bit by bit; the backward pass takes it in place of y.
 cudaError_t bn_forward(const void* x, const void* residual, void* y, int64_t rows, int channels,
                        const float* gamma, const float* beta, float* running_mean, float* running_var,
                        long long* num_batches, float momentum, float eps, int relu, float* mean,
-                       float* invstd, float* ab, float* partial, cudaStream_t stream);
+                       float* invstd, float* ab, float* partial, cudaStream_t stream, uint8_t* mask = nullptr);
 // dy' = relu ? dy*(y > 0) : dy.  dx = d loss / d x; dres (optional) = dy'; dgamma, dbeta fp32;
 // coef = 4*channels floats of scratch.
 cudaError_t bn_backward(const void* dy, const void* x, const void* y, void* dx, void* dres, int64_t rows,
                         int channels, const float* gamma, const float* mean, const float* invstd,
                         int relu, float* dgamma, float* dbeta, float* coef, float* partial,
-                        cudaStream_t stream);
+                        cudaStream_t stream, const uint8_t* mask = nullptr);
 
 // ---------------------------------------------------------------- bias + ReLU (+ 2x2 max pool)
 // Convolution epilogue over channels-last bf16 [n][h][w][c]; c as for batch norm.  With pool,

@@ -36,6 +36,13 @@ const float* opt_f32(const c10::optional<torch::Tensor>& t, int channels, const 
   return t->data_ptr<float>();
 }
 
+uint8_t* opt_mask(const c10::optional<torch::Tensor>& t, const torch::Tensor& x, const Shape& s) {
+  if (!t || !t->defined()) return nullptr;
+  TORCH_CHECK(t->device() == x.device() && t->scalar_type() == torch::kUInt8 && t->is_contiguous() &&
+                  t->numel() == s.rows * s.channels / 8, "mask must be a contiguous uint8 tensor with a bit per element of x");
+  return t->data_ptr<uint8_t>();
+}
+
 }  // namespace
 
 bool bn_supported(const torch::Tensor& x) {
@@ -51,7 +58,7 @@ std::vector<torch::Tensor> bn_forward(const torch::Tensor& x, const c10::optiona
                                       c10::optional<torch::Tensor> running_mean,
                                       c10::optional<torch::Tensor> running_var,
                                       c10::optional<torch::Tensor> num_batches, double momentum, double eps,
-                                      bool relu) {
+                                      bool relu, c10::optional<torch::Tensor> mask) {
   const Shape s = check_activation(x, "x");
   TORCH_CHECK(cuda::bn_supported(s.rows, s.channels), "unsupported channel count ", s.channels);
   const void* res = nullptr;
@@ -78,19 +85,20 @@ std::vector<torch::Tensor> bn_forward(const torch::Tensor& x, const c10::optiona
   HP_BN_CHECK(cuda::bn_forward(x.data_ptr(), res, y.data_ptr(), s.rows, s.channels,
                                opt_f32(weight, s.channels, "weight"), opt_f32(bias, s.channels, "bias"), rm, rv,
                                nb, float(momentum), float(eps), relu ? 1 : 0, st, st + s.channels,
-                               st + 2 * s.channels, partial.data_ptr<float>(), stream));
+                               st + 2 * s.channels, partial.data_ptr<float>(), stream, opt_mask(mask, x, s)));
   return {y, stats};
 }
 
 std::vector<torch::Tensor> bn_backward(const torch::Tensor& dy, const torch::Tensor& x,
                                        const c10::optional<torch::Tensor>& y,
                                        const c10::optional<torch::Tensor>& weight, const torch::Tensor& stats,
-                                       bool relu, bool want_dres) {
+                                       bool relu, bool want_dres, const c10::optional<torch::Tensor>& mask) {
   const Shape s = check_activation(x, "x");
   const Shape g = check_activation(dy, "dy");
   TORCH_CHECK(g.rows == s.rows && g.channels == s.channels, "dy must have x's shape");
   const void* yp = nullptr;
-  if (relu) {
+  const uint8_t* positive = relu ? opt_mask(mask, x, s) : nullptr;
+  if (relu && positive == nullptr) {
     TORCH_CHECK(y && y->defined(), "the fused ReLU needs the forward output");
     const Shape o = check_activation(*y, "y");
     TORCH_CHECK(o.rows == s.rows && o.channels == s.channels, "y must have x's shape");
@@ -111,7 +119,7 @@ std::vector<torch::Tensor> bn_backward(const torch::Tensor& dy, const torch::Ten
   HP_BN_CHECK(cuda::bn_backward(dy.data_ptr(), x.data_ptr(), yp, dx.data_ptr(), want_dres ? dres.data_ptr() : nullptr,
                                 s.rows, s.channels, opt_f32(weight, s.channels, "weight"), st, st + s.channels,
                                 relu ? 1 : 0, dwb.data_ptr<float>(), dwb.data_ptr<float>() + s.channels, sc,
-                                sc + 4 * s.channels, stream));
+                                sc + 4 * s.channels, stream, positive));
   std::vector<torch::Tensor> out{dx, dwb[0], dwb[1]};
   if (want_dres) out.push_back(dres);
   return out;

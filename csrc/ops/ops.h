@@ -117,11 +117,13 @@ std::vector<torch::Tensor> bn_forward(const torch::Tensor& x, const c10::optiona
                                       c10::optional<torch::Tensor> running_mean,
                                       c10::optional<torch::Tensor> running_var,
                                       c10::optional<torch::Tensor> num_batches, double momentum, double eps,
-                                      bool relu);
+                                      bool relu,
+                                      c10::optional<torch::Tensor> mask = c10::nullopt);
 std::vector<torch::Tensor> bn_backward(const torch::Tensor& dy, const torch::Tensor& x,
                                        const c10::optional<torch::Tensor>& y,
                                        const c10::optional<torch::Tensor>& weight, const torch::Tensor& stats,
-                                       bool relu, bool want_dres);
+                                       bool relu, bool want_dres,
+                                       const c10::optional<torch::Tensor>& mask = c10::nullopt);
 
 // 3x3 / stride 2 / padding 1 max pooling of channels-last bf16 activations: {y, idx} forward
 // (idx: winning window position per output element, one byte), gather backward.

@@ -35,18 +35,20 @@ class _FusedBnFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, weight, bias, running_mean, running_var, num_batches,
                 momentum: float, eps: float, relu: bool):
+        # what the backward pass needs of y: a bit per element
+        mask = torch.empty(x.numel() // 8, dtype=torch.uint8, device=x.device) if relu else None
         y, stats = _C.bn_forward(x, residual, weight, bias, running_mean, running_var, num_batches,
-                                 momentum, eps, relu)
-        ctx.save_for_backward(x, y if relu else None, weight, stats)
+                                 momentum, eps, relu, mask)
+        ctx.save_for_backward(x, mask, weight, stats)
         ctx.relu = relu
         ctx.has_residual = residual is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, y, weight, stats = ctx.saved_tensors
+        x, mask, weight, stats = ctx.saved_tensors
         dy = dy.contiguous(memory_format=torch.channels_last)
-        out = _C.bn_backward(dy, x, y, weight, stats, ctx.relu, ctx.has_residual)
+        out = _C.bn_backward(dy, x, None, weight, stats, ctx.relu, ctx.has_residual, mask)
         dres = out[3] if ctx.has_residual else None
         return out[0], dres, out[1], out[2], None, None, None, None, None, None
 

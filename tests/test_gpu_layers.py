@@ -61,6 +61,24 @@ def test_forward_backward_match_fp32_reference(shape, relu, residual):
     assert int(layer.num_batches_tracked) == 1
 
 
+@pytest.mark.parametrize("shape", [(2, 8, 3, 5), (3, 64, 7, 7), (2, 256, 14, 9), (1, 512, 5, 3)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_backward_from_the_bits_equals_backward_from_the_output(shape, residual):
+    torch.manual_seed(3)
+    x, res, dy = ((torch.randn(shape, device="cuda") * s).to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
+                  for s in (1.0, 1e-38, 1.0))   # some sums round to zero or below the smallest normal number
+    w, b = torch.randn(shape[1], device="cuda"), torch.zeros(shape[1], device="cuda")
+    if residual:
+        w[::2] = 0.0
+    mask = torch.full((x.numel() // 8,), 255, dtype=torch.uint8, device="cuda")
+    y, stats = _C.bn_forward(x, res if residual else None, w, b, None, None, None, 0.1, 1e-5, True, mask)
+    bits = (mask[:, None] >> torch.arange(8, device="cuda", dtype=torch.uint8)) & 1
+    assert torch.equal(bits.view(-1).bool(), y.permute(0, 2, 3, 1).reshape(-1) > 0)
+    from_y = _C.bn_backward(dy, x, y, w, stats, True, residual)
+    for a, c in zip(_C.bn_backward(dy, x, None, w, stats, True, residual, mask), from_y):
+        assert torch.equal(a, c)
+
+
 def test_statistics_survive_a_large_mean():
     """Variance of data with |mean| >> std: the per-block + Chan combination must not cancel."""
     torch.manual_seed(1)
