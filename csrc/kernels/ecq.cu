@@ -86,8 +86,9 @@ __device__ __forceinline__ uint32_t ecq_quant_byte(const float* v, float* h, int
 
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
-ecq_absmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ hist, int64_t n,
-                         float alpha, int bw, PushTargets dst, MinMaxScratch* scratch) {
+ecq_absmax_header_kernel(const float* grad, const float* hist, int64_t n, float alpha, int bw, PushTargets dst,
+                         MinMaxScratch* scratch) {
+  wait_for_previous();
   if (push_guarded(dst)) return;
   resolve_epoch(dst);
   float mx = 0.0f, unused = 0.0f;
@@ -103,14 +104,14 @@ ecq_absmax_header_kernel(const float* __restrict__ grad, const float* __restrict
     float4 g[4], h[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      g[u] = __ldg(reinterpret_cast<const float4*>(grad) + q + u * stride);
-      h[u] = __ldg(reinterpret_cast<const float4*>(hist) + q + u * stride);
+      g[u] = reinterpret_cast<const float4*>(grad)[q + u * stride];
+      h[u] = reinterpret_cast<const float4*>(hist)[q + u * stride];
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) fold(g[u], h[u]);
   }
   for (; q < nv; q += stride)
-    fold(__ldg(reinterpret_cast<const float4*>(grad) + q), __ldg(reinterpret_cast<const float4*>(hist) + q));
+    fold(reinterpret_cast<const float4*>(grad)[q], reinterpret_cast<const float4*>(hist)[q]);
   for (int64_t i = (nv << 2) + tid; i < n; i += stride)
     mx = fmaxf(mx, fabsf(ecq_compensated(grad[i], hist[i], alpha)));
   let_next_start();
@@ -431,6 +432,7 @@ ecq_unpack_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add
 template <int WORLD>
 __global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 ecq_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, float post_scale, int* status, int align) {
+  wait_for_previous();
   if (status_guarded(src.guard)) return;
   resolve_epoch(src);
   extern __shared__ __align__(16) float smem[];
@@ -465,7 +467,7 @@ ecq_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, f
 
 template <int WORLD>
 cudaError_t launch_ecq_index(const UnpackSources& src, float* out, int64_t n, float post_scale, int* status,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, bool overlap) {
   constexpr size_t b2 = IndexLayout<2, WORLD, false, true>::kBytes, b4 = IndexLayout<4, WORLD, false, true>::kBytes;
   constexpr size_t smem = b2 > b4 ? b2 : b4;
   if (smem > 40 * 1024) {   // with the static part, past the default limit
@@ -475,16 +477,15 @@ cudaError_t launch_ecq_index(const UnpackSources& src, float* out, int64_t n, fl
   }
   // sized by the smallest chunk (4 bits); at 8 bits the loop strides over what there is
   const int grid = index_grid(n, IndexForm<4>::kChunk, WORLD, smem);
-  ecq_unpack_index_kernel<WORLD><<<grid, index_threads(WORLD), smem, stream>>>(src, out, n, post_scale, status,
-                                                                        payload_alignment(src, kEcqHeaderBytes));
-  return cudaGetLastError();
+  return launch_with(overlap, 1, ecq_unpack_index_kernel<WORLD>, dim3(grid), dim3(index_threads(WORLD)), smem, stream, src, out, n,
+                     post_scale, status, payload_alignment(src, kEcqHeaderBytes));
 }
 
 }  // namespace
 
 cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alpha, float beta,
                          int bitwidth, uint64_t seed, const PushTargets& dst, void* scratch,
-                         cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns) {
+                         cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns, bool overlap) {
   if (n <= 0 || !ecq_bitwidth_ok(bitwidth) || scratch == nullptr) return cudaErrorInvalidValue;
   auto* s = static_cast<MinMaxScratch*>(scratch);
   PushTargets hdr_dst = dst;
@@ -506,8 +507,9 @@ cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alp
     }
   }
   const int hgrid = grid_for((n + 3) >> 2, kThreads, 148 * 4);
-  if (vec) ecq_absmax_header_kernel<true><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
-  else ecq_absmax_header_kernel<false><<<hgrid, kThreads, 0, stream>>>(grad, history, n, alpha, bitwidth, hdr_dst, s);
+  const cudaError_t e = launch_with(overlap, 1, vec ? ecq_absmax_header_kernel<true> : ecq_absmax_header_kernel<false>, dim3(hgrid),
+                                    dim3(kThreads), 0, stream, grad, history, n, alpha, bitwidth, hdr_dst, s);
+  if (e != cudaSuccess) return e;
   // chunked path once there is a chunk per warp of a half-filled GPU
   const int64_t chunks = n / (int64_t(kStageBytes) * (8 / bitwidth));
   const bool wide = vec && shift >= 0 && chunks >= 148 * 2;
@@ -527,10 +529,10 @@ cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alp
 }
 
 cudaError_t ecq_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
-                             float post_scale, int* status, cudaStream_t stream) {
+                             float post_scale, int* status, cudaStream_t stream, bool overlap) {
   if (n <= 0 || src.world < 1 || src.world > kMaxWorld) return cudaErrorInvalidValue;
   if (!add && aligned16(out)) {
-#define HP_INDEX(W) case W: return launch_ecq_index<W>(src, out, n, post_scale, status, stream)
+#define HP_INDEX(W) case W: return launch_ecq_index<W>(src, out, n, post_scale, status, stream, overlap)
     switch (src.world) {
       HP_INDEX(1); HP_INDEX(2); HP_INDEX(3); HP_INDEX(4); HP_INDEX(5); HP_INDEX(6); HP_INDEX(7); HP_INDEX(8);
     }

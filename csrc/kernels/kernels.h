@@ -101,13 +101,15 @@ enum Status : int {
 constexpr uint64_t kGridWaitNs = 2000000000ull;   // of a wait of CTAs for one another
 
 // ---------------------------------------------------------------- TBQ
+// overlap, here and below: the first kernel may be brought in before the one ahead of it in the stream has ended
+// (see launch.cuh).
 // grad and residual hold n floats; each payload destination ceil(n/4) bytes.
 cudaError_t tbq_compress(const float* grad, float* residual, int64_t n, float threshold,
-                         const PushTargets& dst, cudaStream_t stream);
+                         const PushTargets& dst, cudaStream_t stream, bool overlap = false);
 // out[i] = sum_r decode(payload_r)[i] (+ out[i] if add), times post_scale when != 1.
 cudaError_t tbq_unpack_accum(const UnpackSources& src, float threshold, float* out, int64_t n,
                              int add, float post_scale, const SgdApply& apply,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool overlap = false);
 
 // ---------------------------------------------------------------- TernGrad
 // Scratch needed by terngrad_compress / ecq_compress (bytes).
@@ -121,22 +123,22 @@ size_t minmax_scratch_bytes();
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
                               void* scratch, cudaStream_t stream, bool whole_gpu = false, int* status = nullptr,
-                              uint64_t grid_wait_ns = kGridWaitNs);
+                              uint64_t grid_wait_ns = kGridWaitNs, bool overlap = false);
 // Element count per payload is taken from its header and must equal n; all
 // payloads must carry the same bitwidth (kBadHeader otherwise).  bitwidth_hint
 // (0 = unknown) lets the launcher size the decode table for that bitwidth; a
 // payload with another bitwidth is then rejected.
 cudaError_t terngrad_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
                                   float post_scale, const SgdApply& apply, int* status,
-                                  cudaStream_t stream, int bitwidth_hint = 0);
+                                  cudaStream_t stream, int bitwidth_hint = 0, bool overlap = false);
 
 // ---------------------------------------------------------------- ECQ
 cudaError_t ecq_compress(const float* grad, float* history, int64_t n, float alpha, float beta,
                          int bitwidth, uint64_t seed, const PushTargets& dst, void* scratch,
                          cudaStream_t stream, bool whole_gpu = false, int* status = nullptr,
-                         uint64_t grid_wait_ns = kGridWaitNs);   // the last three: see terngrad_compress
+                         uint64_t grid_wait_ns = kGridWaitNs, bool overlap = false);   // see terngrad_compress
 cudaError_t ecq_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
-                             float post_scale, int* status, cudaStream_t stream);
+                             float post_scale, int* status, cudaStream_t stream, bool overlap = false);
 
 // ---------------------------------------------------------------- sparse top-k
 size_t sparse_scratch_bytes(int64_t n);
@@ -179,7 +181,7 @@ cudaError_t sparse_read_stats(const void* scratch, unsigned int* host4, cudaStre
 // per payload.
 cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
                                 float post_scale, int* status, cudaStream_t stream,
-                                unsigned int* redo = nullptr);
+                                unsigned int* redo = nullptr, bool overlap = false);
 
 // Decodes the payloads and applies the optimizer step (exactly one of sgd, adamw) to the parameters in one
 // pass, without a dense gradient.  The indices of each payload must ascend, as the compressor writes them;
@@ -354,17 +356,17 @@ cudaError_t gram_schmidt(float* P, int64_t n, int r, float eps, cudaStream_t str
 // The same, and in the same launch what a projection with P as its operand needs: Xt = P transposed and
 // zero-padded to [16][rows_pad] (null: not wanted), and `zero_count` zeros at `zeros`.
 cudaError_t gram_schmidt_for_projection(float* P, int64_t n, int r, float eps, float* Xt, int64_t rows_pad, float* zeros,
-                                        int64_t zero_count, cudaStream_t stream);
+                                        int64_t zero_count, cudaStream_t stream, bool overlap = false);
 // Mat[:N] = grad + residual, then P = Mat Q, in one pass: ranks 1, 2, 4, 8, m a multiple of 4, and 16-byte
 // aligned arrays (psgd_add_project_eligible).
 bool psgd_add_project_eligible(const float* grad, const float* residual, const float* Mat, const float* Q, int64_t m, int r);
 cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m,
-                             const float* Q, int r, float* P, cudaStream_t stream);
+                             const float* Q, int r, float* P, cudaStream_t stream, bool overlap = false);
 // approx = P Q^T.  mode 0 (API parity): Mat = approx; residual = grad - Mat[:N]; grad = Mat[:N].
 // mode 1 (error feedback in place): grad[:N] = post_scale * approx; Mat -= approx.
 cudaError_t psgd_expand_residual(const float* P, const float* Q, int64_t n, int64_t m, int r,
                                  float* Mat, float* residual, float* grad, int64_t N, int mode,
-                                 float post_scale, cudaStream_t stream);
+                                 float post_scale, cudaStream_t stream, bool overlap = false);
 
 // psgd_expand_sgd for a list of matrices in as few launches as possible (one grid per 32 matrices
 // that take the vectorised form; the others one by one).  `common` carries lr / momentum / weight

@@ -546,6 +546,7 @@ __device__ __forceinline__ void gram_schmidt_cta(float* P, int64_t n, int r, flo
 __global__ void __launch_bounds__(kGsThreads)
 gram_schmidt_kernel(float* __restrict__ P, int64_t n, int r, float eps, float* __restrict__ Xt, int64_t rows_pad,
                     float* __restrict__ zeros, int64_t zero_count) {
+  wait_for_previous();
   let_next_start();
   if (blockIdx.x == 0) {
     gram_schmidt_cta(P, n, r, eps, Xt, rows_pad);
@@ -599,9 +600,9 @@ expand_kernel(const float* __restrict__ P, const float* __restrict__ Q, int64_t 
 // columns in registers, reads P rows as broadcasts, and touches Mat / grad / param / momentum
 // with 16-byte accesses only (no per-element division).
 template <int MODE, int R>
-__device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, const float* __restrict__ Q, int64_t n,
-                                                 int64_t m, float* __restrict__ Mat, float* __restrict__ residual,
-                                                 float* __restrict__ grad, int64_t N, float scale,
+__device__ __forceinline__ void expand_rows_body(const float* P, const float* Q, int64_t n,
+                                                 int64_t m, float* Mat, float* residual,
+                                                 float* grad, int64_t N, float scale,
                                                  const SgdApply& apply, int rows_per_cta, int col_block,
                                                  int row_block) {
   const int64_t col = (int64_t(col_block) * 256 + threadIdx.x) * 4;
@@ -619,8 +620,13 @@ __device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, co
     constexpr int U = 4;
     for (; i + U <= r1 && (i + U - 1) * m + col + 3 < N; i += U) {
       float4 g[U];
+      float p[U][R];   // before the stores, which might lie anywhere for all the compiler knows
 #pragma unroll
-      for (int u = 0; u < U; ++u) g[u] = *reinterpret_cast<const float4*>(grad + (i + u) * m + col);
+      for (int u = 0; u < U; ++u) {
+        g[u] = *reinterpret_cast<const float4*>(grad + (i + u) * m + col);
+#pragma unroll
+        for (int c = 0; c < R; ++c) p[u][c] = P[(i + u) * R + c];
+      }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         float a[4];
@@ -628,7 +634,7 @@ __device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, co
         for (int j = 0; j < 4; ++j) {
           float acc = 0.f;
 #pragma unroll
-          for (int c = 0; c < R; ++c) acc += __ldg(P + (i + u) * R + c) * q[j][c];
+          for (int c = 0; c < R; ++c) acc += p[u][c] * q[j][c];
           a[j] = acc;
         }
         const int64_t e = (i + u) * m + col;
@@ -641,7 +647,7 @@ __device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, co
   for (; i < r1; ++i) {
     float p[R];
 #pragma unroll
-    for (int c = 0; c < R; ++c) p[c] = __ldg(P + i * R + c);
+    for (int c = 0; c < R; ++c) p[c] = P[i * R + c];
     float a[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -690,9 +696,9 @@ __device__ __forceinline__ void expand_rows_body(const float* __restrict__ P, co
 
 template <int MODE, int R>
 __global__ void __launch_bounds__(256)
-expand_rows_kernel(const float* __restrict__ P, const float* __restrict__ Q, int64_t n, int64_t m,
-                   float* __restrict__ Mat, float* __restrict__ residual, float* __restrict__ grad,
+expand_rows_kernel(const float* P, const float* Q, int64_t n, int64_t m, float* Mat, float* residual, float* grad,
                    int64_t N, float scale, SgdApply apply, int rows_per_cta) {
+  wait_for_previous();
   expand_rows_body<MODE, R>(P, Q, n, m, Mat, residual, grad, N, scale, apply, rows_per_cta, int(blockIdx.x),
                             int(blockIdx.y));
 }
@@ -732,7 +738,7 @@ expand_rows_grouped_kernel(const __grid_constant__ GroupedExpand g) {
 template <int MODE>
 bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, int r, float* Mat,
                         float* residual, float* grad, int64_t N, float scale, const SgdApply& apply,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, bool overlap = false) {
   auto al = [](const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if ((m & 3) != 0 || !al(Mat) || !al(residual) || !al(grad) || !al(apply.param) || !al(apply.momentum))
     return false;
@@ -743,8 +749,9 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
   if (row_blocks < 1) row_blocks = 1;
   const int rows_per = int((n + row_blocks - 1) / row_blocks);
   const dim3 grid(col_blocks, unsigned((n + rows_per - 1) / rows_per), 1);
-#define HP_EXPAND(RR) \
-  expand_rows_kernel<MODE, RR><<<grid, 256, 0, stream>>>(P, Q, n, m, Mat, residual, grad, N, scale, apply, rows_per)
+#define HP_EXPAND(RR)                                                                                              \
+  launch_with(overlap, 1, expand_rows_kernel<MODE, RR>, grid, dim3(256), 0, stream, P, Q, n, m, Mat, residual, grad, N, \
+              scale, apply, rows_per)
   switch (r) {
     case 1: HP_EXPAND(1); break;
     case 2: HP_EXPAND(2); break;
@@ -768,9 +775,9 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
 // 15.2.  Error of the three stages against 64 bits 7.4e-4, and 8.4e-4 with the projection in tf32.
 template <int R>
 __global__ void __launch_bounds__(256, 2)
-add_project_kernel(const float* __restrict__ grad, const float* __restrict__ residual, int64_t N, float* __restrict__ Mat,
-                   int64_t n, int64_t m, const float* __restrict__ Q, float* __restrict__ P, int64_t cols_per_cta,
-                   int64_t rows_per_cta, int rows_at_once) {
+add_project_kernel(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m, const float* Q, float* P,
+                   int64_t cols_per_cta, int64_t rows_per_cta, int rows_at_once) {
+  wait_for_previous();
   constexpr int RB = 32 / R;                    // rows at once, at most
   constexpr int RG = 4;                         // rows whose loads are issued together
   __shared__ float sums[8][32];
@@ -786,7 +793,7 @@ add_project_kernel(const float* __restrict__ grad, const float* __restrict__ res
       float q[4 * R];
 #pragma unroll
       for (int k = 0; k < R; ++k) {
-        const float4 t = __ldg(reinterpret_cast<const float4*>(Q + col * R) + k);
+        const float4 t = reinterpret_cast<const float4*>(Q + col * R)[k];
         q[4 * k] = t.x; q[4 * k + 1] = t.y; q[4 * k + 2] = t.z; q[4 * k + 3] = t.w;
       }
 #pragma unroll
@@ -798,8 +805,8 @@ add_project_kernel(const float* __restrict__ grad, const float* __restrict__ res
           a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (g0 + k < rows) {
             if (e + 3 < N) {
-              a[k] = __ldg(reinterpret_cast<const float4*>(grad + e));
-              b[k] = __ldg(reinterpret_cast<const float4*>(residual + e));
+              a[k] = *reinterpret_cast<const float4*>(grad + e);
+              b[k] = *reinterpret_cast<const float4*>(residual + e);
             } else {   // past the gradient the matrix keeps what it holds
               float* x = reinterpret_cast<float*>(&a[k]);
               float* y = reinterpret_cast<float*>(&b[k]);
@@ -922,7 +929,7 @@ bool psgd_add_project_eligible(const float* grad, const float* residual, const f
 }
 
 cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m,
-                             const float* Q, int r, float* P, cudaStream_t stream) {
+                             const float* Q, int r, float* P, cudaStream_t stream, bool overlap) {
   if (n < 1 || m < 1 || N < 0 || N > n * m || !psgd_add_project_eligible(grad, residual, Mat, Q, m, r))
     return cudaErrorInvalidValue;
   // two resident CTAs per SM; columns in steps of 1,024 (one per thread of a CTA, four wide)
@@ -939,16 +946,9 @@ cudaError_t psgd_add_project(const float* grad, const float* residual, int64_t N
     const cudaError_t e = cudaMemsetAsync(P, 0, size_t(n) * r * sizeof(float), stream);
     if (e != cudaSuccess) return e;
   }
-#define HP_ADD_PROJECT(RR) \
-  add_project_kernel<RR><<<grid, 256, 0, stream>>>(grad, residual, N, Mat, n, m, Q, P, cols, rows_per, int(at_once))
-  switch (r) {
-    case 1: HP_ADD_PROJECT(1); break;
-    case 2: HP_ADD_PROJECT(2); break;
-    case 4: HP_ADD_PROJECT(4); break;
-    default: HP_ADD_PROJECT(8); break;
-  }
-#undef HP_ADD_PROJECT
-  return cudaGetLastError();
+  auto kernel = r == 1 ? add_project_kernel<1> : (r == 2 ? add_project_kernel<2> : (r == 4 ? add_project_kernel<4> : add_project_kernel<8>));
+  return launch_with(overlap && grid.y == 1, 1, kernel, grid, dim3(256), 0, stream, grad, residual, N, Mat, n, m, Q, P, cols, rows_per,
+                     int(at_once));
 }
 
 int64_t psgd_kpad(int64_t k) { return (k + kKPad - 1) / kKPad * kKPad; }
@@ -1255,20 +1255,20 @@ cudaError_t gram_schmidt(float* P, int64_t n, int r, float eps, cudaStream_t str
 }
 
 cudaError_t gram_schmidt_for_projection(float* P, int64_t n, int r, float eps, float* Xt, int64_t rows_pad, float* zeros,
-                                        int64_t zero_count, cudaStream_t stream) {
+                                        int64_t zero_count, cudaStream_t stream, bool overlap) {
   if (n < 1 || r < 1 || r > kBN || zero_count < 0 || (Xt != nullptr && rows_pad < n)) return cudaErrorInvalidValue;
   const int64_t side = std::max<int64_t>(zero_count, Xt != nullptr ? (kBN - r) * rows_pad + (rows_pad - n) * r : 0);
   const int64_t blocks = std::min<int64_t>((side + 4 * kGsThreads - 1) / (4 * kGsThreads), 147);
-  gram_schmidt_kernel<<<unsigned(1 + blocks), kGsThreads, 0, stream>>>(P, n, r, eps, Xt, rows_pad, zeros, zero_count);
-  return cudaGetLastError();
+  return launch_with(overlap, 1, gram_schmidt_kernel, dim3(unsigned(1 + blocks)), dim3(kGsThreads), 0, stream, P, n, r, eps, Xt, rows_pad,
+                     zeros, zero_count);
 }
 
 cudaError_t psgd_expand_residual(const float* P, const float* Q, int64_t n, int64_t m, int r,
                                  float* Mat, float* residual, float* grad, int64_t N, int mode,
-                                 float post_scale, cudaStream_t stream) {
+                                 float post_scale, cudaStream_t stream, bool overlap) {
   if (n < 1 || m < 1 || r < 1 || r > kBN || N > n * m) return cudaErrorInvalidValue;
-  if (mode == 0 ? launch_expand_rows<0>(P, Q, n, m, r, Mat, residual, grad, N, post_scale, SgdApply{}, stream)
-                : launch_expand_rows<1>(P, Q, n, m, r, Mat, residual, grad, N, post_scale, SgdApply{}, stream))
+  if (mode == 0 ? launch_expand_rows<0>(P, Q, n, m, r, Mat, residual, grad, N, post_scale, SgdApply{}, stream, overlap)
+                : launch_expand_rows<1>(P, Q, n, m, r, Mat, residual, grad, N, post_scale, SgdApply{}, stream, overlap))
     return cudaGetLastError();
   int64_t blocks = (n * m + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;

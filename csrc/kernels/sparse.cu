@@ -1291,7 +1291,7 @@ struct TileProbes {
 };
 __device__ __forceinline__ int64_t probe_step(uint32_t guess) { return 1 + int64_t(sqrtf(float(guess)) * 0.125f); }
 // guess: entries that fit the slot; no position from there on is read, whatever the header will say.
-__device__ __forceinline__ void first_probes(const uint32_t* __restrict__ idx, uint32_t guess, float inv_n,
+__device__ __forceinline__ void first_probes(const uint32_t* idx, uint32_t guess, float inv_n,
                                              const int64_t (&x)[2], int lane, TileProbes& p) {
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
@@ -1301,7 +1301,7 @@ __device__ __forceinline__ void first_probes(const uint32_t* __restrict__ idx, u
 }
 // Whole warp.  For each end x the first position whose index is not below it lies between two places that
 // depend on x, k and the payload alone; they are brought within `slack` of one another, 32 ways at a time.
-__device__ __forceinline__ TileWindow tile_window(const uint32_t* __restrict__ idx, uint32_t k, uint32_t guess,
+__device__ __forceinline__ TileWindow tile_window(const uint32_t* idx, uint32_t k, uint32_t guess,
                                                   const TileProbes& p, const int64_t (&x)[2], uint32_t slack, int lane) {
   uint32_t a[2], len[2];
   const int64_t step0 = probe_step(guess);
@@ -1496,6 +1496,7 @@ __global__ void __launch_bounds__(kThreads, 6)
 dense_tile_kernel(UnpackSources src, float* __restrict__ out, int64_t n, TilePlan plan, float post_scale, int* status,
                   unsigned int* redo) {
   __shared__ __align__(16) float buf[kDenseTile];
+  wait_for_previous();
   let_next_start();
   const int tid = threadIdx.x;
   const int64_t lo = int64_t(blockIdx.x) * plan.tile;
@@ -1807,7 +1808,7 @@ cudaError_t sparse_apply(const UnpackSources& src, int64_t n, float post_scale, 
 }
 
 cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
-                                float post_scale, int* status, cudaStream_t stream, unsigned int* redo) {
+                                float post_scale, int* status, cudaStream_t stream, unsigned int* redo, bool overlap) {
   if (n <= 0 || src.world < 1 || src.world > kMaxWorld) return cudaErrorInvalidValue;
   if (!add && redo != nullptr && n <= 0x7fffffff && src.epoch_dev == nullptr && src.guard == nullptr) {
     for (int r = 0; r < src.world; ++r)
@@ -1820,8 +1821,8 @@ cudaError_t sparse_unpack_accum(const UnpackSources& src, float* out, int64_t n,
     const bool sparse = per_tile <= kSparseTile;
     auto kernel = sparse ? (vec ? dense_tile_kernel<true, true> : dense_tile_kernel<true, false>)
                          : (vec ? dense_tile_kernel<false, true> : dense_tile_kernel<false, false>);
-    kernel<<<blocks, kThreads, 0, stream>>>(src, out, n, plan, post_scale, status, redo);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_with(overlap, 1, kernel, dim3(blocks), dim3(kThreads), 0, stream, src, out, n, plan, post_scale,
+                                      status, redo);
     if (e != cudaSuccess) return e;
     return launch_after(dense_redo_kernel, dim3(148), dim3(kRedoThreads), 0, stream, src, out, n, post_scale, redo);
   }

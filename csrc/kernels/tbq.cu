@@ -13,6 +13,7 @@
 // optionally scales the sum and applies a fused SGD-momentum update.
 #include "../common/codec_math.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "p2p.cuh"
 #include "unpack_lut.cuh"
 
@@ -33,8 +34,9 @@ constexpr int kStageBytes = 512;  // payload bytes a warp gathers before it stor
 // The rest of the tensor (less than one chunk) takes the word path below.
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
-tbq_compress_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n,
+tbq_compress_kernel(const float* grad, float* residual, int64_t n,
                     float thr, PushTargets dst, int wide) {
+  wait_for_previous();
   if (push_guarded(dst)) return;
   resolve_epoch(dst);
   const int64_t S = dst.shard_elems;
@@ -60,7 +62,7 @@ tbq_compress_kernel(const float* __restrict__ grad, float* __restrict__ residual
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int64_t q = (ebase >> 2) + (j0 + u) * 32 + lane;
-          gv[u] = __ldg(reinterpret_cast<const float4*>(grad) + q);
+          gv[u] = reinterpret_cast<const float4*>(grad)[q];
           rv[u] = reinterpret_cast<const float4*>(residual)[q];
         }
 #pragma unroll
@@ -101,7 +103,7 @@ tbq_compress_kernel(const float* __restrict__ grad, float* __restrict__ residual
     if (q < nquads) {
       float g[4], r[4];
       if (VEC) {
-        const float4 gv = __ldg(reinterpret_cast<const float4*>(grad) + q);
+        const float4 gv = reinterpret_cast<const float4*>(grad)[q];
         const float4 rv = reinterpret_cast<const float4*>(residual)[q];
         g[0] = gv.x; g[1] = gv.y; g[2] = gv.z; g[3] = gv.w;
         r[0] = rv.x; r[1] = rv.y; r[2] = rv.z; r[3] = rv.w;
@@ -151,6 +153,7 @@ template <bool APPLY, int WORLD>
 __global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 tbq_unpack_index_kernel(UnpackSources src, float thr, float* __restrict__ out, int64_t n, int add, float post_scale,
                         SgdApply apply, int align) {
+  wait_for_previous();
   if (unpack_guarded(src)) return;
   resolve_epoch(src);
   extern __shared__ __align__(16) float smem[];
@@ -184,7 +187,7 @@ tbq_unpack_lut_kernel(UnpackSources src, float thr, float* __restrict__ out, int
 
 template <bool APPLY, int WORLD>
 cudaError_t launch_tbq_index(const UnpackSources& src, float thr, float* out, int64_t n, int add, float post_scale,
-                             const SgdApply& apply, cudaStream_t stream) {
+                             const SgdApply& apply, cudaStream_t stream, bool overlap) {
   using L = IndexLayout<2, WORLD, true, false>;
   if (L::kBytes > 40 * 1024) {   // past the default limit; set on every launch rather than remembered per process
     const cudaError_t e = cudaFuncSetAttribute(tbq_unpack_index_kernel<APPLY, WORLD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -192,9 +195,8 @@ cudaError_t launch_tbq_index(const UnpackSources& src, float thr, float* out, in
     if (e != cudaSuccess) return e;
   }
   const int grid = index_grid(n, IndexForm<2>::kChunk, WORLD, L::kBytes);
-  tbq_unpack_index_kernel<APPLY, WORLD><<<grid, index_threads(WORLD), L::kBytes, stream>>>(
-      src, thr, out, n, add, post_scale, apply, payload_alignment(src, 0));
-  return cudaGetLastError();
+  return launch_with(overlap, 1, tbq_unpack_index_kernel<APPLY, WORLD>, dim3(grid), dim3(index_threads(WORLD)), L::kBytes, stream,
+                     src, thr, out, n, add, post_scale, apply, payload_alignment(src, 0));
 }
 
 inline int grid_for(int64_t items, int threads, int max_blocks) {
@@ -209,7 +211,7 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 }  // namespace
 
 cudaError_t tbq_compress(const float* grad, float* residual, int64_t n, float threshold,
-                         const PushTargets& dst, cudaStream_t stream) {
+                         const PushTargets& dst, cudaStream_t stream, bool overlap) {
   if (n <= 0) return cudaErrorInvalidValue;
   const bool vec = aligned16(grad) && aligned16(residual);
   const int64_t S = dst.shard_elems;
@@ -224,16 +226,13 @@ cudaError_t tbq_compress(const float* grad, float* residual, int64_t n, float th
   const int threads = wide ? 128 : kThreads;
   // word path: 148 SMs x 8 resident CTAs of 256 threads
   const int grid = wide ? grid_for(chunks * 32, threads, 148 * 16) : grid_for(n >> 2, kThreads, 148 * 8);
-  if (vec)
-    tbq_compress_kernel<true><<<grid, threads, 0, stream>>>(grad, residual, n, threshold, dst, wide);
-  else
-    tbq_compress_kernel<false><<<grid, threads, 0, stream>>>(grad, residual, n, threshold, dst, wide);
-  return cudaGetLastError();
+  return launch_with(overlap, 1, vec ? tbq_compress_kernel<true> : tbq_compress_kernel<false>, dim3(grid), dim3(threads), 0,
+                     stream, grad, residual, n, threshold, dst, wide);
 }
 
 cudaError_t tbq_unpack_accum(const UnpackSources& src, float threshold, float* out, int64_t n,
                              int add, float post_scale, const SgdApply& apply,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, bool overlap) {
   if (n <= 0 || src.world < 1 || src.world > kMaxWorld) return cudaErrorInvalidValue;
   if (src.shard_elems > 0) {
     // concatenated shards: 16-byte aligned dense arrays only
@@ -248,8 +247,8 @@ cudaError_t tbq_unpack_accum(const UnpackSources& src, float threshold, float* o
 #define HP_INDEX(W)                                                                                               \
   case W:                                                                                                         \
     return apply.param != nullptr                                                                                 \
-               ? launch_tbq_index<true, W>(src, threshold, out, n, add, post_scale, apply, stream)                \
-               : launch_tbq_index<false, W>(src, threshold, out, n, add, post_scale, apply, stream)
+               ? launch_tbq_index<true, W>(src, threshold, out, n, add, post_scale, apply, stream, overlap)                \
+               : launch_tbq_index<false, W>(src, threshold, out, n, add, post_scale, apply, stream, overlap)
     switch (src.world) {
       HP_INDEX(1); HP_INDEX(2); HP_INDEX(3); HP_INDEX(4); HP_INDEX(5); HP_INDEX(6); HP_INDEX(7); HP_INDEX(8);
     }

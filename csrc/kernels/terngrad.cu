@@ -59,8 +59,8 @@ __device__ __forceinline__ void put_header(const PushTargets& dst, const PushCur
 
 template <bool VEC, bool EF>
 __global__ void __launch_bounds__(kThreads)
-minmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ residual, int64_t n,
-                     int bw, PushTargets dst, MinMaxScratch* scratch) {
+minmax_header_kernel(const float* grad, const float* residual, int64_t n, int bw, PushTargets dst, MinMaxScratch* scratch) {
+  wait_for_previous();
   if (push_guarded(dst)) return;
   resolve_epoch(dst);
   // scatter mode: blockIdx.y is the shard; each shard has its own reduction state and header
@@ -93,15 +93,15 @@ minmax_header_kernel(const float* __restrict__ grad, const float* __restrict__ r
       float4 g[4], r[4] = {};
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        g[u] = __ldg(reinterpret_cast<const float4*>(grad) + i + u * stride);
-        if (EF) r[u] = __ldg(reinterpret_cast<const float4*>(residual) + i + u * stride);
+        g[u] = reinterpret_cast<const float4*>(grad)[i + u * stride];
+        if (EF) r[u] = reinterpret_cast<const float4*>(residual)[i + u * stride];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) fold(g[u], r[u]);
     }
     for (; i < nv; i += stride)
-      fold(__ldg(reinterpret_cast<const float4*>(grad) + i),
-           EF ? __ldg(reinterpret_cast<const float4*>(residual) + i) : make_float4(0.f, 0.f, 0.f, 0.f));
+      fold(reinterpret_cast<const float4*>(grad)[i],
+           EF ? reinterpret_cast<const float4*>(residual)[i] : make_float4(0.f, 0.f, 0.f, 0.f));
     for (int64_t i = (nv << 2) + tid; i < n; i += stride) {
       const float v = EF ? hp_add(grad[i], residual[i]) : grad[i];
       mn = fminf(mn, v);
@@ -380,8 +380,8 @@ constexpr int kSmallCtas = 8, kSmallThreads = 1024, kSmallPerThread = 16;
 constexpr int64_t kSmallElems = int64_t(kSmallCtas) * kSmallThreads * kSmallPerThread;
 template <int BW, bool VEC, bool EF>
 __global__ void __cluster_dims__(kSmallCtas, 1, 1) __launch_bounds__(kSmallThreads)
-tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int random, uint64_t seed,
-                  PushTargets dst) {
+tern_small_kernel(const float* grad, float* residual, int64_t n, int random, uint64_t seed, PushTargets dst) {
+  wait_for_previous();
   constexpr int EPT = Unit<BW>::EPT, BPT = Unit<BW>::BPT, UPT = kSmallPerThread / EPT;
   __shared__ float ext_mn[kSmallCtas], ext_mx[kSmallCtas], scale[4];
   const cg::cluster_group cluster = cg::this_cluster();
@@ -397,7 +397,7 @@ tern_small_kernel(const float* __restrict__ grad, float* __restrict__ residual, 
       if (VEC) {
 #pragma unroll
         for (int v = 0; v < EPT / 4; ++v) {
-          float4 g = __ldg(reinterpret_cast<const float4*>(grad + u * EPT) + v);
+          float4 g = reinterpret_cast<const float4*>(grad + u * EPT)[v];
           if (EF) {
             const float4 r = reinterpret_cast<const float4*>(residual + u * EPT)[v];
             g.x = hp_add(g.x, r.x); g.y = hp_add(g.y, r.y);
@@ -624,6 +624,7 @@ template <int BW, bool APPLY, int WORLD>
 __global__ void __launch_bounds__(index_threads(WORLD), index_ctas(WORLD))
 tern_unpack_index_kernel(UnpackSources src, float* __restrict__ out, int64_t n, int add, float post_scale, SgdApply apply,
                          int* status, int align) {
+  wait_for_previous();
   if (unpack_guarded(src)) return;
   resolve_epoch(src);
   extern __shared__ __align__(16) float smem[];
@@ -709,7 +710,7 @@ tern_unpack_lut_kernel(UnpackSources src, float* __restrict__ out, int64_t n, in
 
 template <int BW, bool APPLY, int WORLD>
 cudaError_t launch_tern_index(const UnpackSources& src, float* out, int64_t n, int add, float post_scale,
-                              const SgdApply& apply, int* status, cudaStream_t stream) {
+                              const SgdApply& apply, int* status, cudaStream_t stream, bool overlap) {
   const int align = payload_alignment(src, kTernHeaderBytes);
   int grid = grid_for((n + 3) >> 2, index_threads(WORLD), 148 * 8);
   size_t smem = 0;
@@ -725,14 +726,13 @@ cudaError_t launch_tern_index(const UnpackSources& src, float* out, int64_t n, i
       if (e != cudaSuccess) return e;
     }
   }
-  tern_unpack_index_kernel<BW, APPLY, WORLD><<<grid, index_threads(WORLD), smem, stream>>>(src, out, n, add, post_scale, apply,
-                                                                                  status, align);
-  return cudaGetLastError();
+  return launch_with(overlap, 1, tern_unpack_index_kernel<BW, APPLY, WORLD>, dim3(grid), dim3(index_threads(WORLD)), smem, stream, src,
+                     out, n, add, post_scale, apply, status, align);
 }
 
 template <int BW, bool APPLY>
 cudaError_t launch_tern_unpack(const UnpackSources& src, float* out, int64_t n, int add, float post_scale,
-                               const SgdApply& apply, int* status, cudaStream_t stream) {
+                               const SgdApply& apply, int* status, cudaStream_t stream, bool overlap) {
   bool aligned = aligned16(out);
   if (APPLY) aligned = aligned && aligned16(apply.param) && aligned16(apply.momentum);
   if constexpr (BW == 2) {
@@ -744,7 +744,7 @@ cudaError_t launch_tern_unpack(const UnpackSources& src, float* out, int64_t n, 
   }
   if constexpr (BW > 0) {
     if (aligned) {
-#define HP_INDEX(W) case W: return launch_tern_index<BW, APPLY, W>(src, out, n, add, post_scale, apply, status, stream)
+#define HP_INDEX(W) case W: return launch_tern_index<BW, APPLY, W>(src, out, n, add, post_scale, apply, status, stream, overlap)
       switch (src.world) {
         HP_INDEX(1); HP_INDEX(2); HP_INDEX(3); HP_INDEX(4); HP_INDEX(5); HP_INDEX(6); HP_INDEX(7); HP_INDEX(8);
         default: return cudaErrorInvalidValue;
@@ -774,7 +774,8 @@ size_t minmax_scratch_bytes() { return sizeof(MinMaxScratch); }
 
 cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int bitwidth,
                               int enable_random, uint64_t seed, const PushTargets& dst,
-                              void* scratch, cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns) {
+                              void* scratch, cudaStream_t stream, bool whole_gpu, int* status, uint64_t grid_wait_ns,
+                              bool overlap) {
   if (n <= 0 || !tern_bitwidth_ok(bitwidth) || scratch == nullptr) return cudaErrorInvalidValue;
   auto* s = static_cast<MinMaxScratch*>(scratch);
   const bool ef = residual != nullptr;
@@ -802,10 +803,11 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
   const bool own = hold_alone(whole_gpu, dst);
   if (own && n <= kSmallElems) {
 #define LAUNCH_SMALL(BW, V, E) \
-  tern_small_kernel<BW, V, E><<<kSmallCtas, kSmallThreads, 0, stream>>>(grad, residual, n, enable_random, seed, dst)
+  return launch_with(overlap, 1, tern_small_kernel<BW, V, E>, dim3(kSmallCtas), dim3(kSmallThreads), 0, stream, grad, residual, n, \
+                     enable_random, seed, dst)   /* its clusters are part of the kernel */
     LAUNCH_BITS(LAUNCH_SMALL);
 #undef LAUNCH_SMALL
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
   }
   // 16-byte aligned inputs, and a part per SM that fits its shared memory: one read of them
   if (own && status != nullptr && vec && shift >= 0) {
@@ -842,13 +844,10 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
     int gx = grid_for((per + 3) >> 2, kThreads, 148 * 4);
     if (shards > 1) gx = std::min(gx, std::max(1, (148 * 4 + shards - 1) / shards));
     const dim3 grid(gx, shards);
-#define LAUNCH(V, E) \
-  minmax_header_kernel<V, E><<<grid, kThreads, 0, stream>>>(grad, residual, n, bitwidth, hdr_dst, s)
-    if (vec && ef) LAUNCH(true, true);
-    else if (vec) LAUNCH(true, false);
-    else if (ef) LAUNCH(false, true);
-    else LAUNCH(false, false);
-#undef LAUNCH
+    auto minmax = vec ? (ef ? minmax_header_kernel<true, true> : minmax_header_kernel<true, false>)
+                      : (ef ? minmax_header_kernel<false, true> : minmax_header_kernel<false, false>);
+    const cudaError_t e = launch_with(overlap, 1, minmax, grid, dim3(kThreads), 0, stream, grad, residual, n, bitwidth, hdr_dst, s);
+    if (e != cudaSuccess) return e;
   }
   {
     // chunked path with 16-byte stores once there is a chunk per warp of a half-filled GPU
@@ -873,7 +872,7 @@ cudaError_t terngrad_compress(const float* grad, float* residual, int64_t n, int
 
 cudaError_t terngrad_unpack_accum(const UnpackSources& src, float* out, int64_t n, int add,
                                   float post_scale, const SgdApply& apply, int* status,
-                                  cudaStream_t stream, int bitwidth_hint) {
+                                  cudaStream_t stream, int bitwidth_hint, bool overlap) {
   if (n <= 0 || src.world < 1 || src.world > kMaxWorld) return cudaErrorInvalidValue;
   if (bitwidth_hint != 0 && !tern_bitwidth_ok(bitwidth_hint)) return cudaErrorInvalidValue;
   if (src.shard_elems > 0) {
@@ -885,8 +884,8 @@ cudaError_t terngrad_unpack_accum(const UnpackSources& src, float* out, int64_t 
   }
   const bool ap = apply.param != nullptr;
 #define HP_UNPACK(BW) \
-  (ap ? launch_tern_unpack<BW, true>(src, out, n, add, post_scale, apply, status, stream) \
-      : launch_tern_unpack<BW, false>(src, out, n, add, post_scale, apply, status, stream))
+  (ap ? launch_tern_unpack<BW, true>(src, out, n, add, post_scale, apply, status, stream, overlap) \
+      : launch_tern_unpack<BW, false>(src, out, n, add, post_scale, apply, status, stream, overlap))
   switch (bitwidth_hint) {
     case 1: return HP_UNPACK(1);
     case 2: return HP_UNPACK(2);

@@ -436,15 +436,15 @@ struct PayloadWords {
     if (align == 4) {
 #pragma unroll
       for (int r = 0; r < WORLD; ++r) {
-        lo[r] = __ldg(reinterpret_cast<const uint32_t*>(src.payload[r] + at));
+        lo[r] = *reinterpret_cast<const uint32_t*>(src.payload[r] + at);
         hi[r] = 0;
       }
     } else if (align == 2) {
 #pragma unroll
       for (int r = 0; r < WORLD; ++r) {
         const uint16_t* p = reinterpret_cast<const uint16_t*>(src.payload[r] + at);
-        lo[r] = __ldg(p);
-        hi[r] = __ldg(p + 1);
+        lo[r] = p[0];
+        hi[r] = p[1];
       }
     } else {
 #pragma unroll

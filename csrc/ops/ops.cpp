@@ -77,6 +77,12 @@ void cpu_accumulate(size_t world, int64_t n, float* out, bool add, double post_s
     for (int64_t i = 0; i < n; ++i) out[i] = hp_mul(out[i], float(post_scale));
 }
 
+// Whether a call's first kernel may overlap the end of what the stream holds (launch.cuh).
+bool may_overlap(cudaStream_t stream) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+}
+
 // Places in a stream's scratch (see scratch_for): the min/max state of the quantisers at 0, the
 // sum of squares of DGC's clipping, and from 16,384 the sparse state.
 constexpr size_t kSumsqOffset = 12288, kSparseOffset = 16384;
@@ -173,9 +179,9 @@ void tbq_compress(const torch::Tensor& grad, torch::Tensor residual, torch::Tens
   if (n == 0) return;
   if (grad.is_cuda()) {
     c10::cuda::CUDAGuard guard(grad.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::tbq_compress(grad.data_ptr<float>(), residual.data_ptr<float>(), n,
-                                     float(threshold), local_target(out),
-                                     at::cuda::getCurrentCUDAStream()));
+                                     float(threshold), local_target(out), stream, may_overlap(stream)));
   } else {
     cpu::tbq_compress(grad.data_ptr<float>(), residual.data_ptr<float>(), n, float(threshold),
                       out.data_ptr<uint8_t>());
@@ -193,9 +199,10 @@ void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
   }
   if (out.is_cuda()) {
     c10::cuda::CUDAGuard guard(out.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::tbq_unpack_accum(sources_of(payloads, out), float(threshold),
                                          out.data_ptr<float>(), n, add ? 1 : 0, float(post_scale),
-                                         cuda::SgdApply{}, at::cuda::getCurrentCUDAStream()));
+                                         cuda::SgdApply{}, stream, may_overlap(stream)));
   } else {
     TORCH_CHECK(!payloads.empty() && payloads.size() <= size_t(cuda::kMaxWorld),
                 "between 1 and ", cuda::kMaxWorld, " payloads expected");
@@ -228,10 +235,11 @@ static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int6
   if (grad.is_cuda()) {
     c10::cuda::CUDAGuard guard(grad.device());
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::terngrad_compress(grad.data_ptr<float>(), res, n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed), local_target(out),
-                                          scratch, at::cuda::getCurrentCUDAStream(), whole_gpu,
-                                          whole_gpu ? status_word_for(grad) : nullptr));
+                                          scratch, stream, whole_gpu, whole_gpu ? status_word_for(grad) : nullptr,
+                                          cuda::kGridWaitNs, may_overlap(stream)));
   } else {
     const int rc = cpu::terngrad_compress(grad.data_ptr<float>(), n, int(bitwidth),
                                           enable_random ? 1 : 0, uint64_t(seed),
@@ -268,10 +276,10 @@ void terngrad_decompress(const std::vector<torch::Tensor>& payloads, torch::Tens
   TORCH_CHECK(n > 0, "empty tensor");
   if (out.is_cuda()) {
     c10::cuda::CUDAGuard guard(out.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::terngrad_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
                                               add ? 1 : 0, float(post_scale), cuda::SgdApply{},
-                                              status_word_for(out),
-                                              at::cuda::getCurrentCUDAStream(), int(bitwidth)));
+                                              status_word_for(out), stream, int(bitwidth), may_overlap(stream)));
   } else {
     TORCH_CHECK(!payloads.empty() && payloads.size() <= size_t(cuda::kMaxWorld),
                 "between 1 and ", cuda::kMaxWorld, " payloads expected");
@@ -361,12 +369,11 @@ static void sparse_decompress(const std::vector<torch::Tensor>& payloads, torch:
     auto stream = at::cuda::getCurrentCUDAStream();
     // The one-pass decode shares two words with the stream's other decodes: its launches must not mix with
     // theirs.  A captured graph may run beside later calls on the stream, and takes the form without them.
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    HP_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
-    unsigned int* redo = tiles && !add && capture == cudaStreamCaptureStatusNone ? redo_words_for(out) : nullptr;
+    const bool overlap = may_overlap(stream);   // no capture
+    unsigned int* redo = tiles && !add && overlap ? redo_words_for(out) : nullptr;
     std::lock_guard<std::mutex> one_at_a_time(state().decode);
     HP_CHECK_CUDA(cuda::sparse_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
-                                            add ? 1 : 0, float(post_scale), status_word_for(out), stream, redo));
+                                            add ? 1 : 0, float(post_scale), status_word_for(out), stream, redo, overlap));
   } else {
     TORCH_CHECK(!payloads.empty(), "at least one payload expected");
     if (!add) out.zero_();
@@ -416,10 +423,11 @@ void ecq_compress(const torch::Tensor& grad, torch::Tensor history, torch::Tenso
   if (grad.is_cuda()) {
     c10::cuda::CUDAGuard guard(grad.device());
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::ecq_compress(grad.data_ptr<float>(), history.data_ptr<float>(), n,
                                      float(alpha), float(beta), int(bitwidth), uint64_t(seed),
-                                     local_target(out), scratch, at::cuda::getCurrentCUDAStream(),
-                                     /*whole_gpu=*/true, status_word_for(grad)));
+                                     local_target(out), scratch, stream, /*whole_gpu=*/true, status_word_for(grad),
+                                     cuda::kGridWaitNs, may_overlap(stream)));
   } else {
     const int rc = cpu::ecq_compress(grad.data_ptr<float>(), history.data_ptr<float>(), n,
                                      float(alpha), float(beta), int(bitwidth), uint64_t(seed),
@@ -435,9 +443,9 @@ void ecq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
   TORCH_CHECK(n > 0, "empty tensor");
   if (out.is_cuda()) {
     c10::cuda::CUDAGuard guard(out.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::ecq_unpack_accum(sources_of(payloads, out), out.data_ptr<float>(), n,
-                                         add ? 1 : 0, float(post_scale), status_word_for(out),
-                                         at::cuda::getCurrentCUDAStream()));
+                                         add ? 1 : 0, float(post_scale), status_word_for(out), stream, may_overlap(stream)));
   } else {
     TORCH_CHECK(!payloads.empty(), "at least one payload expected");
     for (size_t r = 0; r < payloads.size(); ++r) {
@@ -672,9 +680,10 @@ void powersgd_encode1(const torch::Tensor& grad, const torch::Tensor& residual,
     c10::cuda::CUDAGuard guard(M.device());
     if (cuda::psgd_add_project_eligible(grad.data_ptr<float>(), residual.data_ptr<float>(), M.data_ptr<float>(),
                                         Q.data_ptr<float>(), s.m, int(s.r))) {
+      const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
       HP_CHECK_CUDA(cuda::psgd_add_project(grad.data_ptr<float>(), residual.data_ptr<float>(), N, M.data_ptr<float>(),
-                                           s.n, s.m, Q.data_ptr<float>(), int(s.r), P.data_ptr<float>(),
-                                           at::cuda::getCurrentCUDAStream()));
+                                           s.n, s.m, Q.data_ptr<float>(), int(s.r), P.data_ptr<float>(), stream,
+                                           may_overlap(stream)));
       return;
     }
     HP_CHECK_CUDA(cuda::add_into(grad.data_ptr<float>(), residual.data_ptr<float>(),
@@ -697,7 +706,7 @@ void powersgd_encode2(torch::Tensor P, const torch::Tensor& M, torch::Tensor Q) 
     if (cuda::psgd_tensor_core_eligible(M.data_ptr<float>(), s.n, s.m)) xt = torch::empty({16, kp}, M.options());
     float* xt_ptr = xt.defined() ? xt.data_ptr<float>() : nullptr;
     HP_CHECK_CUDA(cuda::gram_schmidt_for_projection(P.data_ptr<float>(), s.n, int(s.r), 1e-8f, xt_ptr, kp,
-                                                    Q.data_ptr<float>(), Q.numel(), stream));
+                                                    Q.data_ptr<float>(), Q.numel(), stream, may_overlap(stream)));
     cuda::ReduceTargets red;
     red.world = 1;
     red.dst[0] = Q.data_ptr<float>();
@@ -717,10 +726,10 @@ void powersgd_decode(const torch::Tensor& P, const torch::Tensor& Q, torch::Tens
   TORCH_CHECK(residual.numel() == N && N <= s.n * s.m, "grad/residual must fit in M");
   if (M.is_cuda()) {
     c10::cuda::CUDAGuard guard(M.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::psgd_expand_residual(P.data_ptr<float>(), Q.data_ptr<float>(), s.n, s.m,
                                              int(s.r), M.data_ptr<float>(), residual.data_ptr<float>(),
-                                             grad.data_ptr<float>(), N, 0, 1.0f,
-                                             at::cuda::getCurrentCUDAStream()));
+                                             grad.data_ptr<float>(), N, 0, 1.0f, stream, may_overlap(stream)));
   } else {
     cpu::powersgd_decode(P.data_ptr<float>(), Q.data_ptr<float>(), s.n, s.m, s.r, M.data_ptr<float>(),
                          residual.data_ptr<float>(), grad.data_ptr<float>(), N);

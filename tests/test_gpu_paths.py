@@ -615,3 +615,48 @@ def test_engine_counts_the_kernels_it_launches(codec, n, kw):
         out = torch.zeros(ops.sparse_payload_bytes(n, 1 - (1 - kw["keep_fraction"])), dtype=torch.uint8, device="cuda")
         want = kernels_of(lambda: ops.graddrop_compress(grad, res, kw["sample_rate"], 1 - kw["keep_fraction"], 3, out=out))
     assert push_launches(codec, **kw) == want
+
+
+# ----------------------------------------------------------------------------- calls that overlap the kernel before them
+@pytest.mark.parametrize("n", [4096, 200000, 3000001])
+@pytest.mark.parametrize("codec", ["tbq", "terngrad", "ecq", "graddrop"])
+def test_calls_behind_one_another_and_behind_other_kernels(codec, n):
+    """A pass is three kernels of PyTorch's and two calls, ten passes without a wait between them; every input is
+    written just before it is read, over what the pass before read."""
+    world = 2
+    grads = [gauss(n, seed=s) for s in range(10)]
+    dev = [g.cuda() for g in grads]
+    grad, state, dense = torch.empty(n, device="cuda"), torch.zeros(n, device="cuda"), torch.empty(n, device="cuda")
+    other = torch.zeros(n)
+
+    def call(grad, state, dense, payloads):
+        if codec == "tbq":
+            ops.tbq_compress(grad, state, 0.01, out=payloads[0])
+            ops.tbq_decompress(payloads, dense, 0.01, post_scale=0.5)
+        elif codec == "terngrad":
+            ops.terngrad_compress(grad, 2, True, 3, state, out=payloads[0])
+            ops.terngrad_decompress(payloads, dense, post_scale=0.5, bitwidth=2)
+        elif codec == "ecq":
+            ops.ecq_compress(grad, state, 1.0, 0.9, 4, 3, out=payloads[0])
+            ops.ecq_decompress(payloads, dense, post_scale=0.5)
+        else:
+            ops.graddrop_compress(grad, state, 0.05, 0.99, 3, out=payloads[0])
+            ops.sparse_decompress(payloads, dense, post_scale=0.5)
+
+    size = {"tbq": ops.tbq_payload_bytes(n), "terngrad": ops.terngrad_payload_bytes(n, 2),
+            "ecq": ops.ecq_payload_bytes(n, 4), "graddrop": ops.sparse_payload_bytes(n, 1.0 - 0.99)}[codec]
+    host = [torch.zeros(size, dtype=torch.uint8) for _ in range(world)]
+    call(gauss(n, seed=77), other, torch.empty(n), [host[1], host[1]])
+    payloads = [torch.zeros(size, dtype=torch.uint8, device="cuda"), host[1].cuda()]
+    results = []
+    torch.cuda.synchronize()
+    for g in dev:
+        grad.copy_(g)
+        grad.mul_(2.0)
+        call(grad, state, dense, payloads)
+        results.append(dense.clone())
+    state_host, dense_host = torch.zeros(n), torch.empty(n)
+    for g, got in zip(grads, results):
+        call(g * 2.0, state_host, dense_host, host)
+        assert torch.equal(got.cpu(), dense_host)
+    assert torch.equal(state.cpu(), state_host)
