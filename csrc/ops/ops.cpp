@@ -35,10 +35,11 @@ void check_same_device(const torch::Tensor& a, const torch::Tensor& b) {
   TORCH_CHECK(a.device() == b.device(), "tensors must be on the same device");
 }
 
-cuda::PushTargets local_target(torch::Tensor& out) {
+cuda::PushTargets local_target(torch::Tensor& out, uint8_t* second = nullptr) {
   cuda::PushTargets t;
-  t.world = 1;
+  t.world = second != nullptr ? 2 : 1;
   t.payload[0] = out.data_ptr<uint8_t>();
+  t.payload[1] = second;
   return t;
 }
 
@@ -166,8 +167,8 @@ int64_t ecq_payload_bytes(int64_t n, int64_t bw) {
 }
 
 // ------------------------------------------------------------------ TBQ
-void tbq_compress(const torch::Tensor& grad, torch::Tensor residual, torch::Tensor out,
-                  double threshold) {
+void tbq_compress_beside(const torch::Tensor& grad, torch::Tensor residual, torch::Tensor out,
+                         double threshold, uint8_t* host) {
   check_f32(grad, "grad");
   check_f32(residual, "residual");
   check_u8(out, "out");
@@ -181,11 +182,16 @@ void tbq_compress(const torch::Tensor& grad, torch::Tensor residual, torch::Tens
     c10::cuda::CUDAGuard guard(grad.device());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::tbq_compress(grad.data_ptr<float>(), residual.data_ptr<float>(), n,
-                                     float(threshold), local_target(out), stream, may_overlap(stream)));
+                                     float(threshold), local_target(out, host), stream, may_overlap(stream)));
   } else {
     cpu::tbq_compress(grad.data_ptr<float>(), residual.data_ptr<float>(), n, float(threshold),
                       out.data_ptr<uint8_t>());
   }
+}
+
+void tbq_compress(const torch::Tensor& grad, torch::Tensor residual, torch::Tensor out,
+                  double threshold) {
+  tbq_compress_beside(grad, residual, out, threshold, nullptr);
 }
 
 void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, double threshold,
@@ -216,7 +222,7 @@ void tbq_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor ou
 
 // ------------------------------------------------------------------ TernGrad
 static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
-                              int64_t seed, c10::optional<torch::Tensor> residual, bool whole_gpu) {
+                              int64_t seed, c10::optional<torch::Tensor> residual, bool whole_gpu, uint8_t* host) {
   check_f32(grad, "grad");
   check_u8(out, "out");
   check_same_device(grad, out);
@@ -237,7 +243,7 @@ static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int6
     void* scratch = scratch_for(grad, cuda::minmax_scratch_bytes());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
     HP_CHECK_CUDA(cuda::terngrad_compress(grad.data_ptr<float>(), res, n, int(bitwidth),
-                                          enable_random ? 1 : 0, uint64_t(seed), local_target(out),
+                                          enable_random ? 1 : 0, uint64_t(seed), local_target(out, host),
                                           scratch, stream, whole_gpu, whole_gpu ? status_word_for(grad) : nullptr,
                                           cuda::kGridWaitNs, may_overlap(stream)));
   } else {
@@ -250,7 +256,7 @@ static void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int6
 
 void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth,
                        bool enable_random, int64_t seed, c10::optional<torch::Tensor> residual) {
-  terngrad_compress(grad, out, bitwidth, enable_random, seed, residual, /*whole_gpu=*/true);
+  terngrad_compress(grad, out, bitwidth, enable_random, seed, residual, /*whole_gpu=*/true, nullptr);
 }
 
 int64_t terngrad_resident_wait(const torch::Tensor& grad, torch::Tensor out, torch::Tensor scratch, int64_t wait_us) {
@@ -265,8 +271,8 @@ int64_t terngrad_resident_wait(const torch::Tensor& grad, torch::Tensor out, tor
 }
 
 void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
-                              int64_t seed) {
-  terngrad_compress(grad, out, bitwidth, enable_random, seed, c10::nullopt, /*whole_gpu=*/false);
+                              int64_t seed, uint8_t* host) {
+  terngrad_compress(grad, out, bitwidth, enable_random, seed, c10::nullopt, /*whole_gpu=*/false, host);
 }
 
 void terngrad_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,

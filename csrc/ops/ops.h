@@ -33,8 +33,10 @@ void terngrad_compress(const torch::Tensor& grad, torch::Tensor out, int64_t bit
 // scratch state of the caller's; returns the status word.
 int64_t terngrad_resident_wait(const torch::Tensor& grad, torch::Tensor out, torch::Tensor scratch, int64_t wait_us);
 // The same for a stream beside which the caller's own work runs: it does not ask for all SMs at once.
+// host: null, or a second place for the payload that the device can store to.
+void tbq_compress_beside(const torch::Tensor& grad, torch::Tensor residual, torch::Tensor out, double threshold, uint8_t* host);
 void terngrad_compress_beside(const torch::Tensor& grad, torch::Tensor out, int64_t bitwidth, bool enable_random,
-                              int64_t seed);
+                              int64_t seed, uint8_t* host);
 // bitwidth: 0 = read it from the payload headers on the device; a known bitwidth selects a kernel
 // compiled for it (payloads with another bitwidth are then rejected through the status word).
 void terngrad_decompress(const std::vector<torch::Tensor>& payloads, torch::Tensor out, bool add,

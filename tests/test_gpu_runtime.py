@@ -209,3 +209,37 @@ def test_graddrop_decode_tasks_do_not_wait_for_a_free_gpu(runtime):
     of_task, of_op = medians_beside_matrix_products(task, op)
     assert torch.equal(out, want)
     assert of_task < 0.75 * of_op
+
+
+@pytest.mark.parametrize("alg", ["tbq", "terngrad"])
+@pytest.mark.parametrize("n", [1, 1003, 4 * ((1 << 20) - 10), 4 * (1 << 20) + 4, 5000001])
+@pytest.mark.parametrize("host", ["pinned", "off_a_word", "pageable", "longer"])
+def test_payload_reaches_the_staging_buffer(runtime, alg, n, host):
+    """Stored by the kernel into pinned memory, up to a size, or copied: B and C hold the same payload, and nothing
+    behind it is touched."""
+    if alg == "tbq":
+        runtime.init("tbq", {"threshold": 0.01}, 0, 0, 1)
+        size = ops.tbq_payload_bytes(n)
+    else:
+        runtime.init("terngrad", {"enable_random": 0, "bitwidth": 2}, 0, 0, 1)
+        size = ops.terngrad_payload_bytes(n, 2)
+    g, r = gauss(n, seed=n), gauss(n, 0.004, seed=n + 1)
+    buf = torch.full((size + 64,), 9, dtype=torch.uint8)
+    if host != "pageable":
+        buf = buf.pin_memory()
+    first = 1 if host == "off_a_word" else 0
+    C = buf[first:first + size + (32 if host == "longer" else 0)]
+    B = torch.zeros(size, dtype=torch.uint8, device="cuda")
+    rc, dev, rg = r.clone(), g.cuda(), r.cuda()
+    if alg == "tbq":
+        want = ops.tbq_compress(g, rc, 0.01)
+        runtime.submit_task("t", dev, rg, B, C, 0, runtime.COMP_TASK)
+    else:
+        want = ops.terngrad_compress(g, 2, False)
+        runtime.submit_task("t", dev, B, C, 0, runtime.COMP_TASK)
+    runtime.wait_for(runtime.COMP_TASK, ["t"])
+    assert torch.equal(C[:size], want) and torch.equal(B.cpu(), want)
+    assert int((buf[:first] != 9).sum()) == 0 and int((buf[first + size:] != 9).sum()) == 0
+    if alg == "tbq":
+        assert torch.equal(rg.cpu(), rc)
+    assert runtime.getErrors() == []
