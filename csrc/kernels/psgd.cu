@@ -768,11 +768,13 @@ bool launch_expand_rows(const float* P, const float* Q, int64_t n, int64_t m, in
 // what the SMs can do in the time the matrix takes to stream, while a second launch reads all of M again
 // (and the tensor cores would round it to tf32).  A CTA owns a range of rows and takes up to 32 / R of them at a
 // time; each thread walks its columns four at a time with the Q rows of those columns in registers, used by all of
-// these rows, and four rows' loads in flight.  Two CTAs fit an SM, and the rows are shared out evenly over that many.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across
-// the warps in shared memory.  Few rows are also split by columns; the parts then meet in P by atomics,
-// which the launcher zeroes first.
-// 4096 x 4096, rank 4, in a chain of calls: 37.8 us, 38.4 as 512 CTAs of eight rows.  (ncu, cold) 32 us so; as add 28.9, zero 2.5, transpose 3.5 and tensor-core projection
-// 15.2.  Error of the three stages against 64 bits 7.4e-4, and 8.4e-4 with the projection in tf32.
+// these rows, and four rows' loads in flight.  Two CTAs fit an SM, and the rows are shared out evenly over that
+// many.  The 32 sums of a thread are reduced across the warp by halving (31 shuffles), then across the warps in
+// shared memory.  Few rows are also split by columns; the parts then meet in P by atomics, which the launcher zeroes
+// first.
+// 4096 x 4096, rank 4, in a chain of calls: 37.8 us, 38.4 as 512 CTAs of eight rows.  Cold, alone: 32 us; as
+// separate launches add 28.9, zero 2.5, transpose 3.5 and tensor-core projection 15.2.  Error of the three stages
+// against 64 bits 7.2e-4, and 8.4e-4 with the projection in tf32.
 template <int R>
 __global__ void __launch_bounds__(256, 2)
 add_project_kernel(const float* grad, const float* residual, int64_t N, float* Mat, int64_t n, int64_t m, const float* Q, float* P,
