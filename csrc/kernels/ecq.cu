@@ -285,6 +285,8 @@ ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t 
   __shared__ EcqScale shared_scale;
   uint8_t* const bytes_at = reinterpret_cast<uint8_t*>(hold + part);
   const int tid = threadIdx.x;
+  GridPlace place;
+  grid_arrive(scratch, place);
   const int64_t begin = int64_t(blockIdx.x) * part;       // a multiple of 512
   const int64_t left = n - begin;
   const int len = int(left < 0 ? 0 : (left < part ? left : part));
@@ -312,7 +314,10 @@ ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t 
   for (; q < quads; q += kHoldThreads) take(q, __ldg(g4 + q), h4[q]);
   for (int e = 4 * quads + tid; e < len; e += kHoldThreads)   // fewer than four
     mx = fmaxf(mx, fabsf(ecq_compensated(grad[begin + e], hist[begin + e], alpha)));
-  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status)) return;
+  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status, place)) {
+    grid_leave(scratch, place);
+    return;
+  }
   if (tid == 0) {
     shared_scale = ecq_scale(mx, BW);
     if (blockIdx.x == 0) ecq_put_header(dst, n, BW, shared_scale.mx);
@@ -354,6 +359,7 @@ ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t 
       for (int j = 0; j < count; ++j) hist[begin + e + j] = h[j];
     }
   }
+  grid_leave(scratch, place);
 }
 
 // Headers of all payloads -> mx, gap, bw (shared memory); false, with the status word set, when one of

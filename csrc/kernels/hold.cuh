@@ -25,7 +25,7 @@ inline cudaError_t hold_plan(int64_t n, int bitwidth, HoldPlan& p) {
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return e;
-  if (sms > kReduceMaxBlocks) sms = kReduceMaxBlocks;
+  if (sms > kResidentMaxBlocks) sms = kResidentMaxBlocks;
   const int64_t part = ((n + sms - 1) / sms + 511) / 512 * 512;
   p.smem = size_t(part) * sizeof(float) + size_t(part * bitwidth / 8) + 32;
   if (size_t(part) * sizeof(float) > kHoldBytes || p.smem > kHoldSmem) return cudaSuccess;

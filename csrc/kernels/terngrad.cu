@@ -495,6 +495,8 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
   __shared__ float scale[3];
   uint8_t* const bytes_at = reinterpret_cast<uint8_t*>(hold + part);
   const int tid = threadIdx.x;
+  GridPlace place;
+  grid_arrive(scratch, place);
   const int64_t begin = int64_t(blockIdx.x) * part;       // a multiple of 512
   const int64_t left = n - begin;
   const int len = int(left < 0 ? 0 : (left < part ? left : part));
@@ -528,7 +530,10 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
     mn = fminf(mn, v);
     mx = fmaxf(mx, v);
   }
-  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status)) return;
+  if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status, place)) {
+    grid_leave(scratch, place);
+    return;
+  }
   const PushCursor cur{nullptr};
   if (tid == 0) {
     const float gap = tern_gap(mn, mx, BW);
@@ -560,6 +565,7 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
   hold_put(dst, kTernHeaderBytes, byte0, bytes_at, shift, units * BPT);
   if (tid == 32 && len > 0 && units * EPT < len)
     tern_leftover<BW, EF>(grad, residual, begin + int64_t(units) * EPT, n, mn, inv, gap, random, seed, dst, cur);
+  grid_leave(scratch, place);
 }
 
 struct TernHeader {

@@ -422,6 +422,26 @@ def test_ecq_resident_form(bw, offset):
             assert torch.equal(hg.cpu(), hc), n
 
 
+@pytest.mark.parametrize("n", [65537, 148 * 512, 148 * 512 + 1, 300007, 2359807])
+def test_resident_forms_find_the_extremes_of_every_part(n):
+    """In the first part, the last one and a partial word behind it; zeros of either sign, one sign only."""
+    base = gauss(n, seed=n)
+    inputs = [torch.zeros(n), torch.full((n,), -0.0), torch.full((n,), -3.0), base.abs() + 1, -base.abs() - 1]
+    for at in (0, n // 2, n - 1):
+        for value in (9.0, -9.0):
+            x = base.clone()
+            x[at] = value
+            inputs.append(x)
+    h = gauss(n, 0.4, seed=n + 1)
+    for i, x in enumerate(inputs):
+        want = ops.terngrad_compress(x, 2, True, seed=3)
+        assert torch.equal(ops.terngrad_compress(x.cuda(), 2, True, seed=3).cpu(), want), i
+        hc, hg = h.clone(), h.cuda()
+        want = ops.ecq_compress(x, hc, 1.0, 0.9, 4, 7)
+        assert torch.equal(ops.ecq_compress(x.cuda(), hg, 1.0, 0.9, 4, 7).cpu(), want), i
+        assert torch.equal(hg.cpu(), hc), i
+
+
 def test_terngrad_resident_form_when_its_wait_runs_out():
     """A counter that starts one short: no CTA ever sees all others arrive.  The wait ends, the status word says so, and
     the next call finds its state ready."""
