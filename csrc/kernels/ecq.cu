@@ -274,7 +274,9 @@ ecq_quant_kernel(const float* __restrict__ grad, float* __restrict__ hist, int64
 // once.  What a CTA keeps in shared memory is v = g + alpha * h; the history itself is read again, from L2,
 // where it and the gradient (two tensors of 30 MB at most) still are.  All CTAs have to be resident at once, each
 // with an SM to itself: the exchange engine, whose compressor runs beside the backward pass, keeps the two launches.
-// 25 MB, 4 bits, in a chain of calls: 26.5 us; 28.4 in two launches.  256 KB: 6.4 and 8.1.
+// 25 MB, 4 bits, in a chain of calls: 24.8 us; 28.4 in two launches.  256 KB: 6.4 and 8.1 (with a slower exchange of
+// the extremes).  A thread of 25 MB has eleven words: with the last three loaded one after another, in both walks,
+// compress and decode take 37.9 us, and 37.2 so.
 constexpr int kHoldAhead = 4;   // history words of a thread in flight
 template <int BW>
 __global__ void __launch_bounds__(kHoldThreads, 1)
@@ -300,18 +302,19 @@ ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t 
     mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     reinterpret_cast<float4*>(hold)[i] = v;
   };
-  int q = tid;
-  for (; q + (kHoldAhead - 1) * kHoldThreads < quads; q += kHoldAhead * kHoldThreads) {
+  for (int q = tid; q < quads; q += kHoldAhead * kHoldThreads) {   // the last, partial round keeps its loads together too
     float4 g[kHoldAhead], h[kHoldAhead];
 #pragma unroll
     for (int u = 0; u < kHoldAhead; ++u) {
-      g[u] = __ldg(g4 + q + u * kHoldThreads);
-      h[u] = h4[q + u * kHoldThreads];
+      if (q + u * kHoldThreads < quads) {
+        g[u] = __ldg(g4 + q + u * kHoldThreads);
+        h[u] = h4[q + u * kHoldThreads];
+      }
     }
 #pragma unroll
-    for (int u = 0; u < kHoldAhead; ++u) take(q + u * kHoldThreads, g[u], h[u]);
+    for (int u = 0; u < kHoldAhead; ++u)
+      if (q + u * kHoldThreads < quads) take(q + u * kHoldThreads, g[u], h[u]);
   }
-  for (; q < quads; q += kHoldThreads) take(q, __ldg(g4 + q), h4[q]);
   for (int e = 4 * quads + tid; e < len; e += kHoldThreads)   // fewer than four
     mx = fmaxf(mx, fabsf(ecq_compensated(grad[begin + e], hist[begin + e], alpha)));
   if (!grid_minmax_all<kHoldThreads>(scratch, mn, mx, wait_ns, status, place)) {
@@ -336,15 +339,15 @@ ecq_hold_kernel(const float* __restrict__ grad, float* hist, int64_t n, int64_t 
     h4[u] = make_float4(h[0], h[1], h[2], h[3]);
     hold_unit_bytes<BPT>(bytes_at + shift + u * BPT, bytes);   // shift is even
   };
-  int u = tid;
-  for (; u + (kHoldAhead - 1) * kHoldThreads < quads; u += kHoldAhead * kHoldThreads) {
+  for (int u = tid; u < quads; u += kHoldAhead * kHoldThreads) {
     float4 h[kHoldAhead];
 #pragma unroll
-    for (int k = 0; k < kHoldAhead; ++k) h[k] = h4[u + k * kHoldThreads];
+    for (int k = 0; k < kHoldAhead; ++k)
+      if (u + k * kHoldThreads < quads) h[k] = h4[u + k * kHoldThreads];
 #pragma unroll
-    for (int k = 0; k < kHoldAhead; ++k) quantise(u + k * kHoldThreads, h[k]);
+    for (int k = 0; k < kHoldAhead; ++k)
+      if (u + k * kHoldThreads < quads) quantise(u + k * kHoldThreads, h[k]);
   }
-  for (; u < quads; u += kHoldThreads) quantise(u, h4[u]);
   __syncthreads();
   hold_put(dst, kEcqHeaderBytes, byte0, bytes_at, shift, quads * BPT);
   if (tid == 32) {   // fewer than four leftover elements

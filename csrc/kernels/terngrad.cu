@@ -484,8 +484,10 @@ tern_small_kernel(const float* grad, float* residual, int64_t n, int random, uin
 // exchange engine and the task API, whose compressors run beside the backward pass, keep the two launches.
 // Beside a chain of 16384^3 matrix products a 4 MB task takes 850 us in this form (it waits for SMs to fall
 // free) and 260 in two launches; on an idle GPU 64 and 71 us.
-// 25 MB with error feedback, 2 bits (ncu, cold): 21.3 us; 14.3 + 18.0 in two launches.  9.4 MB at 4 bits, compress
-// and decode: 14.4 and 18.4.
+// 25 MB with error feedback, 2 bits (ncu, cold): 21.3 us with a slower exchange of the extremes; 14.3 + 18.0 in two
+// launches.  9.4 MB at 4 bits, compress and decode: 12.3; two launches were 4 us slower.  A thread of 25 MB has eleven
+// words: with the last three loaded one after another, compress and the decode of eight payloads take 35.3 us, and
+// 34.9 so.  Inside the kernel: 11.5 us for 52 MB of inputs, 1.9 the exchange, 6 the quantiser and its stores.
 template <int BW, bool EF>
 __global__ void __launch_bounds__(kHoldThreads, 1)
 tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, int64_t n, int64_t part, int random,
@@ -513,18 +515,19 @@ tern_hold_kernel(const float* __restrict__ grad, float* __restrict__ residual, i
     mx = fmaxf(mx, fmaxf(fmaxf(g.x, g.y), fmaxf(g.z, g.w)));
     reinterpret_cast<float4*>(hold)[i] = g;
   };
-  int q = tid;
-  for (; q + 3 * kHoldThreads < quads; q += 4 * kHoldThreads) {
+  for (int q = tid; q < quads; q += 4 * kHoldThreads) {   // the last, partial round keeps its loads together too
     float4 g[4], r[4] = {};
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      g[u] = __ldg(g4 + q + u * kHoldThreads);
-      if (EF) r[u] = r4[q + u * kHoldThreads];
+      if (q + u * kHoldThreads < quads) {
+        g[u] = __ldg(g4 + q + u * kHoldThreads);
+        if (EF) r[u] = r4[q + u * kHoldThreads];
+      }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) take(q + u * kHoldThreads, g[u], r[u]);
+    for (int u = 0; u < 4; ++u)
+      if (q + u * kHoldThreads < quads) take(q + u * kHoldThreads, g[u], r[u]);
   }
-  for (; q < quads; q += kHoldThreads) take(q, __ldg(g4 + q), EF ? r4[q] : make_float4(0.f, 0.f, 0.f, 0.f));
   for (int e = 4 * quads + tid; e < len; e += kHoldThreads) {   // fewer than four
     const float v = EF ? hp_add(grad[begin + e], residual[begin + e]) : grad[begin + e];
     mn = fminf(mn, v);
