@@ -1,8 +1,8 @@
 // GELU (x * Phi(x), Phi the normal distribution) of bf16 activations, forward and backward.
 //
-// The framework library's kernels evaluate erf and exp for themselves with some 70 instructions an element, which
-// makes them issue-bound at half the memory rate (16.7 M elements of a BERT-large feed-forward layer at 4,096 tokens:
-// 18 us forward and 34 backward; one pass over memory is 10 and 15).  Here the tail 1 - Phi(|x|) comes from
+// With the library's erf and exp the pass is bound by arithmetic at half the memory rate (16.7 M elements of a
+// BERT-large feed-forward layer at 4,096 tokens: 18 us forward and 34 backward; one pass over memory is 10 and 15).
+// Here the tail 1 - Phi(|x|) comes from
 // Abramowitz and Stegun's formula 7.1.26, a polynomial in 1 / (1 + p z) times exp(-z^2) with an absolute error of
 // 1.5e-7 in erf, and the same exponential gives the density that the backward pass needs.  The tail is used as it
 // is for negative x, so that nothing cancels there, where 1 + erf(z) in 32 bits loses its digits.
